@@ -218,6 +218,76 @@ def run(state):
     return flash_attn_update_out_lse(state["outs"], state["lses"])
 
 
+# ---------------------------------------------------------------------------------------- the same in 64 bits
+def _exact_attention(case, gen, dev):
+    H, G, d, dtype = case["heads"], case["kv_heads"], case["head_dim"], DTYPES[case["dtype"]]
+    raw = _lengths(case)
+    T, blocks = sum(raw), H // case["head_block"]          # rows: head block by head block, in each all tokens
+    hb, gb = H // blocks, G // blocks
+    new = lambda *shape: torch.randn(*shape, generator=gen, device=dev, dtype=torch.float32).to(dtype)
+    q, kv = new(blocks * T, hb, d), new(blocks * T, 2, gb, d)
+    do = new(blocks * T, hb, d) if case["step"] else None
+    mask = torch.from_numpy(masks.to_two_range(_mask(case, raw, raw))).to(dev)        # [T, range, bound]
+    wide = lambda t: torch.zeros(t.shape, dtype=torch.float64, device=dev)
+    out, dq, dkv = wide(q), None if do is None else wide(q), None if do is None else wide(kv)
+    step = 4096
+    for b in range(blocks):
+        lo = 0
+        for n in raw:
+            own = slice(b * T + lo, b * T + lo + n)
+            pos = torch.arange(n, device=dev)
+            for h in range(hb):
+                g = h * gb // hb
+                k, v = kv[own, 0, g].double(), kv[own, 1, g].double()
+                for t in range(0, n, step):
+                    m = min(step, n - t)
+                    rows = slice(own.start + t, own.start + t + m)
+                    r = mask[lo + t:lo + t + m]
+                    sees = ((pos >= r[:, 0, 0, None]) & (pos < r[:, 0, 1, None])) | ((pos >= r[:, 1, 0, None]) & (pos < r[:, 1, 1, None]))
+                    qt = q[rows, h].double()
+                    p = ((qt @ k.t()) * d ** -0.5).masked_fill_(~sees, float("-inf")).softmax(1).nan_to_num_(0.0)
+                    o = p @ v
+                    out[rows, h] = o
+                    if do is not None:
+                        dot = do[rows, h].double()
+                        dkv[own, 1, g] += p.t() @ dot
+                        ds = (dot @ v.t()).sub_((o * dot).sum(1, keepdim=True)).mul_(p).mul_(d ** -0.5)
+                        dq[rows, h] = ds @ k
+                        dkv[own, 0, g] += ds.t() @ qt
+            lo += n
+    return out if do is None else {"out": out, "dq": dq, "dkv": dkv}
+
+
+def _exact_optimizer(case, gen, dev):
+    n = case["params"]
+    p = torch.empty(n, dtype=torch.bfloat16, device=dev).normal_(0.0, 0.02, generator=gen).double()
+    g = torch.empty(n, dtype=torch.bfloat16, device=dev).normal_(0.0, 1e-3, generator=gen).double()
+    if case["clip"]:
+        g *= min(1.0, case["clip"] / (float(g.norm()) + 1e-6))
+    # first step of AdamW with betas 0.9 / 0.95, eps 1e-8, weight decay 0.1: the corrected moments are g and g^2
+    m, v = 0.1 * g, 0.05 * g * g
+    p -= 1e-4 * (g / (g.abs() + 1e-8) + 0.1 * p)
+    return {"params": None, "master": p, "m": m, "v": v}
+
+
+def exact(case, seed):
+    """What ``run`` gives on a fresh state, in 64 bits.  A training step has none here: its layers are bf16
+    throughout, and its kernels are in the other cases."""
+    if case["kind"] == "train":
+        return None
+    dev = torch.device("cuda", torch.cuda.current_device())
+    gen = torch.Generator(device=dev).manual_seed(int(seed))
+    if case["kind"] == "attention":
+        return _exact_attention(case, gen, dev)
+    if case["kind"] == "optimizer":
+        return _exact_optimizer(case, gen, dev)
+    n, t, h = case["partials"], case["tokens"], case["heads"]
+    outs = torch.randn(n, t, h, 128, generator=gen, device=dev, dtype=torch.bfloat16).double()
+    lses = (4.0 + 2.0 * torch.randn(n, t, h, generator=gen, device=dev, dtype=torch.float32)).double()
+    lse = torch.logsumexp(lses, 0)
+    return ((lses - lse).exp()[..., None] * outs).sum(0), lse
+
+
 # ---------------------------------------------------------------------------------------- what a pass needs
 def work(case):
     if case["kind"] == "attention":
