@@ -11,7 +11,7 @@ namespace {
 
 constexpr int64_t kTileN = 128;   // keys per tile
 constexpr int64_t kTileM = 128;   // query rows of one forward tile
-constexpr int64_t kQTileBwd = 64; // query rows of one backward item
+constexpr int64_t kQTileBwd = 128; // query rows of one backward item
 
 // per query tile: union and intersection of each of the two key ranges over the tile's rows
 struct TileBounds {

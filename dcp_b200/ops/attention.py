@@ -294,7 +294,7 @@ def attention_reference(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask:
 
 
 # ----------------------------------------------------------------------------- backward
-Q_TILE_BWD = 64
+Q_TILE_BWD = 128
 
 
 @dataclass
@@ -305,14 +305,16 @@ class BwdTables:
     n_ctas: int
     n_items: int
     flops: float = 0.0
+    max_items: int = 0    # items of the longest key tile (0: not known, head groups are not split over CTAs)
 
     def to(self, device, non_blocking: bool = True) -> "BwdTables":
         mv = lambda t: t.to(device, non_blocking=non_blocking)
-        return BwdTables(mv(self.ctas), mv(self.items), mv(self.masks), self.n_ctas, self.n_items, self.flops)
+        return BwdTables(mv(self.ctas), mv(self.items), mv(self.masks), self.n_ctas, self.n_items, self.flops,
+                         self.max_items)
 
     def pin(self) -> "BwdTables":
         return BwdTables(self.ctas.pin_memory(), self.items.pin_memory(), self.masks.pin_memory(), self.n_ctas,
-                         self.n_items, self.flops)
+                         self.n_items, self.flops, self.max_items)
 
 
 def _tile_bounds(rng: np.ndarray, tile: int):
@@ -341,12 +343,13 @@ def build_bwd_tables(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: int
         return build_bwd_tables_py(rows, block_size, hq, hkv, device)
     c_np, i_np, m_np, pairs = native.build_bwd_tables(_row_tuples(rows), int(block_size), int(hq))
     to = lambda a: torch.from_numpy(a).to(device, non_blocking=True)
-    return BwdTables(to(c_np), to(i_np), to(m_np), int(c_np.shape[0]), int(i_np.shape[0]), flops=10.0 * pairs * HEAD_DIM)
+    return BwdTables(to(c_np), to(i_np), to(m_np), int(c_np.shape[0]), int(i_np.shape[0]), flops=10.0 * pairs * HEAD_DIM,
+                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0)
 
 
 def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: int, device) -> BwdTables:
     """KV-major work lists for the backward kernel: one table entry per key tile (the kernel runs
-    it once per KV head) listing the 64-query tiles that see it; heads are not materialised."""
+    it once per KV head) listing the 128-query tiles that see it; heads are not materialised."""
     masks, mask_row = [], 0
     cta_items = {}  # (kv_row, n_valid, dkv_dev, dkv_row) -> list of item arrays
     pairs = 0.0
@@ -396,7 +399,8 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
     i_np = (np.concatenate(item_chunks, axis=0) if item_chunks else np.zeros((0, 8))).astype(np.int32)
     m_np = np.concatenate(masks, axis=0) if masks else np.zeros((0, 4), np.int32)
     to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device, non_blocking=True)
-    return BwdTables(to(c_np), to(i_np), to(m_np), len(ctas), int(off), flops=10.0 * pairs * HEAD_DIM)
+    return BwdTables(to(c_np), to(i_np), to(m_np), len(ctas), int(off), flops=10.0 * pairs * HEAD_DIM,
+                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0)
 
 
 def attn_delta(out_arena: torch.Tensor, dout_arena: torch.Tensor, delta: torch.Tensor, row0: int, n_rows: int):
@@ -419,7 +423,8 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
     rc = lib.dcpk_attn_bwd(
         _lib.ptr(q_arena), _lib.ptr(do_arena), ctypes.c_long(q_arena.shape[0]), _lib.ptr(kv_arena),
         ctypes.c_long(kv_arena.shape[0]), ctypes.c_int(hq), ctypes.c_int(hkv), _lib.ptr(tables.ctas),
-        ctypes.c_int(tables.n_ctas), _lib.ptr(tables.items), ctypes.c_int(tables.items.shape[0]), _lib.ptr(tables.masks),
+        ctypes.c_int(tables.n_ctas), _lib.ptr(tables.items), ctypes.c_int(tables.items.shape[0]),
+        ctypes.c_int(tables.max_items), _lib.ptr(tables.masks),
         ctypes.c_int(tables.masks.shape[0]), _lib.ptr(lse), _lib.ptr(delta),
         ctypes.c_int(lse.shape[1]), _ptr_array(dq_dsts), _ptr_array(dkv_dsts), ctypes.c_int(len(dq_dsts)),
         ctypes.c_float(scale), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())

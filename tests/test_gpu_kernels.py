@@ -103,6 +103,55 @@ def test_attention_backward(dev, case):
     assert dq[nq:].abs().max() == 0 and dkv[nkv:].abs().max() == 0     # nothing written past the valid rows
 
 
+@pytest.mark.parametrize("nq,nkv,kind,heads", [(1, 1, "causal", (4, 4)), (127, 129, "full", (4, 1)), (129, 127, "causal", (8, 2)),
+                                                (256, 255, "two", (4, 2)), (64, 640, "full", (8, 1)), (700, 700, "two", (8, 2))])
+def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
+    """Edges of the 128 x 128 items, items without and with masking, whole and split head groups, fp64 oracle.
+    P, dS and the operands are bf16: 2^-8 relative each, four of them in a chain, so 2 % of the largest element."""
+    hq, hkv = heads
+    g = torch.Generator().manual_seed(nq * 1000 + nkv)
+    new = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(dev)
+    q, kv, dout = new(nq + 40, hq, 128), new(nkv + 40, 2, hkv, 128), new(nq + 40, hq, 128)
+    i = np.arange(nq)
+    rng = np.zeros((nq, 4), np.int32)
+    off = max(nkv - nq, 0)
+    if kind == "full":
+        rng[:, 1] = nkv
+    elif kind == "causal":
+        rng[:, 1] = np.minimum(i + 1 + off, nkv)
+    else:      # a sink and a window that ends mid-tile, some queries without any key
+        rng[:, 1] = np.minimum(37, nkv)
+        rng[:, 2] = np.clip(i - 70, 37, nkv)
+        rng[:, 3] = np.clip(i + 5, 37, nkv)
+        rng[i % 61 == 60] = 0
+    row = A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)
+    scale = 128 ** -0.5
+    mask = A.ranges_to_dense(rng, nkv).to(dev)
+    k64, v64 = (kv[:nkv, j].double().repeat_interleave(hq // hkv, 1).permute(1, 0, 2) for j in (0, 1))
+    q64, do64 = q[:nq].double().permute(1, 0, 2), dout[:nq].double().permute(1, 0, 2)
+    s = (q64 @ k64.transpose(1, 2) * scale).masked_fill(~mask, float("-inf"))
+    p = s.softmax(-1).nan_to_num(0.0)
+    out64 = p @ v64
+    lse = torch.full((hq, nq + 40), 7.0, device=dev)
+    lse[:, :nq] = torch.logsumexp(s, -1).float()
+    delta = torch.full_like(lse, 7.0)
+    delta[:, :nq] = (out64 * do64).sum(-1).float()
+    ds = p * (do64 @ v64.transpose(1, 2) - (out64 * do64).sum(-1, keepdim=True)) * scale
+    fold = lambda t: t.reshape(hkv, hq // hkv, nkv, 128).sum(1).permute(1, 0, 2)
+    want = ((ds @ k64).permute(1, 0, 2), fold(ds.transpose(1, 2) @ q64), fold(p.transpose(1, 2) @ do64))
+    tables = A.build_bwd_tables([row], 1024, hq, hkv, dev)
+    assert tables.max_items > 0
+    for max_items in (tables.max_items, 0):      # 0: head groups stay whole
+        tables.max_items = max_items
+        dq, dkv = torch.zeros(nq + 40, hq, 128, device=dev), torch.zeros(nkv + 40, 2, hkv, 128, device=dev)
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        A.attn_bwd(q, dout, kv, lse, delta, tables, [dq], [dkv], scale, status)
+        assert status.item() == 0
+        for got, ref in zip((dq[:nq], dkv[:nkv, 0], dkv[:nkv, 1]), want):
+            assert (got - ref).abs().max() <= 2e-2 * ref.abs().max() + 1e-6
+        assert dq[nq:].abs().max() == 0 and dkv[nkv:].abs().max() == 0
+
+
 def test_rmsnorm(dev):
     torch.manual_seed(0)
     for hidden in (1024, 4096):
