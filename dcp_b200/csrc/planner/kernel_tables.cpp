@@ -119,7 +119,13 @@ FwdTablesOut build_fwd_tables(const std::vector<AttnRowDesc>& rows, int64_t bloc
 BwdTablesOut build_bwd_tables(const std::vector<AttnRowDesc>& rows, int64_t block_size, int hq) {
   BwdTablesOut out;
   using Key = std::tuple<int64_t, int64_t, int64_t, int64_t>;  // (kv row, valid keys, dkv device, dkv row)
-  struct Cta { Key key; std::vector<int32_t> items; };
+  struct Cta { Key key; std::vector<int32_t> items; int64_t kv_block; };
+  // KV blocks that some Q block attends to together belong to one group (a sequence)
+  std::map<int64_t, int64_t> parent;
+  auto find = [&](int64_t x) {
+    while (parent[x] != x) x = parent[x] = parent[parent[x]];
+    return x;
+  };
   std::vector<Cta> ctas;               // in order of first appearance
   std::map<Key, size_t> index;
   int64_t mask_row = 0;
@@ -128,6 +134,11 @@ BwdTablesOut build_bwd_tables(const std::vector<AttnRowDesc>& rows, int64_t bloc
     out.masks.insert(out.masks.end(), row.ranges, row.ranges + 4 * row.n_tokens);
     out.pairs += pair_count(row.ranges, row.n_tokens) * double(row.heads.size());
     const TileBounds b = tile_bounds(row.ranges, row.n_tokens, kQTileBwd);
+    for (auto& kv : row.kv) {
+      parent.emplace(kv.first, kv.first);
+      const int64_t a = find(row.kv[0].first), c = find(kv.first);
+      parent[std::max(a, c)] = std::min(a, c);
+    }
     for (size_t e = 0; e < row.kv.size(); ++e) {
       const int64_t kv_row = row.kv[e].first, n_tok = row.kv[e].second;
       const int64_t dkv_dev = row.dkv.empty() ? 0 : row.dkv[e].first, dkv_row = row.dkv.empty() ? kv_row : row.dkv[e].second;
@@ -142,7 +153,7 @@ BwdTablesOut build_bwd_tables(const std::vector<AttnRowDesc>& rows, int64_t bloc
             auto it = index.find(key);
             if (it == index.end()) {
               it = index.emplace(key, ctas.size()).first;
-              ctas.push_back(Cta{key, {}});
+              ctas.push_back(Cta{key, {}, kv_row});
             }
             cta = &ctas[it->second];
           }
@@ -156,10 +167,20 @@ BwdTablesOut build_bwd_tables(const std::vector<AttnRowDesc>& rows, int64_t bloc
     }
     mask_row += row.n_tokens;
   }
-  // key tiles with the most items first (LPT packing of the grid)
+  // group by group, so that key tiles which run at the same time read the same queries and add to the same dQ rows
+  // (they are in L2 then); the group with the longest item list first, and the longest list first inside each
+  std::map<int64_t, size_t> longest;
+  for (const Cta& c : ctas) {
+    size_t& m = longest[find(c.kv_block)];
+    m = std::max(m, c.items.size());
+  }
   std::vector<size_t> order(ctas.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return ctas[a].items.size() > ctas[b].items.size(); });
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+    const int64_t ga = find(ctas[a].kv_block), gb = find(ctas[b].kv_block);
+    if (ga != gb) return longest[ga] != longest[gb] ? longest[ga] > longest[gb] : ga < gb;
+    return ctas[a].items.size() > ctas[b].items.size();
+  });
   int64_t off = 0;
   for (size_t i : order) {
     const Cta& c = ctas[i];

@@ -352,6 +352,14 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
     it once per KV head) listing the 128-query tiles that see it; heads are not materialised."""
     masks, mask_row = [], 0
     cta_items = {}  # (kv_row, n_valid, dkv_dev, dkv_row) -> list of item arrays
+    block_of = {}   # the same key -> first arena row of the KV block the key tile lies in
+    parent = {}     # KV blocks that some Q block attends to together belong to one group (a sequence)
+
+    def find(x):
+        while parent[x] != x:
+            x = parent[x]
+        return x
+
     pairs = 0.0
     for row in rows:
         rng = np.ascontiguousarray(row.ranges, dtype=np.int32).reshape(-1, 4)
@@ -361,6 +369,10 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
         n_qt, (u0s, u0e, u1s, u1e, i0s, i0e, i1s, i1e) = _tile_bounds(rng, Q_TILE_BWD)
         qt = np.arange(n_qt)
         n_rows_t = np.minimum(Q_TILE_BWD, row.n_tokens - qt * Q_TILE_BWD)
+        for kv_row, _ in row.kv:
+            parent.setdefault(kv_row, kv_row)
+            a, c = find(row.kv[0][0]), find(kv_row)
+            parent[max(a, c)] = min(a, c)
         for e, (kv_row, n_tok) in enumerate(row.kv):
             dkv_dev, dkv_row = row.dkv[e] if row.dkv else (0, kv_row)
             n_sub = (n_tok + TILE_N - 1) // TILE_N
@@ -387,11 +399,19 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
             ends = np.cumsum(counts)
             for t in np.nonzero(counts)[0].tolist():
                 key = (kv_row + t * TILE_N, int(nv[t]), dkv_dev, dkv_row + t * TILE_N)
+                block_of.setdefault(key, kv_row)
                 cta_items.setdefault(key, []).append(arr[ends[t] - counts[t]:ends[t]])
         mask_row += row.n_tokens
     ctas, item_chunks, off = [], [], 0
-    for key, chunks in sorted(cta_items.items(), key=lambda kv: -sum(c.shape[0] for c in kv[1])):
-        n = sum(c.shape[0] for c in chunks)
+    # group by group, so that key tiles which run at the same time read the same queries and add to the same dQ
+    # rows (they are in L2 then); the group with the longest item list first, and the longest list first inside each
+    count = {key: sum(c.shape[0] for c in chunks) for key, chunks in cta_items.items()}
+    group = {key: find(block_of[key]) for key in cta_items}
+    longest = {}
+    for key, n in count.items():
+        longest[group[key]] = max(longest.get(group[key], 0), n)
+    for key, chunks in sorted(cta_items.items(), key=lambda kv: (-longest[group[kv[0]]], group[kv[0]], -count[kv[0]])):
+        n = count[key]
         ctas.append((key[0], key[1], off, n, key[2], key[3], 0, 0))
         item_chunks.extend(chunks)
         off += n

@@ -278,3 +278,26 @@ def test_native_table_builders_equal_their_python_twins():
         a, b = A.build_bwd_tables(rows, bs, hq, 1, "cpu"), A.build_bwd_tables_py(rows, bs, hq, 1, "cpu")
         assert torch.equal(a.ctas, b.ctas) and torch.equal(a.items, b.items) and torch.equal(a.masks, b.masks)
         assert (a.n_ctas, a.n_items, a.flops) == (b.n_ctas, b.n_items, b.flops)
+
+
+def test_backward_key_tiles_come_group_by_group():
+    """Key tiles of KV blocks that share a Q block (a sequence) are neighbours in the table, the group with the
+    longest item list first and the longest list first inside each group."""
+    import numpy as np
+    from dcp_b200.ops import attention as A
+    bs, rows, group_of, tok = 256, [], {}, 0
+    for g, n in enumerate((300, 1500, 700, 1500)):
+        blocks = [(tok + b, min(bs, n - b)) for b in range(0, n, bs)]
+        for j, (row, m) in enumerate(blocks):
+            group_of.update({row + t: g for t in range(0, m, 128)})
+            r = np.zeros((m, 4), np.int32)
+            r[:, 1] = j * bs + np.arange(m) + 1
+            rows.append(A.AttnRow(row, m, [0, 1], blocks[:j + 1], r))
+        tok += -(-n // bs) * bs
+    for t in (A.build_bwd_tables(rows, bs, 2, 1, "cpu"), A.build_bwd_tables_py(rows, bs, 2, 1, "cpu")):
+        groups = [group_of[c[0]] for c in t.ctas.tolist()]
+        counts = [c[3] for c in t.ctas.tolist()]
+        seen = list(dict.fromkeys(groups))
+        assert seen == [1, 3, 2, 0] and groups == sorted(groups, key=seen.index)
+        assert all(a >= b for x, y, a, b in zip(groups, groups[1:], counts, counts[1:]) if x == y)
+        assert t.max_items == max(counts) and t.n_items == sum(counts)
