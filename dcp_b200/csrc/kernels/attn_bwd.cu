@@ -134,13 +134,6 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
                : "memory");
 }
 
-// bits [start, start + width) of a word, both clamped to 32
-__device__ __forceinline__ uint32_t bit_range(int start, int width) {
-  uint32_t r;
-  asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(r) : "r"(start), "r"(width));
-  return r;
-}
-
 // lane i holds row i of a 32 x 32 bit matrix; afterwards lane i holds column i
 __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
 #pragma unroll
@@ -154,9 +147,8 @@ __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
 
 // the 32 keys [key0, key0 + 32) of the tile one query sees, from its packed ranges
 __device__ __forceinline__ uint32_t visible_keys(uint32_t rng, int key0) {
-  const int s0 = min(max(int(rng & 0xff) - key0, 0), 32), e0 = min(max(int((rng >> 8) & 0xff) - key0, 0), 32);
-  const int s1 = min(max(int((rng >> 16) & 0xff) - key0, 0), 32), e1 = min(max(int(rng >> 24) - key0, 0), 32);
-  return bit_range(s0, max(e0 - s0, 0)) | bit_range(s1, max(e1 - s1, 0));
+  return bits_between(int(rng & 0xff) - key0, int((rng >> 8) & 0xff) - key0) |
+         bits_between(int((rng >> 16) & 0xff) - key0, int(rng >> 24) - key0);
 }
 
 // P = exp2(S * c - lse) of one key row and 32 queries, in place, and its packed bf16 pairs

@@ -315,7 +315,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                              fmaxf(fmaxf(mxp[4], mxp[5]), fmaxf(mxp[6], mxp[7])));
       const float m_new = fmaxf(m_run, mx);
       const float m_sub = (m_new == -INFINITY) ? 0.f : m_new * sl2;
-      const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2(m_run * sl2 - m_sub);
+      const float alpha = m_new != m_run ? fast_exp2((m_run - m_new) * sl2) : 1.f;   // exactly 1 where the maximum stays
       // packed fp32: one instruction scales two scores, one adds two probabilities to the row sum
       const uint64_t sl2_2 = pack_f32x2(sl2, sl2), negm_2 = pack_f32x2(-m_sub, -m_sub);
       uint64_t ps2[4] = {0ull, 0ull, 0ull, 0ull};

@@ -13,6 +13,16 @@
 // so one warpgroup's exp2 / TMEM round trips run while the other's UMMAs execute.  A query tile
 // that cannot see a KV tile (from the per-tile union of its rows' ranges) skips it: no UMMA is
 // issued for it and its softmax warpgroup does not wait.
+// P of the first 64 keys is handed over while the softmax works on the other 64, so half of PV runs under it.
+// The issuer branches on elect.sync (with a test on the lane number a UMMA took about 90 cycles to issue) and
+// waits for the K and V tiles of a step before it waits for probabilities.
+// What bounds it: the chain of one query tile (scores -> TMEM load and maximum 430, exponentials 1250, hand-over,
+// second half of PV and the next QK 1030 cycles; the other tile's exponentials share the special-function pipe) next
+// to 2180 cycles of tensor time per pair of query tiles.  Exponentials on the FMA pipe (a degree-5 polynomial for
+// 1/8, 1/4 or 3/8 of them) were slower: 1266 / 1184 / 1168 against 1300 TFLOP/s; so was one issuer per query tile (1039).
+// Measured (8192 queries x 16384 keys, 32 / 8 heads, before -> after elected issue, early hand-over, a rescale
+// factor that is exactly 1 where the maximum stays and mask bits): full 2.15 -> 1.69 ms (1299 TFLOP/s), causal
+// 1.65 -> 1.28 ms (1287), sink + window 0.682 -> 0.518 ms (1078).
 // TMEM (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512); P_X overwrites the
 // first 64 columns of S_X as packed bf16 pairs and is the TMEM A operand of O_X += P_X V.
 // S_X = Q_X K^T takes both operands from shared memory (no TMEM columns are left to park Q in).
@@ -32,7 +42,7 @@
 
 namespace dcpk {
 
-static constexpr int kPairThreads = 384;  // 8 softmax warps + producer + UMMA issuer + 2 idle warps (register donors)
+static constexpr int kPairThreads = 384;  // 8 softmax warps + producer + UMMA issuer + 2 fetch warps (all four donate registers)
 static constexpr int kHalfBytesP = 128 * 64 * 2;
 static constexpr int kTileBytesP = 2 * kHalfBytesP;
 
@@ -40,7 +50,7 @@ struct __align__(1024) PairSmem {
   uint8_t q[2][kTileBytesP];
   uint8_t k[2][kTileBytesP];
   uint8_t v[2][kTileBytesP];
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done[2];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2][2], o_done[2];
   uint32_t tmem_base;
   int abort_word;
 };
@@ -79,7 +89,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CopyCtx copy_ctx, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   PairSmem& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const AttnTile tile = tiles[blockIdx.x];
   const int kv_head = tile.head / (hq / hkv);
   {
@@ -103,7 +113,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sm.k_full[i], 1);  mbar_init(&sm.k_empty[i], 1);
       mbar_init(&sm.v_full[i], 1);  mbar_init(&sm.v_empty[i], 1);
-      mbar_init(&sm.s_full[i], 1);  mbar_init(&sm.p_ready[i], 128);
+      mbar_init(&sm.s_full[i], 1);  mbar_init(&sm.p_ready[i][0], 4);  mbar_init(&sm.p_ready[i][1], 4);
       mbar_init(&sm.o_done[i], 1);
     }
     sm.abort_word = 0;
@@ -133,7 +143,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
   // register rebalancing between warpgroups (setmaxnreg inside each role's branch): the four
   // non-softmax warps give registers up, the softmax warps take them
-  // (8 x 32 x 208 + 4 x 32 x 72 = 62464 of 65536)
+  // (256 x 208 + 128 x 72 = 62464 of the 384 x 168 = 64512 the block is launched with)
   if (warp >= 8) {
    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
    if (warp == 8) {
@@ -177,38 +187,37 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // ------------------------------------------------------------ UMMA issuer
     constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
     constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
+    const uint64_t q_desc = make_sdesc_sw128(smem_u32(sm.q[0]), 16, 1024), k_desc = make_sdesc_sw128(smem_u32(sm.k[0]), 16, 1024);
+    const uint64_t v_desc = make_sdesc_sw128(smem_u32(sm.v[0]), kHalfBytesP, 1024);
+    constexpr uint64_t kTileStep = kTileBytesP >> 4, kHalfStep = kHalfBytesP >> 4;   // in a descriptor's 16-byte units
     bool ok = mbar_wait(&sm.q_full, 0, abort_word);
     int j = 0;
     int cnt[2] = {0, 0};                 // KV tiles issued so far per query tile
     bool need_prev[2] = {false, false};  // did query tile X take part in the previous KV tile
     // O_X += P_X V: P from TMEM (TS), V of ring stage `st` is the MN-major B operand; `i` = index
-    // of this KV tile among the ones query tile X takes part in, `jv` = its index in the ring
-    auto issue_pv = [&](int x, int i, int jv) -> bool {
-      const int st = jv & 1;
-      if (!mbar_wait(&sm.p_ready[x], i & 1, abort_word)) return false;
-      if (!mbar_wait(&sm.v_full[st], (jv >> 1) & 1, abort_word)) return false;
-      tc_fence_after();
-      if (lane == 0) {
-        const uint32_t v_addr = smem_u32(sm.v[st]);
+    // of this KV tile among the ones query tile X takes part in
+    auto issue_pv = [&](int x, int i, int st) -> bool {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          uint64_t bdesc = make_sdesc_sw128(v_addr + k * 2048, kHalfBytesP, 1024);
-          umma_ts(tmem + 256 + x * 128, tmem + x * 128 + k * 8, bdesc, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+      for (int h = 0; h < 2; ++h) {   // the first 64 keys while the softmax warps still work on the others
+        if (!mbar_wait(&sm.p_ready[x][h], i & 1, abort_word)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 4 * h; k < 4 * h + 4; ++k)
+            umma_ts(tmem + 256 + x * 128, tmem + x * 128 + k * 8, v_desc + st * kTileStep + k * 128, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+          if (h == 1) umma_commit(&sm.o_done[x]);
         }
-        umma_commit(&sm.o_done[x]);
+        __syncwarp();
       }
-      __syncwarp();
       return true;
     };
     // S_X = Q_X K^T, both operands from shared memory
     auto issue_qk = [&](int x, int st) {
-      if (lane == 0) {
-        const uint32_t q_addr = smem_u32(sm.q[x]), k_addr = smem_u32(sm.k[st]);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          uint64_t adesc = make_sdesc_sw128(q_addr + (k >> 2) * kHalfBytesP + (k & 3) * 32, 16, 1024);
-          uint64_t bdesc = make_sdesc_sw128(k_addr + (k >> 2) * kHalfBytesP + (k & 3) * 32, 16, 1024);
-          umma_ss(tmem + x * 128, adesc, bdesc, idesc_qk, k > 0 ? 1u : 0u);
+          const uint64_t off = (k >> 2) * kHalfStep + (k & 3) * 2;
+          umma_ss(tmem + x * 128, q_desc + x * kTileStep + off, k_desc + st * kTileStep + off, idesc_qk, k > 0 ? 1u : 0u);
         }
         umma_commit(&sm.s_full[x]);
       }
@@ -216,7 +225,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     };
     while (ok && it.next()) {
       const int st = j & 1, u = j >> 1;
+      // the operands of this step are waited for before the probabilities: nothing then stands between the
+      // products once a softmax warpgroup has delivered
       ok = mbar_wait(&sm.k_full[st], u & 1, abort_word);
+      if (ok && j > 0) ok = mbar_wait(&sm.v_full[st ^ 1], ((j - 1) >> 1) & 1, abort_word);
       if (!ok) break;
       tc_fence_after();
       bool need_cur[2];
@@ -224,11 +236,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       for (int x = 0; x < 2; ++x) {
         need_cur[x] = (it.cur.w >> x) & 1;
         // S_X may only be overwritten after P_X of the previous tile was consumed: its PV goes first
-        if (need_prev[x]) { ok = issue_pv(x, cnt[x] - 1, j - 1); if (!ok) break; }
+        if (need_prev[x]) { ok = issue_pv(x, cnt[x] - 1, st ^ 1); if (!ok) break; }
         if (need_cur[x]) { issue_qk(x, st); ++cnt[x]; }
       }
       if (!ok) break;
-      if (lane == 0) {
+      if (elect_one()) {
         umma_commit(&sm.k_empty[st]);                   // both query tiles are through with K(j)
         if (j > 0) umma_commit(&sm.v_empty[st ^ 1]);    // ... and with V(j-1)
       }
@@ -236,9 +248,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       need_prev[0] = need_cur[0]; need_prev[1] = need_cur[1];
       ++j;
     }
+    if (ok && j > 0) ok = mbar_wait(&sm.v_full[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_word);
 #pragma unroll
     for (int x = 0; x < 2; ++x)
-      if (ok && need_prev[x]) ok = issue_pv(x, cnt[x] - 1, j - 1);
+      if (ok && need_prev[x]) ok = issue_pv(x, cnt[x] - 1, (j - 1) & 1);
     // keep TMEM alive until the last accumulate retired (the epilogues also wait on it)
 #pragma unroll
     for (int x = 0; x < 2; ++x)
@@ -254,7 +267,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t s_addr = tmem + lane_base + X * 128, o_addr = tmem + lane_base + 256 + X * 128;
     const float sl2 = scale * 1.4426950408889634f;
     const float rescale_gap = 8.0f / sl2;   // 8 in the base-2 exponent, expressed in raw score units
-    const int len0 = e0 - s0, len1 = e1 - s1;
     float m_run = -INFINITY, l_run = 0.f;
     int j = 0;   // KV tiles this query tile took part in
     bool ok = true;
@@ -277,14 +289,18 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int c = 0; c < 64; ++c)
           mxp[c & 7] = fmax3(mxp[c & 7], __uint_as_float(sreg[2 * c]), __uint_as_float(sreg[2 * c + 1]));
       } else {
-        const int rel0 = it.cur.y - s0, rel1 = it.cur.y - s1, n_valid = it.cur.z;
+        // the keys this row sees as one bit each: a range costs a handful of instructions per 32 keys and an
+        // element one test, where comparing every key with four bounds costs six per element
+        const int a0 = s0 - it.cur.y, b0 = min(e0 - it.cur.y, it.cur.z), a1 = s1 - it.cur.y, b1 = min(e1 - it.cur.y, it.cur.z);
 #pragma unroll
-        for (int c = 0; c < 128; ++c) {
-          bool allow = (unsigned(rel0 + c) < unsigned(len0)) || (unsigned(rel1 + c) < unsigned(len1));
-          allow = allow && (c < n_valid);
-          float sv = allow ? __uint_as_float(sreg[c]) : -INFINITY;
-          sreg[c] = __float_as_uint(sv);
-          mxp[c & 7] = fmaxf(mxp[c & 7], sv);
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t see = bits_between(a0 - 32 * w, b0 - 32 * w) | bits_between(a1 - 32 * w, b1 - 32 * w);
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const float sv = (see >> c) & 1u ? __uint_as_float(sreg[32 * w + c]) : -INFINITY;
+            sreg[32 * w + c] = __float_as_uint(sv);
+            mxp[c & 7] = fmaxf(mxp[c & 7], sv);
+          }
         }
       }
       const float mx = fmaxf(fmaxf(fmaxf(mxp[0], mxp[1]), fmaxf(mxp[2], mxp[3])),
@@ -295,7 +311,22 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // in most tiles.  out = O / l and lse = m + ln l are exact for any reference value m.
       const float m_new = (mx > m_run + rescale_gap) ? mx : m_run;
       const float m_sub = (m_new == -INFINITY) ? 0.f : m_new * sl2;
-      const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2(m_run * sl2 - m_sub);
+      // exactly 1 where the maximum stays: m_run * sl2 - m_sub would be contracted to an FMA, whose residue of m_sub's
+      // rounding made most tiles rescale O
+      const bool moved = m_new != m_run;
+      const float alpha = moved ? fast_exp2((m_run - m_new) * sl2) : 1.f;
+      // S_X(j) was issued behind the previous accumulate into O_X, so that one has retired too
+      if (j > 0 && __any_sync(0xffffffffu, moved)) {
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {   // rare: few registers and little code matter more than its speed
+          uint32_t oreg[16];
+          tmem_ld16(o_addr + c * 16, oreg);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
+          tmem_st16(o_addr + c * 16, oreg);
+        }
+      }
       // packed fp32: one instruction scales two scores, one adds two probabilities to the row sum
       // every probability carries the factor kTruncScale (folded into the exponent), so cutting it to
       // bf16 is unbiased; the row sum carries the same factor, which cancels in O / l and is taken
@@ -317,6 +348,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           preg[c] = pack_bf16x2_trunc(p0, p1);
         }
         tmem_st32(s_addr + 32 * h, preg);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.p_ready[X][h]);
       }
       float psp[8];
 #pragma unroll
@@ -324,26 +359,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const float psum = ((psp[0] + psp[1]) + (psp[2] + psp[3])) + ((psp[4] + psp[5]) + (psp[6] + psp[7]));
       l_run = l_run * alpha + psum;
       m_run = m_new;
-      if (j > 0) {
-        // O_X may only be rescaled once the previous accumulate into it retired
-        ok = mbar_wait(&sm.o_done[X], (j - 1) & 1, abort_word);
-        if (!ok) break;
-        tc_fence_after();
-      }
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t oreg[32];
-          tmem_ld32(o_addr + c * 32, oreg);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-          tmem_st32(o_addr + c * 32, oreg);
-        }
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&sm.p_ready[X]);
       ++j;
     }
     if (ok && j > 0) {

@@ -272,28 +272,6 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// 2^x of two values on the FMA and integer pipes: x = n + f with n = round(x), |f| <= 1/2; 2^f is the
-// degree-5 polynomial with the smallest relative error on [-1/2, 1/2] (fitted numerically; 2.1e-7 evaluated
-// in fp32, ex2.approx is good to 2.4e-7), and n is added to the exponent field.  Inputs below -126 give
-// 2^-126 (ex2.approx.ftz gives 0).  The special-function pipe does 4 exponentials per clock and scheduler and
-// also the bf16 conversions; the softmax loops send part of their exponentials through here instead.
-__device__ __forceinline__ void exp2_poly_f32x2(float x0, float x1, float& y0, float& y1) {
-  const uint64_t magic = pack_f32x2(12582912.f, 12582912.f);   // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
-  const uint64_t x = pack_f32x2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
-  const uint64_t t = add_f32x2(x, magic);
-  const uint64_t n = add_f32x2(t, pack_f32x2(-12582912.f, -12582912.f));
-  const uint64_t f = fma_f32x2(n, pack_f32x2(-1.f, -1.f), x);
-  uint64_t p = fma_f32x2(f, pack_f32x2(1.3276472454890609e-3f, 1.3276472454890609e-3f), pack_f32x2(9.675540961325169e-3f, 9.675540961325169e-3f));
-  p = fma_f32x2(p, f, pack_f32x2(5.550713092088699e-2f, 5.550713092088699e-2f));
-  p = fma_f32x2(p, f, pack_f32x2(0.24022120237350464f, 0.24022120237350464f));
-  p = fma_f32x2(p, f, pack_f32x2(0.6931469440460205f, 0.6931469440460205f));
-  p = fma_f32x2(p, f, pack_f32x2(1.0000001192092896f, 1.0000001192092896f));
-  float p0, p1, t0, t1;
-  unpack_f32x2(p, p0, p1);
-  unpack_f32x2(t, t0, t1);
-  y0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
-  y1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
-}
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -315,6 +293,13 @@ static constexpr float kTruncLn = 0.0026964f;     // ln(kTruncScale)
 __device__ __forceinline__ uint32_t pack_bf16x2_trunc(float lo, float hi) {
   uint32_t r;
   asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(r) : "r"(__float_as_uint(lo)), "r"(__float_as_uint(hi)));
+  return r;
+}
+// bits [from, to) of a word, both clamped to [0, 32]; empty when to <= from
+__device__ __forceinline__ uint32_t bits_between(int from, int to) {
+  const int a = min(max(from, 0), 32), b = min(max(to, 0), 32);
+  uint32_t r;
+  asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(max(b - a, 0)));
   return r;
 }
 __device__ __forceinline__ uint64_t global_timer_ns() {

@@ -103,6 +103,37 @@ def test_attention_backward(dev, case):
     assert dq[nq:].abs().max() == 0 and dkv[nkv:].abs().max() == 0     # nothing written past the valid rows
 
 
+@pytest.mark.parametrize("nq,nkv,kind", [(1, 1, "full"), (130, 129, "window"), (256, 384, "window"), (300, 700, "climb")])
+def test_attention_forward_masks_and_rescale(dev, nq, nkv, kind):
+    """Mask words at the edges of 32 keys and of a tile, and a running maximum that moves in later tiles, fp64
+    oracle.  P and V are bf16 (2^-9 of the largest value each, and P is cut, not rounded: 2^-8), the result is rounded
+    to bf16 once more: 2^-6 of the largest value; the row sum is fp32 and unbiased to 1e-3 in the LSE."""
+    g = torch.Generator().manual_seed(nq + nkv)
+    q, kv = (torch.randn(n + 17, *s, generator=g).bfloat16().to(dev) for n, s in ((nq, (4, 128)), (nkv, (2, 2, 128))))
+    i = np.arange(nq)
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = nkv
+    if kind == "window":       # windows that start and end at every offset inside a word, disjoint, some rows empty
+        rng[:, 1] = np.minimum(i % 67, nkv)
+        rng[:, 2] = np.clip(i % 67 + i % 35, 0, nkv)
+        rng[:, 3] = np.clip(i % 67 + i % 35 + i % 131, 0, nkv)
+    if kind == "climb":        # later key tiles score far higher: O is rescaled
+        q[:, :, 0] = 4.0
+        kv[:nkv, 0, :, 0] = (torch.arange(nkv, device=dev) // 128 * 16.0)[:, None].bfloat16()
+    row = A.AttnRow(0, nq, [0, 1, 2, 3], [(0, nkv)], rng)
+    out, lse = torch.zeros_like(q), torch.zeros(4, nq + 17, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 1024, dev), [out], [lse], 128 ** -0.5, status)
+    assert status.item() == 0
+    k64, v64 = (kv[:nkv, j].double().repeat_interleave(2, 1).permute(1, 0, 2) for j in (0, 1))
+    s = (q[:nq].double().permute(1, 0, 2) @ k64.transpose(1, 2) * 128 ** -0.5).masked_fill(~A.ranges_to_dense(rng, nkv).to(dev), float("-inf"))
+    ref, rl = (s.softmax(-1).nan_to_num(0.0) @ v64).permute(1, 0, 2), torch.logsumexp(s, -1)
+    empty = torch.isinf(rl)
+    assert (out[:nq] - ref).abs().max() <= 2.0 ** -6 * ref.abs().max()
+    assert torch.equal(torch.isinf(lse[:, :nq]), empty) and ((lse[:, :nq] - rl)[~empty].abs() < 1e-3).all()
+    assert out[nq:].abs().max() == 0
+
+
 @pytest.mark.parametrize("nq,nkv,kind,heads", [(1, 1, "causal", (4, 4)), (127, 129, "full", (4, 1)), (129, 127, "causal", (8, 2)),
                                                 (256, 255, "two", (4, 2)), (64, 640, "full", (8, 1)), (700, 700, "two", (8, 2))])
 def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
