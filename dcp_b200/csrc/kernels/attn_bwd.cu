@@ -631,28 +631,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-// delta[h][row] = sum_d dO[row][h][d] * O[row][h][d]; one warp per (row, head)
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int n_rows, int hq, int stat_stride, int row0) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gw >= n_rows * hq) return;
-  const int row = gw / hq, h = gw % hq;
-  const size_t off = (size_t(row0 + row) * hq + h) * kHeadDim + lane * 4;
-  const uint2 a = *reinterpret_cast<const uint2*>(o + off);
-  const uint2 b = *reinterpret_cast<const uint2*>(d_o + off);
-  const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-  const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
-  float acc = 0.f;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(b2[i]);
-    acc += x.x * y.x + x.y * y.y;
-  }
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) delta[size_t(h) * stat_stride + row0 + row] = acc;
-}
-
 static constexpr int kSms = 148;
 static int g_bwd_attr_set[2] = {0, 0};
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
@@ -662,18 +640,6 @@ static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instru
 void dcpk_fill_copy_ctx(dcpk::CopyCtx* ctx, void* const* src_ptrs, void* const* dst_ptrs, int stat_stride);
 
 using namespace dcpk;
-
-extern "C" int dcpk_attn_delta(const void* o, const void* d_o, float* delta, int n_rows, int hq, int stat_stride,
-                               int row0, void* stream) {
-  if (n_rows <= 0) return 0;
-  const long warps = long(n_rows) * hq;
-  const int threads = 256;
-  const long blocks = (warps * 32 + threads - 1) / threads;
-  attn_delta_kernel<<<unsigned(blocks), threads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
-      row0);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
 
 // Points the kernel's cycle-counter timeline at `buf` (>= 16 int64, device memory) or disables it (null).
 extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {

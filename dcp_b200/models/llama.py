@@ -132,9 +132,13 @@ class _DecoderLayerFn(torch.autograd.Function):
         del h1
         model_ops.qkv_rope_split(qkv, cos, sin, ex.q, ex.kv, cfg.n_heads, cfg.n_kv_heads)
         ex.inputs_written()
-        out, lse = ex.forward()
-        a = out.reshape(T, -1).clone()
-        lse_c = lse.clone()
+        if ex.world == 1:      # nobody else reads the arena: results of the layer's own
+            out, lse_c = ex.forward(None, None, *ex.new_results())
+            a = out.view(T, -1)
+        else:
+            out, lse = ex.forward()
+            a = out.reshape(T, -1).clone()
+            lse_c = lse.clone()
         x_mid = model.row_parallel(x, a, p[f"l{l}.wo"])
         h2, rstd2 = model_ops.rmsnorm_fwd_raw(x_mid, p[f"l{l}.norm2"], cfg.eps)
         gu = torch.mm(h2, p[f"l{l}.wgu"].t())
@@ -205,9 +209,11 @@ class _DecoderLayerFn(torch.autograd.Function):
             # another layer used the arenas since this forward ran: put this layer's operands back
             model_ops.qkv_rope_split(qkv, cos, sin, ex.q, ex.kv, cfg.n_heads, cfg.n_kv_heads)
             ex.inputs_written()
-            ex.out_local().copy_(a.view(-1, cfg.n_heads, cfg.head_dim))
-            ex.lse_local().copy_(lse_c)
-        dq, dkv = ex.backward(da.view(-1, cfg.n_heads, cfg.head_dim))
+            if ex.world > 1:
+                ex.out_local().copy_(a.view(-1, cfg.n_heads, cfg.head_dim))
+                ex.lse_local().copy_(lse_c)
+        heads = lambda t: t.view(-1, cfg.n_heads, cfg.head_dim)
+        dq, dkv = ex.backward(heads(da), None, None, heads(a), lse_c) if ex.world == 1 else ex.backward(heads(da))
         del da
         dqkv = model_ops.qkv_rope_pack_bwd(dq, dkv, cos, sin, T, cfg.n_heads, cfg.n_kv_heads)
         h1, _ = model_ops.rmsnorm_fwd_raw(x, w1, cfg.eps)

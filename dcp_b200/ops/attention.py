@@ -423,13 +423,62 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
                      max_items=int(c_np[0, 3]) if c_np.shape[0] else 0)
 
 
+def attn_bwd_prep(out: torch.Tensor, dout: torch.Tensor, delta: torch.Tensor, n_rows: int, row0: int = 0, zero=()) -> None:
+    """One launch: delta[h, row] = sum_d dO*O for rows [row0, row0+n_rows) of bf16 [rows, hq, 128] tensors, and up to
+    two contiguous fp32 tensors (``zero``) cleared."""
+    lib = _lib.load()
+    hq = out.shape[1]
+    assert out.is_contiguous() and dout.is_contiguous() and delta.stride(1) == 1 and delta.stride(0) == delta.shape[1]
+    assert row0 >= 0 and row0 + n_rows <= min(out.shape[0], dout.shape[0], delta.shape[1]) and len(zero) <= 2
+    args = []
+    for t in list(zero) + [None] * (2 - len(zero)):
+        assert t is None or (t.is_contiguous() and t.dtype == torch.float32 and t.numel() % 4 == 0)
+        args += [ctypes.c_void_p(0), ctypes.c_long(0)] if t is None else [_lib.ptr(t), ctypes.c_long(t.numel())]
+    rc = lib.dcpk_attn_bwd_prep(_lib.ptr(out[row0:]), _lib.ptr(dout[row0:]), ctypes.c_void_p(delta.data_ptr() + 4 * row0),
+                                ctypes.c_int(n_rows), ctypes.c_int(hq), ctypes.c_int(delta.shape[1]), *args,
+                                _lib.stream_handle())
+    _lib.check(rc, "dcpk_attn_bwd_prep")
+
+
 def attn_delta(out_arena: torch.Tensor, dout_arena: torch.Tensor, delta: torch.Tensor, row0: int, n_rows: int):
     """delta[h, row] = sum_d dO*O for rows [row0, row0+n_rows) of bf16 [rows, hq, 128] arenas."""
-    lib = _lib.load()
-    rc = lib.dcpk_attn_delta(_lib.ptr(out_arena), _lib.ptr(dout_arena), _lib.ptr(delta), ctypes.c_int(n_rows),
-                             ctypes.c_int(out_arena.shape[1]), ctypes.c_int(delta.shape[1]), ctypes.c_int(row0),
-                             _lib.stream_handle())
-    _lib.check(rc, "dcpk_attn_delta")
+    attn_bwd_prep(out_arena, dout_arena, delta, n_rows, row0)
+
+
+_ROW_TYPES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
+
+
+def _row_pairs(pairs, d: int):
+    args = []
+    for src, dst in list(pairs) + [None] * (2 - len(pairs)):
+        rows = src.numel() // max(src.shape[-1], 1)
+        assert src.is_contiguous() and dst.is_contiguous() and src.data_ptr() % 16 == 0 and dst.data_ptr() % 16 == 0
+        assert dst.numel() // dst.shape[-1] == rows
+        args += [_lib.ptr(src), _lib.ptr(dst), ctypes.c_long(rows)]
+    return args + [ctypes.c_int(d), _lib.stream_handle()]
+
+
+def pad_cast_rows(pairs) -> None:
+    """Two (src, dst) pairs in one launch: contiguous rows of d channels (fp32 / fp16 / bf16, one type for both) ->
+    bf16 rows of 128 channels, zero-padded."""
+    (src, _), _ = pairs
+    assert all(a.dtype == src.dtype and a.shape[-1] == src.shape[-1] and b.dtype == torch.bfloat16 and b.shape[-1] == HEAD_DIM
+               for a, b in pairs)
+    rc = _lib.load().dcpk_pad_cast_rows(ctypes.c_int(_ROW_TYPES[src.dtype]), *_row_pairs(pairs, src.shape[-1]))
+    _lib.check(rc, "dcpk_pad_cast_rows")
+
+
+def cut_cast_rows(pairs) -> None:
+    """One or two (src, dst) pairs in one launch: rows of 128 channels (fp32 or bf16) -> rows of d channels of a type of
+    ``pad_cast_rows``."""
+    src, dst = pairs[0]
+    assert all(a.dtype == src.dtype and a.shape[-1] == HEAD_DIM and b.dtype == dst.dtype and b.shape[-1] == dst.shape[-1]
+               for a, b in pairs)
+    if len(pairs) == 1:
+        pairs = [pairs[0], (src[:0], dst[:0])]
+    rc = _lib.load().dcpk_cut_cast_rows(ctypes.c_int(src.dtype == torch.float32), ctypes.c_int(_ROW_TYPES[dst.dtype]),
+                                        *_row_pairs(pairs, dst.shape[-1]))
+    _lib.check(rc, "dcpk_cut_cast_rows")
 
 
 def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts, dkv_dsts, scale: float,

@@ -120,6 +120,13 @@ class FusedAttentionExecutor:
                                                 if isinstance(getattr(tabs, f.name), torch.Tensor)})
 
         self.program = program
+        # rows that a tile or a merge writes; a Q block without any work has none and stays zero
+        written = int(program.merge_ops[:, 1].sum())
+        for t in program.fwd:
+            if t is not None:
+                tile = t.tiles.numpy() if isinstance(t.tiles, torch.Tensor) else t.tiles
+                written += int(tile[(tile[:, 2] == 0) & (tile[:, 6] == program.world + program.rank), 1].sum())
+        self._all_rows_written = written >= program.q_local_rows
         # copy jobs per stage: Q + KV rows (forward, and backward when the staging rows were
         # overwritten since), dO + statistics (backward)
         self.jobs_qkv = [up(x) for x in program.jobs_qkv]
@@ -224,10 +231,32 @@ class FusedAttentionExecutor:
         self._marks = []
         return tot
 
+    def new_results(self):
+        """Fresh (out, lse) for a ``forward`` call with a single rank."""
+        new = torch.empty if self._all_rows_written else torch.zeros
+        n = self.program.q_local_rows
+        return (new(n, self.hq, HEAD_DIM, dtype=torch.bfloat16, device=self.q.device),
+                new(self.hq, n, dtype=torch.float32, device=self.q.device))
+
+    def usable(self, t: torch.Tensor) -> bool:
+        """Can the kernels read / write ``t`` in place (the address and layout an arena region has)?"""
+        return t.device == self.q.device and t.is_contiguous() and t.data_ptr() % 16 == 0
+
     # ---- forward
-    def forward(self):
+    def forward(self, q: Optional[torch.Tensor] = None, kv: Optional[torch.Tensor] = None,
+                out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None):
         """Attention over the Q/KV already present in ``q_local()`` / ``kv_local()``.
-        Returns views (out [rows, hq, d] bf16, lse [hq, rows] fp32) of this rank's own tokens."""
+        Returns views (out [rows, hq, d] bf16, lse [hq, rows] fp32) of this rank's own tokens.
+
+        With a single rank nobody else reads the arena, so the operands may be read from the caller's
+        tensors (``q`` / ``kv``: bf16, local rows, ``usable``) and the results written to them (``out`` /
+        ``lse``, both or none; contiguous) with no copy on either side."""
+        assert self.world == 1 or (q is None and kv is None and out is None), "peers read the arenas"
+        q = self.q if q is None else q
+        kv = self.kv if kv is None else kv
+        own = out is None
+        if own:
+            out, lse = self.out, self.lse
         p, a = self.program, self.arena
         main = torch.cuda.current_stream(self.device)
         tok = self._call_begin("fwd")
@@ -236,8 +265,8 @@ class FusedAttentionExecutor:
             self._poison_staging(False)
         a.barrier()                                   # every rank's inputs are in place
         self._mark("fwd:wait inputs of peers")
-        out_dsts = a.peer_ptrs("part_out") + a.peer_ptrs("out")
-        lse_dsts = a.peer_ptrs("part_lse") + a.peer_ptrs("lse")
+        out_dsts = a.peer_ptrs("part_out") + (a.peer_ptrs("out") if own else [out])
+        lse_dsts = a.peer_ptrs("part_lse") + (a.peer_ptrs("lse") if own else [lse])
         self._fetch_standalone(self._jobs_of(self.jobs_qkv, 0))
         for s in range(p.n_stages):
             nxt = self._jobs_of(self.jobs_qkv, s + 1)
@@ -246,47 +275,59 @@ class FusedAttentionExecutor:
                 self._fetch_standalone(nxt)
                 nxt = None
             if t is not None:
-                self._launch_fwd(t, out_dsts, lse_dsts, nxt)
+                self._launch_fwd(t, q, kv, out_dsts, lse_dsts, lse.shape[1], nxt)
         self._mark("fwd:kernels (with operand fetch)")
         if self.world > 1:
             a.barrier()                               # all partials have landed at their owners
         self._mark("fwd:wait partials of peers")
         if self.merge_ops.shape[0]:
-            block_ops.merge_out_lse(self.merge_ops, self.merge_src, self.part_out, self.part_lse, self.out, self.lse)
+            block_ops.merge_out_lse(self.merge_ops, self.merge_src, self.part_out, self.part_lse, out, lse)
             if self.check_reductions:
                 block_ops.check_merge_against_reference(
-                    self.merge_ops, self.merge_src, self.part_out, self.part_lse, self.out, self.lse,
+                    self.merge_ops, self.merge_src, self.part_out, self.part_lse, out, lse,
                     os.path.join(os.environ.get("DCP_LOGGING_DEBUG_DIR", "./debug"), "executor"))
             self.kernel_launches += 1
         self._mark("fwd:merge")
         torch.cuda.nvtx.range_pop()
         self._call_end(tok)
         self._staging_valid = True
-        return self.out_local(), self.lse_local()
+        return (self.out_local(), self.lse_local()) if own else (out, lse)
 
-    def _launch_fwd(self, t, out_dsts, lse_dsts, jobs=None) -> None:
-        # destinations 0..world-1 are partial arenas (row stride cap[2]), the rest final buffers (cap[0]);
+    def _launch_fwd(self, t, q, kv, out_dsts, lse_dsts, lse_rows, jobs=None) -> None:
+        # destinations 0..world-1 are partial arenas (row stride cap[2]), the rest final buffers (`lse_rows`);
         # `jobs`: the next stage's operand fetch, carried by this kernel
-        attn_ops.attn_fwd(self.q, self.kv, t, out_dsts, lse_dsts, self.scale, a_status(self), self.variant,
-                          lse_stride=self.cap[2], lse_stride_b=self.cap[0], n_dst_a=self.world, jobs=jobs,
+        attn_ops.attn_fwd(q, kv, t, out_dsts, lse_dsts, self.scale, a_status(self), self.variant,
+                          lse_stride=self.cap[2], lse_stride_b=lse_rows, n_dst_a=self.world, jobs=jobs,
                           job_ctx=self.copy_ctx)
         self.kernel_launches += 1
 
     # ---- backward
-    def backward(self, dout_local: torch.Tensor):
+    def backward(self, dout_local: torch.Tensor, q: Optional[torch.Tensor] = None, kv: Optional[torch.Tensor] = None,
+                 out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None):
         """dout_local [rows, hq, d] bf16 for this rank's tokens; returns fp32 accumulator views
-        (dq [rows, hq, d], dkv [rows, 2, hkv, d]) valid until the next backward call."""
+        (dq [rows, hq, d], dkv [rows, 2, hkv, d]) valid until the next backward call.  ``q`` / ``kv`` / ``out`` /
+        ``lse``: as in ``forward``, instead of what the arenas hold (single rank; ``out`` and ``lse`` both or none)."""
         p, a = self.program, self.arena
+        assert self.world == 1 or (q is None and kv is None and out is None), "peers read the arenas"
         main = torch.cuda.current_stream(self.device)
         n = p.q_local_rows
         tok = self._call_begin("bwd")
         self._mark("bwd:start")
         if self.poison and not self._staging_valid:
             self._poison_staging(True)
-        self.dout[:n].copy_(dout_local.reshape(n, self.hq, HEAD_DIM))
-        attn_ops.attn_delta(self.out, self.dout, self.delta, 0, n)
-        self.dq[:p.q_rows].zero_()
-        self.dkv[:p.kv_rows].zero_()
+        dout = dout_local.reshape(n, self.hq, HEAD_DIM)
+        if self.world > 1 or dout.dtype != torch.bfloat16 or not self.usable(dout):
+            self.dout[:n].copy_(dout)
+            dout = self.dout
+        q = self.q if q is None else q
+        kv = self.kv if kv is None else kv
+        if out is None:
+            out, lse, delta = self.out, self.lse, self.delta
+        else:
+            delta = torch.empty_like(lse)
+        if self.world == 1:      # one row count for Q and dO, whichever of them lives in an arena
+            q, dout = q[:n], dout[:n]
+        attn_ops.attn_bwd_prep(out, dout, delta, n, zero=(self.dq[:p.q_rows], self.dkv[:p.kv_rows]))
         self.kernel_launches += 1
         self._mark("bwd:dout copy, delta, zero accumulators")
         a.barrier()
@@ -299,7 +340,7 @@ class FusedAttentionExecutor:
             if t is None:
                 self._fetch_standalone(nxt)
                 continue
-            attn_ops.attn_bwd(self.q, self.dout, self.kv, self.lse, self.delta, t, [self.dq], [self.dkv], self.scale,
+            attn_ops.attn_bwd(q, dout, kv, lse, delta, t, [self.dq], [self.dkv], self.scale,
                               a_status(self), jobs=nxt, job_ctx=self.copy_ctx)
             self.kernel_launches += 1
         self._mark("bwd:kernels (with operand fetch)")

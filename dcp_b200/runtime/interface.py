@@ -17,6 +17,7 @@ import torch
 from ..core.blocks import Device, WorkloadSpec
 from ..core.common import ExecutionContext
 from ..core.instructions import BufferType, ExecutionPlan
+from ..ops import attention as attn_ops
 from ..planner import masks
 from ..planner.compiler import CompilerConfig, InstrCompiler
 from ..planner.workload import generate_workload, pad_seqlens
@@ -182,6 +183,81 @@ class FusedPlanExecutor:
         d = self.head_dim
         return dq[..., :d].to(q.dtype).contiguous(), dkv[..., :d].to(kv.dtype).contiguous()
 
+    # ---- the same two calls for DCPAttention: results belong to the caller, and with a single rank the kernels read
+    # bf16 tensors of 128 channels where they are; other types and widths are converted in one pass each way
+    def _as_kernel_rows(self, t, like) -> torch.Tensor:
+        """``t`` on the executor's device as contiguous, aligned [..., head_dim] rows of a type the row kernels take."""
+        t = t.reshape(like.shape[:-1] + (self.head_dim,)).to(like.device).contiguous()
+        if t.dtype not in (torch.float32, torch.float16, torch.bfloat16):
+            t = t.to(torch.bfloat16)
+        return t if self.impl.usable(t) else t.clone()
+
+    def _in_place(self, *tensors) -> bool:
+        return self.head_dim == self.impl.q_local().shape[-1] and all(t.dtype == torch.bfloat16 for t in tensors)
+
+    def _load_arena(self, q, kv) -> None:
+        """q / kv (``_as_kernel_rows``) into the arenas."""
+        ex = self.impl
+        if q.dtype != kv.dtype:
+            q, kv = q.to(torch.bfloat16), kv.to(torch.bfloat16)
+        attn_ops.pad_cast_rows([(q, ex.q_local()), (kv, ex.kv_local())])
+        ex.inputs_written()
+        self._epoch = ex.arena_epoch
+
+    def _cut(self, pairs):
+        """fp32 or bf16 [..., 128] kernel results -> fresh tensors [..., head_dim] of the given types."""
+        res = []
+        for src, dtype in pairs:
+            res.append(torch.empty(src.shape[:-1] + (self.head_dim,), device=src.device,
+                                   dtype=dtype if dtype in (torch.float16, torch.bfloat16) else torch.float32))
+        srcs = [s for s, _ in pairs]
+        if len(pairs) == 2 and res[0].dtype == res[1].dtype:
+            attn_ops.cut_cast_rows(list(zip(srcs, res)))
+        else:
+            for s, r in zip(srcs, res):
+                attn_ops.cut_cast_rows([(s, r)])
+        return [r.to(dtype) for r, (_, dtype) in zip(res, pairs)]
+
+    def forward_fresh(self, q: torch.Tensor, kv: torch.Tensor):
+        """(out, lse, token): results the caller owns; ``token`` goes to ``backward_fresh``."""
+        ex = self.impl
+        if ex.world > 1:
+            out, lse = self.forward(q, kv)
+            return out.clone(), lse.clone(), self._epoch
+        qk, kvk = self._as_kernel_rows(q, ex.q_local()), self._as_kernel_rows(kv, ex.kv_local())
+        out, lse = ex.new_results()
+        if self._in_place(qk, kvk):
+            self._epoch = -1          # the arenas do not hold this call's operands
+            ex.forward(qk, kvk, out, lse)
+        else:
+            self._load_arena(qk, kvk)
+            ex.forward(out=out, lse=lse)
+        if self.head_dim != out.shape[-1] or out.dtype != q.dtype:
+            out, = self._cut([(out, q.dtype)])
+        return out, lse, self._epoch
+
+    def backward_fresh(self, q, kv, out, dout, lse, token):
+        ex = self.impl
+        if ex.world > 1:
+            dq, dkv = self.backward(q, kv, out, dout, lse)
+            return dq.clone(), dkv.clone()
+        qk, kvk = self._as_kernel_rows(q, ex.q_local()), self._as_kernel_rows(kv, ex.kv_local())
+        ok, dok = self._as_kernel_rows(out, ex.q_local()), self._as_kernel_rows(dout, ex.q_local())
+        lse = lse.reshape(ex.lse_local().shape).to(out.device, torch.float32).contiguous()
+        if self._in_place(qk, kvk):
+            args = (qk, kvk)
+        else:
+            if token != ex.arena_epoch or not ex._staging_valid:   # another call's operands took the arenas meanwhile
+                self._load_arena(qk, kvk)
+            args = (None, None)
+        if not self._in_place(ok, dok):
+            if ok.dtype != dok.dtype:
+                ok, dok = ok.to(torch.bfloat16), dok.to(torch.bfloat16)
+            attn_ops.pad_cast_rows([(ok, ex.out_local()), (dok, ex.dout[:ex.program.q_local_rows])])
+            ok, dok = ex.out_local(), ex.dout[:ex.program.q_local_rows]
+        dq, dkv = ex.backward(dok, *args, ok, lse)
+        return self._cut([(dq, q.dtype), (dkv, kv.dtype)])
+
     def capture_cudagraph(self, *a, **k) -> None:
         """Nothing to capture: a call is a handful of launches whose tables change every batch."""
         return None
@@ -214,8 +290,11 @@ class DCPAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, executor: AttentionExecutor, capture_fwd_graph, capture_bwd_graph, q, kv):
-        out, lse = executor.forward(q, kv)
-        out, lse = out.clone(), lse.clone()
+        if hasattr(executor, "forward_fresh"):
+            out, lse, ctx.token = executor.forward_fresh(q, kv)
+        else:
+            out, lse = executor.forward(q, kv)
+            out, lse = out.clone(), lse.clone()
         ctx.executor = executor
         ctx.save_for_backward(q, kv, out, lse)
         return out
@@ -223,8 +302,12 @@ class DCPAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, kv, out, lse = ctx.saved_tensors
-        dq, dkv = ctx.executor.backward(q, kv, out, dout.contiguous(), lse)
-        return None, None, None, dq.clone().view_as(q), dkv.clone().view_as(kv)
+        if hasattr(ctx.executor, "backward_fresh"):
+            dq, dkv = ctx.executor.backward_fresh(q, kv, out, dout, lse, ctx.token)
+        else:
+            dq, dkv = ctx.executor.backward(q, kv, out, dout.contiguous(), lse)
+            dq, dkv = dq.clone(), dkv.clone()
+        return None, None, None, dq.view_as(q), dkv.view_as(kv)
 
 
 # ---------------------------------------------------------------------------------------- test glue

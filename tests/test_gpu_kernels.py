@@ -183,6 +183,43 @@ def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
         assert dq[nq:].abs().max() == 0 and dkv[nkv:].abs().max() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("d", [8, 96, 128])
+def test_row_conversions(dev, dtype, d):
+    """Padding and cutting rows of d channels round exactly as a torch conversion does, odd row counts, NaN and
+    infinities included, and write nothing next to their rows."""
+    g = torch.Generator().manual_seed(d)
+    x = [(torch.randn(n, 3, d, generator=g) * 100).to(dtype).to(dev) for n in (1, 37)]
+    x[1][5, 1, 0], x[1][6, 0, 1] = float("nan"), float("inf")
+    dst = [torch.full((t.shape[0] + 1, 3, 128), 7.0, device=dev, dtype=torch.bfloat16) for t in x]
+    A.pad_cast_rows([(t, y[:-1]) for t, y in zip(x, dst)])
+    for t, y in zip(x, dst):
+        want = torch.nn.functional.pad(t.to(torch.bfloat16), (0, 128 - d))
+        assert torch.equal(y[:-1].nan_to_num(3.0), want.nan_to_num(3.0)) and (y[-1] == 7).all()
+    for src_dtype in (torch.float32, torch.bfloat16):
+        src = [torch.randn(n, 3, 128, generator=g).to(src_dtype).to(dev) for n in (37, 2)]
+        src[0][5, 1, 0], src[0][6, 0, 1] = float("nan"), -float("inf")
+        out = [torch.full((t.shape[0] + 1, 3, d), 7.0, device=dev, dtype=dtype) for t in src]
+        A.cut_cast_rows([(t, y[:-1]) for t, y in zip(src, out)])
+        for t, y in zip(src, out):
+            assert torch.equal(y[:-1].nan_to_num(3.0), t[..., :d].to(dtype).nan_to_num(3.0)) and (y[-1] == 7).all()
+
+
+@pytest.mark.parametrize("n,hq", [(1, 1), (33, 3), (257, 8), (2500, 32)])
+def test_backward_preparation(dev, n, hq):
+    """delta is an fp32 sum of 128 products (2^-24 each step of the tree, 1e-5 of the sum of magnitudes), rows beside the
+    range stay, both accumulators are cleared as a whole."""
+    o, do = torch.randn(n + 5, hq, 128, device=dev).bfloat16(), torch.randn(n + 5, hq, 128, device=dev).bfloat16()
+    delta = torch.full((hq, n + 5), 7.0, device=dev)
+    z = [torch.ones(k, 128, device=dev) for k in (n, 3)]
+    A.attn_bwd_prep(o, do, delta, n, 2, zero=[t[:-1] for t in z])
+    prod = o.double() * do.double()
+    want, mag = prod.sum(-1).t()[:, 2:n + 2], prod.abs().sum(-1).t()[:, 2:n + 2]
+    assert ((delta[:, 2:n + 2] - want).abs() <= 1e-5 * mag).all()
+    assert (delta[:, :2] == 7).all() and (delta[:, n + 2:] == 7).all()
+    assert all((t[:-1] == 0).all() and (t[-1] == 1).all() for t in z)
+
+
 def test_rmsnorm(dev):
     torch.manual_seed(0)
     for hidden in (1024, 4096):
