@@ -134,6 +134,16 @@ def flash_attn_update_out_lse(out_blocks: torch.Tensor, lse_blocks: torch.Tensor
     if not out_blocks.is_cuda:
         o, l = merge_out_lse_reference(out_blocks, lse_blocks)
         return o.to(out_blocks.dtype), l
+    if out_blocks.dtype == torch.bfloat16 and lse_blocks.dtype == torch.float32 and d == 128 and n > 0 and \
+            lse_blocks.shape == (n, t, h) and lse_blocks.device == out_blocks.device:
+        out_blocks, lse_blocks = out_blocks.contiguous(), lse_blocks.contiguous()
+        if out_blocks.data_ptr() % 16:
+            out_blocks = out_blocks.clone()
+        out = torch.empty(t, h, d, dtype=torch.bfloat16, device=out_blocks.device)
+        lse = torch.empty(t, h, dtype=torch.float32, device=out_blocks.device)
+        _lib.check(_lib.load().dcpk_merge_stacked(_lib.ptr(out_blocks), _lib.ptr(lse_blocks), _c_int(n), ctypes.c_long(t * h),
+                                                  _lib.ptr(out), _lib.ptr(lse), _lib.stream_handle()), "merge_stacked")
+        return out, lse
     part_out = out_blocks.reshape(n * t, h, d).contiguous()
     part_lse = lse_blocks.permute(2, 0, 1).reshape(h, n * t).contiguous()
     out = torch.empty(t, h, d, dtype=out_blocks.dtype, device=out_blocks.device)

@@ -220,6 +220,47 @@ def test_backward_preparation(dev, n, hq):
     assert all((t[:-1] == 0).all() and (t[-1] == 1).all() for t in z)
 
 
+@pytest.mark.parametrize("n,t,h", [(1, 3, 1), (2, 17, 5), (3, 1, 4), (4, 100, 32), (5, 7, 3), (6, 33, 2), (7, 2, 8), (8, 64, 4), (11, 9, 3)])
+def test_merge_of_stacked_partials(dev, n, t, h):
+    """The stacked merge equals the table-driven one bit for bit: every count of sources with a kernel of its own and
+    one without, ragged item counts, invalid (-inf, +inf, NaN) partials, strided and misaligned inputs."""
+    g = torch.Generator().manual_seed(n * 100 + t)
+    outs = torch.randn(n, t, h, 128, generator=g).bfloat16().to(dev)
+    lses = (4 + 2 * torch.randn(n, t, h, generator=g)).to(dev)
+    kind = torch.randint(0, 8, (n, t, h), generator=g).to(dev)
+    for k, v in ((0, float("-inf")), (1, float("nan")), (2, float("inf"))):
+        lses[kind == k] = v
+    lses[:, 0, 0] = float("-inf")
+    ops = torch.tensor([[0, t, 0, n]], dtype=torch.int32, device=dev)
+    src = torch.arange(0, n * t, t, dtype=torch.int32, device=dev)
+    want, want_lse = torch.empty(t, h, 128, device=dev, dtype=torch.bfloat16), torch.empty(h, t, device=dev)
+    block_ops.merge_out_lse(ops, src, outs.view(n * t, h, 128), lses.permute(2, 0, 1).reshape(h, n * t).contiguous(), want, want_lse)
+    shifted = torch.cat([outs.new_zeros(1), outs.flatten()])[1:].view(outs.shape)
+    for o, l in ((outs, lses), (outs.transpose(1, 2).contiguous().transpose(1, 2), lses.transpose(1, 2).contiguous().transpose(1, 2)), (shifted, lses)):
+        out, lse = block_ops.flash_attn_update_out_lse(o, l)
+        assert torch.equal(out, want) and torch.equal(lse, want_lse.t())
+
+
+@pytest.mark.parametrize("n", [8, 8 * 1023, 8 * 1025, 8 * (148 * 8 * 256 * 4 + 3)])
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+def test_gradient_norm_and_clip_coefficient(dev, n, scale):
+    """fp32 sums of at most a few hundred terms per thread and a few thousand partial sums: 1e-5 relative; a norm below
+    the limit gives exactly 1, a NaN gradient a NaN coefficient."""
+    from dcp_b200.parallel.dist_optimizer import FlatBuffers, ShardedAdamW
+    bufs = FlatBuffers(n, dev)
+    opt = ShardedAdamW(bufs, clip_grad=0.25)
+    bufs.grads.normal_()
+    norm = float(bufs.grads.double().norm()) * scale
+    opt.step(scale)
+    assert abs(opt.grad_norm() / norm - 1) < 1e-5 and abs(float(opt.clip_coef) / (0.25 / (norm + 1e-6)) - 1) < 2e-5
+    bufs.grads.mul_(0.1 / norm)
+    opt.step(scale)
+    assert float(opt.clip_coef) == 1.0
+    bufs.grads[n // 2] = float("nan")
+    opt.step(scale)
+    assert bool(torch.isnan(opt.clip_coef))
+
+
 def test_rmsnorm(dev):
     torch.manual_seed(0)
     for hidden in (1024, 4096):
