@@ -217,7 +217,9 @@ class ShardedAdamW:
         grads, params = _ptr_array(a.peer_ptrs("grads")), _ptr_array(a.peer_ptrs("params"))
         clip_ptr = ctypes.c_void_p(0)
         if self.clip is not None:
-            self.sq_norm.zero_(); self.sq_parts.zero_()
+            self.sq_norm.zero_()
+            if self.tp_group is not None:
+                self.sq_parts.zero_()
             for s in self.shards:
                 _lib.check(lib.dcpk_grad_sqnorm(grads, ctypes.c_int(b.world), ctypes.c_long(s.flat_off),
                                                 ctypes.c_long(s.length), ctypes.c_float(grad_scale),
@@ -243,7 +245,8 @@ class ShardedAdamW:
             self.sq_norm.copy_(self.sq_parts.sum().reshape(1))
         elif self.bufs.world > 1:
             dist.all_reduce(self.sq_norm, group=self.group)
-        torch.clamp(self.clip / (self.sq_norm.sqrt() + 1e-6), max=1.0, out=self.clip_coef)
+        _lib.check(_lib.load().dcpk_clip_coef(_lib.ptr(self.sq_norm), ctypes.c_float(self.clip), _lib.ptr(self.clip_coef),
+                                              _lib.stream_handle()), "clip_coef")
 
     def _step_overlapped(self, lib, st_a, st_b) -> None:
         b, a = self.bufs, self.bufs.arena
