@@ -232,13 +232,17 @@ class _DecoderLayerFn(torch.autograd.Function):
 
 class _LMHeadLossFn(torch.autograd.Function):
     """Chunked LM head + cross entropy: logits never exist for more than ``chunk`` tokens, and
-    the gradients of the hidden states and of the head weight are formed in the same pass."""
+    the gradients of the hidden states and of the head weight are formed in the same pass.
+
+    ``write_grad``: the weight gradient is added to ``weight.grad`` by the backward itself, as the
+    hand-written decoder layers do with theirs, instead of being handed to autograd (a product and an
+    accumulation over the whole matrix)."""
 
     @staticmethod
-    def forward(ctx, h, weight, labels, grad_scale, chunk):
+    def forward(ctx, h, weight, labels, grad_scale, chunk, write_grad=False):
         T = h.shape[0]
         dh = torch.empty_like(h)
-        dweight = torch.zeros_like(weight)
+        dweight = torch.zeros_like(weight) if T == 0 else None
         total = torch.zeros((), dtype=torch.float32, device=h.device)
         for t0 in range(0, T, chunk):
             hc = h[t0:t0 + chunk]
@@ -246,15 +250,40 @@ class _LMHeadLossFn(torch.autograd.Function):
             loss = model_ops.cross_entropy_inplace(logits, labels[t0:t0 + chunk], grad_scale)
             total += loss.sum()
             dh[t0:t0 + chunk] = logits @ weight
-            dweight.addmm_(logits.t(), hc)
+            if t0 == 0:
+                dweight = torch.mm(logits.t(), hc)
+            else:
+                dweight.addmm_(logits.t(), hc)
         ctx.save_for_backward(dh, dweight)
+        ctx.grad = weight.grad if write_grad else None
         return total * grad_scale
 
     @staticmethod
     def backward(ctx, g):
         dh, dweight = ctx.saved_tensors
         # g is the upstream gradient of the (already scaled) loss; it is 1 in the training loop
-        return dh * g, dweight * g, None, None, None
+        dh = model_ops.scale_rows(dh, g)
+        if ctx.grad is not None:
+            model_ops.scale_rows(dweight, g, ctx.grad)
+            return dh, None, None, None, None, None
+        return dh, model_ops.scale_rows(dweight, g), None, None, None, None
+
+
+class _EmbeddingFn(torch.autograd.Function):
+    """Embedding whose backward adds the rows that occur straight into ``weight.grad`` (CUDA, bf16): autograd
+    forms a dense gradient of the whole table and accumulates that."""
+
+    @staticmethod
+    def forward(ctx, tokens, weight):
+        ctx.save_for_backward(tokens)
+        ctx.grad = weight.grad
+        return F.embedding(tokens, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        tokens, = ctx.saved_tensors
+        model_ops.embedding_grad(tokens, dy, ctx.grad)
+        return None, None
 
 
 class LlamaModel:
@@ -436,8 +465,9 @@ class LlamaModel:
         self._attn_stash.clear()
         self._stash_enabled = self.cache_attention and self.recompute and torch.is_grad_enabled()
         cos, sin = model_ops.rope_tables(positions, cfg.rope_theta, cfg.head_dim)
-        x = F.embedding(tokens, self.p["embed"])
-        manual = self.layer_levels is not None and x.is_cuda and torch.is_grad_enabled()
+        embed = self.p["embed"]
+        manual = self.layer_levels is not None and embed.is_cuda and torch.is_grad_enabled()
+        x = _EmbeddingFn.apply(tokens, embed) if manual else F.embedding(tokens, embed)
         for l in range(cfg.n_layers):
             if manual:
                 x = _DecoderLayerFn.apply(x, self, l, cos, sin, self.layer_levels[l])
@@ -446,4 +476,4 @@ class LlamaModel:
             else:
                 x = self._layer(x, l, cos, sin)
         h = model_ops.rmsnorm(x, self.p["norm_f"], cfg.eps)
-        return _LMHeadLossFn.apply(h, self.p["lm_head"], labels, grad_scale, self.lm_head_chunk)
+        return _LMHeadLossFn.apply(h, self.p["lm_head"], labels, grad_scale, self.lm_head_chunk, manual)

@@ -89,6 +89,31 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> torch.Tensor
     return _RMSNorm.apply(x, w, eps)
 
 
+# --------------------------------------------------------------------------- scaled and gathered gradients
+def scale_rows(src: torch.Tensor, g: torch.Tensor, dst: torch.Tensor = None) -> torch.Tensor:
+    """bf16(src * g) for bf16 ``src`` and a one-element ``g``; with ``dst`` (bf16, contiguous) it is added to ``dst``
+    in the same pass."""
+    plain = src.is_cuda and src.dtype == torch.bfloat16 and src.is_contiguous() and src.numel() % 8 == 0 and src.data_ptr() % 16 == 0
+    if not plain or (dst is not None and not (dst.is_contiguous() and dst.dtype == src.dtype and dst.data_ptr() % 16 == 0)):
+        return src * g if dst is None else dst.add_(src * g)
+    g32 = g.detach().to(src.device, torch.float32).reshape(1)
+    out = torch.empty_like(src) if dst is None else dst
+    _lib.check(_lib.load().dcpk_scale_rows(_lib.ptr(src), _lib.ptr(g32), _lib.ptr(out), _c_long(src.numel()),
+                                           _c_int(dst is not None), _lib.stream_handle()), "scale_rows")
+    return out
+
+
+def embedding_grad(tokens: torch.Tensor, dy: torch.Tensor, grad: torch.Tensor) -> None:
+    """grad[id] += sum of dy over the tokens with that id (fp32 sums, bf16 tensors on the GPU)."""
+    ids, order = torch.sort(tokens.reshape(-1).to(torch.int64))
+    dy = dy.reshape(ids.shape[0], grad.shape[1]).contiguous()
+    assert dy.dtype == grad.dtype == torch.bfloat16 and grad.is_contiguous() and grad.shape[1] % 8 == 0
+    assert dy.data_ptr() % 16 == 0 and grad.data_ptr() % 16 == 0
+    _lib.check(_lib.load().dcpk_embedding_grad(_lib.ptr(ids), _lib.ptr(order), _lib.ptr(dy), _lib.ptr(grad), _c_int(ids.shape[0]),
+                                               _c_int(grad.shape[1]), _c_long(grad.shape[0]), _lib.stream_handle()),
+               "embedding_grad")
+
+
 # --------------------------------------------------------------------------- SwiGLU
 def swiglu_fwd_raw(gu: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up for contiguous 2-D bf16 [T, 2F] laid out gate | up; no autograd."""

@@ -291,6 +291,54 @@ def test_swiglu(dev):
     assert ((gu.grad.float() - gr.grad).abs() / (gr.grad.abs() + 1.0)).max() < 2e-2
 
 
+@pytest.mark.parametrize("n,f", [(1, 8), (3, 2040), (2, 2048), (5, 8200), (300, 1024)])
+def test_swiglu_row_lengths(dev, n, f):
+    """Row lengths around a multiple of the CTA's stride, fp64 oracle: the result is rounded to bf16 once (2^-8), plus
+    1e-5 for the fast exponential."""
+    g = torch.Generator().manual_seed(f)
+    gu, dy = (4 * torch.randn(n, 2 * f, generator=g)).bfloat16().to(dev), torch.randn(n, f, generator=g).bfloat16().to(dev)
+    x = gu.double().requires_grad_(True)
+    a, u = x.chunk(2, dim=-1)
+    y = torch.nn.functional.silu(a) * u
+    y.backward(dy.double())
+    for got, want in ((model_ops.swiglu_fwd_raw(gu), y), (model_ops.swiglu_bwd_raw(gu, dy), x.grad)):
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * (1 + want.abs())).all()
+
+
+@pytest.mark.parametrize("n", [8, 8 * 257, 8 * (148 * 8 * 256 + 5)])
+def test_scaled_gradients(dev, n):
+    """The roundings are those of an fp32 product (the scalar is not rounded to bf16 first) and an accumulation of
+    their own, bit for bit."""
+    src, old = torch.randn(n, device=dev).bfloat16(), torch.randn(n, device=dev).bfloat16()
+    src[0] = float("inf")
+    for v in (1.0, 0.37):
+        g = torch.tensor(v, device=dev)
+        prod = (src.float() * g).bfloat16()
+        assert torch.equal(model_ops.scale_rows(src, g), prod)
+        dst = old.clone()
+        model_ops.scale_rows(src, g, dst)
+        assert torch.equal(dst, old + prod)
+
+
+@pytest.mark.parametrize("tokens", ["one", "same", "mixed"])
+@pytest.mark.parametrize("hidden", [8, 520, 1024])
+def test_embedding_gradient(dev, tokens, hidden):
+    """fp32 sums (1e-5 of the magnitudes) rounded to bf16 before and after they are added to the old gradient (2^-8 of
+    both); rows that no token names keep theirs."""
+    g = torch.Generator().manual_seed(hidden)
+    ids = {"one": torch.tensor([3]), "same": torch.full((1030,), 6), "mixed": torch.randint(0, 40, (700,), generator=g)}[tokens].to(dev)
+    dy = torch.randn(ids.shape[0], hidden, generator=g).bfloat16().to(dev)
+    grad = torch.randn(50, hidden, generator=g).bfloat16().to(dev)
+    add = torch.zeros(50, hidden, dtype=torch.float64, device=dev).index_add_(0, ids, dy.double())
+    mag = torch.zeros(50, hidden, dtype=torch.float64, device=dev).index_add_(0, ids, dy.double().abs())
+    want, old = grad.double() + add, grad.clone()
+    model_ops.embedding_grad(ids, dy, grad)
+    assert ((grad.double() - want).abs() <= 2.0 ** -8 * (add.abs() + want.abs()) + 1e-5 * mag + 1e-9).all()
+    rest = torch.ones(50, dtype=torch.bool, device=dev)
+    rest[ids] = False
+    assert torch.equal(grad[rest], old[rest])
+
+
 def test_cross_entropy(dev):
     torch.manual_seed(0)
     logits = (3 * torch.randn(129, 4096, device=dev)).bfloat16()
