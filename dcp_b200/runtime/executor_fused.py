@@ -258,7 +258,6 @@ class FusedAttentionExecutor:
         if own:
             out, lse = self.out, self.lse
         p, a = self.program, self.arena
-        main = torch.cuda.current_stream(self.device)
         tok = self._call_begin("fwd")
         self._mark("fwd:start")
         if self.poison:
@@ -309,7 +308,6 @@ class FusedAttentionExecutor:
         ``lse``: as in ``forward``, instead of what the arenas hold (single rank; ``out`` and ``lse`` both or none)."""
         p, a = self.program, self.arena
         assert self.world == 1 or (q is None and kv is None and out is None), "peers read the arenas"
-        main = torch.cuda.current_stream(self.device)
         n = p.q_local_rows
         tok = self._call_begin("bwd")
         self._mark("bwd:start")

@@ -185,15 +185,20 @@ class FusedPlanExecutor:
 
     # ---- the same two calls for DCPAttention: results belong to the caller, and with a single rank the kernels read
     # bf16 tensors of 128 channels where they are; other types and widths are converted in one pass each way
-    def _as_kernel_rows(self, t, like) -> torch.Tensor:
-        """``t`` on the executor's device as contiguous, aligned [..., head_dim] rows of a type the row kernels take."""
-        t = t.reshape(like.shape[:-1] + (self.head_dim,)).to(like.device).contiguous()
-        if t.dtype not in (torch.float32, torch.float16, torch.bfloat16):
+    def _as_kernel_rows(self, t, kv: bool = False) -> torch.Tensor:
+        """``t`` (Q-like, or KV-like) on the executor's device as contiguous, aligned [..., head_dim] rows of a type
+        the row kernels take."""
+        ex, p = self.impl, self.impl.program
+        t = t.reshape((p.kv_local_rows, 2, ex.hkv, self.head_dim) if kv else (p.q_local_rows, ex.hq, self.head_dim))
+        if t.device != ex.q.device:
+            t = t.to(ex.q.device)
+        if t.dtype not in (torch.bfloat16, torch.float16, torch.float32):
             t = t.to(torch.bfloat16)
-        return t if self.impl.usable(t) else t.clone()
+        t = t.contiguous()
+        return t if t.data_ptr() % 16 == 0 else t.clone()
 
-    def _in_place(self, *tensors) -> bool:
-        return self.head_dim == self.impl.q_local().shape[-1] and all(t.dtype == torch.bfloat16 for t in tensors)
+    def _in_place(self, a, b) -> bool:
+        return self.head_dim == 128 and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
 
     def _load_arena(self, q, kv) -> None:
         """q / kv (``_as_kernel_rows``) into the arenas."""
@@ -224,7 +229,7 @@ class FusedPlanExecutor:
         if ex.world > 1:
             out, lse = self.forward(q, kv)
             return out.clone(), lse.clone(), self._epoch
-        qk, kvk = self._as_kernel_rows(q, ex.q_local()), self._as_kernel_rows(kv, ex.kv_local())
+        qk, kvk = self._as_kernel_rows(q), self._as_kernel_rows(kv, True)
         out, lse = ex.new_results()
         if self._in_place(qk, kvk):
             self._epoch = -1          # the arenas do not hold this call's operands
@@ -241,9 +246,9 @@ class FusedPlanExecutor:
         if ex.world > 1:
             dq, dkv = self.backward(q, kv, out, dout, lse)
             return dq.clone(), dkv.clone()
-        qk, kvk = self._as_kernel_rows(q, ex.q_local()), self._as_kernel_rows(kv, ex.kv_local())
-        ok, dok = self._as_kernel_rows(out, ex.q_local()), self._as_kernel_rows(dout, ex.q_local())
-        lse = lse.reshape(ex.lse_local().shape).to(out.device, torch.float32).contiguous()
+        qk, kvk = self._as_kernel_rows(q), self._as_kernel_rows(kv, True)
+        ok, dok = self._as_kernel_rows(out), self._as_kernel_rows(dout)
+        lse = lse.reshape(ex.hq, ex.program.q_local_rows).to(ok.device, torch.float32).contiguous()
         if self._in_place(qk, kvk):
             args = (qk, kvk)
         else:
