@@ -198,9 +198,8 @@ class _DecoderLayerFn(torch.autograd.Function):
         dh2 = model.tp_sum(torch.mm(dgu, wgu))     # the norm output feeds every rank's gate/up shard
         wgrad(wgu, dgu.t(), h2)
         del dgu, h2
-        dx_mid, dw2 = model_ops.rmsnorm_bwd_raw(x_mid, w2, rstd2, dh2)
+        dx_mid, dw2 = model_ops.rmsnorm_bwd_raw(x_mid, w2, rstd2, dh2, dy)
         del dh2
-        dx_mid.add_(dy)
         ngrad(w2, dw2)
         # ---- attention
         da = torch.mm(dx_mid, wo)
@@ -220,8 +219,7 @@ class _DecoderLayerFn(torch.autograd.Function):
         dh1 = model.tp_sum(torch.mm(dqkv, wqkv))
         wgrad(wqkv, dqkv.t(), h1)
         del dqkv, h1
-        dx, dw1 = model_ops.rmsnorm_bwd_raw(x, w1, rstd1, dh1)
-        dx.add_(dx_mid)
+        dx, dw1 = model_ops.rmsnorm_bwd_raw(x, w1, rstd1, dh1, dx_mid)
         ngrad(w1, dw1)
         if model.grad_ready_hook is not None and not model.accumulate_grads:
             # every matrix gradient of this layer is final: its bucket can be reduced over the
@@ -249,7 +247,7 @@ class _LMHeadLossFn(torch.autograd.Function):
             logits = hc @ weight.t()
             loss = model_ops.cross_entropy_inplace(logits, labels[t0:t0 + chunk], grad_scale)
             total += loss.sum()
-            dh[t0:t0 + chunk] = logits @ weight
+            torch.mm(logits, weight, out=dh[t0:t0 + chunk])
             if t0 == 0:
                 dweight = torch.mm(logits.t(), hc)
             else:

@@ -58,13 +58,14 @@ def rmsnorm_fwd_raw(x: torch.Tensor, w: torch.Tensor, eps: float):
     return y, rstd
 
 
-def rmsnorm_bwd_raw(x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, dy: torch.Tensor):
-    """(dx bf16, dw fp32) for contiguous 2-D x / dy; no autograd."""
+def rmsnorm_bwd_raw(x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, dy: torch.Tensor, residual: torch.Tensor = None):
+    """(dx bf16, dw fp32) for contiguous 2-D x / dy; ``residual`` (bf16, contiguous, like dx) is added to dx; no autograd."""
+    assert residual is None or (residual.is_contiguous() and residual.shape == x.shape and residual.dtype == x.dtype)
     dx = torch.empty_like(x)
     dw = torch.zeros(x.shape[1], dtype=torch.float32, device=x.device)
-    _lib.check(_lib.load().dcpk_rmsnorm_bwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(dy), _lib.ptr(rstd), _lib.ptr(dx),
-                                            _lib.ptr(dw), _c_int(x.shape[0]), _c_int(x.shape[1]), _lib.stream_handle()),
-               "rmsnorm_bwd")
+    _lib.check(_lib.load().dcpk_rmsnorm_bwd_add(_lib.ptr(x), _lib.ptr(w), _lib.ptr(dy), _lib.ptr(rstd), _lib.ptr(dx), _lib.ptr(dw),
+                                                ctypes.c_void_p(0) if residual is None else _lib.ptr(residual), _c_int(x.shape[0]),
+                                                _c_int(x.shape[1]), _lib.stream_handle()), "rmsnorm_bwd")
     return dx, dw
 
 

@@ -291,6 +291,41 @@ def test_swiglu(dev):
     assert ((gu.grad.float() - gr.grad).abs() / (gr.grad.abs() + 1.0)).max() < 2e-2
 
 
+@pytest.mark.parametrize("rows", [1, 7, 9, 300, 4000])
+@pytest.mark.parametrize("hidden", [1024, 4096])
+def test_rmsnorm_backward_with_residual(dev, rows, hidden):
+    """One rounding to bf16 of the sum (2^-8 of it) plus 1e-5 for the fp32 row sums; dW is an fp32 sum over the rows
+    (1e-5 of the magnitudes), whatever the number of CTAs."""
+    g = torch.Generator().manual_seed(rows + hidden)
+    x, dy, res = (torch.randn(rows, hidden, generator=g).bfloat16().to(dev) for _ in range(3))
+    w = (1 + 0.1 * torch.randn(hidden, generator=g)).bfloat16().to(dev)
+    _, rstd = model_ops.rmsnorm_fwd_raw(x, w, 1e-5)
+    x64, r64 = x.double(), rstd.double()[:, None]
+    gw = dy.double() * w.double()
+    base = r64 * (gw - x64 * r64 * (gw * x64 * r64).mean(-1, keepdim=True))
+    terms = dy.double() * x64 * r64
+    for residual in (None, res):
+        dx, dw = model_ops.rmsnorm_bwd_raw(x, w, rstd, dy, residual)
+        want = base if residual is None else base + res.double()
+        assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * (1 + base.abs())).all()
+        assert ((dw.double() - terms.sum(0)).abs() <= 1e-5 * (terms.abs().sum(0) + 1)).all()
+
+
+@pytest.mark.parametrize("vocab", [8, 32760, 32768, 40008])
+def test_cross_entropy_row_widths(dev, vocab):
+    """Both CTA widths, fp64 oracle: the gradient is rounded to bf16 once (2^-8) and the fast exponentials are good to
+    1e-5 of a probability; the loss is an fp32 logarithm of an fp32 sum."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = (3 * torch.randn(5, vocab, generator=g)).bfloat16().to(dev)
+    labels = torch.tensor([0, vocab - 1, vocab // 2, -100, 7], device=dev)
+    l64 = logits.double()
+    want = torch.nn.functional.cross_entropy(l64, labels.clamp(min=0), reduction="none") * (labels >= 0)
+    grad = (l64.softmax(-1) - torch.nn.functional.one_hot(labels.clamp(min=0), vocab)) * (labels >= 0)[:, None] * 0.5
+    loss = model_ops.cross_entropy_inplace(logits, labels, 0.5)
+    assert ((loss - want).abs() < 1e-4).all()
+    assert ((logits.double() - grad).abs() <= 2.0 ** -8 * grad.abs() + 1e-5 * l64.softmax(-1) + 1e-7).all()
+
+
 @pytest.mark.parametrize("n,f", [(1, 8), (3, 2040), (2, 2048), (5, 8200), (300, 1024)])
 def test_swiglu_row_lengths(dev, n, f):
     """Row lengths around a multiple of the CTA's stride, fp64 oracle: the result is rounded to bf16 once (2^-8), plus
