@@ -148,6 +148,7 @@ class ShardedAdamW:
         self._side_used = False
         self.sq_norm = torch.zeros(1, dtype=torch.float32, device=dev)
         self.sq_parts = torch.zeros(2, dtype=torch.float32, device=dev)   # [replicated, sharded]
+        self.sq_sum = torch.zeros(2, dtype=torch.float64, device=dev)     # one rank's buckets, [replicated or all, sharded]
         self.clip_coef = torch.ones(1, dtype=torch.float32, device=dev)
         self.grad_scale = 1.0
         self.extra_status = extra_status
@@ -217,14 +218,16 @@ class ShardedAdamW:
         grads, params = _ptr_array(a.peer_ptrs("grads")), _ptr_array(a.peer_ptrs("params"))
         clip_ptr = ctypes.c_void_p(0)
         if self.clip is not None:
-            self.sq_norm.zero_()
-            if self.tp_group is not None:
-                self.sq_parts.zero_()
+            self.sq_sum.zero_()
             for s in self.shards:
+                sharded = self.tp_group is not None and self.buckets[s.bucket][0] >= self.n_replicated
                 _lib.check(lib.dcpk_grad_sqnorm(grads, ctypes.c_int(b.world), ctypes.c_long(s.flat_off),
                                                 ctypes.c_long(s.length), ctypes.c_float(grad_scale),
-                                                _lib.ptr(self._sq_slot(s)), _lib.stream_handle()), "grad_sqnorm")
-            self._finish_norm()
+                                                ctypes.c_void_p(self.sq_sum.data_ptr() + 8 * sharded), _lib.stream_handle()),
+                           "grad_sqnorm")
+            if self.tp_group is not None:
+                self.sq_parts.copy_(self.sq_sum)
+            self._finish_norm(self.tp_group is None)
             clip_ptr = _lib.ptr(self.clip_coef)
         for s in self.shards:
             _lib.check(lib.dcpk_fused_rs_adamw_ag(
@@ -235,8 +238,9 @@ class ShardedAdamW:
                 ctypes.c_int(self.step_count), clip_ptr, st_a, st_b, _lib.stream_handle()), "fused_rs_adamw_ag")
         self.kernel_launches += 2 * len(self.shards)
 
-    def _finish_norm(self) -> None:
-        """Total squared gradient norm over all ranks (one scalar all-reduce) -> clip coefficient."""
+    def _finish_norm(self, from_sum: bool = False) -> None:
+        """Total squared gradient norm over all ranks (one scalar all-reduce) -> clip coefficient.  ``from_sum``: the
+        norm is the 64-bit sum this rank has."""
         import torch.distributed as dist
         if self.tp_group is not None:
             if self.bufs.world > 1:
@@ -245,8 +249,9 @@ class ShardedAdamW:
             self.sq_norm.copy_(self.sq_parts.sum().reshape(1))
         elif self.bufs.world > 1:
             dist.all_reduce(self.sq_norm, group=self.group)
-        _lib.check(_lib.load().dcpk_clip_coef(_lib.ptr(self.sq_norm), ctypes.c_float(self.clip), _lib.ptr(self.clip_coef),
-                                              _lib.stream_handle()), "clip_coef")
+        _lib.check(_lib.load().dcpk_clip_coef(_lib.ptr(self.sq_sum) if from_sum else ctypes.c_void_p(0), _lib.ptr(self.sq_norm),
+                                              ctypes.c_float(self.clip), _lib.ptr(self.clip_coef), _lib.stream_handle()),
+                   "clip_coef")
 
     def _step_overlapped(self, lib, st_a, st_b) -> None:
         b, a = self.bufs, self.bufs.arena

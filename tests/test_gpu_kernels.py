@@ -244,7 +244,7 @@ def test_merge_of_stacked_partials(dev, n, t, h):
 @pytest.mark.parametrize("n", [8, 8 * 1023, 8 * 1025, 8 * (148 * 8 * 256 * 4 + 3)])
 @pytest.mark.parametrize("scale", [1.0, 0.5])
 def test_gradient_norm_and_clip_coefficient(dev, n, scale):
-    """fp32 sums of at most a few hundred terms per thread and a few thousand partial sums: 1e-5 relative; a norm below
+    """fp32 sums of at most a few hundred terms per thread, added in 64 bits: 1e-6 relative; a norm below
     the limit gives exactly 1, a NaN gradient a NaN coefficient."""
     from dcp_b200.parallel.dist_optimizer import FlatBuffers, ShardedAdamW
     bufs = FlatBuffers(n, dev)
@@ -252,7 +252,7 @@ def test_gradient_norm_and_clip_coefficient(dev, n, scale):
     bufs.grads.normal_()
     norm = float(bufs.grads.double().norm()) * scale
     opt.step(scale)
-    assert abs(opt.grad_norm() / norm - 1) < 1e-5 and abs(float(opt.clip_coef) / (0.25 / (norm + 1e-6)) - 1) < 2e-5
+    assert abs(opt.grad_norm() / norm - 1) < 1e-6 and abs(float(opt.clip_coef) / (0.25 / (norm + 1e-6)) - 1) < 1e-6
     bufs.grads.mul_(0.1 / norm)
     opt.step(scale)
     assert float(opt.clip_coef) == 1.0
