@@ -10,8 +10,10 @@
 //   dK  += dS^T Q     (SS, A = dS^T tile in shared memory, K-major)
 //   dQ   = dS   K     (SS, A = the same dS^T bytes read MN-major)           -> the TMEM columns of dP^T
 // TMEM (512 columns): S^T / P^T [0,128)  dP^T / dQ [128,256)  dK [256,384)  dV [384,512).
-// Per item t the issuer emits  S(t+1) | dQ(t) dK(t) | dP(t+1) | dV(t+1):  the exponentials of t+1 run
-// under dQ(t) / dK(t), the drain of dQ(t) under dK(t), and dS(t+1) under dV(t+1) and S(t+2).
+// Per item t the issuer emits  S(t+1) | dK(t) dQ(t) | dP(t+1) | dV(t+1):  the exponentials of t+1 run
+// under dK(t) / dQ(t), and dS(t+1) under dV(t+1) and S(t+2).  dK comes before dQ although the drain of dQ is not
+// hidden behind it then: it hands the Q tile back 580 cycles earlier, and a Q tile that arrives late holds up all
+// that follows (full 5.02 -> 4.98 ms, causal 3.82 -> 3.77, sink + window 1.41 -> 1.38 at the size below).
 // Warps: 0-15 gradient (warp = 32 key rows x 32 queries), 16-23 drain dQ (thread = 64 channels of a query row; a
 // [32 queries x 32 channels] swizzled fp32 tile per step, added to the accumulator with one tiled TMA
 // reduce-add, or red.global.add.v4 for a peer's accumulator), 24 TMA producer, 25 UMMA issuer, 26
@@ -28,8 +30,8 @@
 // What bounds it now: the shared-memory pipe.  An item moves 2304 wavefronts of UMMA operands, about 1800 of
 // loads and stores (dS^T, dQ staging, statistics) and about 1000 of TMA traffic in its 4100 to 4300 cycles;
 // the tensor pipe is 55 % busy.  Without the dQ drain an item takes 15 % less.
-// Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 5.02 ms (1095
-// TFLOP/s), causal 4.99 -> 3.81 ms (1081), sink + window 1.84 -> 1.41 ms (990).
+// Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104
+// TFLOP/s), causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
 //
 // The first `n_copy_rows` rows of the grid are fetch CTAs: they compute nothing and bring the next plan
 // stage's remote operands (Q, dO, KV rows and the lse / delta statistics of the queries) from peer
@@ -449,15 +451,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (elect_one()) {
           const uint32_t q_addr = smem_u32(sm.q[t & 1]);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)  // 16 keys per step
-            umma_ss(tmem + cdP, make_sdesc_sw128(ds_addr + k * 2048, kHalf, 1024), make_sdesc_sw128(k_addr + k * 2048, kHalf, 1024),
-                    idesc_dq, k > 0 ? 1u : 0u);
-          umma_commit(&sm.dq_full);
-#pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 queries per step
             umma_ss(tmem + cdK, make_sdesc_sw128(ds_addr + (k >> 2) * kHalf + (k & 3) * 32, 16, 1024),
                     make_sdesc_sw128(q_addr + k * 2048, kHalf, 1024), idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&sm.q_empty[t & 1]);   // Q(t) and the dS^T tile are free
+          umma_commit(&sm.q_empty[t & 1]);   // Q(t) is free
+#pragma unroll
+          for (int k = 0; k < 8; ++k)  // 16 keys per step
+            umma_ss(tmem + cdP, make_sdesc_sw128(ds_addr + k * 2048, kHalf, 1024), make_sdesc_sw128(k_addr + k * 2048, kHalf, 1024),
+                    idesc_dq, k > 0 ? 1u : 0u);
+          umma_commit(&sm.dq_full);            // and so is the dS^T tile
         }
         __syncwarp();
         TL_ADD(13, tl_t);
@@ -574,8 +576,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       TL_ADD(3, tl_t);
       ok = mbar_wait(&sm.delta_full, t & 1, abort_word);
       ok = ok && mbar_wait(&sm.dp_full, t & 1, abort_word);
-      // dK of the previous item must have finished reading the dS^T tile
-      if (t > 0) ok = ok && mbar_wait(&sm.q_empty[st ^ 1], ((t - 1) >> 1) & 1, abort_word);
+      // dK and dQ of the previous item must have finished reading the dS^T tile
+      if (t > 0) ok = ok && mbar_wait(&sm.dq_full, (t - 1) & 1, abort_word);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       TL_ADD(4, tl_t);
