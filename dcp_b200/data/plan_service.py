@@ -129,13 +129,21 @@ def plan_iteration_all(spec: PlanSpec, iteration: int) -> Dict[int, RankPlan]:
     return plan_batch_all(spec, iteration, seqlens, batch, info, group_members=members)
 
 
+# Part of the key of a cached plan: raised whenever what a plan file holds, or what the kernels expect of the tables in
+# it, changes.
+PLAN_FORMAT = 1
+
+
 def batch_signature(spec: PlanSpec, rank: int, seqlens: Sequence[int], mask_fn_info, group_members) -> str:
-    """Stable key of everything a rank's plan depends on (the iteration number is not part of it:
-    the same batch planned at another step gives the same plan)."""
+    """Stable key of everything a rank's plan depends on, the format of the kernel tables and their tile sizes
+    included (the iteration number is not part of it: the same batch planned at another step gives the same plan)."""
     import hashlib
+
+    from ..ops import attention as attn_ops
+    form = (PLAN_FORMAT, attn_ops.TILE_M_PAIR, attn_ops.TILE_N, attn_ops.Q_TILE_BWD)
     fields = {k: v for k, v in vars(spec).items() if k not in ("cache_dir", "seed")}
     fields["length_dist"] = vars(spec.length_dist) if hasattr(spec.length_dist, "__dict__") else str(spec.length_dist)
-    text = repr((sorted(fields.items(), key=lambda kv: kv[0]), rank, list(map(int, seqlens)), mask_fn_info, group_members))
+    text = repr((form, sorted(fields.items(), key=lambda kv: kv[0]), rank, list(map(int, seqlens)), mask_fn_info, group_members))
     return hashlib.sha1(text.encode()).hexdigest()
 
 

@@ -196,6 +196,20 @@ def test_plan_cache_reuses_plans_by_batch_signature(tmp_path):
     assert s0 != batch_signature(mk(cache_dir=str(tmp_path), mem_imbalance_epsilon=0.2), 0, [100, 200], None, None)
 
 
+def test_cached_plan_of_another_table_format_is_planned_again(tmp_path, monkeypatch):
+    """A plan file written for other kernel tables is not used: its key holds the format and the tile sizes."""
+    from dcp_b200.data import plan_service
+    from dcp_b200.ops import attention
+    spec = plan_service.PlanSpec(world=1, dcp_size=1, tokens_per_step=1024, n_heads=8, n_kv_heads=2, block_size=256, vocab=100)
+    key = lambda: plan_service.batch_signature(spec, 0, [700, 324], None, None)
+    keys = {key()}
+    monkeypatch.setattr(plan_service, "PLAN_FORMAT", plan_service.PLAN_FORMAT + 1)
+    keys.add(key())
+    monkeypatch.setattr(attention, "Q_TILE_BWD", 64)
+    keys.add(key())
+    assert len(keys) == 3
+
+
 def test_plan_service_validate_mode(monkeypatch):
     """DCP_B200_VALIDATE=1: every rank's tables are lowered and cross-checked before the rank's own
     program is handed out; the program is the same as without the check."""
