@@ -15,7 +15,7 @@ import concurrent.futures as cf
 import multiprocessing as mp
 import os
 import time
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 from typing import Dict, List, Optional, Sequence
 
 import numpy as np
@@ -130,8 +130,8 @@ def plan_iteration_all(spec: PlanSpec, iteration: int) -> Dict[int, RankPlan]:
 
 
 # Part of the key of a cached plan: raised whenever what a plan file holds, or what the kernels expect of the tables in
-# it, changes.
-PLAN_FORMAT = 1
+# it, changes.  2: rows of the packed batch in place of the token arrays.
+PLAN_FORMAT = 2
 
 
 def batch_signature(spec: PlanSpec, rank: int, seqlens: Sequence[int], mask_fn_info, group_members) -> str:
@@ -148,23 +148,28 @@ def batch_signature(spec: PlanSpec, rank: int, seqlens: Sequence[int], mask_fn_i
 
 
 def _cached_plan(spec, iteration, rank, seqlens, batch, mask_fn_info, group_members):
-    """Plan-cache lookup / fill around ``plan_batch``; token arrays are re-derived from the batch on
-    every call, so only planning work is saved."""
+    """Plan-cache lookup / fill around ``plan_batch``.  A file holds the plan and, in place of its token arrays, the
+    rows of the packed batch that this rank takes (``tokens``): tokens, labels and positions are always cut from
+    ``batch``, so only planning work is saved."""
     import pickle
     key = batch_signature(spec, rank, seqlens, mask_fn_info, group_members)
     path = os.path.join(spec.cache_dir, f"plan_{key}.pkl")
     if os.path.exists(path):
         with open(path, "rb") as f:
             plan = pickle.load(f)
-        plan.iteration = iteration
-        return plan
-    plan = plan_batch(spec, iteration, rank, seqlens, batch, mask_fn_info, group_members=group_members)
-    os.makedirs(spec.cache_dir, exist_ok=True)
-    tmp = f"{path}.{os.getpid()}.tmp"
-    with open(tmp, "wb") as f:
-        pickle.dump(plan, f)
-    os.replace(tmp, path)            # atomic: a concurrent reader never sees a partial file
-    return plan
+    else:
+        rows = np.arange(int(sum(seqlens)), dtype=np.int64)
+        plan = plan_batch(spec, iteration, rank, seqlens, {"tokens": rows, "labels": rows, "positions": rows}, mask_fn_info,
+                          group_members=group_members)
+        plan = replace(plan, labels=plan.labels[:0].clone(), positions=plan.positions[:0].clone())
+        os.makedirs(spec.cache_dir, exist_ok=True)
+        tmp = f"{path}.{os.getpid()}.tmp"
+        with open(tmp, "wb") as f:
+            pickle.dump(plan, f)
+        os.replace(tmp, path)            # atomic: a concurrent reader never sees a partial file
+    take = plan.tokens.numpy()
+    own = {k: torch.from_numpy(np.ascontiguousarray(np.asarray(batch[k])[take])) for k in ("tokens", "labels", "positions")}
+    return replace(plan, iteration=iteration, **own)
 
 
 def plan_batch(spec: PlanSpec, iteration: int, rank: int, seqlens: Sequence[int], batch: Dict[str, np.ndarray],

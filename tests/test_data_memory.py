@@ -196,6 +196,22 @@ def test_plan_cache_reuses_plans_by_batch_signature(tmp_path):
     assert s0 != batch_signature(mk(cache_dir=str(tmp_path), mem_imbalance_epsilon=0.2), 0, [100, 200], None, None)
 
 
+def test_cached_plan_takes_the_tokens_of_its_own_batch(tmp_path):
+    """Batches of equal lengths share a cached plan, never the tokens, labels or positions in it."""
+    from dcp_b200.data import synth
+    from dcp_b200.data.plan_service import PlanSpec, plan_iteration
+    mk = lambda **kw: PlanSpec(world=2, dcp_size=2, tokens_per_step=2048, n_heads=8, n_kv_heads=2, block_size=256,
+                               length_dist=synth.LengthDist("fixed", fixed=512), vocab=1000, **kw)
+    for it in (0, 1, 0):
+        for rank in (0, 1):
+            got, want = plan_iteration(mk(cache_dir=str(tmp_path)), it, rank), plan_iteration(mk(), it, rank)
+            assert got.iteration == it and got.seqlens == want.seqlens
+            for name in ("tokens", "labels", "positions"):
+                a, b = getattr(got, name), getattr(want, name)
+                assert a.dtype == b.dtype and torch.equal(a, b)
+    assert len(list(tmp_path.iterdir())) == 2          # one plan per rank
+
+
 def test_cached_plan_of_another_table_format_is_planned_again(tmp_path, monkeypatch):
     """A plan file written for other kernel tables is not used: its key holds the format and the tile sizes."""
     from dcp_b200.data import plan_service
