@@ -244,7 +244,9 @@ class FusedPlanExecutor:
     def backward_fresh(self, q, kv, out, dout, lse, token):
         ex = self.impl
         if ex.world > 1:
-            dq, dkv = self.backward(q, kv, out, dout, lse)
+            if token != ex.arena_epoch:      # another call's operands took the arenas meanwhile, on every rank
+                self._epoch = -1
+            dq, dkv = self.backward(q, kv, out, dout.contiguous(), lse)
             return dq.clone(), dkv.clone()
         qk, kvk = self._as_kernel_rows(q), self._as_kernel_rows(kv, True)
         ok, dok = self._as_kernel_rows(out), self._as_kernel_rows(dout)

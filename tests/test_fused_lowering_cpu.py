@@ -301,3 +301,37 @@ def test_backward_key_tiles_come_group_by_group():
         assert seen == [1, 3, 2, 0] and groups == sorted(groups, key=seen.index)
         assert all(a >= b for x, y, a, b in zip(groups, groups[1:], counts, counts[1:]) if x == y)
         assert t.max_items == max(counts) and t.n_items == sum(counts)
+
+
+def test_backward_of_an_earlier_call_gets_its_own_operands_on_several_ranks():
+    """Two forwards before the first one's backward: the arenas hold the second call's operands by then, and on several
+    ranks too the first call's have to be put back (an executor that records what its backward finds in the arenas)."""
+    from dcp_b200.runtime.interface import DCPAttention, FusedPlanExecutor
+
+    class Arenas:
+        world, arena_epoch, _staging_valid = 2, 0, False
+
+        def __init__(self):
+            self.q, self.kv, self.out, self.lse = (torch.zeros(*s) for s in ((6, 4, 128), (6, 2, 2, 128), (6, 4, 128), (4, 6)))
+
+        q_local, kv_local, out_local, lse_local = (lambda self, n=n: getattr(self, n) for n in ("q", "kv", "out", "lse"))
+
+        def inputs_written(self):
+            self.arena_epoch += 1
+            self._staging_valid = False
+
+        def forward(self):
+            self._staging_valid = True
+            self.out.copy_(self.q)
+            return self.out, self.lse
+
+        def backward(self, dout):
+            return self.q.clone(), self.kv.clone()
+
+    ex = FusedPlanExecutor.__new__(FusedPlanExecutor)
+    ex.impl, ex.head_dim, ex._epoch = Arenas(), 128, -1
+    calls = [(torch.randn(6, 4, 128, requires_grad=True), torch.randn(6, 2, 2, 128, requires_grad=True)) for _ in range(2)]
+    outs = [DCPAttention.apply(ex, False, False, *c) for c in calls]
+    for out, (q, kv) in zip(outs, calls):
+        dq, dkv = torch.autograd.grad(out, (q, kv), torch.ones_like(out))
+        assert torch.equal(dq, q) and torch.equal(dkv, kv)
