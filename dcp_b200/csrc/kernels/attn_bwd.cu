@@ -18,7 +18,10 @@
 // [32 queries x 32 channels] swizzled fp32 tile per step, added to the accumulator with one tiled TMA
 // reduce-add, or red.global.add.v4 for a peer's accumulator), 24 TMA producer, 25 UMMA issuer, 26
 // per-query statistics, 27 idle.  dK/dV stay in TMEM for the CTA's lifetime and are added once
-// with red.global.add.v4.f32.
+// with red.global.add.v4.f32; the CTAs of a split head group first add their shares up through distributed
+// shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
+// (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
+// every key tile as it comes: its last bits may differ from run to run.
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
@@ -43,6 +46,7 @@
 // that follow it (dcp/ops/fused_ops.py:1087-1360), which the atomics make unnecessary.
 #include <limits.h>
 #include <math.h>
+#include <stddef.h>
 
 #include "attn_common.cuh"
 #include "copy_jobs.cuh"
@@ -126,6 +130,7 @@ struct __align__(1024) BwdSmem {
 // a separately instantiated kernel (kTL) so the production kernel carries no probe branches; each
 // phase includes the cost of one probe (about 110 cycles).
 __device__ long long* g_bwd_timeline = nullptr;
+static_assert(offsetof(BwdSmem, dout) == 256 * kHeadDim * sizeof(float), "K, V and Q tiles hold a gradient share");
 #define TL_ADD(idx, t_prev)                                                        \
   do {                                                                             \
     if constexpr (kTL) if (tl) { long long now_ = clock64(); if (lane == 0) atomicAdd(reinterpret_cast<unsigned long long*>(tl + (idx)), (unsigned long long)(now_ - (t_prev))); (t_prev) = now_; } \
@@ -135,6 +140,9 @@ __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");
 }
+
+// row `row` (0-127 dK, 128-255 dV) of a CTA's gradient share: 128 floats, 16-byte pieces swizzled by the row
+__device__ __forceinline__ float* share_of(BwdSmem& sm, int row) { return reinterpret_cast<float*>(sm.k) + row * kHeadDim; }
 
 // lane i holds row i of a 32 x 32 bit matrix; afterwards lane i holds column i
 __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
@@ -605,7 +613,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       ok = __all_sync(0xffffffffu, mbar_wait(&sm.acc_full, 0, abort_word));
       if (ok) {
         tc_fence_after();
-        // lane = key row; warps 0-7 add dK, warps 8-15 dV, half of the channels each
+        // lane = key row; warps 0-7 take dK, warps 8-15 dV, half of the channels each
         const int ch = (hf & 1) * 64;
         float* dst = ptrs.dkv[cta.dkv_dev] + ((size_t(cta.dkv_row + r) * 2 + (hf >> 1)) * hkv + kv_head) * kHeadDim + ch;
         const uint32_t acc = tmem + lane_base + (hf >> 1 ? cdV : cdK) + ch;
@@ -614,7 +622,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           uint32_t reg[32];
           tmem_ld32(acc + 32 * c, reg);
           tmem_wait_ld();
-          if (r < cta.n_valid) {
+          if (parts > 1) {   // K, V and Q have been read for the last time: their 128 KB take the CTA's share
+            float* row = share_of(sm, (hf >> 1) * 128 + r);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              *reinterpret_cast<uint4*>(row + (((ch >> 2) + 8 * c + i) ^ (r & 7)) * 4) =
+                  make_uint4(reg[4 * i], reg[4 * i + 1], reg[4 * i + 2], reg[4 * i + 3]);
+          } else if (r < cta.n_valid) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               red_add_v4(dst + 32 * c + 4 * i, __uint_as_float(reg[4 * i]), __uint_as_float(reg[4 * i + 1]),
@@ -630,10 +644,34 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  if (parts > 1) {
+    // the CTAs of a split head group (a cluster) add their shares up in the order of their heads, each for a part of
+    // the rows: one addition to the accumulator per element, and the same bits in every run
+    cluster_sync();
+    if (warp < 16) {
+      const int rank = blockIdx.x % parts;
+      bool all_ok = n_items > 0;   // an empty list leaves no share behind
+      for (int p = 0; p < parts; ++p) all_ok = all_ok && ld_cluster_u32(smem_u32(&sm.abort_word), p) == 0;
+      if (all_ok)
+        for (int row = rank * 16 + warp; row < 256; row += parts * 16) {   // 0-127 dK, 128-255 dV; lane = 4 channels
+          const int r = row & 127;
+          if (r >= cta.n_valid) continue;
+          const uint32_t addr = smem_u32(share_of(sm, row) + (lane ^ (r & 7)) * 4);
+          float4 sum = ld_cluster_f4(addr, 0);
+          for (int p = 1; p < parts; ++p) {
+            const float4 v = ld_cluster_f4(addr, p);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+          }
+          red_add_v4(ptrs.dkv[cta.dkv_dev] + ((size_t(cta.dkv_row + r) * 2 + (row >> 7)) * hkv + kv_head) * kHeadDim + 4 * lane,
+                     sum.x, sum.y, sum.z, sum.w);
+        }
+    }
+    cluster_sync();   // no CTA's shared memory goes away while another reads it
+  }
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-static constexpr int kSms = 148;
+static constexpr int kSms = 148, kMaxParts = 8;
 static int g_bwd_attr_set[2] = {0, 0};
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
 
@@ -685,15 +723,34 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
   // A CTA visits its items once per query head of the group, unless that would leave SMs idle: when the
   // longest item list times the group is more than the average SM's share of all visits, the group is
-  // split over as many CTAs (each adds its part of dK / dV) as it takes to get below that share.
-  // Four sequences of 300 to 2100 tokens, 8 / 2 heads: 64 key tiles with up to 68 visits, 11 per SM on average.
+  // split over as many CTAs (a cluster, at most the portable 8, which adds its parts of dK / dV up in a fixed order)
+  // as it takes to get below that share.  CTAs that all run at once add to a row of dQ in the order of their items, which
+  // in practice gives a short batch the same bits in every run; they become more than one wave only where that takes 32
+  // visits (about 70 us) off the longest list.  Four sequences of 300 to 2100 tokens, 8 / 2 heads: 66 key tiles with up to
+  // 68 visits, 11 per SM on average: 171 us whole, 95 us in two parts (132 CTAs), 69 us in four, and the call, which waits
+  // for its launches, takes 231 us with two and 229 with four.  512 to 4096 tokens: 120 key tiles with up to 128 visits,
+  // 317 us whole, 163 us in four parts (480 CTAs), the call 457 and 319 us.
   const int group = hq / hkv;
   int parts = 1;
-  while (parts < group && (group % parts != 0 || long(max_items) * (group / parts) * kSms > long(n_items_total) * hq)) ++parts;
+  for (int p = 2; p <= group && p <= kMaxParts && long(max_items) * (group / parts) * kSms > long(n_items_total) * hq; ++p) {
+    const bool leaves_wave = long(n_ctas) * hkv * parts <= kSms && long(n_ctas) * hkv * p > kSms;
+    if (group % p == 0 && !(leaves_wave && long(max_items) * (group / parts - group / p) < 32)) parts = p;
+  }
   const int heads_per_cta = group / parts;
-  kernel<<<dim3(hkv * parts, n_ctas + n_copy_rows), kBwdThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      tm_q, tm_do, tm_kv, tm_dq, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = unsigned(parts);
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(hkv * parts, n_ctas + n_copy_rows);
+  cfg.blockDim = dim3(kBwdThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = &cluster;
+  cfg.numAttrs = parts > 1 ? 1 : 0;
+  const cudaError_t rc = cudaLaunchKernelEx(
+      &cfg, kernel, tm_q, tm_do, tm_kv, tm_dq, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
       static_cast<const int4*>(masks), lse, delta, pp, hq, hkv, heads_per_cta, stat_stride, n_dst, int(q_rows), int(kv_rows),
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

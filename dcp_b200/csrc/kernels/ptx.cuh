@@ -209,6 +209,29 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
+// ---------------------------------------------------------------- clusters: distributed shared memory
+// all threads of all CTAs of the cluster; what was written before is visible to every CTA afterwards
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// the word / four floats at shared-memory address `addr` of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, int rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr(addr, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr(addr, rank)) : "memory");
+  return v;
+}
+
 // ---------------------------------------------------------------- descriptors
 // Instruction descriptor for kind::f16 with bf16 A/B and fp32 accumulate.
 // Bit layout: [4,6) D format (1 = f32); [7,10) A format (1 = bf16); [10,13) B format;

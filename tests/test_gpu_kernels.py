@@ -183,6 +183,42 @@ def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
         assert dq[nq:].abs().max() == 0 and dkv[nkv:].abs().max() == 0
 
 
+@pytest.mark.parametrize("hq,hkv,parts", [(8, 2, 1), (8, 2, 2), (8, 2, 4), (16, 2, 4), (6, 2, 3), (12, 2, 2), (4, 1, 4), (16, 1, 8), (12, 1, 6)])
+def test_attention_backward_split_head_groups(dev, hq, hkv, parts):
+    """A head group over 1, some or all of its possible CTAs (at most 8), partial key and query tiles, fp64 oracle with the
+    bound of ``test_attention_backward_tile_edges``; dK and dV are the same bits in every run."""
+    n = 1500
+    g = torch.Generator().manual_seed(hq * 10 + parts)
+    new = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(dev)
+    q, kv, dout = new(n, hq, 128), new(n, 2, hkv, 128), new(n, hq, 128)
+    rng = np.zeros((n, 4), np.int32)
+    rng[:, 1] = np.arange(n) + 1
+    row = A.AttnRow(0, n, list(range(hq)), [(0, n)], rng)
+    scale = 128 ** -0.5
+    heads = lambda t: t.double().repeat_interleave(hq // t.shape[1], 1).permute(1, 0, 2)
+    q64, k64, v64, do64 = heads(q), heads(kv[:, 0]), heads(kv[:, 1]), heads(dout)
+    s = (q64 @ k64.transpose(1, 2) * scale).masked_fill(~A.ranges_to_dense(rng, n).to(dev), float("-inf"))
+    p = s.softmax(-1)
+    d64 = (p @ v64 * do64).sum(-1)
+    ds = p * (do64 @ v64.transpose(1, 2) - d64[..., None]) * scale
+    fold = lambda t: t.reshape(hkv, hq // hkv, n, 128).sum(1).permute(1, 0, 2)
+    want = ((ds @ k64).permute(1, 0, 2), fold(ds.transpose(1, 2) @ q64), fold(p.transpose(1, 2) @ do64))
+    lse, delta = torch.logsumexp(s, -1).float(), d64.float()
+    tables = A.build_bwd_tables([row], 1024, hq, hkv, dev)
+    # the group is split until the longest list x (heads of a CTA) x 148 SMs is within all visits
+    tables.max_items = tables.n_items * hkv * parts // 148 if parts > 1 else 0
+    first = None
+    for _ in range(10):
+        dq, dkv = torch.zeros(n, hq, 128, device=dev), torch.zeros(n, 2, hkv, 128, device=dev)
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        A.attn_bwd(q, dout, kv, lse, delta, tables, [dq], [dkv], scale, status)
+        assert status.item() == 0
+        first = dkv if first is None else first
+        assert torch.equal(dkv, first)
+    for got, ref in zip((dq, dkv[:, 0], dkv[:, 1]), want):
+        assert (got - ref).abs().max() <= 2e-2 * ref.abs().max()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [8, 96, 128])
 def test_row_conversions(dev, dtype, d):
