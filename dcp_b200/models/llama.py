@@ -228,12 +228,20 @@ class _DecoderLayerFn(torch.autograd.Function):
         return dx, None, None, None, None, None
 
 
+def _direct_grad(weight: torch.Tensor) -> bool:
+    """May a backward add to ``weight.grad`` itself?  Only a gradient buffer that is there when the backward runs, of a
+    form the kernels write, and of a weight that no hook waits for; anything else goes through autograd."""
+    g = weight.grad
+    return g is not None and weight.requires_grad and not weight._backward_hooks and not weight._post_accumulate_grad_hooks and \
+        g.dtype == weight.dtype == torch.bfloat16 and g.is_contiguous() and g.data_ptr() % 16 == 0 and not g.requires_grad
+
+
 class _LMHeadLossFn(torch.autograd.Function):
     """Chunked LM head + cross entropy: logits never exist for more than ``chunk`` tokens, and
     the gradients of the hidden states and of the head weight are formed in the same pass.
 
-    ``write_grad``: the weight gradient is added to ``weight.grad`` by the backward itself, as the
-    hand-written decoder layers do with theirs, instead of being handed to autograd (a product and an
+    ``write_grad``: the weight gradient is added to ``weight.grad`` by the backward itself where that makes no
+    difference to the caller (see ``_direct_grad``), instead of being handed to autograd (a product and an
     accumulation over the whole matrix)."""
 
     @staticmethod
@@ -253,7 +261,7 @@ class _LMHeadLossFn(torch.autograd.Function):
             else:
                 dweight.addmm_(logits.t(), hc)
         ctx.save_for_backward(dh, dweight)
-        ctx.grad = weight.grad if write_grad else None
+        ctx.weight = weight if write_grad else None
         return total * grad_scale
 
     @staticmethod
@@ -261,27 +269,30 @@ class _LMHeadLossFn(torch.autograd.Function):
         dh, dweight = ctx.saved_tensors
         # g is the upstream gradient of the (already scaled) loss; it is 1 in the training loop
         dh = model_ops.scale_rows(dh, g)
-        if ctx.grad is not None:
-            model_ops.scale_rows(dweight, g, ctx.grad)
+        if ctx.weight is not None and _direct_grad(ctx.weight):
+            model_ops.scale_rows(dweight, g, ctx.weight.grad)
             return dh, None, None, None, None, None
         return dh, model_ops.scale_rows(dweight, g), None, None, None, None
 
 
 class _EmbeddingFn(torch.autograd.Function):
-    """Embedding whose backward adds the rows that occur straight into ``weight.grad`` (CUDA, bf16): autograd
-    forms a dense gradient of the whole table and accumulates that."""
+    """Embedding whose backward adds the rows that occur straight into ``weight.grad`` (CUDA, bf16) where that makes
+    no difference to the caller (see ``_direct_grad``): autograd forms a dense gradient of the whole table and
+    accumulates that."""
 
     @staticmethod
     def forward(ctx, tokens, weight):
         ctx.save_for_backward(tokens)
-        ctx.grad = weight.grad
+        ctx.weight = weight
         return F.embedding(tokens, weight)
 
     @staticmethod
     def backward(ctx, dy):
         tokens, = ctx.saved_tensors
-        model_ops.embedding_grad(tokens, dy, ctx.grad)
-        return None, None
+        if _direct_grad(ctx.weight):
+            model_ops.embedding_grad(tokens, dy, ctx.weight.grad)
+            return None, None
+        return None, torch.ops.aten.embedding_dense_backward(dy, tokens, ctx.weight.shape[0], -1, False)
 
 
 class LlamaModel:
@@ -456,16 +467,22 @@ class LlamaModel:
         x = x + F.linear(model_ops.swiglu(gu), p[f"l{l}.wd"])
         return x
 
-    def loss(self, tokens: torch.Tensor, labels: torch.Tensor, positions: torch.Tensor, grad_scale: float) -> torch.Tensor:
+    def loss(self, tokens: torch.Tensor, labels: torch.Tensor, positions: torch.Tensor, grad_scale: float,
+             write_grads: bool = False) -> torch.Tensor:
         """Sum over this rank's tokens of the token losses times ``grad_scale`` (1 / global token
-        count); ``labels`` < 0 are ignored.  Call ``.backward()`` on the result."""
+        count); ``labels`` < 0 are ignored.  Call ``.backward()`` on the result.  With ``layer_levels`` set the
+        decoder layers write their gradients to ``.grad`` themselves.  ``write_grads``: the embedding and the LM head
+        may do so as well, which saves passes over the two tables; only for a caller that runs ``.backward()`` (not
+        ``torch.autograd.grad``) and has no hooks on their gradient-accumulation nodes.  Hooks on the two tensors, a
+        missing ``.grad`` and one that was replaced in between are respected either way."""
         cfg = self.cfg
         self._attn_stash.clear()
         self._stash_enabled = self.cache_attention and self.recompute and torch.is_grad_enabled()
         cos, sin = model_ops.rope_tables(positions, cfg.rope_theta, cfg.head_dim)
         embed = self.p["embed"]
         manual = self.layer_levels is not None and embed.is_cuda and torch.is_grad_enabled()
-        x = _EmbeddingFn.apply(tokens, embed) if manual else F.embedding(tokens, embed)
+        write_grads = write_grads and manual
+        x = _EmbeddingFn.apply(tokens, embed) if write_grads else F.embedding(tokens, embed)
         for l in range(cfg.n_layers):
             if manual:
                 x = _DecoderLayerFn.apply(x, self, l, cos, sin, self.layer_levels[l])
@@ -474,4 +491,4 @@ class LlamaModel:
             else:
                 x = self._layer(x, l, cos, sin)
         h = model_ops.rmsnorm(x, self.p["norm_f"], cfg.eps)
-        return _LMHeadLossFn.apply(h, self.p["lm_head"], labels, grad_scale, self.lm_head_chunk, manual)
+        return _LMHeadLossFn.apply(h, self.p["lm_head"], labels, grad_scale, self.lm_head_chunk, write_grads)

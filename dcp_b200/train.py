@@ -224,7 +224,7 @@ class TrainEngine:
     def run_step(self, toks, labels, pos, n_global_tokens: int) -> torch.Tensor:
         """Forward + backward + optimizer on staged inputs; returns the device loss tensor."""
         self.model.zero_grad()
-        loss = self.model.loss(toks, labels, pos, 1.0 / max(n_global_tokens, 1))
+        loss = self.model.loss(toks, labels, pos, 1.0 / max(n_global_tokens, 1), write_grads=True)
         loss.backward()
         if self.time_optimizer:
             # what the optimizer still costs after the backward: the reduce-scatters of the layer buckets

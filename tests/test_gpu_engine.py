@@ -79,6 +79,54 @@ def test_tensor_parallel_step_two_gpus():
     assert res.returncode == 0 and "TP_OK" in res.stdout, res.stdout[-3000:]
 
 
+def test_head_and_embedding_gradients_reach_autograd():
+    """With hand-written layers the gradients of the embedding and the LM head still answer ``torch.autograd.grad``,
+    tensor hooks, a ``.grad`` that is not there and one replaced before the backward; writing them directly gives the
+    same (the embedding sums fp32 in another order and rounds to bf16 once: 2^-7 of the largest element)."""
+    _need_gpu()
+    from dcp_b200.data import synth
+    from dcp_b200.models.llama import tiny_config
+    from dcp_b200.train import EngineConfig, TrainEngine
+    eng = TrainEngine(EngineConfig(tiny_config(n_layers=1, hidden=1024, n_heads=8, n_kv_heads=2, ffn=2048, vocab=512), tokens_per_step=512,
+                                   block_size=256, length_dist=synth.LengthDist("lognormal", 200.0, 0.6, 64, 512), planner_workers=0,
+                                   activation_budget_gb=0.0), torch.device("cuda", 0))
+    model, plan = eng.model, eng.plans.get(0)
+    assert model.layer_levels is not None
+    inputs = (*eng.stage_inputs(plan), 1.0 / plan.n_global_tokens)
+    pair = [model.p["embed"], model.p["lm_head"]]
+    want = [g.float() for g in torch.autograd.grad(model.loss(*inputs), pair)]
+    assert all(w.abs().max() > 0 for w in want)
+
+    def check(grads):
+        for g, w in zip(grads, want):
+            assert (g.float() - w).abs().max() <= 2.0 ** -7 * w.abs().max()
+
+    for write in (False, True):
+        model.zero_grad()
+        loss = model.loss(*inputs, write_grads=write)
+        old, new = [t.grad for t in pair], [torch.zeros_like(t) for t in pair]
+        for t, g in zip(pair, new):
+            t.grad = g
+        loss.backward()
+        check(new)
+        assert all(t.grad is g for t, g in zip(pair, new)) and all(not g.any() for g in old)
+        for t in pair:
+            t.grad = None
+        model.loss(*inputs, write_grads=write).backward()
+        check([t.grad for t in pair])
+        seen = []
+        handles = [t.register_hook(lambda g, i=i: seen.append(i)) for i, t in enumerate(pair)]
+        handles += [t.register_post_accumulate_grad_hook(lambda t, i=i: seen.append(2 + i)) for i, t in enumerate(pair)]
+        for t, g in zip(pair, old):
+            t.grad = g
+        model.loss(*inputs, write_grads=write).backward()
+        assert sorted(seen) == [0, 1, 2, 3]
+        check([t.grad for t in pair])
+        for h in handles:
+            h.remove()
+    eng.close()
+
+
 @pytest.mark.parametrize("layer_path", ["autograd", "level0", "level1+2", "auto"])
 def test_tiny_model_step_matches_pytorch(layer_path):
     """Every layer implementation (autograd + checkpoint, hand-written backward at each activation
