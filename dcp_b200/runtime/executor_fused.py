@@ -124,7 +124,7 @@ class FusedAttentionExecutor:
         written = int(program.merge_ops[:, 1].sum())
         for t in program.fwd:
             if t is not None:
-                tile = t.tiles.numpy() if isinstance(t.tiles, torch.Tensor) else t.tiles
+                tile = t.tiles.cpu().numpy() if isinstance(t.tiles, torch.Tensor) else t.tiles
                 written += int(tile[(tile[:, 2] == 0) & (tile[:, 6] == program.world + program.rank), 1].sum())
         self._all_rows_written = written >= program.q_local_rows
         # copy jobs per stage: Q + KV rows (forward, and backward when the staging rows were

@@ -316,6 +316,22 @@ def test_reference_api_with_fused_backend(impl):
     assert set(ex.log_memory_usage()) >= {"q", "kv", "dq", "dkv"}
 
 
+def test_program_tables_may_be_on_the_gpu_already():
+    """``prepare`` takes a program whose tables were moved to the device before: the same results."""
+    _need_gpu()
+    import dataclasses
+    from dcp_b200.core.common import get_default_execution_context
+    from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test
+    dev = torch.device("cuda", 0)
+    ex, lq, lkv, *_ = prepare_dcp_distributed_attn_for_test([300, 129], 4, 2, 128, 256, 4, get_default_execution_context(1, 1), 0, "causal",
+                                                            torch.bfloat16, device=dev, executor_impl="fused")
+    want = DCPAttention.apply(ex, False, False, lq, lkv)
+    p = ex.impl.program
+    moved = dataclasses.replace(p, fwd=[t.to(dev) for t in p.fwd], bwd=[t.to(dev) for t in p.bwd])
+    ex.impl.prepare(moved)
+    assert torch.equal(DCPAttention.apply(ex, False, False, lq, lkv), want)
+
+
 @pytest.mark.parametrize("head_dim,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.float32)])
 def test_fused_backend_other_head_dims_and_dtypes(head_dim, dtype):
     """Head dimensions below 128 run zero-padded on the 128-channel kernels and fp16 / fp32 tensors
