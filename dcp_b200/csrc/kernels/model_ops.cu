@@ -303,41 +303,105 @@ __global__ void __launch_bounds__(256) scale_rows_kernel(const uint4* __restrict
 }
 
 // grad[id] += sum over the tokens with that id of dy[token], fp32 sums.  `ids` sorted, `order` the token at each sorted
-// place.  One CTA per (sorted place, 512 channels); only the first place of a run of equal ids works, on the
-// whole run, so each gradient row has one writer and rows no token names are not touched.
-__global__ void __launch_bounds__(64) embedding_grad_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ order,
-                                                            const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ grad,
-                                                            int n_tok, int hidden, long vocab) {
-  const int i = blockIdx.x;
-  const int64_t id = ids[i];
-  if ((i > 0 && ids[i - 1] == id) || id < 0 || id >= vocab) return;
-  const int c = (blockIdx.y * 64 + threadIdx.x) * 8;
-  if (c >= hidden) return;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int j = i; j < n_tok && ids[j] == id; j += 4) {
-    uint4 raw[4];
-    bool in[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      in[k] = j + k < n_tok && ids[j + k] == id;
-      raw[k] = in[k] ? *reinterpret_cast<const uint4*>(dy + size_t(order[j + k]) * hidden + c) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float v[8];
-      unpack8(raw[k], v);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += v[e];
-    }
-  }
+// place.  A run of equal ids is cut at every kSegment-th place, and one CTA per (segment, 512 channels) works on it: the
+// first place of a segment is the first of a run or a multiple of kSegment.  A run that lies in one segment is added to
+// its gradient row at once.  The segments of a longer one leave fp32 sums in `part` (block of kSegment places; 0: from
+// the block's start, 1: a run that begins inside it), which embedding_grad_combine_kernel adds in order: one writer per
+// gradient row, the same bits in every run, and rows no token names are not touched.
+static constexpr int kSegment = 64;
+
+__device__ __forceinline__ void add_rounded(__nv_bfloat16* dst, const float (&acc)[8]) {
   // rounded to bf16 before it is added, as a gradient tensor of its own would be
-  uint4* dst = reinterpret_cast<uint4*>(grad + size_t(id) * hidden + c);
+  uint4* d = reinterpret_cast<uint4*>(dst);
   float old[8], sum[8];
   unpack8(pack8(acc), sum);
-  unpack8(*dst, old);
+  unpack8(*d, old);
 #pragma unroll
   for (int e = 0; e < 8; ++e) sum[e] += old[e];
-  *dst = pack8(sum);
+  *d = pack8(sum);
+}
+
+__global__ void __launch_bounds__(kSegment) embedding_grad_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ order,
+                                                                  const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ grad,
+                                                                  float* __restrict__ part, int n_tok, int hidden, long vocab) {
+  const int i = blockIdx.x, block = i / kSegment, t = threadIdx.x;
+  const int64_t id = ids[i];
+  const bool first = i == 0 || ids[i - 1] != id;
+  if (!(first || i % kSegment == 0) || id < 0 || id >= vocab) return;
+  const int stop = min(n_tok, (block + 1) * kSegment);
+  // the tokens of the segment, read at once: no gradient row waits for a place and its token first
+  __shared__ int64_t token[kSegment];
+  const bool in = i + t < stop && ids[i + t] == id;
+  if (in) token[t] = order[i + t];
+  const int n = __syncthreads_count(in);
+  const bool more = stop < n_tok && ids[stop] == id;
+  const int c = (blockIdx.y * kSegment + t) * 8;
+  if (c >= hidden) return;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const auto row = [&](int j) { return *reinterpret_cast<const uint4*>(dy + size_t(token[j]) * hidden + c); };
+  const auto add = [&](const uint4& raw) {
+    float v[8];
+    unpack8(raw, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] += v[e];
+  };
+  int j = 0;
+  for (; j + 8 <= n; j += 8) {      // eight rows in flight
+    uint4 raw[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) raw[k] = row(j + k);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) add(raw[k]);
+  }
+#pragma unroll 4
+  for (; j < n; ++j) add(row(j));
+  if (first && !more) {
+    add_rounded(grad + size_t(id) * hidden + c, acc);
+  } else {
+    float4* dst = reinterpret_cast<float4*>(part + (size_t(block) * 2 + (i % kSegment != 0)) * hidden + c);
+    dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+}
+
+// One CTA per (block of places, 512 channels): the run that begins in the block and goes on past its end.  Eight rows of
+// 64 threads take every eighth of its sums.
+__global__ void __launch_bounds__(512) embedding_grad_combine_kernel(const int64_t* __restrict__ ids, const float* __restrict__ part,
+                                                                     __nv_bfloat16* __restrict__ grad, int n_tok, int hidden, long vocab) {
+  const int block = blockIdx.x, next = (block + 1) * kSegment;
+  if (next >= n_tok) return;
+  const int64_t id = ids[next];
+  if (ids[next - 1] != id || id < 0 || id >= vocab) return;
+  const bool whole = ids[block * kSegment] == id;          // the run covers the block from its start
+  if (whole && block > 0 && ids[block * kSegment - 1] == id) return;   // and began before it
+  int n = 1;                                               // blocks the run has a sum in
+  for (long b = block + 1;; b += 512) {
+    const long place = (b + threadIdx.x) * kSegment;
+    const int k = __syncthreads_count(place < n_tok && ids[place] == id);
+    n += k;
+    if (k < 512) break;
+  }
+  const int lane = threadIdx.x & 63, row = threadIdx.x >> 6, c = (blockIdx.y * 64 + lane) * 8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  __shared__ float sums[8][64][9];
+  if (c < hidden) {
+#pragma unroll 4
+    for (int k = row; k < n; k += 8) {
+      const float4* src = reinterpret_cast<const float4*>(part + (size_t(block + k) * 2 + (k == 0 && !whole)) * hidden + c);
+      const float4 x = src[0], y = src[1];
+      acc[0] += x.x; acc[1] += x.y; acc[2] += x.z; acc[3] += x.w;
+      acc[4] += y.x; acc[5] += y.y; acc[6] += y.z; acc[7] += y.w;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sums[row][lane][e] = acc[e];
+  }
+  __syncthreads();
+  if (row == 0 && c < hidden) {
+    for (int r = 1; r < 8; ++r)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += sums[r][lane][e];
+    add_rounded(grad + size_t(id) * hidden + c, acc);
+  }
 }
 
 // ------------------------------------------------------------------ cross entropy (loss + dlogits)
@@ -510,13 +574,18 @@ extern "C" int dcpk_scale_rows(const void* src, const float* g, void* dst, long 
   return LAUNCH_OK;
 }
 
-extern "C" int dcpk_embedding_grad(const void* ids, const void* order, const void* dy, void* grad, int n_tok, int hidden,
+// part: fp32 [2 * ceil(n_tok / 64), hidden] of scratch, not read before it is written
+extern "C" int dcpk_embedding_grad(const void* ids, const void* order, const void* dy, void* grad, float* part, int n_tok, int hidden,
                                    long vocab, void* stream) {
   if (n_tok <= 0) return 0;
   if (hidden % 8 != 0 || hidden <= 0) return -3;
-  embedding_grad_kernel<<<dim3(unsigned(n_tok), unsigned((hidden + 511) / 512)), 64, 0, STREAM>>>(
+  const unsigned slices = unsigned((hidden + 511) / 512), blocks = unsigned((n_tok + kSegment - 1) / kSegment);
+  embedding_grad_kernel<<<dim3(unsigned(n_tok), slices), kSegment, 0, STREAM>>>(
       static_cast<const int64_t*>(ids), static_cast<const int64_t*>(order), static_cast<const __nv_bfloat16*>(dy),
-      static_cast<__nv_bfloat16*>(grad), n_tok, hidden, vocab);
+      static_cast<__nv_bfloat16*>(grad), part, n_tok, hidden, vocab);
+  if (blocks > 1)
+    embedding_grad_combine_kernel<<<dim3(blocks - 1, slices), 512, 0, STREAM>>>(
+        static_cast<const int64_t*>(ids), part, static_cast<__nv_bfloat16*>(grad), n_tok, hidden, vocab);
   return LAUNCH_OK;
 }
 

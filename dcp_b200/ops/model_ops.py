@@ -110,9 +110,11 @@ def embedding_grad(tokens: torch.Tensor, dy: torch.Tensor, grad: torch.Tensor) -
     dy = dy.reshape(ids.shape[0], grad.shape[1]).contiguous()
     assert dy.dtype == grad.dtype == torch.bfloat16 and grad.is_contiguous() and grad.shape[1] % 8 == 0
     assert dy.data_ptr() % 16 == 0 and grad.data_ptr() % 16 == 0
-    _lib.check(_lib.load().dcpk_embedding_grad(_lib.ptr(ids), _lib.ptr(order), _lib.ptr(dy), _lib.ptr(grad), _c_int(ids.shape[0]),
-                                               _c_int(grad.shape[1]), _c_long(grad.shape[0]), _lib.stream_handle()),
-               "embedding_grad")
+    # sums of the runs of equal ids that go over the end of a 64-token segment
+    part = torch.empty(2 * -(-ids.shape[0] // 64), grad.shape[1], dtype=torch.float32, device=dy.device)
+    _lib.check(_lib.load().dcpk_embedding_grad(_lib.ptr(ids), _lib.ptr(order), _lib.ptr(dy), _lib.ptr(grad), _lib.ptr(part),
+                                               _c_int(ids.shape[0]), _c_int(grad.shape[1]), _c_long(grad.shape[0]),
+                                               _lib.stream_handle()), "embedding_grad")
 
 
 # --------------------------------------------------------------------------- SwiGLU

@@ -391,6 +391,26 @@ def test_scaled_gradients(dev, n):
         assert torch.equal(dst, old + prod)
 
 
+@pytest.mark.parametrize("runs", [[64], [65], [63, 2, 64, 1], [1, 63, 64, 128, 3], [5, 700, 59], [200, 1, 1, 1, 4500], [40000]])
+def test_embedding_gradient_of_long_runs(dev, runs):
+    """Runs of equal ids that end at, before and past the 64-place segments, with the bound of ``test_embedding_gradient``;
+    the same bits in every run."""
+    g = torch.Generator().manual_seed(len(runs))
+    ids = torch.repeat_interleave(torch.arange(len(runs)) * 3 + 1, torch.tensor(runs))
+    ids = ids[torch.randperm(ids.shape[0], generator=g)].to(dev)
+    dy = torch.randn(ids.shape[0], 520, generator=g).bfloat16().to(dev)
+    old = torch.randn(50, 520, generator=g).bfloat16().to(dev)
+    add = torch.zeros(50, 520, dtype=torch.float64, device=dev).index_add_(0, ids, dy.double())
+    mag = torch.zeros(50, 520, dtype=torch.float64, device=dev).index_add_(0, ids, dy.double().abs())
+    want, first = old.double() + add, None
+    for _ in range(3):
+        grad = old.clone()
+        model_ops.embedding_grad(ids, dy, grad)
+        first = grad if first is None else first
+        assert torch.equal(grad, first)
+    assert ((first.double() - want).abs() <= 2.0 ** -8 * (add.abs() + want.abs()) + 1e-5 * mag + 1e-9).all()
+
+
 @pytest.mark.parametrize("tokens", ["one", "same", "mixed"])
 @pytest.mark.parametrize("hidden", [8, 520, 1024])
 def test_embedding_gradient(dev, tokens, hidden):
