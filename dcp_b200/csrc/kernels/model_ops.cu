@@ -97,8 +97,9 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   }
 }
 
-// persistent CTAs: each walks rows blockIdx.x, +gridDim.x, ... and keeps its dW slice in registers
-template <int kVecs>
+// persistent CTAs: each walks rows blockIdx.x, +gridDim.x, ... and keeps its dW slice in registers.  kResidual is a
+// template parameter: tested at run time it cost rows of 8192 (255 registers) 6 % (16384 rows: 186 -> 199 us)
+template <int kVecs, bool kResidual>
 __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                           const __nv_bfloat16* __restrict__ w,
                                                           const __nv_bfloat16* __restrict__ dy,
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const __nv_bfloat16* _
     for (int i = 0; i < kVecs; ++i) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) g[i][j] = r * (g[i][j] - xh[i][j] * dot);
-      if (residual) {   // the gradient that by-passed the norm, added before the one rounding
+      if (kResidual) {   // the gradient that by-passed the norm, added before the one rounding
         float add[8];
         unpack8(reinterpret_cast<const uint4*>(residual + row * hidden)[threadIdx.x + i * 128], add);
 #pragma unroll
@@ -501,22 +502,26 @@ extern "C" int dcpk_rmsnorm_bwd_add(const void* x, const void* w, const void* dy
   auto X = static_cast<const __nv_bfloat16*>(x); auto W = static_cast<const __nv_bfloat16*>(w);
   auto G = static_cast<const __nv_bfloat16*>(dy); auto DX = static_cast<__nv_bfloat16*>(dx);
   auto R = static_cast<const __nv_bfloat16*>(residual);
-  // persistent CTAs: exactly as many as are resident at once (registers decide), so no CTA waits for a
-  // slot while others already finished their share; at least eight rows each, because every CTA adds its whole
-  // dW slice to the same few lines (2048 rows of 1024: 28 us with 1.4 rows
-  // per CTA, 14 us now)
-  auto launch = [&](auto kernel) {
+  // Persistent CTAs: at most as many as are resident at once (registers decide), so no CTA waits for a slot while
+  // others already finished their share.  Fewer where there are few rows: a CTA's chain of rows grows with rows / CTAs,
+  // and the additions to each line of dW with the CTAs, so the best count grows with the root of the rows.  Counts from
+  // 32 to 1332 timed at 1 to 16384 rows are best at 6.5 roots (rows of 8192, which take twice as long: 9.3), us against as
+  // many CTAs as rows or residents: 256 rows of 1024 10 / 12, 2048 of 1024 17 / 33, 1024 of 4096 18 / 20, 512 of 8192 22 / 23.
+  auto launch = [&](auto kernel, float per_root) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm < 1) per_sm = 2;
-    const int cap = 148 * per_sm, want = (n_rows + 7) / 8;
-    const int grid = want < cap ? want : cap;
-    kernel<<<grid, 128, 0, STREAM>>>(X, W, G, rstd, DX, dw, R, n_rows, hidden);
+    const int root = int(per_root * sqrtf(float(n_rows)) + 0.5f), want = root < 64 ? 64 : root, cap = want < 148 * per_sm ? want : 148 * per_sm;
+    kernel<<<n_rows < cap ? n_rows : cap, 128, 0, STREAM>>>(X, W, G, rstd, DX, dw, R, n_rows, hidden);
+  };
+  const auto sized = [&](auto plain, auto with_residual, float per_root) {
+    if (R) launch(with_residual, per_root);
+    else launch(plain, per_root);
   };
   switch (hidden) {
-    case 1024: launch(rmsnorm_bwd_kernel<1>); break;
-    case 2048: launch(rmsnorm_bwd_kernel<2>); break;
-    case 4096: launch(rmsnorm_bwd_kernel<4>); break;
-    case 8192: launch(rmsnorm_bwd_kernel<8>); break;
+    case 1024: sized(rmsnorm_bwd_kernel<1, false>, rmsnorm_bwd_kernel<1, true>, 6.5f); break;
+    case 2048: sized(rmsnorm_bwd_kernel<2, false>, rmsnorm_bwd_kernel<2, true>, 6.5f); break;
+    case 4096: sized(rmsnorm_bwd_kernel<4, false>, rmsnorm_bwd_kernel<4, true>, 6.5f); break;
+    case 8192: sized(rmsnorm_bwd_kernel<8, false>, rmsnorm_bwd_kernel<8, true>, 9.3f); break;
     default: return -3;
   }
   return LAUNCH_OK;

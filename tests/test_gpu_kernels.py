@@ -376,6 +376,13 @@ def test_swiglu_row_lengths(dev, n, f):
         assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * (1 + want.abs())).all()
 
 
+@pytest.mark.parametrize("rows,hidden", [(2, 2048), (43, 8192), (1000, 8192), (5000, 2048)])
+def test_rmsnorm_backward_grid(dev, rows, hidden):
+    """One, some and all of the CTAs the row count allows, with and without a residual, with the bounds of
+    ``test_rmsnorm_backward_with_residual``."""
+    test_rmsnorm_backward_with_residual(dev, rows, hidden)
+
+
 @pytest.mark.parametrize("n", [8, 8 * 257, 8 * (148 * 8 * 256 + 5)])
 def test_scaled_gradients(dev, n):
     """The roundings are those of an fp32 product (the scalar is not rounded to bf16 first) and an accumulation of
