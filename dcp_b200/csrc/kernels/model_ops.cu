@@ -408,9 +408,12 @@ __global__ void __launch_bounds__(512) embedding_grad_combine_kernel(const int64
 // ------------------------------------------------------------------ cross entropy (loss + dlogits)
 // one CTA per row; vocab must be a multiple of 8.  Rows whose label is < 0 are ignored
 // (loss 0, zero gradient).  dlogits overwrite logits: (softmax - onehot) * grad_scale.
-// The logits are read twice and overwritten.  Wide rows take 1024 threads, so that the rows of all CTAs at work (296 x
-// 256 KB) stay in L2 until they are read again; with 256 threads four times as many rows are under way (4096 rows of
-// 128256: 523 -> 477 us; 2.17 -> 2.09 ms per training step of 16384 tokens).
+// The logits are read twice and overwritten, so the rows under way should stay in L2 until they are read again.  With 256
+// threads 1184 rows are under way, with 1024 threads 296: 1024 from 49152 classes on, where 1184 rows fill L2 (4096 rows
+// of 128256: 517 -> 471 us, of 65536: 264 -> 248, of 50304: 203 -> 199).  Below that 256 threads, which hide latency across
+// rows better (4096 rows of 40008: 164 against 168 us, of 32768: 125 / 139), unless all rows are under way at once
+// anyway: then 1024 threads read a row faster (1184 rows of 40008: 53 against 59 us, of 32768: 45 / 47; of 16384 no
+// more: 31 / 25).
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
                                                             const int64_t* __restrict__ labels,
@@ -602,7 +605,7 @@ extern "C" int dcpk_cross_entropy(void* logits, const void* labels, float* loss,
     kernel<<<n_rows, threads, 0, STREAM>>>(static_cast<__nv_bfloat16*>(logits), static_cast<const int64_t*>(labels), loss,
                                            vocab, grad_scale);
   };
-  if (vocab >= 32768) launch(cross_entropy_kernel<1024>, 1024);
+  if (vocab >= 49152 || (vocab >= 32768 && n_rows <= 148 * 8)) launch(cross_entropy_kernel<1024>, 1024);
   else launch(cross_entropy_kernel<256>, 256);
   return LAUNCH_OK;
 }

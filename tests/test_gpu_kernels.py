@@ -383,6 +383,25 @@ def test_rmsnorm_backward_grid(dev, rows, hidden):
     test_rmsnorm_backward_with_residual(dev, rows, hidden)
 
 
+@pytest.mark.parametrize("rows,vocab", [(1184, 32768), (1185, 32768), (3, 49144), (1185, 49144), (1185, 49152)])
+def test_cross_entropy_dispatch(dev, rows, vocab):
+    """Both sides of the rule that picks the CTA width, with the bounds of ``test_cross_entropy_row_widths``."""
+    g = torch.Generator(device=dev).manual_seed(vocab)
+    logits = (3 * torch.randn(rows, vocab, generator=g, device=dev)).bfloat16()
+    labels = torch.randint(-1, vocab, (rows,), generator=g, device=dev)
+    want = logits.clone()
+    loss = model_ops.cross_entropy_inplace(logits, labels, 0.5)
+    for lo in range(0, rows, 256):
+        l64, lab, got = want[lo:lo + 256].double(), labels[lo:lo + 256], logits[lo:lo + 256].double()
+        grad = l64.softmax(-1)
+        tol = 1e-5 * grad + 1e-7
+        grad[torch.arange(len(lab), device=dev), lab.clamp(min=0)] -= 1.0
+        grad *= 0.5 * (lab >= 0)[:, None]
+        assert ((got - grad).abs() <= 2.0 ** -8 * grad.abs() + tol).all()
+        ref = torch.nn.functional.cross_entropy(l64, lab.clamp(min=0), reduction="none") * (lab >= 0)
+        assert ((loss[lo:lo + 256] - ref).abs() < 1e-4).all()
+
+
 @pytest.mark.parametrize("n", [8, 8 * 257, 8 * (148 * 8 * 256 + 5)])
 def test_scaled_gradients(dev, n):
     """The roundings are those of an fp32 product (the scalar is not rounded to bf16 first) and an accumulation of
