@@ -240,13 +240,18 @@ __global__ void qkv_rope_pack_bwd_kernel(const float* __restrict__ dq, const flo
 }
 
 // ------------------------------------------------------------------ SwiGLU
-// One CTA per row: a flat index over the tensor costs two 64-bit divisions per vector.  Bound by HBM (16384 rows,
-// F = 14336: forward 287 -> 243 us, 5.8 TB/s; backward 437 -> 393 us, 6.0 TB/s).  Two or four vectors per thread
-// in flight were slower (259 / 261 and 415 / 434 us).
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint4* __restrict__ gu, uint4* __restrict__ y, int f_vec) {
-  const uint4* gr = gu + size_t(blockIdx.x) * 2 * f_vec;
-  uint4* yr = y + size_t(blockIdx.x) * f_vec;
-  for (int c = threadIdx.x; c < f_vec; c += 256) {
+// Bound by HBM; a flat index over the tensor would cost two 64-bit divisions per vector.  kWide: one CTA of 256 threads
+// per row (16384 rows, F = 14336: forward 287 -> 243 us, 5.8 TB/s; backward 437 -> 393 us, 6.0 TB/s against the flat
+// index; two or four vectors per thread in flight were slower: 259 / 261 and 415 / 434 us).  Otherwise as many rows per
+// CTA as fit its threads, and wide rows over several CTAs; see swiglu_launch for the choice.
+template <bool kWide>
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint4* __restrict__ gu, uint4* __restrict__ y, size_t n_rows, int f_vec) {
+  const size_t row = kWide ? size_t(blockIdx.x) : size_t(blockIdx.x) * blockDim.y + threadIdx.y;
+  if (!kWide && row >= n_rows) return;
+  const int first = kWide ? threadIdx.x : blockIdx.y * blockDim.x + threadIdx.x, step = kWide ? 256 : gridDim.y * blockDim.x;
+  const uint4* gr = gu + row * 2 * f_vec;
+  uint4* yr = y + row * f_vec;
+  for (int c = first; c < f_vec; c += step) {
     float g[8], u[8];
     unpack8(gr[c], g);
     unpack8(gr[f_vec + c], u);
@@ -255,12 +260,16 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint4* __restrict
     yr[c] = pack8(g);
   }
 }
+template <bool kWide>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const uint4* __restrict__ gu, const uint4* __restrict__ dy,
-                                                         uint4* __restrict__ dgu, int f_vec) {
-  const uint4* gr = gu + size_t(blockIdx.x) * 2 * f_vec;
-  const uint4* dr = dy + size_t(blockIdx.x) * f_vec;
-  uint4* out = dgu + size_t(blockIdx.x) * 2 * f_vec;
-  for (int c = threadIdx.x; c < f_vec; c += 256) {
+                                                         uint4* __restrict__ dgu, size_t n_rows, int f_vec) {
+  const size_t row = kWide ? size_t(blockIdx.x) : size_t(blockIdx.x) * blockDim.y + threadIdx.y;
+  if (!kWide && row >= n_rows) return;
+  const int first = kWide ? threadIdx.x : blockIdx.y * blockDim.x + threadIdx.x, step = kWide ? 256 : gridDim.y * blockDim.x;
+  const uint4* gr = gu + row * 2 * f_vec;
+  const uint4* dr = dy + row * f_vec;
+  uint4* out = dgu + row * 2 * f_vec;
+  for (int c = first; c < f_vec; c += step) {
     float g[8], u[8], d[8], dg[8], du[8];
     unpack8(gr[c], g);
     unpack8(gr[f_vec + c], u);
@@ -556,18 +565,39 @@ extern "C" int dcpk_qkv_rope_pack_bwd(const float* dq, const float* dkv, const f
   return LAUNCH_OK;
 }
 
+// Grid and block of a SwiGLU pass.  A CTA per row pays when at least half of its 256 threads have work (32768 rows of
+// F = 1024, backward: 59 us, two rows per CTA 64) and the rows fill the GPU twice (148 x 8 CTAs at once).  Narrower rows share a CTA (32768 rows of F = 64, forward:
+// 25 us with a CTA per row, 10 so), few wide ones are cut into pieces of 256 vectors (64 rows of F = 14336: 14 us / 8).
+static bool swiglu_launch(long n_rows, int f_vec, dim3* grid, dim3* block) {
+  const long full = 148 * 8 * 2;
+  if (f_vec >= 128 && n_rows >= full) {
+    *grid = dim3(unsigned(n_rows));
+    *block = dim3(256);
+    return true;
+  }
+  const int tx = f_vec < 256 ? f_vec : 256, ty = 256 / tx;
+  const long gx = (n_rows + ty - 1) / ty, pieces = (f_vec + tx - 1) / tx, want = (full + gx - 1) / gx;
+  *grid = dim3(unsigned(gx), unsigned(pieces < want ? pieces : want));
+  *block = dim3(unsigned(tx), unsigned(ty));
+  return false;
+}
+
 extern "C" int dcpk_swiglu_fwd(const void* gu, void* y, long n_rows, int f, void* stream) {
-  if (n_rows <= 0) return 0;
-  if (f % 8 != 0 || n_rows > 0x7fffffffl) return -3;
-  swiglu_fwd_kernel<<<unsigned(n_rows), 256, 0, STREAM>>>(static_cast<const uint4*>(gu), static_cast<uint4*>(y), f / 8);
+  if (n_rows <= 0 || f == 0) return 0;
+  if (f < 0 || f % 8 != 0 || n_rows / (f >= 1024 ? 1 : 2) > 0x7fffffffl) return -3;   // narrower rows share a CTA
+  dim3 grid, block;
+  auto kernel = swiglu_launch(n_rows, f / 8, &grid, &block) ? swiglu_fwd_kernel<true> : swiglu_fwd_kernel<false>;
+  kernel<<<grid, block, 0, STREAM>>>(static_cast<const uint4*>(gu), static_cast<uint4*>(y), size_t(n_rows), f / 8);
   return LAUNCH_OK;
 }
 
 extern "C" int dcpk_swiglu_bwd(const void* gu, const void* dy, void* dgu, long n_rows, int f, void* stream) {
-  if (n_rows <= 0) return 0;
-  if (f % 8 != 0 || n_rows > 0x7fffffffl) return -3;
-  swiglu_bwd_kernel<<<unsigned(n_rows), 256, 0, STREAM>>>(static_cast<const uint4*>(gu), static_cast<const uint4*>(dy),
-                                                          static_cast<uint4*>(dgu), f / 8);
+  if (n_rows <= 0 || f == 0) return 0;
+  if (f < 0 || f % 8 != 0 || n_rows / (f >= 1024 ? 1 : 2) > 0x7fffffffl) return -3;   // narrower rows share a CTA
+  dim3 grid, block;
+  auto kernel = swiglu_launch(n_rows, f / 8, &grid, &block) ? swiglu_bwd_kernel<true> : swiglu_bwd_kernel<false>;
+  kernel<<<grid, block, 0, STREAM>>>(static_cast<const uint4*>(gu), static_cast<const uint4*>(dy), static_cast<uint4*>(dgu),
+                                     size_t(n_rows), f / 8);
   return LAUNCH_OK;
 }
 

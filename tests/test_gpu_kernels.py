@@ -402,6 +402,18 @@ def test_cross_entropy_dispatch(dev, rows, vocab):
         assert ((loss[lo:lo + 256] - ref).abs() < 1e-4).all()
 
 
+@pytest.mark.parametrize("n,f", [(5, 72), (33, 320), (7, 1024), (2367, 1536), (2368, 1536), (2369, 1016), (2368, 1032), (3, 14336), (1300, 4104)])
+def test_swiglu_dispatch(dev, n, f):
+    """A CTA per row, several rows per CTA and several CTAs per row, with the bounds of ``test_swiglu_row_lengths``."""
+    g = torch.Generator(device=dev).manual_seed(f)
+    gu, dy = (4 * torch.randn(n, 2 * f, generator=g, device=dev)).bfloat16(), torch.randn(n, f, generator=g, device=dev).bfloat16()
+    a, u = gu.double().chunk(2, dim=-1)
+    sg = torch.sigmoid(a)
+    want = (a * sg * u, torch.cat([dy.double() * u * (sg + a * sg * (1 - sg)), dy.double() * a * sg], -1))
+    for got, ref in zip((model_ops.swiglu_fwd_raw(gu), model_ops.swiglu_bwd_raw(gu, dy)), want):
+        assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * (1 + ref.abs())).all()
+
+
 @pytest.mark.parametrize("n", [8, 8 * 257, 8 * (148 * 8 * 256 + 5)])
 def test_scaled_gradients(dev, n):
     """The roundings are those of an fp32 product (the scalar is not rounded to bf16 first) and an accumulation of
