@@ -59,8 +59,10 @@ def rmsnorm_fwd_raw(x: torch.Tensor, w: torch.Tensor, eps: float):
 
 
 def rmsnorm_bwd_raw(x: torch.Tensor, w: torch.Tensor, rstd: torch.Tensor, dy: torch.Tensor, residual: torch.Tensor = None):
-    """(dx bf16, dw fp32) for contiguous 2-D x / dy; ``residual`` (bf16, contiguous, like dx) is added to dx; no autograd."""
-    assert residual is None or (residual.is_contiguous() and residual.shape == x.shape and residual.dtype == x.dtype)
+    """(dx bf16, dw fp32) for contiguous 2-D x / dy; ``residual`` (bf16, like dx, any layout) is added to dx; no autograd."""
+    if residual is not None:
+        assert residual.shape == x.shape and residual.dtype == x.dtype
+        residual = _aligned(residual)
     dx = torch.empty_like(x)
     dw = torch.zeros(x.shape[1], dtype=torch.float32, device=x.device)
     _lib.check(_lib.load().dcpk_rmsnorm_bwd_add(_lib.ptr(x), _lib.ptr(w), _lib.ptr(dy), _lib.ptr(rstd), _lib.ptr(dx), _lib.ptr(dw),
@@ -91,6 +93,12 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> torch.Tensor
 
 
 # --------------------------------------------------------------------------- scaled and gathered gradients
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels' 16-byte accesses take it: contiguous, on a 16-byte boundary."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def scale_rows(src: torch.Tensor, g: torch.Tensor, dst: torch.Tensor = None) -> torch.Tensor:
     """bf16(src * g) for bf16 ``src`` and a one-element ``g``; with ``dst`` (bf16, contiguous) it is added to ``dst``
     in the same pass."""
@@ -107,9 +115,9 @@ def scale_rows(src: torch.Tensor, g: torch.Tensor, dst: torch.Tensor = None) -> 
 def embedding_grad(tokens: torch.Tensor, dy: torch.Tensor, grad: torch.Tensor) -> None:
     """grad[id] += sum of dy over the tokens with that id (fp32 sums, bf16 tensors on the GPU)."""
     ids, order = torch.sort(tokens.reshape(-1).to(torch.int64))
-    dy = dy.reshape(ids.shape[0], grad.shape[1]).contiguous()
+    dy = _aligned(dy.reshape(ids.shape[0], grad.shape[1]))
     assert dy.dtype == grad.dtype == torch.bfloat16 and grad.is_contiguous() and grad.shape[1] % 8 == 0
-    assert dy.data_ptr() % 16 == 0 and grad.data_ptr() % 16 == 0
+    assert grad.data_ptr() % 16 == 0
     # sums of the runs of equal ids that go over the end of a 64-token segment
     part = torch.empty(2 * -(-ids.shape[0] // 64), grad.shape[1], dtype=torch.float32, device=dy.device)
     _lib.check(_lib.load().dcpk_embedding_grad(_lib.ptr(ids), _lib.ptr(order), _lib.ptr(dy), _lib.ptr(grad), _lib.ptr(part),

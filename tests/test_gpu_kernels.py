@@ -347,6 +347,23 @@ def test_rmsnorm_backward_with_residual(dev, rows, hidden):
         assert ((dw.double() - terms.sum(0)).abs() <= 1e-5 * (terms.abs().sum(0) + 1)).all()
 
 
+@pytest.mark.parametrize("how", ["strided", "shifted"])
+def test_gradients_of_any_layout(dev, how):
+    """The gradient that by-passes a norm and the one that reaches the embedding may be strided or start off a 16-byte
+    boundary: the same result bit for bit."""
+    change = {"strided": lambda t: torch.stack([t, t * 2], dim=-1)[..., 0],
+              "shifted": lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)}[how]
+    x, dy, res = (torch.randn(9, 1024, device=dev).bfloat16() for _ in range(3))
+    w = torch.ones(1024, device=dev).bfloat16()
+    _, rstd = model_ops.rmsnorm_fwd_raw(x, w, 1e-5)
+    assert torch.equal(model_ops.rmsnorm_bwd_raw(x, w, rstd, dy, change(res))[0], model_ops.rmsnorm_bwd_raw(x, w, rstd, dy, res)[0])
+    ids = torch.tensor([0, 3, 3, 1, 7, 7, 7, 2, 0], device=dev)
+    a, b = torch.zeros(8, 1024, device=dev).bfloat16(), torch.zeros(8, 1024, device=dev).bfloat16()
+    model_ops.embedding_grad(ids, dy, a)
+    model_ops.embedding_grad(ids, change(dy), b)
+    assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("vocab", [8, 32760, 32768, 40008])
 def test_cross_entropy_row_widths(dev, vocab):
     """Both CTA widths, fp64 oracle: the gradient is rounded to bf16 once (2^-8) and the fast exponentials are good to
