@@ -15,8 +15,8 @@
 // hidden behind it then: it hands the Q tile back 580 cycles earlier, and a Q tile that arrives late holds up all
 // that follows (full 5.02 -> 4.98 ms, causal 3.82 -> 3.77, sink + window 1.41 -> 1.38 at the size below).
 // Warps: 0-15 gradient (warp = 32 key rows x 32 queries), 16-23 drain dQ (thread = 64 channels of a query row; a
-// [32 queries x 32 channels] swizzled fp32 tile per step, added to the accumulator with one tiled TMA
-// reduce-add, or red.global.add.v4 for a peer's accumulator), 24 TMA producer, 25 UMMA issuer, 26
+// [32 queries x 32 channels] fp32 tile per step, added to the accumulator with one tiled TMA
+// reduce-add, or to a peer's with a 128-byte bulk reduce-add per row), 24 TMA producer, 25 UMMA issuer, 26
 // per-query statistics, 27 idle.  dK/dV stay in TMEM for the CTA's lifetime and are added once
 // with red.global.add.v4.f32; the CTAs of a split head group first add their shares up through distributed
 // shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
@@ -510,19 +510,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.dq_drained);
       if (!any_row) continue;
-      if (cur.dq_dev == 0) {
-        // rows past n_rows hold exact zeros (their probabilities are masked to 0): adding them is harmless
-        float* stage = sm.dq_stage[warp - 16];
+      // this GPU's accumulator takes a swizzled tile with one tiled reduce, any other one 128 bytes of a row per lane
+      // (rows past n_rows of the tile hold exact zeros, their probabilities are masked to 0: adding them is harmless)
+      float* stage = sm.dq_stage[warp - 16];
+      const int swizzle = cur.dq_dev == 0 ? lane & 7 : 0;
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the earlier tile has left the buffer
-          __syncwarp();
+      for (int b = 0; b < 2; ++b) {
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // what this lane reduced before has left the buffer
+        __syncwarp();
 #pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<uint4*>(stage + lane * 32 + ((c ^ (lane & 7)) << 2)) =
-                make_uint4(reg[32 * b + 4 * c], reg[32 * b + 4 * c + 1], reg[32 * b + 4 * c + 2], reg[32 * b + 4 * c + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
+        for (int c = 0; c < 8; ++c)
+          *reinterpret_cast<uint4*>(stage + lane * 32 + ((c ^ swizzle) << 2)) =
+              make_uint4(reg[32 * b + 4 * c], reg[32 * b + 4 * c + 1], reg[32 * b + 4 * c + 2], reg[32 * b + 4 * c + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (cur.dq_dev == 0) {
           if (lane == 0) {
             asm volatile(
                 "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
@@ -531,13 +533,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
+        } else if (quad * 32 + lane < cur.n_rows) {
+          float* dq = ptrs.dq[cur.dq_dev] + (size_t(cur.dq_row + quad * 32 + lane) * hq + cur.head) * kHeadDim + ch0 + b * 32;
+          asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], 128;"
+                       ::"l"(dq), "r"(smem_u32(stage + lane * 32)) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-      } else if (quad * 32 + lane < cur.n_rows) {
-        float* dq = ptrs.dq[cur.dq_dev] + (size_t(cur.dq_row + quad * 32 + lane) * hq + cur.head) * kHeadDim + ch0;
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          red_add_v4(dq + 4 * c, __uint_as_float(reg[4 * c]), __uint_as_float(reg[4 * c + 1]),
-                     __uint_as_float(reg[4 * c + 2]), __uint_as_float(reg[4 * c + 3]));
       }
     }
     // no staged dQ tile may still be in flight when the CTA retires (also on the abort path)

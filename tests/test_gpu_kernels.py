@@ -219,6 +219,43 @@ def test_attention_backward_split_head_groups(dev, hq, hkv, parts):
         assert (got - ref).abs().max() <= 2e-2 * ref.abs().max()
 
 
+def test_attention_backward_into_a_second_accumulator(dev):
+    """Items that name another accumulator than the first (a peer's, here a second local one) add the rows the first
+    would have got, and nothing beside them; items that want no dQ add none.  dQ is a sum of fp32 in changing order:
+    1e-5 of the largest element."""
+    n, hq, hkv = 700, 4, 2
+    g = torch.Generator().manual_seed(1)
+    new = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(dev)
+    q, kv, dout = new(n, hq, 128), new(n, 2, hkv, 128), new(n, hq, 128)
+    rng = np.zeros((n, 4), np.int32)
+    rng[:, 1] = np.arange(n) + 1
+    row = A.AttnRow(0, n, list(range(hq)), [(0, n)], rng)
+    out, lse = torch.zeros_like(q), torch.zeros(hq, n, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 1024, dev), [out], [lse], 128 ** -0.5, status)
+    delta = torch.zeros_like(lse)
+    A.attn_delta(out, dout, delta, 0, n)
+    runs = []
+    for split in (False, True):
+        tables = A.build_bwd_tables([row], 1024, hq, hkv, dev)
+        tile = tables.items[:, 0] // 128           # query tile: 1 and 4 to the second accumulator, 2 to none
+        if split:
+            tables.items[:, 4] = ((tile == 1) | (tile >= 4)).int() - (tile == 2).int()
+        dq = [torch.zeros(n, hq, 128, device=dev) for _ in range(2)]
+        dkv = [torch.zeros(n, 2, hkv, 128, device=dev) for _ in range(2)]
+        A.attn_bwd(q, dout, kv, lse, delta, tables, dq, dkv, 128 ** -0.5, status)
+        assert status.item() == 0 and dkv[1].abs().max() == 0
+        runs.append((dq, dkv[0]))
+    (want, _), want_kv = runs[0]
+    (first, second), got_kv = runs[1]
+    assert torch.equal(got_kv, want_kv)
+    tile = torch.arange(n, device=dev) // 128
+    other = (tile == 1) | (tile >= 4)
+    close = lambda a, b: (a - b).abs().max() <= 1e-5 * want.abs().max()
+    assert close(first[(tile == 0) | (tile == 3)], want[(tile == 0) | (tile == 3)]) and close(second[other], want[other])
+    assert first[other | (tile == 2)].abs().max() == 0 and second[~other].abs().max() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [8, 96, 128])
 def test_row_conversions(dev, dtype, d):
