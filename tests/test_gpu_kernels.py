@@ -219,6 +219,39 @@ def test_attention_backward_split_head_groups(dev, hq, hkv, parts):
         assert (got - ref).abs().max() <= 2e-2 * ref.abs().max()
 
 
+def test_attention_backward_split_group_carries_copy_jobs(dev):
+    """Head groups over several CTAs (clusters) in a launch whose first CTAs only copy rows and statistics from a peer's
+    region (here a local one): the copies arrive, dK and dV are those of a launch without them."""
+    from dcp_b200.planner.lowering import row_copy_jobs, stat_copy_jobs
+    n, hq, hkv = 700, 8, 2
+    g = torch.Generator().manual_seed(2)
+    new = lambda *shape: torch.randn(*shape, generator=g).bfloat16().to(dev)
+    q, kv, dout = new(n, hq, 128), new(n, 2, hkv, 128), new(n, hq, 128)
+    rng = np.zeros((n, 4), np.int32)
+    rng[:, 1] = np.arange(n) + 1
+    row = A.AttnRow(0, n, list(range(hq)), [(0, n)], rng)
+    out, lse = torch.zeros_like(q), torch.zeros(hq, n, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 1024, dev), [out], [lse], 128 ** -0.5, status)
+    delta = torch.zeros_like(lse)
+    A.attn_delta(out, dout, delta, 0, n)
+    regions = {"q": q, "kv": kv, "dout": dout, "lse": lse, "delta": delta}
+    staged = {k: torch.zeros_like(t) for k, t in regions.items()}
+    ctx = A.CopyContext(lambda name: [regions[name].data_ptr(), staged[name].data_ptr()], 1, n)
+    pulls = np.array([[0, 3, 10, 600]], np.int32)
+    jobs = np.concatenate([row_copy_jobs(pulls, 0, hq * 16), row_copy_jobs(pulls, 1, 2 * hkv * 16), stat_copy_jobs(pulls, 3, hq)])
+    tables = A.build_bwd_tables([row], 1024, hq, hkv, dev)
+    runs = []
+    for j in (None, torch.from_numpy(jobs).to(dev)):
+        dq, dkv = torch.zeros(n, hq, 128, device=dev), torch.zeros(n, 2, hkv, 128, device=dev)
+        A.attn_bwd(q, dout, kv, lse, delta, tables, [dq], [dkv], 128 ** -0.5, status, jobs=j, job_ctx=ctx)
+        runs.append(dkv)
+    assert status.item() == 0 and torch.equal(*runs)
+    for name in ("q", "kv"):
+        assert torch.equal(staged[name][10:610], regions[name][3:603]) and not staged[name][:10].any() and not staged[name][610:].any()
+    assert torch.equal(staged["lse"][:, 10:610], lse[:, 3:603]) and not staged["delta"].any() and not staged["lse"][:, 610:].any()
+
+
 def test_attention_backward_into_a_second_accumulator(dev):
     """Items that name another accumulator than the first (a peer's, here a second local one) add the rows the first
     would have got, and nothing beside them; items that want no dQ add none.  dQ is a sum of fp32 in changing order:
