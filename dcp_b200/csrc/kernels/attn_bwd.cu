@@ -30,9 +30,12 @@
 // 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
 // 13 stall cycles per issue; 0.5 of 19 now).  8 drain warps keep their part of dQ in registers, so the columns
 // are free before the shared-memory tile and the L2 have taken it (4 warps with half of it at a time: 7 % slower).
-// What bounds it now: the shared-memory pipe.  An item moves 2304 wavefronts of UMMA operands, about 1800 of
-// loads and stores (dS^T, dQ staging, statistics) and about 1000 of TMA traffic in its 4100 to 4300 cycles;
-// the tensor pipe is 55 % busy.  Without the dQ drain an item takes 15 % less.
+// What bounds it now: the shared-memory pipe.  An item moves 2304 wavefronts of UMMA operands and 1870 of loads
+// and stores (dS^T, dQ staging, statistics).  Over the whole kernel (causal, below, under ncu: 3.92 ms at 1.62
+// GHz, 1335 items per SM, so 4760 cycles per item with prologues, ends of CTAs and the last wave) the counters show
+// 49 and 40 % of that pipe and 56 % of the tensor pipe; inside the loop an item takes 4100 to 4300 cycles, which the
+// 4174 wavefronts fill.  TMA traffic (128 KB per item: Q, dO, dQ) is in neither counter.  Without the dQ drain an item takes 15 %
+// less.
 // Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104
 // TFLOP/s), causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
 //

@@ -485,7 +485,8 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
              status: torch.Tensor, jobs: Optional[torch.Tensor] = None, job_ctx: Optional[CopyContext] = None):
     """Run the backward kernel; dq_dsts/dkv_dsts are fp32 accumulators (zeroed by the caller),
     [rows, hq, 128] and [rows, 2, hkv, 128]; lse/delta are fp32 [hq, rows].  ``jobs`` / ``job_ctx``: copy
-    jobs two spare warps per CTA perform meanwhile (the next stage's operands, see attn_fwd)."""
+    jobs (the next stage's operands, see attn_fwd) that about sixteen CTAs of their own, the first of the grid,
+    perform meanwhile."""
     lib = _lib.load()
     hq, hkv = q_arena.shape[1], kv_arena.shape[2]
     assert q_arena.shape == do_arena.shape and lse.shape == delta.shape
