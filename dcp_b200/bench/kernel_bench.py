@@ -86,7 +86,7 @@ def bench_attention(kind, args):
     if kind == "attn_fwd":
         ms = time_fn(fwd, args.iters, 3, flush)
         flops = ft.flops
-        if args.timeline:
+        if args.timeline and args.variant != 2:    # only the one-tile kernel has counters
             from ..ops import _lib
             tl = torch.zeros(16, dtype=torch.int64, device=dev)
             _lib.load().dcpk_attn_fwd_set_timeline(_lib.ptr(tl))
@@ -278,7 +278,7 @@ def main():
     ap.add_argument("--mask", default="causal", choices=["full", "causal", "lambda"])
     ap.add_argument("--variant", type=int, default=2, help="forward kernel: 2 = two query tiles per CTA (default), 0 / 1 = one tile per CTA with P in TMEM / shared memory")
     ap.add_argument("--iters", type=int, default=10)
-    ap.add_argument("--timeline", action="store_true", help="print per-phase cycle counts of one backward CTA")
+    ap.add_argument("--timeline", action="store_true", help="print per-phase cycle counts of one CTA (attn_bwd; attn_fwd with --variant 0 or 1)")
     ap.add_argument("--skip-dq", action="store_true", help="backward without the dQ drain (upper bound probe)")
     args = ap.parse_args()
     if args.kind == "nvlink":
