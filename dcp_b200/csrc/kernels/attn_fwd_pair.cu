@@ -1,39 +1,58 @@
-// Blockwise range-masked attention forward for sm_100a, two query tiles per CTA.
+// Blockwise range-masked attention forward for sm_100a: pairs of CTAs, 256 queries of one head per pair, persistent.
 //
-// One CTA = up to 256 queries (two 128-row tiles A and B of one Q block) of one head.  Warps:
-//   0-3  softmax of tile A, 4-7 softmax of tile B (one thread per query row),
-//   8    TMA producer (Q of both tiles once, 2-deep rings of K and V tiles),
-//   9    UMMA issuer,
-//   10-11 fetch the next plan stage's remote operands (copy jobs: peer loads over NVLink into this
-//        GPU's staging rows, see copy_jobs.cuh) while the tiles are computed; they also donate
-//        registers (setmaxnreg).
-// K and V tiles are loaded once and used by both query tiles, and the two softmax warpgroups
-// alternate on the tensor core: per KV tile j the issuer emits
-//   PV(A, j-1), QK(A, j), PV(B, j-1), QK(B, j)
-// so one warpgroup's exp2 / TMEM round trips run while the other's UMMAs execute.  A query tile
-// that cannot see a KV tile (from the per-tile union of its rows' ranges) skips it: no UMMA is
-// issued for it and its softmax warpgroup does not wait.
-// P of the first 64 keys is handed over while the softmax works on the other 64, so half of PV runs under it.
-// The issuer branches on elect.sync (with a test on the lane number a UMMA took about 90 cycles to issue) and
-// waits for the K and V tiles of a step before it waits for probabilities.
-// What bounds it: the chain of one query tile (scores -> TMEM load and maximum 430, exponentials 1250, hand-over,
-// second half of PV and the next QK 1030 cycles; the other tile's exponentials share the special-function pipe) next
-// to 2180 cycles of tensor time per pair of query tiles.  Exponentials on the FMA pipe (a degree-5 polynomial for
-// 1/8, 1/4 or 3/8 of them) were slower: 1266 / 1184 / 1168 against 1300 TFLOP/s; so was one issuer per query tile (1039).
-// Measured (8192 queries x 16384 keys, 32 / 8 heads, before -> after elected issue, early hand-over, a rescale
-// factor that is exactly 1 where the maximum stays and mask bits): full 2.15 -> 1.69 ms (1299 TFLOP/s), causal
-// 1.65 -> 1.28 ms (1287), sink + window 0.682 -> 0.518 ms (1078).
-// TMEM (512 columns): S_A [0,128) S_B [128,256) O_A [256,384) O_B [384,512); P_X overwrites the
-// first 64 columns of S_X as packed bf16 pairs and is the TMEM A operand of O_X += P_X V.
-// S_X = Q_X K^T takes both operands from shared memory (no TMEM columns are left to park Q in).
+// A pair of CTAs (a cluster of two, cta_group::2) takes one 256-row tile after another; the even CTA has query rows
+// 0-127 (tile A), the odd one 128-255 (tile B).  Warps of a CTA:
+//   0-3, 4-7  softmax of every second KV tile (one thread per query row), each half of the channels in the epilogue,
+//   8         TMA producer: this CTA's Q rows and its halves of the K and V tiles,
+//   9         UMMA issuer (even CTA only: a product covers both CTAs' rows),
+//   10-11     fetch the next plan stage's remote operands (copy jobs: peer loads over NVLink into this
+//             GPU's staging rows, see copy_jobs.cuh) while the tiles are computed.
+// All four non-softmax warps donate registers (setmaxnreg).
+//   S(j) = Q K(j)^T   M = 256, each CTA holds 64 of the 128 keys             -> TMEM
+//   O   += P(j) V(j)  P as packed bf16 in the TMEM columns S(j) came from, each CTA holds 64 of the channels
+// TMEM (512 columns): three score buffers [0,384), O [384,512).  Per KV tile j the issuer emits PV(j), QK(j+3), also
+// across the end of a tile: the next tile's Q has a buffer of its own and its products wait only until the epilogue has
+// taken O to registers.
+//
+// Why pairs: with one query tile per CTA there is room for three score buffers, so a softmax warp finds its next scores
+// ready.  (Two query tiles per CTA, the earlier form, leave one buffer each: scores, exponentials and both products of a
+// tile were one serial chain of 3200 cycles per 2180 of tensor time.)  One query tile per CTA alone would read every K
+// and V tile twice as often from L2; in a pair each CTA reads half of it, and the tensor core reads half as much of
+// B from shared memory.
+//
+// Why no running maximum: out = O / l and lse = m + ln l are exact for any reference m, and bf16 has the exponent range of
+// fp32, so m has to be near the row's largest score only within what fp32 holds.  A row keeps the maximum of the first
+// tile it sees anything of; while some row of a warp has none, the two warps that share the rows hand the references on
+// from KV tile to KV tile.  Afterwards no maximum is taken and nothing is handed on.  Where a row's sum exceeds 2^64 (a
+// score 44 above the reference) or is not a number, the pair goes through the tile again when it is done with all tiles,
+// with the reference following the maximum to within 2^8 and O rescaled in TMEM where it moves.
+//
+// P of the first 64 keys is handed over while the softmax works on the other 64, so half of PV runs under it.  The next
+// scores' barrier is asked before the last probabilities are stored: a look at shared memory queues behind the
+// exponentials of the other warp, 200 cycles and more.  Arrivals on the other CTA's barriers carry no release at cluster
+// scope (a fence that waits for everything the warp has stored; 1.6 times slower): what they announce is in TMEM.
+//
+// What bounds it: the issuing thread and the softmax warps that share its scheduler.  Where both are in time a KV tile takes
+// 1250 cycles per CTA; the exponentials need 1024 of them and the products 1024.  Every look at a barrier costs the issuer
+// 200 cycles, so it asks for its three at once, and K(j+3) and V(j), which one step consumes, share a barrier.  Between
+// two tiles of a pair: the last product, the sums of the two warpgroups, O out of TMEM, about 4000 cycles; as a launch
+// with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
+// Measured against two query tiles per CTA (32 / 8 heads, queries x keys; one box): full 8192 x 16384 1.71 -> 1.57 ms
+// (1283 -> 1404 TFLOP/s), causal 1.29 -> 1.17 ms (1397), sink + window 0.568 -> 0.505 ms, causal 4096 x 4096 0.163 ->
+// 0.153 ms; in long runs under the power cap full 2.01 -> 1.74 ms.  Slower where the tiles are many and short: causal
+// 2048 x 2048 0.059 -> 0.061 ms.  Tried and left: a pair per tile instead of persistent pairs (4096 x 4096 0.159 ms, 16384
+// tokens in sequences of 8192 6 % slower); the result written after the next tile's first exponentials (the longer loop
+// costs more than it hides: 1.57 -> 1.66 ms); the maximum taken beside the exponentials (1.75 ms).
 //
 // The partial (out, lse) of a tile is stored straight to its destination arena, which may be a
-// peer GPU's memory (plain st.global over the NVLink mapping).
+// peer GPU's memory (plain st.global over the NVLink mapping), through shared memory in 64-byte pieces of a row.
 //
 // Reference behaviour covered: the varlen forward with block tables and per-query KV ranges that
 // dcp/runtime/flash_attention/executor.py:884-913 calls.
 #include <limits.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "attn_common.cuh"
 #include "copy_jobs.cuh"
@@ -43,19 +62,46 @@
 namespace dcpk {
 
 static constexpr int kPairThreads = 384;  // 8 softmax warps + producer + UMMA issuer + 2 fetch warps (all four donate registers)
-static constexpr int kHalfBytesP = 128 * 64 * 2;
-static constexpr int kTileBytesP = 2 * kHalfBytesP;
+static constexpr int kPairs = 148 / 2;    // one CTA per SM
+static constexpr int kSlots = 4;          // slot i holds this CTA's halves of K(i) and V(i-3): what one step of the issuer consumes
+static constexpr int kSBufs = 3;
+static constexpr int kQHalf = 128 * 64 * 2;      // [128 queries x 64 channels]
+static constexpr int kKHalf = 64 * 64 * 2;       // [64 keys x 64 channels]
+static constexpr int kKvBytes = 64 * 128 * 2;    // a CTA's half of a K or V tile
+static constexpr int kRedoWords = 16;
+static constexpr int kInfos = 4;
+static constexpr float kGap = 8.f;            // exponent (base 2) by which a score may exceed a reference that can still move
+static constexpr float kMaxSum = 1.8447e19f;  // 2^64: a row sum above it sends the tile through the second pass
 
-struct __align__(1024) PairSmem {
-  uint8_t q[2][kTileBytesP];
-  uint8_t k[2][kTileBytesP];
-  uint8_t v[2][kTileBytesP];
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2][2], o_done[2];
-  uint32_t tmem_base;
-  int abort_word;
+// What the softmax warps of a CTA need of a tile, put into shared memory by the TMA producer, which is some KV tiles
+// ahead of them: from the tables it would take three dependent trips to memory between two tiles.
+struct __align__(16) TileInfo {
+  int4 mask[kTileM];        // ranges of this CTA's rows
+  int4 first[2];            // first KV tiles
+  __nv_bfloat16* out;       // where the first row goes
+  float* lse;
+  int n_rows, n_kv, kv_off, round;  // rows of this CTA; n_kv < 0: there are no more tiles
 };
 
-// One 128-key tile of the CTA's KV walk, prepared by the host (build_fwd_tables with tile_m = 256).
+struct __align__(1024) PairSmem {
+  uint8_t q[2][2 * kQHalf];
+  uint8_t k[kSlots][kKvBytes];      // 64 of the 128 keys, all channels
+  uint8_t v[kSlots][kKvBytes];      // all 128 keys, 64 of the channels
+  uint8_t o_stage[8][32 * 64];      // per softmax warp: 32 rows x 32 channels on their way out
+  TileInfo info[kInfos];
+  float m[kTileM];                  // reference of a row
+  float l[2][2][kTileM];            // its sums over the KV tiles of either warpgroup, of two tiles in turn
+  uint32_t redo[kRedoWords];        // rounds that go through the second pass
+  // of the even CTA (bytes and arrivals of both CTAs): q_full, kv_full, p_ready, o_empty; the others are signalled in
+  // both
+  uint64_t q_full[2], q_empty[2], kv_full[kSlots], kv_empty[kSlots], s_full[kSBufs], p_ready[kSBufs][2], o_empty, acc_full,
+      m_ready[4], l_ready[4], info_full[kInfos], info_empty[kInfos];
+  uint32_t tmem_base;
+  int abort_word;
+  int any_redo;
+};
+
+// One 128-key tile of the pair's KV walk, prepared by the host (build_fwd_tables with tile_m = 256).
 struct KvSub {
   int row;       // first arena row of the 128 keys
   int pos0;      // position of the first key in the Q block's concatenated KV
@@ -63,347 +109,511 @@ struct KvSub {
   int flags;     // bit 0 / 1: query tile A / B sees at least one key; bit 2 / 3: A / B sees every pair
 };
 
-// walks the list with the next entry already in registers, so a step never waits on global memory
-struct SubIter {
-  const int4* p;
-  int n, i;
-  int4 cur, ahead;
-  __device__ __forceinline__ void init(const int4* base, int count) {
-    p = base; n = count; i = -1;
-    ahead = count > 0 ? base[0] : make_int4(0, 0, 0, 0);
-  }
-  __device__ __forceinline__ bool next() {
-    if (++i >= n) return false;
-    cur = ahead;
-    if (i + 1 < n) ahead = p[i + 1];
-    return true;
-  }
-};
+template <typename F>
+__device__ __forceinline__ void for_each_barrier(PairSmem& sm, F f) {   // f(barrier, arrivals)
+  for (int i = 0; i < 2; ++i) { f(&sm.q_full[i], 1); f(&sm.q_empty[i], 1); }
+  for (int i = 0; i < kSlots; ++i) { f(&sm.kv_full[i], 1); f(&sm.kv_empty[i], 1); }
+  for (int i = 0; i < kSBufs; ++i) { f(&sm.s_full[i], 1); f(&sm.p_ready[i][0], 8); f(&sm.p_ready[i][1], 8); }   // four warps of either CTA
+  f(&sm.o_empty, 16);   // eight warps of either CTA
+  f(&sm.acc_full, 1);
+  for (int i = 0; i < 4; ++i) { f(&sm.m_ready[i], 1); f(&sm.l_ready[i], 2); }
+  for (int i = 0; i < kInfos; ++i) { f(&sm.info_full[i], 1); f(&sm.info_empty[i], 8); }
+}
 
-__global__ void __launch_bounds__(kPairThreads, 1)
-attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
-                     const AttnTile* __restrict__ tiles, const int4* __restrict__ kv_subs,
-                     const int4* __restrict__ masks, PeerPtrs ptrs, int hq, int hkv, int lse_stride_a,
-                     int lse_stride_b, int n_dst_a, int n_dst, int q_rows, int block_size, int n_mask_rows,
+// P = exp2(S * c - m) of 64 keys of a row, cut to bf16, to TMEM; `ps2` collects the row sum.  Packed fp32: one
+// instruction scales two scores, one adds two probabilities.  Every probability carries the factor kTruncScale (folded
+// into the exponent), so cutting it to bf16 is unbiased; the row sum carries the same factor, which cancels in O / l
+// and is taken out of the LSE in the epilogue.
+__device__ __forceinline__ void softmax_half(const uint32_t* s, uint64_t sl2_2, uint64_t negm_2, uint64_t* ps2, uint32_t p_addr) {
+  uint32_t preg[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(s[2 * c]), __uint_as_float(s[2 * c + 1])), sl2_2, negm_2);
+    float x0, x1;
+    unpack_f32x2(x2, x0, x1);
+    const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+    ps2[c & 3] = add_f32x2(ps2[c & 3], pack_f32x2(p0, p1));
+    preg[c] = pack_bf16x2_trunc(p0, p1);
+  }
+  tmem_st32(p_addr, preg);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const AttnTile* __restrict__ tiles, int n_tiles,
+                     const int4* __restrict__ kv_subs, const int4* __restrict__ masks, PeerPtrs ptrs, int hq, int hkv,
+                     int lse_stride_a, int lse_stride_b, int n_dst_a, int n_dst, int q_rows, int n_mask_rows,
                      int n_kv_subs, float scale, const CopyJob* __restrict__ jobs, int n_jobs,
                      const __grid_constant__ CopyCtx copy_ctx, int* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   PairSmem& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const AttnTile tile = tiles[blockIdx.x];
-  const int kv_head = tile.head / (hq / hkv);
-  {
-    // table sanity before anything is allocated: a tile that would store outside its destination
-    // arena, or read a head / row / table entry that does not exist, is reported and skipped
-    const int dst_rows = tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b;
-    const bool bad = tile.out_dev < 0 || tile.out_dev >= n_dst || tile.out_row < 0 || tile.n_rows < 0 ||
-                     tile.n_rows > 2 * kTileM || tile.out_row + tile.n_rows > dst_rows || tile.head < 0 ||
-                     tile.head >= hq || tile.q_row < 0 || tile.q_row + tile.n_rows > q_rows || tile.n_kv < 0 ||
-                     tile.mask_row < 0 || tile.mask_row + tile.n_rows > n_mask_rows || tile.kv_off < 0 ||
-                     tile.kv_off + tile.n_kv > n_kv_subs;
-    if (bad) {
-      if (threadIdx.x == 0) atomicExch(status, kStatusBadArgs);
-      return;
-    }
-  }
+  const int X = blockIdx.x & 1;   // query tile of this CTA == its rank in the cluster
   if (threadIdx.x == 256) {
     tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_kv);
-    mbar_init(&sm.q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&sm.k_full[i], 1);  mbar_init(&sm.k_empty[i], 1);
-      mbar_init(&sm.v_full[i], 1);  mbar_init(&sm.v_empty[i], 1);
-      mbar_init(&sm.s_full[i], 1);  mbar_init(&sm.p_ready[i][0], 4);  mbar_init(&sm.p_ready[i][1], 4);
-      mbar_init(&sm.o_done[i], 1);
-    }
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+    for_each_barrier(sm, [](uint64_t* bar, int count) { mbar_init(bar, count); });
     sm.abort_word = 0;
+    sm.any_redo = 0;
+    for (int i = 0; i < kRedoWords; ++i) sm.redo[i] = 0;
     mbar_fence_init();
   }
-  if (warp == 9) {
-    tmem_alloc(&sm.tmem_base, 512);
-    tmem_relinquish();
-  }
-  // this thread's query row (softmax warps): X = which tile, r = row inside it
-  const int X = warp >> 2, r = threadIdx.x & 127;
-  int s0 = 0, e0 = 0, s1 = 0, e1 = 0;
-  if (warp < 8) {
-    const bool valid = X * kTileM + r < tile.n_rows;
-    if (valid) {
-      int4 m = masks[tile.mask_row + X * kTileM + r];
-      s0 = m.x; e0 = max(m.y, m.x); s1 = m.z; e1 = max(m.w, m.z);
-    }
-  }
+  if (warp == 9) tmem_alloc_pair(&sm.tmem_base, 512);
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();   // barriers and TMEM of both CTAs are there
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   volatile int* abort_word = &sm.abort_word;
-  SubIter it;
-  it.init(kv_subs + tile.kv_off, tile.n_kv);
+  const int4 none = make_int4(0, 0, 0, 0);
+
+  // The pairs of CTAs take the tiles, which are ordered by length, in rounds and every second round backwards.
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  auto index_of = [&](int round) { return round * n_pairs + ((round & 1) ? n_pairs - 1 - pair : pair); };
+  // the first tile from `round` on that has work for the pass and at least `min_kv` KV tiles; false: there is none
+  auto find_tile = [&](int pass, int& round, AttnTile& t, int min_kv) -> bool {
+    for (;; ++round) {
+      const int i = index_of(round);
+      if (i >= n_tiles) return false;
+      if (pass > 0 && !((sm.redo[(round >> 5) & (kRedoWords - 1)] >> (round & 31)) & 1u)) continue;
+      t = tiles[i];
+      // table sanity: a tile that would store outside its destination arena, or read a head / row / table entry that
+      // does not exist, is reported and skipped (by all warps of both CTAs)
+      const int dst_rows = t.out_dev < n_dst_a ? lse_stride_a : lse_stride_b;
+      const bool bad = t.out_dev < 0 || t.out_dev >= n_dst || t.out_row < 0 || t.n_rows < 0 ||
+                       t.n_rows > 2 * kTileM || t.out_row + t.n_rows > dst_rows || t.head < 0 ||
+                       t.head >= hq || t.q_row < 0 || t.q_row + t.n_rows > q_rows || t.n_kv < 0 ||
+                       t.mask_row < 0 || t.mask_row + t.n_rows > n_mask_rows || t.kv_off < 0 ||
+                       t.kv_off + t.n_kv > n_kv_subs;
+      if (bad) atomicExch(status, kStatusBadArgs);
+      if (!bad && t.n_kv >= min_kv) return true;
+    }
+  };
+  // End of a pass over the tiles, by all threads of both CTAs; true: a second pass follows.
+  auto next_pass = [&](int pass) -> bool {
+    // a CTA that gave up tells the other, which waits for it
+    if (threadIdx.x == 0 && sm.abort_word) st_cluster_u32(smem_u32(&sm.abort_word), X ^ 1, 1u);
+    tc_fence_before();
+    cluster_sync();
+    tc_fence_after();
+    if (pass > 0 || !sm.any_redo) return false;
+    if (threadIdx.x == 256) {
+      for_each_barrier(sm, [](uint64_t* bar, int count) { mbar_inval(bar); mbar_init(bar, count); });
+      mbar_fence_init();
+    }
+    cluster_sync();
+    return true;
+  };
 
   // register rebalancing between warpgroups (setmaxnreg inside each role's branch): the four
   // non-softmax warps give registers up, the softmax warps take them
-  // (256 x 208 + 128 x 72 = 62464 of the 384 x 168 = 64512 the block is launched with)
+  // (256 x 216 + 128 x 72 = 64512 = 384 x 168, what the block is launched with)
   if (warp >= 8) {
    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
    if (warp == 8) {
-    // ------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------ TMA producer: this CTA's rows and halves
+   for (int pass = 0;; ++pass) {
     if (lane == 0) {
-      mbar_expect_tx(&sm.q_full, 2 * kTileBytesP);
-      for (int x = 0; x < 2; ++x) {
-        tma_load_3d(sm.q[x], &tm_q, &sm.q_full, 0, tile.head, tile.q_row + x * kTileM);
-        tma_load_3d(sm.q[x] + kHalfBytesP, &tm_q, &sm.q_full, 64, tile.head, tile.q_row + x * kTileM);
-      }
-      int j = 0;
+      const uint32_t q_bar = cluster_addr(smem_u32(&sm.q_full[0]), 0), kv_bar = cluster_addr(smem_u32(&sm.kv_full[0]), 0);
       bool ok = true;
-      int k_pending[2] = {-1, -1}, v_pending[2] = {-1, -1};
-      while (ok && it.next()) {
-        const int st = j & 1, u = j >> 1;
-        ok = mbar_wait(&sm.k_empty[st], (u & 1) ^ 1, abort_word);
+      int qi = 0, qph = 1, slot = 0, ph = 1, info = 0, iph = 1, used = 0;   // used: slots and, above them, Q buffers
+      // V is loaded three KV tiles after K: where the last three are (oldest in the third)
+      int row1 = 0, row2 = 0, row3 = 0, head1 = 0, head2 = 0, head3 = 0, behind = 0;
+      auto load_slot = [&](bool with_k, bool with_v, int row, int kv_head) -> bool {
+        if (!mbar_wait(&sm.kv_empty[slot], ph, abort_word)) return false;
+        used |= 1 << slot;
+        if (X == 0) mbar_expect_tx(&sm.kv_full[slot], 2 * kKvBytes * (with_k + with_v));
+        if (with_v) tma_load_3d_pair(sm.v[slot], &tm_v, kv_bar + 8 * slot, 64 * X, hkv + head3, row3);
+        if (with_k) {
+          tma_load_3d_pair(sm.k[slot], &tm_k, kv_bar + 8 * slot, 0, kv_head, row + 64 * X);
+          tma_load_3d_pair(sm.k[slot] + kKHalf, &tm_k, kv_bar + 8 * slot, 64, kv_head, row + 64 * X);
+        }
+        if (++slot == kSlots) { slot = 0; ph ^= 1; }
+        return true;
+      };
+      AttnTile tile;
+      for (int round = 0; ok; ++round) {
+        const bool more = find_tile(pass, round, tile, 0);
+        ok = mbar_wait(&sm.info_empty[info], iph, abort_word);
         if (!ok) break;
-        mbar_expect_tx(&sm.k_full[st], kTileBytesP);
-        tma_load_3d(sm.k[st], &tm_kv, &sm.k_full[st], 0, kv_head, it.cur.x);
-        tma_load_3d(sm.k[st] + kHalfBytesP, &tm_kv, &sm.k_full[st], 64, kv_head, it.cur.x);
-        k_pending[st] = u & 1;
-        ok = mbar_wait(&sm.v_empty[st], (u & 1) ^ 1, abort_word);
+        TileInfo& ti = sm.info[info];
+        if (!more) {
+          ti.n_kv = -1;
+          mbar_arrive(&sm.info_full[info]);
+          break;
+        }
+        const int4* subs = kv_subs + tile.kv_off;
+        const int kv_head = tile.head / (hq / hkv), n = tile.n_kv;
+        const int4 sub0 = n > 0 ? subs[0] : none;
+        ti.first[0] = sub0;
+        if (n > 1) ti.first[1] = subs[1];
+        ti.n_kv = n;
+        ti.kv_off = tile.kv_off;
+        ti.round = round;
+        ti.n_rows = tile.n_rows - X * kTileM;
+        ti.out = reinterpret_cast<__nv_bfloat16*>(ptrs.out[tile.out_dev]) + (size_t(tile.out_row + X * kTileM) * hq + tile.head) * kHeadDim;
+        ti.lse = ptrs.lse[tile.out_dev] + size_t(tile.head) * (tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b) + tile.out_row + X * kTileM;
+        const int mask_bytes = 16 * min(max(tile.n_rows - X * kTileM, 0), kTileM);
+        mbar_expect_tx(&sm.info_full[info], mask_bytes);
+        if (mask_bytes > 0) bulk_load(ti.mask, masks + tile.mask_row + X * kTileM, mask_bytes, &sm.info_full[info]);
+        if (++info == kInfos) { info = 0; iph ^= 1; }
+        if (n == 0) continue;
+        int ahead = sub0.x;
+        ok = mbar_wait(&sm.q_empty[qi], qph, abort_word);
         if (!ok) break;
-        mbar_expect_tx(&sm.v_full[st], kTileBytesP);
-        tma_load_3d(sm.v[st], &tm_kv, &sm.v_full[st], 0, hkv + kv_head, it.cur.x);
-        tma_load_3d(sm.v[st] + kHalfBytesP, &tm_kv, &sm.v_full[st], 64, hkv + kv_head, it.cur.x);
-        v_pending[st] = u & 1;
-        ++j;
-      }
-      if (!ok) {
-        // give copies already in flight a bounded chance to land before the CTA retires
-        for (int st = 0; st < 2; ++st) {
-          if (k_pending[st] >= 0)
-            for (int spin = 0; spin < 200000 && !mbar_try_wait(&sm.k_full[st], k_pending[st]); ++spin) {}
-          if (v_pending[st] >= 0)
-            for (int spin = 0; spin < 200000 && !mbar_try_wait(&sm.v_full[st], v_pending[st]); ++spin) {}
+        used |= 1 << (kSlots + qi);
+        if (X == 0) mbar_expect_tx(&sm.q_full[qi], 4 * kQHalf);
+        tma_load_3d_pair(sm.q[qi], &tm_q, q_bar + 8 * qi, 0, tile.head, tile.q_row + X * kTileM);
+        tma_load_3d_pair(sm.q[qi] + kQHalf, &tm_q, q_bar + 8 * qi, 64, tile.head, tile.q_row + X * kTileM);
+        if (++qi == 2) { qi = 0; qph ^= 1; }
+        for (int j = 0; j < n && ok; ++j) {
+          const int row = ahead;
+          if (j + 1 < n) ahead = subs[j + 1].x;
+          ok = load_slot(true, behind == 3, row, kv_head);
+          behind = min(behind + 1, 3);
+          row3 = row2; row2 = row1; row1 = row;
+          head3 = head2; head2 = head1; head1 = kv_head;
         }
       }
+      // the last three V: slots 3, 4 and 5 at the earliest
+      if (behind > 0 && behind < 3) slot = 3;
+      for (; ok && behind > 0; --behind) {
+        if (behind < 3) { row3 = behind == 2 ? row2 : row1; head3 = behind == 2 ? head2 : head1; }
+        ok = load_slot(false, true, 0, 0);
+      }
+      // arrivals from the even CTA's issuer have all come in before this CTA may retire
+      for (int i = 0; ok && i < kSlots; ++i) {
+        if ((used >> slot) & 1) ok = mbar_wait(&sm.kv_empty[slot], ph, abort_word);
+        if (++slot == kSlots) { slot = 0; ph ^= 1; }
+      }
+      for (int i = 0; ok && i < 2; ++i) {
+        if ((used >> (kSlots + qi)) & 1) ok = mbar_wait(&sm.q_empty[qi], qph, abort_word);
+        if (++qi == 2) { qi = 0; qph ^= 1; }
+      }
+      // copies already in flight get a millisecond to land before the CTAs retire
+      if (!ok)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
+    __syncwarp();
+    if (!next_pass(pass)) break;
+   }
    } else if (warp == 9) {
-    // ------------------------------------------------------------ UMMA issuer
-    constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, 0, 0);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(128, 128, 0, 1);
-    const uint64_t q_desc = make_sdesc_sw128(smem_u32(sm.q[0]), 16, 1024), k_desc = make_sdesc_sw128(smem_u32(sm.k[0]), 16, 1024);
-    const uint64_t v_desc = make_sdesc_sw128(smem_u32(sm.v[0]), kHalfBytesP, 1024);
-    constexpr uint64_t kTileStep = kTileBytesP >> 4, kHalfStep = kHalfBytesP >> 4;   // in a descriptor's 16-byte units
-    bool ok = mbar_wait(&sm.q_full, 0, abort_word);
-    int j = 0;
-    int cnt[2] = {0, 0};                 // KV tiles issued so far per query tile
-    bool need_prev[2] = {false, false};  // did query tile X take part in the previous KV tile
-    // O_X += P_X V: P from TMEM (TS), V of ring stage `st` is the MN-major B operand; `i` = index
-    // of this KV tile among the ones query tile X takes part in
-    auto issue_pv = [&](int x, int i, int st) -> bool {
+    // ------------------------------------------------------------ UMMA issuer (even CTA), for both CTAs
+   for (int pass = 0;; ++pass) {
+    if (X == 0 && elect_one()) {   // one thread from here on
+      constexpr uint32_t idesc_qk = make_idesc_bf16(256, 128, 0, 0);
+      constexpr uint32_t idesc_pv = make_idesc_bf16(256, 128, 0, 1);
+      // descriptors differ in the address field of the low word only
+      const uint64_t some = make_sdesc_sw128(0, 16, 1024);
+      const uint32_t hi = uint32_t(some >> 32);
+      const uint32_t q_lo = uint32_t(some) + (smem_u32(sm.q[0]) >> 4), k_lo = uint32_t(some) + (smem_u32(sm.k[0]) >> 4),
+                     v_lo = uint32_t(some) + (smem_u32(sm.v[0]) >> 4);
+      auto desc = [&](uint32_t lo) { return (uint64_t(hi) << 32) | lo; };
+      constexpr uint32_t kKvStep = kKvBytes >> 4, kQStep = 2 * kQHalf >> 4;   // in a descriptor's 16-byte units
+      bool ok = true;
+      // two walks over the KV tiles of all this pair's tiles: scores three ahead of products
+      AttnTile t;
+      int q_round = 0, q_left = 0, qi = 0, qph = 0;
+      // the next KV tile's scores can be issued: its Q is there
+      auto next_q = [&]() -> bool {
+        if (q_left == 0) {
+          q_left = -1;
+          if (find_tile(pass, q_round, t, 1)) {
+            ++q_round;
+            q_left = t.n_kv;
+            ok = mbar_wait(&sm.q_full[qi], qph, abort_word);
+          }
+        }
+        return ok && q_left > 0;
+      };
+      auto issue_qk = [&](int slot, int b) {
+        const uint32_t q0 = q_lo + qi * kQStep, k0 = k_lo + slot * kKvStep, d = tmem + b * 128;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {   // the first 64 keys while the softmax warps still work on the others
-        if (!mbar_wait(&sm.p_ready[x][h], i & 1, abort_word)) return false;
+        for (int k = 0; k < 8; ++k)
+          umma_ss_pair(d, desc(q0 + (k >> 2) * (kQHalf >> 4) + (k & 3) * 2), desc(k0 + (k >> 2) * (kKHalf >> 4) + (k & 3) * 2),
+                       idesc_qk, k > 0 ? 1u : 0u);
+        umma_commit_pair(&sm.s_full[b]);
+        if (--q_left == 0) {
+          umma_commit_pair(&sm.q_empty[qi]);
+          if (++qi == 2) { qi = 0; qph ^= 1; }
+        }
+      };
+      for (int i = 0; i < kSBufs && next_q(); ++i) {
+        ok = mbar_wait(&sm.kv_full[i], 0, abort_word);
+        if (!ok) break;
         tc_fence_after();
-        if (elect_one()) {
+        issue_qk(i, i);
+        umma_commit_pair(&sm.kv_empty[i]);
+      }
+      int slot = kSBufs, ph = 0, b = 0, bph = 0, n_tiles_done = 0;
+      for (int round = 0; ok && find_tile(pass, round, t, 1); ++round) {
+        const int n = t.n_kv;
+        const int4* subs = kv_subs + t.kv_off;
+        int flags = subs[0].w;
+        for (int j = 0; j < n && ok; ++j) {
+          // the three barriers are asked at once: an answer takes 200 cycles and more
+          const bool kv_there = mbar_test_wait(&sm.kv_full[slot], ph), p0_there = mbar_test_wait(&sm.p_ready[b][0], bph),
+                     p1_there = mbar_test_wait(&sm.p_ready[b][1], bph);
+          const uint32_t hold_a = (flags & 1) - 1u, hold_b = ((flags >> 1) & 1) - 1u;   // all ones: the query tile sees none of the keys
+          if (j + 1 < n) flags = subs[j + 1].w;
+          if (!kv_there) ok = mbar_wait(&sm.kv_full[slot], ph, abort_word);
+          if (ok && j == 0 && n_tiles_done > 0) ok = mbar_wait(&sm.o_empty, (n_tiles_done - 1) & 1, abort_word);   // the last result is in registers
+          const uint32_t v0 = v_lo + slot * kKvStep, a = tmem + b * 128;
 #pragma unroll
-          for (int k = 4 * h; k < 4 * h + 4; ++k)
-            umma_ts(tmem + 256 + x * 128, tmem + x * 128 + k * 8, v_desc + st * kTileStep + k * 128, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
-          if (h == 1) umma_commit(&sm.o_done[x]);
+          for (int h = 0; h < 2 && ok; ++h) {   // O += P V: the first 64 keys while the softmax warps still work on the others
+            if (!(h ? p1_there : p0_there)) ok = mbar_wait(&sm.p_ready[b][h], bph, abort_word);
+            if (!ok) break;
+            tc_fence_after();
+            if ((hold_a | hold_b) == 0) {
+#pragma unroll
+              for (int k = 4 * h; k < 4 * h + 4; ++k)
+                umma_ts_pair(tmem + kSBufs * 128, a + k * 8, desc(v0 + k * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+            } else {
+#pragma unroll 1
+              for (int k = 4 * h; k < 4 * h + 4; ++k)
+                umma_ts_pair_hold(tmem + kSBufs * 128, a + k * 8, desc(v0 + k * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u, hold_a, hold_b);
+            }
+          }
+          if (!ok) break;
+          if (j + 1 == n) umma_commit_pair(&sm.acc_full);
+          // S(j+3) goes where P(j) was: behind the product that reads it
+          if (next_q()) issue_qk(slot, b);
+          umma_commit_pair(&sm.kv_empty[slot]);
+          if (++slot == kSlots) { slot = 0; ph ^= 1; }
+          if (++b == kSBufs) { b = 0; bph ^= 1; }
         }
-        __syncwarp();
+        n_tiles_done += ok;
       }
-      return true;
-    };
-    // S_X = Q_X K^T, both operands from shared memory
-    auto issue_qk = [&](int x, int st) {
-      if (elect_one()) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint64_t off = (k >> 2) * kHalfStep + (k & 3) * 2;
-          umma_ss(tmem + x * 128, q_desc + x * kTileStep + off, k_desc + st * kTileStep + off, idesc_qk, k > 0 ? 1u : 0u);
-        }
-        umma_commit(&sm.s_full[x]);
-      }
-      __syncwarp();
-    };
-    while (ok && it.next()) {
-      const int st = j & 1, u = j >> 1;
-      // the operands of this step are waited for before the probabilities: nothing then stands between the
-      // products once a softmax warpgroup has delivered
-      ok = mbar_wait(&sm.k_full[st], u & 1, abort_word);
-      if (ok && j > 0) ok = mbar_wait(&sm.v_full[st ^ 1], ((j - 1) >> 1) & 1, abort_word);
-      if (!ok) break;
-      tc_fence_after();
-      bool need_cur[2];
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        need_cur[x] = (it.cur.w >> x) & 1;
-        // S_X may only be overwritten after P_X of the previous tile was consumed: its PV goes first
-        if (need_prev[x]) { ok = issue_pv(x, cnt[x] - 1, st ^ 1); if (!ok) break; }
-        if (need_cur[x]) { issue_qk(x, st); ++cnt[x]; }
-      }
-      if (!ok) break;
-      if (elect_one()) {
-        umma_commit(&sm.k_empty[st]);                   // both query tiles are through with K(j)
-        if (j > 0) umma_commit(&sm.v_empty[st ^ 1]);    // ... and with V(j-1)
-      }
-      __syncwarp();
-      need_prev[0] = need_cur[0]; need_prev[1] = need_cur[1];
-      ++j;
+      // TMEM and operands stay until all has retired
+      if (!ok) { umma_commit_pair(&sm.acc_full); ++n_tiles_done; }
+      for (int spin = 0; spin < 200000 && n_tiles_done > 0 && !mbar_try_wait(&sm.acc_full, (n_tiles_done - 1) & 1); ++spin) {}
+      // ... and no arrival from the other CTA is on its way any more
+      if (ok && n_tiles_done > 0) mbar_wait(&sm.o_empty, (n_tiles_done - 1) & 1, abort_word);
     }
-    if (ok && j > 0) ok = mbar_wait(&sm.v_full[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_word);
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-      if (ok && need_prev[x]) ok = issue_pv(x, cnt[x] - 1, (j - 1) & 1);
-    // keep TMEM alive until the last accumulate retired (the epilogues also wait on it)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-      if (ok && cnt[x] > 0) ok = mbar_wait(&sm.o_done[x], (cnt[x] - 1) & 1, abort_word);
+    __syncwarp();
+    if (!next_pass(pass)) break;
+   }
    } else {
     // ------------------------------------------------------------ operand fetch for the next stage
     run_copy_jobs(jobs, n_jobs, copy_ctx, blockIdx.x, gridDim.x, threadIdx.x - 320, 64);
+    __syncwarp();
+    if (next_pass(0)) next_pass(1);
    }
   } else {
-    // ------------------------------------------------------------ softmax + epilogue of tile X
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
-    const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem + lane_base + X * 128, o_addr = tmem + lane_base + 256 + X * 128;
+    // ------------------------------------------------------------ softmax of every second KV tile, epilogue of half the channels
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    const int wg = warp >> 2, quad = warp & 3, r = threadIdx.x & 127;
+    const uint32_t lane_base = uint32_t(quad * 32) << 16;
+    const uint32_t o_addr = tmem + lane_base + kSBufs * 128;
+    const uint32_t p_bar = cluster_addr(smem_u32(&sm.p_ready[0][0]), 0);
     const float sl2 = scale * 1.4426950408889634f;
-    const float rescale_gap = 8.0f / sl2;   // 8 in the base-2 exponent, expressed in raw score units
-    float m_run = -INFINITY, l_run = 0.f;
-    int j = 0;   // KV tiles this query tile took part in
-    bool ok = true;
-    while (ok && it.next()) {
-      if (!((it.cur.w >> X) & 1)) continue;
-      ok = mbar_wait(&sm.s_full[X], j & 1, abort_word);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t sreg[128];
+   for (int pass = 0;; ++pass) {
+    bool ok = true, ready = false;
+    int b = wg, bph = 0;       // buffer of this warpgroup's next KV tile, counted over all tiles
+    int g0 = 0;                // KV tiles before this tile
+    int published = 0;         // references handed on before this tile
+    int acc_ph = 0, turn = 0;  // parities of the tiles with a product and of all tiles so far
+    for (int info = 0, iph = 0;;) {
+      // ---- next tile
+      const TileInfo& ti = sm.info[info];
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&sm.info_full[info], iph, abort_word));
+      if (!ok || ti.n_kv < 0) break;
+      const int n = ti.n_kv;
+      const int4* subs = kv_subs + ti.kv_off;
+      const int4 mk = r < ti.n_rows ? ti.mask[r] : none;
+      const int first = wg ^ (g0 & 1);
+      int4 ahead = ti.first[first];
+      const bool sees = mk.y > mk.x || mk.w > mk.z;
+      float m_ref = sees ? -INFINITY : 0.f, l_run = 0.f;   // the row's reference, as far as this warpgroup knows; its own sum
+      bool exchange = pass > 0 || __any_sync(0xffffffffu, m_ref == -INFINITY);
+      int n_pub = exchange ? n : 0;
+      if (n > 0 && !((ti.first[0].w >> X) & 1)) {   // then no product sets O of this one; this warpgroup's channels here
+        uint32_t zero[32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + c * 32, sreg + c * 32);
-      tmem_wait_ld();
-      // Row maximum and row sum are reduced through 8 independent partial chains: a single running
-      // value would be a 128-long dependent chain with nothing to hide its latency behind.
-      float mxp[8];
+        for (int c = 0; c < 32; ++c) zero[c] = 0;
+        tmem_st32(o_addr + wg * 64, zero);
+        tmem_st32(o_addr + wg * 64 + 32, zero);
+        tmem_wait_st();
+      }
+      for (int j = first; j < n; j += 2) {
+        const int4 sub = ahead;
+        if (j + 2 < n) ahead = subs[j + 2];
+        const uint32_t s_addr = tmem + lane_base + b * 128;
+        const bool need = (sub.w >> X) & 1;
+        if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(&sm.s_full[b], bph, abort_word));
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t sreg[128];
+        if (need) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) mxp[i] = -INFINITY;
-      if ((it.cur.w >> (2 + X)) & 1) {
+          for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + c * 32, sreg + c * 32);
+          tmem_wait_ld();
+          if (!((sub.w >> (2 + X)) & 1)) {
+            // the keys this row sees as one bit each: a range costs a handful of instructions per 32 keys and an
+            // element one test, where comparing every key with four bounds costs six per element
+            const int a0 = mk.x - sub.y, b0 = min(max(mk.y, mk.x) - sub.y, sub.z), a1 = mk.z - sub.y,
+                      b1 = min(max(mk.w, mk.z) - sub.y, sub.z);
 #pragma unroll
-        for (int c = 0; c < 64; ++c)
-          mxp[c & 7] = fmax3(mxp[c & 7], __uint_as_float(sreg[2 * c]), __uint_as_float(sreg[2 * c + 1]));
-      } else {
-        // the keys this row sees as one bit each: a range costs a handful of instructions per 32 keys and an
-        // element one test, where comparing every key with four bounds costs six per element
-        const int a0 = s0 - it.cur.y, b0 = min(e0 - it.cur.y, it.cur.z), a1 = s1 - it.cur.y, b1 = min(e1 - it.cur.y, it.cur.z);
+            for (int w = 0; w < 4; ++w) {
+              const uint32_t see = bits_between(a0 - 32 * w, b0 - 32 * w) | bits_between(a1 - 32 * w, b1 - 32 * w);
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const uint32_t see = bits_between(a0 - 32 * w, b0 - 32 * w) | bits_between(a1 - 32 * w, b1 - 32 * w);
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const float sv = (see >> c) & 1u ? __uint_as_float(sreg[32 * w + c]) : -INFINITY;
-            sreg[32 * w + c] = __float_as_uint(sv);
-            mxp[c & 7] = fmaxf(mxp[c & 7], sv);
+              for (int c = 0; c < 32; ++c)
+                if (!((see >> c) & 1u)) sreg[32 * w + c] = 0xff800000u;   // -inf
+            }
           }
         }
-      }
-      const float mx = fmaxf(fmaxf(fmaxf(mxp[0], mxp[1]), fmaxf(mxp[2], mxp[3])),
-                             fmaxf(fmaxf(mxp[4], mxp[5]), fmaxf(mxp[6], mxp[7])));
-      // The running maximum only moves when the tile's maximum exceeds it by more than 2^8 in the
-      // exponent (or on the first tile): probabilities may then reach 256 instead of 1, which fp32 /
-      // bf16 hold without loss, and O has to be rescaled in TMEM only a few times per row instead of
-      // in most tiles.  out = O / l and lse = m + ln l are exact for any reference value m.
-      const float m_new = (mx > m_run + rescale_gap) ? mx : m_run;
-      const float m_sub = (m_new == -INFINITY) ? 0.f : m_new * sl2;
-      // exactly 1 where the maximum stays: m_run * sl2 - m_sub would be contracted to an FMA, whose residue of m_sub's
-      // rounding made most tiles rescale O
-      const bool moved = m_new != m_run;
-      const float alpha = moved ? fast_exp2((m_run - m_new) * sl2) : 1.f;
-      // S_X(j) was issued behind the previous accumulate into O_X, so that one has retired too
-      if (j > 0 && __any_sync(0xffffffffu, moved)) {
+        if (exchange) {
+          // what the warp that has the previous tile left behind
+          float m_cur = m_ref;
+          if (j > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.m_ready[quad], (published + j - 1) & 1, abort_word));
+            if (!ok) break;
+            m_cur = sm.m[r];
+          }
+          float m_new = m_cur;
+          if (pass == 0 && __all_sync(0xffffffffu, m_cur != -INFINITY)) {
+            exchange = false;   // settled by the other warpgroup
+            n_pub = j;
+          } else {
+            if (need) {
+              float mxp[8];   // eight chains: a single one would be 64 dependent steps
+#pragma unroll
+              for (int i = 0; i < 8; ++i) mxp[i] = -INFINITY;
+#pragma unroll
+              for (int c = 0; c < 64; ++c)
+                mxp[c & 7] = fmax3(mxp[c & 7], __uint_as_float(sreg[2 * c]), __uint_as_float(sreg[2 * c + 1]));
+              const float mx = fmaxf(fmaxf(fmaxf(mxp[0], mxp[1]), fmaxf(mxp[2], mxp[3])),
+                                     fmaxf(fmaxf(mxp[4], mxp[5]), fmaxf(mxp[6], mxp[7])));
+              m_new = (mx > m_cur + kGap / sl2) ? mx : m_cur;
+            }
+            sm.m[r] = m_new;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.m_ready[quad]);
+            exchange = pass > 0 || __any_sync(0xffffffffu, m_new == -INFINITY);
+            if (!exchange) n_pub = j + 1;
+            if (j > 0 && __any_sync(0xffffffffu, m_new != m_cur)) {
+              // no product may be adding to O; that of KV tile j - 3 has retired, as S(j) came after it, so the phase is
+              // unambiguous
+              const int i = g0 + j - 1 + kSBufs;   // its slot
+              ok = __all_sync(0xffffffffu, mbar_wait(&sm.kv_empty[i % kSlots], (i / kSlots) & 1, abort_word));
+              if (!ok) break;
+              tc_fence_after();
+              const float alpha = m_new != m_cur ? fast_exp2((m_cur - m_new) * sl2) : 1.f;   // exactly 1 where m stays
 #pragma unroll 1
-        for (int c = 0; c < 8; ++c) {   // rare: few registers and little code matter more than its speed
-          uint32_t oreg[16];
-          tmem_ld16(o_addr + c * 16, oreg);
-          tmem_wait_ld();
+              for (int c = 0; c < 8; ++c) {
+                uint32_t oreg[16];
+                tmem_ld16(o_addr + c * 16, oreg);
+                tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-          tmem_st16(o_addr + c * 16, oreg);
+                for (int i = 0; i < 16; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
+                tmem_st16(o_addr + c * 16, oreg);
+              }
+            }
+          }
+          if (m_ref != m_new) l_run *= fast_exp2((m_ref - m_new) * sl2);
+          m_ref = m_new;
+        }
+        if (need) {
+          const float m_sub = (m_ref == -INFINITY) ? 0.f : m_ref * sl2;
+          const uint64_t sl2_2 = pack_f32x2(sl2, sl2), negm_2 = pack_f32x2(kTruncLog2 - m_sub, kTruncLog2 - m_sub);
+          uint64_t ps2[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            softmax_half(sreg + 64 * h, sl2_2, negm_2, ps2, s_addr + 32 * h);
+            // the next scores: asked for here, where the answer is not waited for
+            if (h == 1) ready = __all_sync(0xffffffffu, mbar_test_wait(&sm.s_full[b >= 1 ? b - 1 : 2], b >= 1 ? bph ^ 1 : bph));
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(p_bar + 16 * b + 8 * h);
+          }
+          float psp[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) unpack_f32x2(ps2[i], psp[2 * i], psp[2 * i + 1]);
+          l_run += ((psp[0] + psp[1]) + (psp[2] + psp[3])) + ((psp[4] + psp[5]) + (psp[6] + psp[7]));
+        } else {
+          // Only the other query tile sees these keys: the product leaves O of this one alone (P times V would not,
+          // where V is not finite).
+          ready = false;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) { mbar_arrive_cluster(p_bar + 16 * b); mbar_arrive_cluster(p_bar + 16 * b + 8); }
+        }
+        b += 2;
+        if (b >= kSBufs) { b -= kSBufs; bph ^= 1; }
+      }
+      // ---- epilogue
+      float m_fin = m_ref;
+      if (n > 0 && ok) {
+        ok = mbar_wait(&sm.acc_full, acc_ph, abort_word);
+        acc_ph ^= 1;
+        tc_fence_after();
+        if (ok && exchange && ((g0 + n - 1) & 1) != wg) {
+          ok = mbar_wait(&sm.m_ready[quad], (published + n - 1) & 1, abort_word);
+          m_fin = sm.m[r];
         }
       }
-      // packed fp32: one instruction scales two scores, one adds two probabilities to the row sum
-      // every probability carries the factor kTruncScale (folded into the exponent), so cutting it to
-      // bf16 is unbiased; the row sum carries the same factor, which cancels in O / l and is taken
-      // out of the LSE in the epilogue
-      const uint64_t sl2_2 = pack_f32x2(sl2, sl2), negm_2 = pack_f32x2(kTruncLog2 - m_sub, kTruncLog2 - m_sub);
-      uint64_t ps2[4] = {0ull, 0ull, 0ull, 0ull};
-      // P goes back in two 32-column stores so fewer registers stay live
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t preg[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int cc = 32 * h + c;
-          const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(sreg[2 * cc]), __uint_as_float(sreg[2 * cc + 1])), sl2_2, negm_2);
-          float x0, x1;
-          unpack_f32x2(x2, x0, x1);
-          const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-          ps2[c & 3] = add_f32x2(ps2[c & 3], pack_f32x2(p0, p1));
-          preg[c] = pack_bf16x2_trunc(p0, p1);
-        }
-        tmem_st32(s_addr + 32 * h, preg);
-        tmem_wait_st();
+      float (*sums)[kTileM] = sm.l[turn];
+      sums[wg][r] = l_run != 0.f ? l_run * fast_exp2((m_ref - m_fin) * sl2) : 0.f;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.l_ready[quad]);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&sm.l_ready[quad], turn, abort_word));
+      if (!ok) break;
+      turn ^= 1;
+      published += n_pub;
+      g0 += n;
+      uint32_t oreg[64];
+      if (n > 0) {  // warp-uniform: the TMEM load is a warp-collective instruction
+        tmem_ld32(o_addr + wg * 64, oreg);
+        tmem_ld32(o_addr + wg * 64 + 32, oreg + 32);
+        tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.p_ready[X][h]);
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&sm.o_empty), 0));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) oreg[i] = 0;
       }
-      float psp[8];
+      const int n_rows = ti.n_rows;
+      const float l_sum = sums[0][r] + sums[1][r];
+      if (pass == 0 && __any_sync(0xffffffffu, r < n_rows && !(l_sum < kMaxSum)) && lane == 0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) unpack_f32x2(ps2[i], psp[2 * i], psp[2 * i + 1]);
-      const float psum = ((psp[0] + psp[1]) + (psp[2] + psp[3])) + ((psp[4] + psp[5]) + (psp[6] + psp[7]));
-      l_run = l_run * alpha + psum;
-      m_run = m_new;
-      ++j;
-    }
-    if (ok && j > 0) {
-      ok = mbar_wait(&sm.o_done[X], (j - 1) & 1, abort_word);
-      tc_fence_after();
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
-      const int row = X * kTileM + r;
-      const bool store = row < tile.n_rows;
-      const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
-      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(ptrs.out[tile.out_dev]) +
-                           (size_t(tile.out_row + row) * hq + tile.head) * kHeadDim;
-      if (store)
-        ptrs.lse[tile.out_dev][size_t(tile.head) * (tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b) + tile.out_row + row] =
-            l_run > 0.f ? m_run * scale + logf(l_run) - kTruncLn : -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t oreg[32];
-        if (j > 0) {  // warp-uniform: the TMEM load is a warp-collective instruction
-          tmem_ld32(o_addr + c * 32, oreg);
-          tmem_wait_ld();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) oreg[i] = 0;
-        }
-        if (store) {
-          uint32_t packed[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
-          uint4* dst = reinterpret_cast<uint4*>(out + c * 32);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+        for (int c = 0; c < 2; ++c) {
+          st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
+          or_cluster_u32(smem_u32(&sm.redo[(ti.round >> 5) & (kRedoWords - 1)]), c, 1u << (ti.round & 31));
         }
       }
+      const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
+      if (r < n_rows && wg == 0) ti.lse[r] = l_sum > 0.f ? m_fin * scale + logf(l_sum) - kTruncLn : -INFINITY;
+      __nv_bfloat16* out = ti.out + size_t(quad * 32 + (lane >> 2)) * hq * kHeadDim + wg * 64 + (lane & 3) * 8;
+      uint8_t* stage = sm.o_stage[warp];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {   // 32 channels: four 16-byte pieces per row, swizzled, out with four lanes per row
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t packed[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            packed[k] = pack_bf16x2(__uint_as_float(oreg[32 * c + 8 * i + 2 * k]) * inv_l, __uint_as_float(oreg[32 * c + 8 * i + 2 * k + 1]) * inv_l);
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = 8 * i + (lane >> 2);
+          const uint4 piece = *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4));
+          if (quad * 32 + row < n_rows) *reinterpret_cast<uint4*>(out + size_t(8 * i) * hq * kHeadDim + c * 32) = piece;
+        }
+        __syncwarp();
+      }
+      if (lane == 0) mbar_arrive(&sm.info_empty[info]);
+      if (++info == kInfos) { info = 0; iph ^= 1; }
     }
+    if (!next_pass(pass)) break;
+   }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 9) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
-  }
+  // nobody reads or signals the other CTA's shared memory any more
+  if (warp == 9) tmem_dealloc_pair(tmem, 512);
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, kStatusBarrierTimeout);
 }
 
@@ -426,9 +636,10 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
                                   void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream) {
   if (n_tiles <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
   if (n_dst > kMaxPeers || hq % hkv != 0) return -3;
-  CUtensorMap tm_q, tm_kv;
+  CUtensorMap tm_q, tm_k, tm_v;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, 128)) return -1;
-  if (encode_arena_map(&tm_kv, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 128)) return -1;
+  if (encode_arena_map(&tm_k, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 64)) return -1;
+  if (encode_arena_map(&tm_v, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 128)) return -1;
   PeerPtrs pp;
   for (int i = 0; i < kMaxPeers; ++i) {
     pp.out[i] = i < n_dst ? out_ptrs[i] : nullptr;
@@ -442,9 +653,9 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
       return -4;
     g_pair_attr_set = 1;
   }
-  attn_fwd_pair_kernel<<<n_tiles, kPairThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      tm_q, tm_kv, static_cast<const AttnTile*>(tiles), static_cast<const int4*>(kv_entries),
+  attn_fwd_pair_kernel<<<2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+      tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
       static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, int(q_rows),
-      block_size, n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);
+      n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

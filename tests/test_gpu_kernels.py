@@ -134,6 +134,61 @@ def test_attention_forward_masks_and_rescale(dev, nq, nkv, kind):
     assert out[nq:].abs().max() == 0
 
 
+@pytest.mark.parametrize("nkv", [128, 256, 300, 384, 512, 640, 1100])
+@pytest.mark.parametrize("kind", ["plain", "late", "jump", "apart", "short", "many"])
+def test_attention_forward_pairs_of_tiles(dev, nkv, kind):
+    """Two query tiles that share a walk over the keys, every remainder of the three score buffers and two
+    warpgroups, fp64 oracle.  late: rows whose first key lies in a later tile than their neighbours'; jump: scores that
+    rise by 2^70 and more after the first tile (the second pass); apart: key tiles that only one of the query tiles
+    sees, with values that are not finite where the other one does not look; short: the second query tile is empty; many:
+    more tiles than pairs of CTAs, some of them with a second pass, some without any key.
+    Bound as above: P and V are bf16, P is cut, the result is rounded once more, 2^-6 of the largest value."""
+    nq, hq = {"short": (100, 4), "many": (2300, 16)}.get(kind, (256, 4))
+    g = torch.Generator().manual_seed(nkv)
+    q, kv = (torch.randn(n + 29, *s, generator=g).bfloat16().to(dev) for n, s in ((nq, (hq, 128)), (nkv, (2, 2, 128))))
+    i = np.arange(nq)
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = nkv
+    if kind == "late":
+        rng[:, 0] = np.minimum(i * 5 % 700, nkv)          # the last ones see nothing at all
+    if kind == "many":
+        rng[512:800, 1] = 0
+        q[1000:1300, 1, 0] = 16.0
+    if kind in ("jump", "many"):
+        q[:, 0, 0] = 16.0                                 # one head
+        kv[128:nkv, 0, 0, 0] = (40.0 * (1 + torch.arange(nkv - 128, device=dev) // 128))[:].bfloat16()
+    if kind == "apart":
+        half = nkv // 256 * 128
+        rng[:128, 1], rng[128:, 0] = half, half
+        if half:
+            kv[half:nkv, 1, 0, 5] = float("inf")          # first value head: only the second query tile sees these keys
+            kv[:half, 1, 1, 7] = float("nan")             # second value head: only the first one does
+    row = A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)
+    out, lse = torch.zeros_like(q), torch.zeros(hq, nq + 29, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 2048, dev), [out], [lse], 128 ** -0.5, status)
+    assert status.item() == 0
+    k64, v64 = (kv[:nkv, j].double().repeat_interleave(hq // 2, 1).permute(1, 0, 2) for j in (0, 1))
+    sees = A.ranges_to_dense(rng, nkv).to(dev)
+    s = (q[:nq].double().permute(1, 0, 2) @ k64.transpose(1, 2) * 128 ** -0.5).masked_fill(~sees, float("-inf"))
+    p, rl = s.softmax(-1).nan_to_num(0.0), torch.logsumexp(s, -1)
+    got = out[:nq].double()
+    if kind == "apart":
+        fine = torch.ones(nq, 4, dtype=torch.bool, device=dev)
+        if nkv >= 256:
+            fine[128:, :2], fine[:128, 2:] = False, False
+        assert torch.isfinite(got[fine]).all()
+        v64, got = v64.nan_to_num(0.0, 0.0, 0.0), torch.where(fine[..., None], got, torch.zeros_like(got))
+        ref = torch.where(fine[..., None], (p @ v64).permute(1, 0, 2), torch.zeros_like(got))
+    else:
+        ref = (p @ v64).permute(1, 0, 2)
+    empty = torch.isinf(rl)
+    assert (got - ref).abs().max() <= 2.0 ** -6 * ref.abs().max()
+    assert torch.equal(torch.isinf(lse[:, :nq]), empty)
+    assert ((lse[:, :nq] - rl)[~empty].abs() < 1e-3 + 2.0 ** -22 * rl[~empty].abs()).all()
+    assert out[nq:].abs().max() == 0
+
+
 @pytest.mark.parametrize("nq,nkv,kind,heads", [(1, 1, "causal", (4, 4)), (127, 129, "full", (4, 1)), (129, 127, "causal", (8, 2)),
                                                 (256, 255, "two", (4, 2)), (64, 640, "full", (8, 1)), (700, 700, "two", (8, 2))])
 def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
