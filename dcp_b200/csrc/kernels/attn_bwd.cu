@@ -7,13 +7,16 @@
 //   dP^T = V  dO^T    (SS)                                                  -> TMEM
 //   P^T  = exp2(S^T*c - lse),  dS^T = P^T o (dP^T - delta) * scale          (16 gradient warps)
 //   dV  += P^T  dO    (TS, P^T as packed bf16 in the TMEM columns S^T came from)
-//   dK  += dS^T Q     (SS, A = dS^T tile in shared memory, K-major)
-//   dQ   = dS   K     (SS, A = the same dS^T bytes read MN-major)           -> the TMEM columns of dP^T
-// TMEM (512 columns): S^T / P^T [0,128)  dP^T / dQ [128,256)  dK [256,384)  dV [384,512).
+//   dK  += dS^T Q     (TS, dS^T as packed bf16 in the TMEM columns dP^T came from)
+//   dQ   = dS   K     (SS, A = dS^T in shared memory, read MN-major)         -> the TMEM columns of dP^T, behind dK
+// TMEM (512 columns): S^T / P^T [0,128)  dP^T / dS^T / dQ [128,256)  dK [256,384)  dV [384,512).
 // Per item t the issuer emits  S(t+1) | dK(t) dQ(t) | dP(t+1) | dV(t+1):  the exponentials of t+1 run
-// under dK(t) / dQ(t), and dS(t+1) under dV(t+1) and S(t+2).  dK comes before dQ although the drain of dQ is not
-// hidden behind it then: it hands the Q tile back 580 cycles earlier, and a Q tile that arrives late holds up all
-// that follows (full 5.02 -> 4.98 ms, causal 3.82 -> 3.77, sink + window 1.41 -> 1.38 at the size below).
+// under dK(t) / dQ(t), and dS(t+1) under dV(t+1) and S(t+2).  dK comes before dQ, which overwrites its A
+// operand.  With dS^T in TMEM the product dK takes 64 instead of 72 cycles per UMMA and leaves 256 wavefronts per
+// item of shared memory to others.  The gradient warps wait twice per item, where it was five times: the statistics
+// of the queries arrive on the barriers of S and dP, and dP says that dQ of the item before is done with dS^T.  Both
+// together (8192 queries x 16384 keys, one box, long runs): full 5.59 -> 5.41 ms, causal 4.23 -> 4.09, sink + window
+// 1.49 -> 1.47; each alone up to 1 %.
 // Warps: 0-15 gradient (warp = 32 key rows x 32 queries), 16-23 drain dQ (thread = 64 channels of a query row; a
 // [32 queries x 32 channels] fp32 tile per step, added to the accumulator with one tiled TMA
 // reduce-add, or to a peer's with a 128-byte bulk reduce-add per row), 24 TMA producer, 25 UMMA issuer, 26
@@ -30,11 +33,11 @@
 // 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
 // 13 stall cycles per issue; 0.5 of 19 now).  8 drain warps keep their part of dQ in registers, so the columns
 // are free before the shared-memory tile and the L2 have taken it (4 warps with half of it at a time: 7 % slower).
-// What bounds it now: the shared-memory pipe.  An item moves 2304 wavefronts of UMMA operands and 1870 of loads
-// and stores (dS^T, dQ staging, statistics).  Over the whole kernel (causal, below, under ncu: 3.92 ms at 1.62
+// What bounds it now: the shared-memory pipe.  An item moves 2048 wavefronts of UMMA operands and 1870 of loads
+// and stores (dS^T, dQ staging, statistics).  Before dK took its operand from TMEM (256 more), over the whole kernel (causal, below, under ncu: 3.92 ms at 1.62
 // GHz, 1335 items per SM, so 4760 cycles per item with prologues, ends of CTAs and the last wave) the counters show
-// 49 and 40 % of that pipe and 56 % of the tensor pipe; inside the loop an item takes 4100 to 4300 cycles, which the
-// 4174 wavefronts fill.  TMA traffic (128 KB per item: Q, dO, dQ) is in neither counter.  Without the dQ drain an item takes 15 %
+// 49 and 40 % of that pipe and 56 % of the tensor pipe; inside the loop an item took 4100 to 4300 cycles, which the
+// 4174 wavefronts filled.  TMA traffic (128 KB per item: Q, dO, dQ) is in neither counter.  Without the dQ drain an item takes 15 %
 // less.
 // Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104
 // TFLOP/s), causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
@@ -121,7 +124,7 @@ struct __align__(1024) BwdSmem {
   alignas(16) float nlse[2][kQTile];
   uint32_t rng[2][kQTile];
   alignas(16) float ndelta[kQTile];
-  uint64_t kv_full, q_full[2], q_empty[2], stats_full[2], do_full, do_empty, delta_full, s_full, p_ready, dp_full,
+  uint64_t kv_full, q_full[2], q_empty[2], do_full, do_empty, s_full[2], p_ready, dp_full,
       ds_ready, dq_full, dq_drained, acc_full;
   int fast[2];                      // item of the stage needs no masking at all
   uint32_t tmem_base;
@@ -256,13 +259,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_kv);
     tma_prefetch_desc(&tm_dq);
     mbar_init(&sm.kv_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&sm.q_full[i], 1); mbar_init(&sm.q_empty[i], 1); mbar_init(&sm.stats_full[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sm.q_full[i], 1); mbar_init(&sm.q_empty[i], 1); mbar_init(&sm.s_full[i], 2); }
     mbar_init(&sm.do_full, 1);
     mbar_init(&sm.do_empty, 1);
-    mbar_init(&sm.delta_full, 1);
-    mbar_init(&sm.s_full, 1);
     mbar_init(&sm.p_ready, 16);
-    mbar_init(&sm.dp_full, 1);
+    mbar_init(&sm.dp_full, 2);
     mbar_init(&sm.ds_ready, 16);
     mbar_init(&sm.dq_full, 1);
     mbar_init(&sm.dq_drained, 8);
@@ -393,14 +394,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           sm.rng[st][lane + 32 * h] = cur.rg[h];
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.stats_full[st]);  // release: the stores above are visible to waiters
+        if (lane == 0) mbar_arrive(&sm.s_full[st]);  // release: the stores above are visible to waiters
         // the gradient warps are through with the previous item's delta once its dS is written
         if (i > 0) ok = __all_sync(0xffffffffu, mbar_wait(&sm.ds_ready, (i - 1) & 1, abort_word));
         if (!ok) break;
 #pragma unroll
         for (int h = 0; h < 4; ++h) sm.ndelta[lane + 32 * h] = -cur.d[h] * scale;
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.delta_full);
+        if (lane == 0) mbar_arrive(&sm.dp_full);
         cur = nxt;
       }
     } else if (warp == 25) {
@@ -427,7 +428,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       auto issue_s = [&](int t) -> bool {
         if (!mbar_wait(&sm.q_full[t & 1], (t >> 1) & 1, abort_word)) return false;
         TL_ADD(8, tl_t);
-        issue_kk(cS, k_addr, smem_u32(sm.q[t & 1]), &sm.s_full);   // P(t-1) was consumed by dV(t-1), issued before
+        issue_kk(cS, k_addr, smem_u32(sm.q[t & 1]), &sm.s_full[t & 1]);   // P(t-1) was consumed by dV(t-1), issued before
         TL_ADD(12, tl_t);
         return true;
       };
@@ -463,8 +464,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint32_t q_addr = smem_u32(sm.q[t & 1]);
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 queries per step
-            umma_ss(tmem + cdK, make_sdesc_sw128(ds_addr + (k >> 2) * kHalf + (k & 3) * 32, 16, 1024),
-                    make_sdesc_sw128(q_addr + k * 2048, kHalf, 1024), idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
+            umma_ts(tmem + cdK, tmem + cdP + (k >> 1) * 32 + (k & 1) * 8, make_sdesc_sw128(q_addr + k * 2048, kHalf, 1024),
+                    idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.q_empty[t & 1]);   // Q(t) is free
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 keys per step
@@ -559,7 +560,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     for (int t = 0; t < n_items && ok; ++t) {
       const int st = t & 1;
-      ok = mbar_wait(&sm.stats_full[st], (t >> 1) & 1, abort_word);
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.s_full[st], (t >> 1) & 1, abort_word));
+      if (!ok) break;
       TL_ADD(0, tl_t);
       // The tile-level "no masking needed" switch is taken once, outside the element loops.  Otherwise
       // every lane turns the ranges of one query into a bit word over the warp's 32 keys, and a bit
@@ -567,8 +569,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const bool fast = sm.fast[st];
       uint32_t see = 0;
       if (!fast) see = warp_transpose_bits(visible_keys(sm.rng[st][hf * 32 + lane], quad * 32), lane);
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(&sm.s_full, t & 1, abort_word));
-      if (!ok) break;
       TL_ADD(1, tl_t);
       tc_fence_after();
       uint32_t p[32];
@@ -586,11 +586,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.p_ready);
       TL_ADD(3, tl_t);
-      ok = mbar_wait(&sm.delta_full, t & 1, abort_word);
-      ok = ok && mbar_wait(&sm.dp_full, t & 1, abort_word);
-      // dK and dQ of the previous item must have finished reading the dS^T tile
-      if (t > 0) ok = ok && mbar_wait(&sm.dq_full, (t - 1) & 1, abort_word);
-      ok = __all_sync(0xffffffffu, ok);
+      // dP(t) was issued behind dK(t-1) and dQ(t-1), which have finished reading dS^T then
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.dp_full, t & 1, abort_word));
       if (!ok) break;
       TL_ADD(4, tl_t);
       tc_fence_after();
@@ -605,7 +602,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int c = 0; c < 2; ++c)
           *reinterpret_cast<uint4*>(ds_row + ((((hf & 1) * 4 + 2 * h + c) ^ (r & 7)) << 4)) =
               make_uint4(packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
+        tmem_st8(dp_addr + 8 * h, packed);   // over the dP^T columns read above
       }
+      tmem_wait_st();
       TL_ADD(5, tl_t);
       fence_proxy_async_smem();
       tc_fence_before();
