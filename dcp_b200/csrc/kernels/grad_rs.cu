@@ -23,6 +23,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace dcpk {
 
 static constexpr int kMaxRanks = 16;
@@ -100,41 +102,57 @@ __global__ void adamw_all_gather_kernel(float* __restrict__ master, float* __res
   }
 }
 
-// squared norm of the scaled, rank-summed gradient slice; nothing is written but the scalar.  Four vectors of a
-// thread are in flight at once (one at a time read at 3.4 TB/s: 253 us for 436M gradients, 212 us now; with a
-// thread's four vectors 4 KB apart instead of a grid apart 235 us).
+// squared norm of the scaled, rank-summed gradient slice; nothing is written but the scalar.  Bound by reading.
+// One rank (kOne): a vector at a time in 148 x 4 CTAs whose loads leave L1 alone reads 436M gradients at 6.2 TB/s (141 us);
+// four vectors of a thread in flight, which over peers' buffers hide the link, 4.4 TB/s (197 us; a grid apart or 4 KB apart,
+// in twice as many CTAs or half as many: 152 to 350 us), and 32-byte loads 5.7 TB/s.
+template <bool kOne>
 __global__ void __launch_bounds__(256) grad_sqnorm_kernel(GradPtrs grads, int world, size_t shard_off, size_t shard_len,
                                                           float scale, double* __restrict__ sq_norm) {
+  constexpr int kFlight = kOne ? 1 : 4;
   const size_t n_vec = shard_len / 8, stride = size_t(gridDim.x) * blockDim.x;
-  float local_sq = 0.f;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec; i += 4 * stride) {
-    float acc[4][8];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[u][j] = 0.f;
-    for (int r = 0; r < world; ++r) {
+  const uint64_t scale_2 = pack_f32x2(scale, scale);
+  uint64_t sq_2[4] = {0ull, 0ull, 0ull, 0ull};
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec; i += kFlight * stride) {
+    uint64_t acc[kFlight][4];
+    for (int r = 0; r < (kOne ? 1 : world); ++r) {
       const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(grads.p[r]) + shard_off);
-      uint4 raw[4];
+      uint4 raw[kFlight];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) raw[u] = i + u * stride < n_vec ? src[i + u * stride] : make_uint4(0, 0, 0, 0);
+      for (int u = 0; u < kFlight; ++u) {
+        if (kOne) {
+          asm("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
+              : "=r"(raw[u].x), "=r"(raw[u].y), "=r"(raw[u].z), "=r"(raw[u].w) : "l"(src + i));
+        } else {
+          raw[u] = i + u * stride < n_vec ? src[i + u * stride] : make_uint4(0, 0, 0, 0);
+        }
+      }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
+      for (int u = 0; u < kFlight; ++u) {
+        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 f = __bfloat1622float2(v[j]);
-          acc[u][2 * j] += f.x; acc[u][2 * j + 1] += f.y;
+          const uint64_t g = pack_f32x2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+          acc[u][j] = r == 0 ? g : add_f32x2(acc[u][j], g);
         }
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < kFlight; ++u)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { const float g = acc[u][j] * scale; local_sq += g * g; }
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t g = mul_f32x2(acc[u][j], scale_2);
+        sq_2[j] = fma_f32x2(g, g, sq_2[j]);
+      }
   }
   // from the threads' sums on in 64 bits: a thousand partial sums added one by one in 32 bits cost 1e-6
-  double t = local_sq;
+  double t = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float lo, hi;
+    unpack_f32x2(sq_2[j], lo, hi);
+    t += double(lo) + double(hi);
+  }
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
   __shared__ double part[8];
@@ -229,9 +247,11 @@ extern "C" int dcpk_grad_sqnorm(const void* const* grad_ptrs, int world, long sh
   if (world > kMaxRanks || shard_off % 8 || shard_len % 8) return -3;
   GradPtrs g;
   for (int i = 0; i < kMaxRanks; ++i) g.p[i] = i < world ? grad_ptrs[i] : nullptr;
-  const long blocks = (shard_len / 8 + 4 * 256 - 1) / (4 * 256);
-  grad_sqnorm_kernel<<<int(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(g, world, size_t(shard_off),
-                                                                             size_t(shard_len), scale, sq_norm);
+  const bool one = world == 1;
+  const long per_block = one ? 256 : 4 * 256, most = one ? 148 * 4 : 148 * 8, blocks = (shard_len / 8 + per_block - 1) / per_block;
+  auto kernel = one ? grad_sqnorm_kernel<true> : grad_sqnorm_kernel<false>;
+  kernel<<<int(blocks < most ? blocks : most), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      g, world, size_t(shard_off), size_t(shard_len), scale, sq_norm);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
