@@ -28,8 +28,12 @@
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
-// products ran at half rate.  The issuer's branch is taken by elect.sync: with a test on the lane number
-// each UMMA took about 90 cycles to issue (128 x 128 tiles: 839 against 1053 TFLOP/s).  16 gradient warps of
+// products ran at half rate.  The issuer is one thread, taken by elect.sync: with a test on the lane number
+// each UMMA took about 90 cycles to issue (128 x 128 tiles: 839 against 1053 TFLOP/s).  Its descriptors cost an addition of 32
+// bits each, and it asks for operands that are long there while it has something to issue: an answer takes 200 cycles and
+// more, behind the exponentials of the warps that share its scheduler (full 5.52 -> 5.45 ms, causal 4.18 -> 4.13, sink +
+// window 1.52 -> 1.51 in long runs; 1000 queries x 2100 keys, causal, 101 -> 99 us).  Handing dS^T to dK before it is stored
+// for dQ costs more registers than it gains time (5.69 ms).  16 gradient warps of
 // 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
 // 13 stall cycles per issue; 0.5 of 19 now).  8 drain warps keep their part of dQ in registers, so the columns
 // are free before the shared-memory tile and the L2 have taken it (4 warps with half of it at a time: 7 % slower).
@@ -139,7 +143,7 @@ __device__ long long* g_bwd_timeline = nullptr;
 static_assert(offsetof(BwdSmem, dout) == 256 * kHeadDim * sizeof(float), "K, V and Q tiles hold a gradient share");
 #define TL_ADD(idx, t_prev)                                                        \
   do {                                                                             \
-    if constexpr (kTL) if (tl) { long long now_ = clock64(); if (lane == 0) atomicAdd(reinterpret_cast<unsigned long long*>(tl + (idx)), (unsigned long long)(now_ - (t_prev))); (t_prev) = now_; } \
+    if constexpr (kTL) if (tl) { long long now_ = clock64(); if (lane == 0 || warp == 25) atomicAdd(reinterpret_cast<unsigned long long*>(tl + (idx)), (unsigned long long)(now_ - (t_prev))); (t_prev) = now_; } \
   } while (0)
 
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
@@ -405,89 +409,90 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         cur = nxt;
       }
     } else if (warp == 25) {
-      // ------------------------------------------------------------ UMMA issuer
-      constexpr uint32_t idesc_sdp = make_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1);
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, 1, 1);
-      const uint32_t k_addr = smem_u32(sm.k), v_addr = smem_u32(sm.v), ds_addr = smem_u32(sm.ds), do_addr = smem_u32(sm.dout);
-      bool ok = mbar_wait(&sm.kv_full, 0, abort_word);
-      // D = A B^T, both operands K-major (K = channels)
-      auto issue_kk = [&](uint32_t col, uint32_t a_addr, uint32_t b_addr, uint64_t* done) {
-        tc_fence_after();
-        if (elect_one()) {
+      // ------------------------------------------------------------ UMMA issuer (one thread)
+      if (elect_one()) {
+        constexpr uint32_t idesc_sdp = make_idesc_bf16(128, 128, 0, 0);
+        constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1);
+        constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, 1, 1);
+        // descriptors: K-major operands and MN-major ones differ in the leading offset, all others in the address field only
+        const uint64_t some = make_sdesc_sw128(0, 16, 1024), some_mn = make_sdesc_sw128(0, kHalf, 1024);
+        const uint32_t hi = uint32_t(some >> 32), lo = uint32_t(some), lo_mn = uint32_t(some_mn);
+        auto desc = [&](uint32_t low) { return (uint64_t(hi) << 32) | low; };
+        const uint32_t k_at = sdesc_addr(sm.k), v_at = sdesc_addr(sm.v), ds_at = sdesc_addr(sm.ds), do_at = sdesc_addr(sm.dout),
+                       q_at = sdesc_addr(sm.q[0]);
+        constexpr uint32_t kTile = 2 * kHalf >> 4;
+        bool ok = mbar_wait(&sm.kv_full, 0, abort_word);
+        // D = A B^T, both operands K-major (K = channels)
+        auto issue_kk = [&](uint32_t col, uint32_t a_at, uint32_t b_at, uint64_t* done) {
+          tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            const uint32_t off = (k >> 2) * kHalf + (k & 3) * 32;
-            umma_ss(tmem + col, make_sdesc_sw128(a_addr + off, 16, 1024), make_sdesc_sw128(b_addr + off, 16, 1024), idesc_sdp,
-                    k > 0 ? 1u : 0u);
+            const uint32_t off = (k >> 2) * (kHalf >> 4) + (k & 3) * 2;
+            umma_ss(tmem + col, desc(lo + a_at + off), desc(lo + b_at + off), idesc_sdp, k > 0 ? 1u : 0u);
           }
           umma_commit(done);
-        }
-        __syncwarp();
-      };
-      auto issue_s = [&](int t) -> bool {
-        if (!mbar_wait(&sm.q_full[t & 1], (t >> 1) & 1, abort_word)) return false;
-        TL_ADD(8, tl_t);
-        issue_kk(cS, k_addr, smem_u32(sm.q[t & 1]), &sm.s_full[t & 1]);   // P(t-1) was consumed by dV(t-1), issued before
-        TL_ADD(12, tl_t);
-        return true;
-      };
-      auto issue_dp = [&](int t) -> bool {
-        if (t > 0 && !mbar_wait(&sm.dq_drained, (t - 1) & 1, abort_word)) return false;
-        TL_ADD(10, tl_t);
-        if (!mbar_wait(&sm.do_full, t & 1, abort_word)) return false;
-        TL_ADD(14, tl_t);
-        issue_kk(cdP, v_addr, do_addr, &sm.dp_full);
-        TL_ADD(15, tl_t);
-        return true;
-      };
-      auto issue_dv = [&](int t) -> bool {
-        if (!mbar_wait(&sm.p_ready, t & 1, abort_word)) return false;
-        TL_ADD(11, tl_t);
-        tc_fence_after();
-        if (elect_one()) {
+        };
+        auto issue_s = [&](int t, bool there) -> bool {
+          if (!there && !mbar_wait(&sm.q_full[t & 1], (t >> 1) & 1, abort_word)) return false;
+          TL_ADD(8, tl_t);
+          issue_kk(cS, k_at, q_at + (t & 1) * kTile, &sm.s_full[t & 1]);   // P(t-1) was consumed by dV(t-1), issued before
+          TL_ADD(12, tl_t);
+          return true;
+        };
+        auto issue_dp = [&](int t, bool there) -> bool {
+          if (t > 0 && !mbar_wait(&sm.dq_drained, (t - 1) & 1, abort_word)) return false;
+          TL_ADD(10, tl_t);
+          if (!there && !mbar_wait(&sm.do_full, t & 1, abort_word)) return false;
+          TL_ADD(14, tl_t);
+          issue_kk(cdP, v_at, do_at, &sm.dp_full);
+          TL_ADD(15, tl_t);
+          return true;
+        };
+        auto issue_dv = [&](int t) -> bool {
+          if (!mbar_wait(&sm.p_ready, t & 1, abort_word)) return false;
+          TL_ADD(11, tl_t);
+          tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 queries per step; P^T: queries 32 i .. 32 i + 31 in columns [32 i, 32 i + 16) of S^T
-            umma_ts(tmem + cdV, tmem + cS + (k >> 1) * 32 + (k & 1) * 8, make_sdesc_sw128(do_addr + k * 2048, kHalf, 1024),
-                    idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
+            umma_ts(tmem + cdV, tmem + cS + (k >> 1) * 32 + (k & 1) * 8, desc(lo_mn + do_at + k * 128), idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.do_empty);
-        }
-        __syncwarp();
-        TL_ADD(7, tl_t);
-        return true;
-      };
-      auto issue_dqk = [&](int t) -> bool {
-        if (!mbar_wait(&sm.ds_ready, t & 1, abort_word)) return false;
-        TL_ADD(9, tl_t);
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t q_addr = smem_u32(sm.q[t & 1]);
+          TL_ADD(7, tl_t);
+          return true;
+        };
+        auto issue_dqk = [&](int t) -> bool {
+          if (!mbar_wait(&sm.ds_ready, t & 1, abort_word)) return false;
+          TL_ADD(9, tl_t);
+          tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 queries per step
-            umma_ts(tmem + cdK, tmem + cdP + (k >> 1) * 32 + (k & 1) * 8, make_sdesc_sw128(q_addr + k * 2048, kHalf, 1024),
-                    idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
+            umma_ts(tmem + cdK, tmem + cdP + (k >> 1) * 32 + (k & 1) * 8, desc(lo_mn + q_at + (t & 1) * kTile + k * 128), idesc_acc,
+                    (t > 0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.q_empty[t & 1]);   // Q(t) is free
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 keys per step
-            umma_ss(tmem + cdP, make_sdesc_sw128(ds_addr + k * 2048, kHalf, 1024), make_sdesc_sw128(k_addr + k * 2048, kHalf, 1024),
-                    idesc_dq, k > 0 ? 1u : 0u);
+            umma_ss(tmem + cdP, desc(lo_mn + ds_at + k * 128), desc(lo_mn + k_at + k * 128), idesc_dq, k > 0 ? 1u : 0u);
           umma_commit(&sm.dq_full);            // and so is the dS^T tile
-        }
-        __syncwarp();
-        TL_ADD(13, tl_t);
-        return true;
-      };
-      if (n_items > 0) {
-        ok = ok && issue_s(0) && issue_dp(0) && issue_dv(0);
-        for (int t = 0; t + 1 < n_items && ok; ++t)
-          ok = issue_s(t + 1) && issue_dqk(t) && issue_dp(t + 1) && issue_dv(t + 1);
-        ok = ok && issue_dqk(n_items - 1);
-        if (ok) {
-          if (elect_one()) umma_commit(&sm.acc_full);
-          __syncwarp();
-          mbar_wait(&sm.acc_full, 0, abort_word);   // keep TMEM alive until everything retired
+          TL_ADD(13, tl_t);
+          return true;
+        };
+        if (n_items > 0) {
+          ok = ok && issue_s(0, false) && issue_dp(0, false) && issue_dv(0);
+          for (int t = 0; t + 1 < n_items && ok; ++t) {
+            // an answer takes 200 cycles and more: the operands that are long there are asked for together
+            const bool q_there = mbar_test_wait(&sm.q_full[(t + 1) & 1], ((t + 1) >> 1) & 1);
+            ok = issue_s(t + 1, q_there);
+            if (!ok) break;
+            const bool do_there = mbar_test_wait(&sm.do_full, (t + 1) & 1);
+            ok = issue_dqk(t) && issue_dp(t + 1, do_there) && issue_dv(t + 1);
+          }
+          ok = ok && issue_dqk(n_items - 1);
+          if (ok) {
+            umma_commit(&sm.acc_full);
+            mbar_wait(&sm.acc_full, 0, abort_word);   // keep TMEM alive until everything retired
+          }
         }
       }
+      __syncwarp();
     }
   } else if (warp >= 16) {
     // ------------------------------------------------------------ dQ drain: thread = query row

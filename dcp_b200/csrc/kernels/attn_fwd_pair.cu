@@ -306,8 +306,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // descriptors differ in the address field of the low word only
       const uint64_t some = make_sdesc_sw128(0, 16, 1024);
       const uint32_t hi = uint32_t(some >> 32);
-      const uint32_t q_lo = uint32_t(some) + (smem_u32(sm.q[0]) >> 4), k_lo = uint32_t(some) + (smem_u32(sm.k[0]) >> 4),
-                     v_lo = uint32_t(some) + (smem_u32(sm.v[0]) >> 4);
+      const uint32_t q_lo = uint32_t(some) + sdesc_addr(sm.q[0]), k_lo = uint32_t(some) + sdesc_addr(sm.k[0]),
+                     v_lo = uint32_t(some) + sdesc_addr(sm.v[0]);
       auto desc = [&](uint32_t lo) { return (uint64_t(hi) << 32) | lo; };
       constexpr uint32_t kKvStep = kKvBytes >> 4, kQStep = 2 * kQHalf >> 4;   // in a descriptor's 16-byte units
       bool ok = true;

@@ -344,6 +344,10 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_
   return d;
 }
 
+// address field of a descriptor: the offset in the CTA's own window (in a cluster the upper bits of a shared-memory
+// address name the CTA and must not reach the fields above)
+__device__ __forceinline__ uint32_t sdesc_addr(const void* p) { return (smem_u32(p) & 0x3FFFFu) >> 4; }
+
 // ---------------------------------------------------------------- misc math
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
