@@ -218,7 +218,12 @@ __device__ __forceinline__ void grad_scores(const uint32_t* p, const uint32_t* d
   }
 }
 
-template <bool kTL>
+// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and products over zeros
+// and accumulators of zeros are left out: for up to 64 channels half of S and dP (K steps), half of dK, dV and dQ (N) and
+// of their traffic; for up to 96 a quarter of S, dP and the drain of dQ (N stays 128: an operand that is not K-major comes in
+// 64s).  8192 queries x 16384 keys, 32 / 8 heads, causal, against all 128
+// channels: 64 channels 3.56 -> 2.61 ms, 96 channels 3.99 -> 3.45 ms; 1000 x 2100: 110 -> 83 us and 122 -> 110 us.
+template <bool kTL, int kD>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_dq,
@@ -238,6 +243,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // grid = (kv heads x parts of the head group, key tiles): neighbouring CTAs share the item list and the mask rows
   const BwdCta cta = ctas[blockIdx.y - n_copy_rows];
+  constexpr int kHalves = kD > 64 ? 2 : 1;   // of 64 channels
   const int group = hq / hkv, parts = group / heads_per_cta;
   const int kv_head = blockIdx.x / parts, head0 = kv_head * group + (blockIdx.x % parts) * heads_per_cta;
   const BwdItemDesc* my_items = items + cta.item_off;
@@ -295,11 +301,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (warp == 24) {
       // ------------------------------------------------------------ TMA producer
       if (lane == 0) {
-        mbar_expect_tx(&sm.kv_full, 4 * kHalf);
-        tma_load_3d(sm.k, &tm_kv, &sm.kv_full, 0, kv_head, cta.kv_row);
-        tma_load_3d(sm.k + kHalf, &tm_kv, &sm.kv_full, 64, kv_head, cta.kv_row);
-        tma_load_3d(sm.v, &tm_kv, &sm.kv_full, 0, hkv + kv_head, cta.kv_row);
-        tma_load_3d(sm.v + kHalf, &tm_kv, &sm.kv_full, 64, hkv + kv_head, cta.kv_row);
+        mbar_expect_tx(&sm.kv_full, 2 * kHalves * kHalf);
+#pragma unroll
+        for (int h = 0; h < kHalves; ++h) {
+          tma_load_3d(sm.k + h * kHalf, &tm_kv, &sm.kv_full, 64 * h, kv_head, cta.kv_row);
+          tma_load_3d(sm.v + h * kHalf, &tm_kv, &sm.kv_full, 64 * h, hkv + kv_head, cta.kv_row);
+        }
       }
       bool ok = true;
       int q_pending[2] = {-1, -1}, do_pending = -1;
@@ -320,25 +327,28 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         ok = __all_sync(0xffffffffu, mbar_wait(&sm.q_empty[st], (u & 1) ^ 1, abort_word));
         if (!ok) break;
         if (lane == 0) {
-          mbar_expect_tx(&sm.q_full[st], 2 * kHalf);
-          tma_load_3d(sm.q[st], &tm_q, &sm.q_full[st], 0, itx.head, itx.q_row);
-          tma_load_3d(sm.q[st] + kHalf, &tm_q, &sm.q_full[st], 64, itx.head, itx.q_row);
+          mbar_expect_tx(&sm.q_full[st], kHalves * kHalf);
+#pragma unroll
+          for (int h = 0; h < kHalves; ++h)
+            tma_load_3d(sm.q[st] + h * kHalf, &tm_q, &sm.q_full[st], 64 * h, itx.head, itx.q_row);
           q_pending[st] = u & 1;
         }
         ok = __all_sync(0xffffffffu, mbar_wait(&sm.do_empty, (i & 1) ^ 1, abort_word));
         if (!ok) break;
         if (lane == 0) {
-          mbar_expect_tx(&sm.do_full, 2 * kHalf);
-          tma_load_3d(sm.dout, &tm_do, &sm.do_full, 0, itx.head, itx.q_row);
-          tma_load_3d(sm.dout + kHalf, &tm_do, &sm.do_full, 64, itx.head, itx.q_row);
+          mbar_expect_tx(&sm.do_full, kHalves * kHalf);
+#pragma unroll
+          for (int h = 0; h < kHalves; ++h)
+            tma_load_3d(sm.dout + h * kHalf, &tm_do, &sm.do_full, 64 * h, itx.head, itx.q_row);
           do_pending = i & 1;
           // the visit after the next is pulled into L2 now, so that its loads find it there
           const BwdItem& nx = ring[2];
           if (i + 2 < n_items && nx.q_row >= 0 && nx.q_row < q_rows && nx.head < hq) {
-            tma_prefetch_l2_3d(&tm_q, 0, nx.head, nx.q_row);
-            tma_prefetch_l2_3d(&tm_q, 64, nx.head, nx.q_row);
-            tma_prefetch_l2_3d(&tm_do, 0, nx.head, nx.q_row);
-            tma_prefetch_l2_3d(&tm_do, 64, nx.head, nx.q_row);
+#pragma unroll
+            for (int h = 0; h < kHalves; ++h) {
+              tma_prefetch_l2_3d(&tm_q, 64 * h, nx.head, nx.q_row);
+              tma_prefetch_l2_3d(&tm_do, 64 * h, nx.head, nx.q_row);
+            }
           }
         }
         ring[0] = ring[1]; ring[1] = ring[2];
@@ -412,8 +422,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // ------------------------------------------------------------ UMMA issuer (one thread)
       if (elect_one()) {
         constexpr uint32_t idesc_sdp = make_idesc_bf16(128, 128, 0, 0);
-        constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1);
-        constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, 1, 1);
+        constexpr uint32_t idesc_acc = make_idesc_bf16(128, 64 * kHalves, 0, 1);
+        constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64 * kHalves, 1, 1);
         // descriptors: K-major operands and MN-major ones differ in the leading offset, all others in the address field only
         const uint64_t some = make_sdesc_sw128(0, 16, 1024), some_mn = make_sdesc_sw128(0, kHalf, 1024);
         const uint32_t hi = uint32_t(some >> 32), lo = uint32_t(some), lo_mn = uint32_t(some_mn);
@@ -426,7 +436,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         auto issue_kk = [&](uint32_t col, uint32_t a_at, uint32_t b_at, uint64_t* done) {
           tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
+          for (int k = 0; k < kD / 16; ++k) {
             const uint32_t off = (k >> 2) * (kHalf >> 4) + (k & 3) * 2;
             umma_ss(tmem + col, desc(lo + a_at + off), desc(lo + b_at + off), idesc_sdp, k > 0 ? 1u : 0u);
           }
@@ -497,8 +507,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   } else if (warp >= 16) {
     // ------------------------------------------------------------ dQ drain: thread = query row
     asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
-    // warps 16-19 channels 0-63, warps 20-23 channels 64-127
-    const int quad = warp & 3, ch0 = (warp >= 20) * 64;
+    // warps 16-19 the first half of the channels, warps 20-23 the others (of 96: 64 and 32)
+    constexpr int kMine = kD > 64 ? 2 : 1;   // steps of 32 channels
+    const int quad = warp & 3, ch0 = (warp >= 20) * 32 * kMine;
     const uint32_t lane_base = uint32_t(quad * 32) << 16;
     bool ok = true;
     BwdItem itx{};
@@ -511,9 +522,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       tc_fence_after();
       // the warp's part goes to registers as a whole: dP of the next item waits for the columns
-      uint32_t reg[64];
-      tmem_ld32(tmem + lane_base + cdP + ch0, reg);
-      tmem_ld32(tmem + lane_base + cdP + ch0 + 32, reg + 32);
+      uint32_t reg[32 * kMine];
+#pragma unroll
+      for (int b = 0; b < kMine; ++b) tmem_ld32(tmem + lane_base + cdP + ch0 + 32 * b, reg + 32 * b);
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
@@ -524,7 +535,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       float* stage = sm.dq_stage[warp - 16];
       const int swizzle = cur.dq_dev == 0 ? lane & 7 : 0;
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
+      for (int b = 0; b < kMine; ++b) {
+        if (ch0 + 32 * b >= kD) break;
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // what this lane reduced before has left the buffer
         __syncwarp();
 #pragma unroll
@@ -622,11 +634,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (ok) {
         tc_fence_after();
         // lane = key row; warps 0-7 take dK, warps 8-15 dV, half of the channels each
-        const int ch = (hf & 1) * 64;
+        constexpr int kMine = kD > 64 ? 2 : 1;   // steps of 32 channels
+        const int ch = (hf & 1) * 32 * kMine;
         float* dst = ptrs.dkv[cta.dkv_dev] + ((size_t(cta.dkv_row + r) * 2 + (hf >> 1)) * hkv + kv_head) * kHeadDim + ch;
         const uint32_t acc = tmem + lane_base + (hf >> 1 ? cdV : cdK) + ch;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < kMine; ++c) {
+          if (ch + 32 * c >= kD) break;
           uint32_t reg[32];
           tmem_ld32(acc + 32 * c, reg);
           tmem_wait_ld();
@@ -663,7 +677,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (all_ok)
         for (int row = rank * 16 + warp; row < 256; row += parts * 16) {   // 0-127 dK, 128-255 dV; lane = 4 channels
           const int r = row & 127;
-          if (r >= cta.n_valid) continue;
+          if (r >= cta.n_valid || 4 * lane >= kD) continue;
           const uint32_t addr = smem_u32(share_of(sm, row) + (lane ^ (r & 7)) * 4);
           float4 sum = ld_cluster_f4(addr, 0);
           for (int p = 1; p < parts; ++p) {
@@ -680,7 +694,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 }
 
 static constexpr int kSms = 148, kMaxParts = 8;
-static int g_bwd_attr_set[2] = {0, 0};
+static int g_bwd_attr_set[4] = {0, 0, 0, 0};
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
 
 }  // namespace dcpk
@@ -696,17 +710,18 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
   return cudaMemcpyToSymbol(g_bwd_timeline, &p, sizeof(p)) == cudaSuccess ? 0 : -5;
 }
 
-// Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  n_items_total / n_mask_rows are the
+// Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  channels: of the arenas' 128, those that may be other
+// than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are the
 // lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
 // length of the longest item list (0: not known, the head groups stay whole).
 extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena,
                              long kv_rows, int hq, int hkv, const void* ctas, int n_ctas, const void* items,
                              int n_items_total, int max_items, const void* masks, int n_mask_rows, const float* lse, const float* delta,
-                             int stat_stride, float* const* dq_ptrs, float* const* dkv_ptrs, int n_dst, float scale,
+                             int stat_stride, float* const* dq_ptrs, float* const* dkv_ptrs, int n_dst, float scale, int channels,
                              const void* jobs, int n_jobs, void* const* job_src_ptrs, void* const* job_dst_ptrs,
                              int job_stat_stride, int* status, void* stream) {
   if (n_ctas <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
-  if (n_dst > kMaxPeers || hq % hkv != 0) return -3;
+  if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
   CUtensorMap tm_q, tm_do, tm_kv, tm_dq;
   if (encode_f32_tile_map(&tm_dq, dq_ptrs[0], uint64_t(q_rows), uint32_t(hq), kHeadDim, 32, 32)) return -1;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
@@ -721,8 +736,9 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   dcpk_fill_copy_ctx(&ctx, n_jobs > 0 ? job_src_ptrs : nullptr, n_jobs > 0 ? job_dst_ptrs : nullptr, job_stat_stride);
   const int smem = int(sizeof(BwdSmem));
   static_assert(sizeof(BwdSmem) <= 227 * 1024, "shared memory of one CTA");
-  const int v = g_bwd_timeline_host ? 1 : 0;
-  auto kernel = v ? attn_bwd_kernel<true> : attn_bwd_kernel<false>;
+  const int v = g_bwd_timeline_host ? 3 : channels > 96 ? 0 : channels > 64 ? 1 : 2;
+  auto kernel = v == 3 ? attn_bwd_kernel<true, 128> : v == 2 ? attn_bwd_kernel<false, 64>
+              : v == 1 ? attn_bwd_kernel<false, 96> : attn_bwd_kernel<false, 128>;
   if (!g_bwd_attr_set[v]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
     g_bwd_attr_set[v] = 1;

@@ -138,6 +138,10 @@ __device__ __forceinline__ void softmax_half(const uint32_t* s, uint64_t sl2_2, 
   tmem_st32(p_addr, preg);
 }
 
+// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and what S adds up over
+// zeros is left out.  PV stays as it is, so that the output's padding is written.  8192 queries x 16384 keys, 32 / 8 heads, against all 128
+// channels: 64 channels 1.43 -> 1.33 ms (causal 1.08 -> 1.04: the exponentials bound it then), 96 channels 1.51 -> 1.47 ms.
+template <int kD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const AttnTile* __restrict__ tiles, int n_tiles,
@@ -145,6 +149,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      int lse_stride_a, int lse_stride_b, int n_dst_a, int n_dst, int q_rows, int n_mask_rows,
                      int n_kv_subs, float scale, const CopyJob* __restrict__ jobs, int n_jobs,
                      const __grid_constant__ CopyCtx copy_ctx, int* __restrict__ status) {
+  constexpr int kHalves = kD > 64 ? 2 : 1;   // of 64 channels of Q and K
   extern __shared__ uint8_t smem_raw[];
   PairSmem& sm = *reinterpret_cast<PairSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -222,11 +227,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       auto load_slot = [&](bool with_k, bool with_v, int row, int kv_head) -> bool {
         if (!mbar_wait(&sm.kv_empty[slot], ph, abort_word)) return false;
         used |= 1 << slot;
-        if (X == 0) mbar_expect_tx(&sm.kv_full[slot], 2 * kKvBytes * (with_k + with_v));
+        if (X == 0) mbar_expect_tx(&sm.kv_full[slot], 2 * (kHalves * kKHalf * with_k + kKvBytes * with_v));
         if (with_v) tma_load_3d_pair(sm.v[slot], &tm_v, kv_bar + 8 * slot, 64 * X, hkv + head3, row3);
         if (with_k) {
           tma_load_3d_pair(sm.k[slot], &tm_k, kv_bar + 8 * slot, 0, kv_head, row + 64 * X);
-          tma_load_3d_pair(sm.k[slot] + kKHalf, &tm_k, kv_bar + 8 * slot, 64, kv_head, row + 64 * X);
+          if (kHalves > 1) tma_load_3d_pair(sm.k[slot] + kKHalf, &tm_k, kv_bar + 8 * slot, 64, kv_head, row + 64 * X);
         }
         if (++slot == kSlots) { slot = 0; ph ^= 1; }
         return true;
@@ -262,9 +267,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         ok = mbar_wait(&sm.q_empty[qi], qph, abort_word);
         if (!ok) break;
         used |= 1 << (kSlots + qi);
-        if (X == 0) mbar_expect_tx(&sm.q_full[qi], 4 * kQHalf);
+        if (X == 0) mbar_expect_tx(&sm.q_full[qi], 2 * kHalves * kQHalf);
         tma_load_3d_pair(sm.q[qi], &tm_q, q_bar + 8 * qi, 0, tile.head, tile.q_row + X * kTileM);
-        tma_load_3d_pair(sm.q[qi] + kQHalf, &tm_q, q_bar + 8 * qi, 64, tile.head, tile.q_row + X * kTileM);
+        if (kHalves > 1) tma_load_3d_pair(sm.q[qi] + kQHalf, &tm_q, q_bar + 8 * qi, 64, tile.head, tile.q_row + X * kTileM);
         if (++qi == 2) { qi = 0; qph ^= 1; }
         for (int j = 0; j < n && ok; ++j) {
           const int row = ahead;
@@ -329,7 +334,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       auto issue_qk = [&](int slot, int b) {
         const uint32_t q0 = q_lo + qi * kQStep, k0 = k_lo + slot * kKvStep, d = tmem + b * 128;
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < kD / 16; ++k)
           umma_ss_pair(d, desc(q0 + (k >> 2) * (kQHalf >> 4) + (k & 3) * 2), desc(k0 + (k >> 2) * (kKHalf >> 4) + (k & 3) * 2),
                        idesc_qk, k > 0 ? 1u : 0u);
         umma_commit_pair(&sm.s_full[b]);
@@ -617,7 +622,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, kStatusBarrierTimeout);
 }
 
-static int g_pair_attr_set = 0;
+static int g_pair_attr_set[3] = {0, 0, 0};
 
 }  // namespace dcpk
 
@@ -632,10 +637,10 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
                                   int hkv, const void* tiles, int n_tiles, const void* kv_entries, int n_kv_entries,
                                   const void* masks, int n_mask_rows, void* const* out_ptrs, float* const* lse_ptrs,
                                   int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a, int block_size,
-                                  float scale, const void* jobs, int n_jobs, void* const* job_src_ptrs,
+                                  float scale, int channels, const void* jobs, int n_jobs, void* const* job_src_ptrs,
                                   void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream) {
   if (n_tiles <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
-  if (n_dst > kMaxPeers || hq % hkv != 0) return -3;
+  if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
   CUtensorMap tm_q, tm_k, tm_v;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, 128)) return -1;
   if (encode_arena_map(&tm_k, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 64)) return -1;
@@ -648,12 +653,14 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
   CopyCtx ctx;
   dcpk_fill_copy_ctx(&ctx, n_jobs > 0 ? job_src_ptrs : nullptr, n_jobs > 0 ? job_dst_ptrs : nullptr, job_stat_stride);
   const int smem = int(sizeof(PairSmem)) + 1024;
-  if (!g_pair_attr_set) {
-    if (cudaFuncSetAttribute(attn_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  const int v = channels > 96 ? 0 : channels > 64 ? 1 : 2;
+  auto kernel = v == 2 ? attn_fwd_pair_kernel<64> : v == 1 ? attn_fwd_pair_kernel<96> : attn_fwd_pair_kernel<128>;
+  if (!g_pair_attr_set[v]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return -4;
-    g_pair_attr_set = 1;
+    g_pair_attr_set[v] = 1;
   }
-  attn_fwd_pair_kernel<<<2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+  kernel<<<2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream)>>>(
       tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
       static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, int(q_rows),
       n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);

@@ -224,7 +224,7 @@ def copy_jobs(jobs: torch.Tensor, ctx: CopyContext) -> None:
 def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, out_dsts, lse_dsts,
              scale: float, status: torch.Tensor, variant: int = 0, lse_stride: Optional[int] = None,
              lse_stride_b: Optional[int] = None, n_dst_a: Optional[int] = None, jobs: Optional[torch.Tensor] = None,
-             job_ctx: Optional[CopyContext] = None):
+             job_ctx: Optional[CopyContext] = None, channels: int = HEAD_DIM):
     """Run the forward kernel the tables were built for (``tables.tile_m``); ``variant`` only applies to
     the one-tile kernel (0: P in TMEM, 1: P through shared memory).  ``jobs`` (int32 [n, 4] on the
     device, see copy_jobs.cuh) is a list of peer -> local copies the two-tile kernel performs with
@@ -232,7 +232,8 @@ def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, o
 
     q_arena: bf16 [rows, hq, 128]; kv_arena: bf16 [rows, 2, hkv, 128]; out_dsts / lse_dsts: lists of
     destination arenas (tensors or raw device addresses; index 0 = this rank), every out arena
-    bf16 [rows_o, hq, 128] with its lse fp32 [hq, rows_o].
+    bf16 [rows_o, hq, 128] with its lse fp32 [hq, rows_o].  ``channels``: all channels of Q and K from there on are zero,
+    and the products need not go over them (the two-tile kernel makes use of it).
     """
     lib = _lib.load()
     assert q_arena.dtype == torch.bfloat16 and kv_arena.dtype == torch.bfloat16
@@ -250,7 +251,7 @@ def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, o
             ctypes.c_int(len(out_dsts)), ctypes.c_int(lse_stride),
             ctypes.c_int(lse_stride if lse_stride_b is None else lse_stride_b),
             ctypes.c_int(len(out_dsts) if n_dst_a is None else n_dst_a), ctypes.c_int(tables.block_size),
-            ctypes.c_float(scale), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
+            ctypes.c_float(scale), ctypes.c_int(channels), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
         _lib.check(rc, "dcpk_attn_fwd_pair")
         return
     assert jobs is None or jobs.shape[0] == 0, "only the two-tile forward kernel carries copy jobs"
@@ -482,11 +483,13 @@ def cut_cast_rows(pairs) -> None:
 
 
 def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts, dkv_dsts, scale: float,
-             status: torch.Tensor, jobs: Optional[torch.Tensor] = None, job_ctx: Optional[CopyContext] = None):
+             status: torch.Tensor, jobs: Optional[torch.Tensor] = None, job_ctx: Optional[CopyContext] = None,
+             channels: int = HEAD_DIM):
     """Run the backward kernel; dq_dsts/dkv_dsts are fp32 accumulators (zeroed by the caller),
     [rows, hq, 128] and [rows, 2, hkv, 128]; lse/delta are fp32 [hq, rows].  ``jobs`` / ``job_ctx``: copy
     jobs (the next stage's operands, see attn_fwd) that about sixteen CTAs of their own, the first of the grid,
-    perform meanwhile."""
+    perform meanwhile.  ``channels``: all channels of the operands from there on are zero, and the gradients' need not be
+    added to."""
     lib = _lib.load()
     hq, hkv = q_arena.shape[1], kv_arena.shape[2]
     assert q_arena.shape == do_arena.shape and lse.shape == delta.shape
@@ -497,7 +500,7 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
         ctypes.c_int(tables.max_items), _lib.ptr(tables.masks),
         ctypes.c_int(tables.masks.shape[0]), _lib.ptr(lse), _lib.ptr(delta),
         ctypes.c_int(lse.shape[1]), _ptr_array(dq_dsts), _ptr_array(dkv_dsts), ctypes.c_int(len(dq_dsts)),
-        ctypes.c_float(scale), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
+        ctypes.c_float(scale), ctypes.c_int(channels), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
     _lib.check(rc, "dcpk_attn_bwd")
 
 

@@ -36,11 +36,13 @@ HEAD_DIM = 128
 class FusedAttentionExecutor:
     def __init__(self, heads_q: int, heads_kv: int, max_q_rows: int, max_kv_rows: int, max_part_rows: int,
                  device: torch.device, group=None, softmax_scale: Optional[float] = None, timeout_s: float = 10.0,
-                 variant: int = 0):
+                 variant: int = 0, channels: int = HEAD_DIM):
+        """``channels``: every head's channels from there on are zero in all operands (a smaller head dimension in the
+        arenas' rows of 128)."""
         self.hq, self.hkv = heads_q, heads_kv
         self.device = device
         self.scale = softmax_scale if softmax_scale is not None else HEAD_DIM ** -0.5
-        self.variant = variant
+        self.variant, self.channels = variant, channels
         self.group, self.timeout_s = group, timeout_s
         self.arena = None
         self.n_reallocations = 0
@@ -297,7 +299,7 @@ class FusedAttentionExecutor:
         # `jobs`: the next stage's operand fetch, carried by this kernel
         attn_ops.attn_fwd(q, kv, t, out_dsts, lse_dsts, self.scale, a_status(self), self.variant,
                           lse_stride=self.cap[2], lse_stride_b=lse_rows, n_dst_a=self.world, jobs=jobs,
-                          job_ctx=self.copy_ctx)
+                          job_ctx=self.copy_ctx, channels=self.channels)
         self.kernel_launches += 1
 
     # ---- backward
@@ -339,7 +341,7 @@ class FusedAttentionExecutor:
                 self._fetch_standalone(nxt)
                 continue
             attn_ops.attn_bwd(q, dout, kv, lse, delta, t, [self.dq], [self.dkv], self.scale,
-                              a_status(self), jobs=nxt, job_ctx=self.copy_ctx)
+                              a_status(self), jobs=nxt, job_ctx=self.copy_ctx, channels=self.channels)
             self.kernel_launches += 1
         self._mark("bwd:kernels (with operand fetch)")
         if self.world > 1:

@@ -127,7 +127,8 @@ class FusedPlanExecutor:
         device = device or torch.device("cuda", torch.cuda.current_device())
         rq, rkv, rp = self.program.need_all
         self.impl = FusedAttentionExecutor(self.program.heads_q, self.program.heads_kv, rq, rkv, max(rp, 128), device,
-                                           process_group if exec_context.n_devices > 1 else None, softmax_scale)
+                                           process_group if exec_context.n_devices > 1 else None, softmax_scale,
+                                           channels=head_dim)
         self.impl.synchronous = self.impl.synchronous or synchronous
         self.impl.prepare(self.program)
         self.fw_plan, self.bw_plan, self.fw_workload, self.bw_workload = fw_exec_plan, bw_exec_plan, fw_workload, bw_workload

@@ -344,6 +344,42 @@ def test_attention_backward_into_a_second_accumulator(dev):
     assert first[other | (tile == 2)].abs().max() == 0 and second[~other].abs().max() == 0
 
 
+@pytest.mark.parametrize("d", [8, 40, 64, 72, 96, 104])
+@pytest.mark.parametrize("nq,nkv,heads", [(130, 300, (4, 2)), (600, 520, (16, 2))])   # head groups whole; split over clusters
+def test_attention_over_fewer_channels(dev, d, nq, nkv, heads):
+    """Products that leave the zeros of padded heads out, against products over all 128 channels of the same arenas: the
+    terms left out are exact zeros, so S, P and the output agree to the bit; the gradients are sums of the same terms
+    that the accumulators take in any order (float32, at most 600 of them: 600 x 2^-24 of the largest partial sum)."""
+    hq, hkv = heads
+    torch.manual_seed(0)
+    q = torch.zeros(nq + 128, hq, 128, device=dev, dtype=torch.bfloat16)
+    kv = torch.zeros(nkv + 128, 2, hkv, 128, device=dev, dtype=torch.bfloat16)
+    dout = torch.zeros_like(q)
+    q[:nq, :, :d], kv[:nkv, ..., :d], dout[:nq, :, :d] = (torch.randn(n, *h, d, device=dev).bfloat16() for n, h in
+                                                          ((nq, (hq,)), (nkv, (2, hkv)), (nq, (hq,))))
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    rng = np.zeros((nq, 4), dtype=np.int32)
+    rng[:, 1] = np.minimum(np.arange(nq) + 33, nkv)
+    rng[5:9] = 0
+    row = A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)
+    ft, bt = A.build_fwd_tables([row], 1024, dev), A.build_bwd_tables([row], 1024, hq, hkv, dev)
+    res = []
+    for channels in (128, d):
+        out, lse, delta = torch.full_like(q, 7), torch.zeros(hq, nq + 128, device=dev), torch.zeros(hq, nq + 128, device=dev)
+        A.attn_fwd(q, kv, ft, [out], [lse], d ** -0.5, status, channels=channels)
+        out = out[:nq]
+        A.attn_delta(out, dout, delta, 0, nq)
+        dq, dkv = torch.zeros(nq + 128, hq, 128, device=dev), torch.zeros(nkv + 128, 2, hkv, 128, device=dev)
+        A.attn_bwd(q, dout, kv, lse, delta, bt, [dq], [dkv], d ** -0.5, status, channels=channels)
+        torch.cuda.synchronize()
+        assert status.item() == 0
+        res.append((out, lse, dq, dkv))
+    (out, lse, dq, dkv), (out_d, lse_d, dq_d, dkv_d) = res
+    assert torch.equal(out, out_d) and torch.equal(lse, lse_d) and dq.abs().max() > 0.1 and dkv.abs().max() > 0.1
+    assert (dq - dq_d).abs().max() <= 600 * 2.0 ** -24 * dq.abs().max()
+    assert (dkv - dkv_d).abs().max() <= 600 * 2.0 ** -24 * dkv.abs().max()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("d", [8, 96, 128])
 def test_row_conversions(dev, dtype, d):
