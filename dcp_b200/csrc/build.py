@@ -1,6 +1,7 @@
-"""In-tree native build: CUDA kernels (sm_100a) -> dcp_b200/_kernels.so, C++ planner -> dcp_b200/_planner*.so.
+"""In-tree native build: CUDA kernels (sm_100a) -> dcp_b200/_kernels.so, C++ planner -> dcp_b200/_planner*.so, host
+side of single-rank attention calls -> dcp_b200/_calls*.so.
 
-Both libraries are built with plain nvcc / g++ command lines (no JIT cache), so the
+The libraries are built with plain nvcc / g++ command lines (no JIT cache), so the
 resulting shared objects sit next to the Python sources and travel with the tree.
 Run as ``python -m dcp_b200.csrc.build`` or through ``__graft_entry__.build()``.
 """
@@ -18,6 +19,7 @@ HERE = Path(__file__).resolve().parent
 PKG = HERE.parent
 KERNEL_DIR = HERE / "kernels"
 PLANNER_DIR = HERE / "planner"
+HOST_DIR = HERE / "host"
 OBJ_DIR = HERE / "build"
 
 NVCC_FLAGS = [
@@ -109,10 +111,35 @@ def build_planner(force: bool = False) -> Path:
     return out
 
 
+def calls_lib_path() -> Path:
+    return PKG / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_calls(force: bool = False) -> Path:
+    """Links to the kernel library next to it, which has to be there."""
+    import torch
+
+    OBJ_DIR.mkdir(exist_ok=True)
+    srcs = sorted(HOST_DIR.glob("*.cpp"))
+    out = calls_lib_path()
+    stamp = OBJ_DIR / "calls.stamp"
+    digest = _digest(srcs + [KERNEL_DIR / "entries.h"]) + " " + torch.__version__
+    if not force and out.exists() and stamp.exists() and stamp.read_text() == digest:
+        return out
+    pt = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent / "include" if os.path.isabs(_nvcc()) else Path("/usr/local/cuda/include")
+    inc = [pt / "include", pt / "include/torch/csrc/api/include", sysconfig.get_paths()["include"], cuda, KERNEL_DIR]
+    _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+          "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, *["-I%s" % i for i in inc], *map(str, srcs),
+          "-o", str(out), "-L%s" % PKG, "-l:" + kernels_lib_path().name, "-Wl,-rpath,$ORIGIN", "-L%s" % (pt / "lib"),
+          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-ldl"])
+    stamp.write_text(digest)
+    return out
+
+
 def build_all(force: bool = False, verbose: bool = False):
-    return build_kernels(force, verbose), build_planner(force)
+    return build_kernels(force, verbose), build_planner(force), build_calls(force)
 
 
 if __name__ == "__main__":
-    k, p = build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print("built", k, p)
+    print("built", *build_all(force="--force" in sys.argv, verbose="-v" in sys.argv))

@@ -60,6 +60,7 @@
 
 #include "attn_common.cuh"
 #include "copy_jobs.cuh"
+#include "entries.h"
 #include "ptx.cuh"
 #include "tmap.cuh"
 

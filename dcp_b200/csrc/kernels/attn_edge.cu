@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
+
 namespace dcpk {
 
 static constexpr int kEdgeHeadDim = 128;

@@ -48,6 +48,22 @@ def stream_handle():
 LAUNCHES = 0  # kernel-entry calls made through this library since import (each launches >= 1 kernel)
 
 
+def calls():
+    """The native host side of single-rank attention calls (``csrc/host/calls.cpp``)."""
+    load()
+    try:
+        from .. import _calls
+    except ImportError as e:
+        raise RuntimeError("dcp_b200/_calls is missing: build it with `python -m dcp_b200.csrc.build`") from e
+    return _calls
+
+
+def count(n: int):
+    """``n`` kernel entries were called by native code."""
+    global LAUNCHES
+    LAUNCHES += n
+
+
 def check(rc: int, what: str):
     global LAUNCHES
     LAUNCHES += 1

@@ -25,6 +25,7 @@ from typing import Optional
 import numpy as np
 import torch
 
+from ..ops import _lib
 from ..ops import attention as attn_ops
 from ..ops import block_ops
 from ..planner.lowering import FusedProgram
@@ -45,6 +46,7 @@ class FusedAttentionExecutor:
         self.variant, self.channels = variant, channels
         self.group, self.timeout_s = group, timeout_s
         self.arena = None
+        self._native = None           # host side of this program's calls in native code (single rank)
         self.n_reallocations = 0
         self._allocate((max_q_rows, max_kv_rows, max_part_rows))
         self.program: Optional[FusedProgram] = None
@@ -85,6 +87,7 @@ class FusedAttentionExecutor:
             "part_out": ((rp, hq, HEAD_DIM), bf), "part_lse": ((hq, rp), f32),
             "dq": ((rq, hq, HEAD_DIM), f32), "dkv": ((rkv, 2, hkv, HEAD_DIM), f32),
         }
+        self._native = None           # it holds the arenas
         if self.arena is not None:
             torch.cuda.synchronize(self.device)
             for name in regions:
@@ -140,6 +143,29 @@ class FusedAttentionExecutor:
         self.dq_push, self.dkv_push = up(program.dq_push), up(program.dkv_push)
         self._host_keep = keep
         self._staging_valid = False
+        self._native = self._native_calls()
+
+    def _native_calls(self):
+        """Calls of one launch each way, one rank's whole work: no stages, merges or peers in between."""
+        p = self.program
+        f, b = self.fwd_tabs, self.bwd_tabs
+        if self.world > 1 or p.n_stages != 1 or self.merge_ops.shape[0] or f[0] is None or f[0].tile_m != attn_ops.TILE_M_PAIR:
+            return None
+        f, b = f[0], b[0] if len(b) else None
+        d = {"q": self.q, "kv": self.kv, "dout": self.dout, "out": self.out, "lse": self.lse, "dq": self.dq, "dkv": self.dkv,
+             "part_out": self.part_out, "part_lse": self.part_lse, "status": self.arena.status, "tiles": f.tiles,
+             "kv_entries": f.kv_entries, "fwd_masks": f.masks, "n_tiles": f.n_tiles, "block_size": f.block_size,
+             "q_local_rows": p.q_local_rows, "kv_local_rows": p.kv_local_rows, "q_rows": p.q_rows, "kv_rows": p.kv_rows,
+             "all_rows_written": self._all_rows_written, "channels": self.channels}
+        if b is not None:
+            d.update(ctas=b.ctas, items=b.items, bwd_masks=b.masks, n_ctas=b.n_ctas, max_items=b.max_items)
+        return _lib.calls().SingleRankAttention(d)
+
+    def native(self):
+        """The native calls of the program, None where there are none or a debugging aid wants to see the phases."""
+        if self.profile or self.poison or self.synchronous or self.time_calls or self.check_reductions:
+            return None
+        return self._native
 
     # ---- views the model writes into / reads from
     def q_local(self) -> torch.Tensor:
@@ -259,6 +285,12 @@ class FusedAttentionExecutor:
         own = out is None
         if own:
             out, lse = self.out, self.lse
+        native = self.native()
+        if native is not None and native.forward_into(q, kv, out, lse, self.scale):
+            _lib.count(1)
+            self.kernel_launches += 1
+            self._staging_valid = True
+            return (self.out_local(), self.lse_local()) if own else (out, lse)
         p, a = self.program, self.arena
         tok = self._call_begin("fwd")
         self._mark("fwd:start")
@@ -311,6 +343,13 @@ class FusedAttentionExecutor:
         p, a = self.program, self.arena
         assert self.world == 1 or (q is None and kv is None and out is None), "peers read the arenas"
         n = p.q_local_rows
+        native = self.native()
+        if native is not None and native.backward_from(
+                dout_local, self.q if q is None else q, self.kv if kv is None else kv, self.out if out is None else out,
+                self.lse if out is None else lse, self.delta if out is None else None, self.scale):
+            _lib.count(2)
+            self.kernel_launches += 2
+            return self.dq[:n], self.dkv[:p.kv_local_rows]
         tok = self._call_begin("bwd")
         self._mark("bwd:start")
         if self.poison and not self._staging_valid:

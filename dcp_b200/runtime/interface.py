@@ -17,6 +17,7 @@ import torch
 from ..core.blocks import Device, WorkloadSpec
 from ..core.common import ExecutionContext
 from ..core.instructions import BufferType, ExecutionPlan
+from ..ops import _lib
 from ..ops import attention as attn_ops
 from ..planner import masks
 from ..planner.compiler import CompilerConfig, InstrCompiler
@@ -230,6 +231,19 @@ class FusedPlanExecutor:
         if ex.world > 1:
             out, lse = self.forward(q, kv)
             return out.clone(), lse.clone(), self._epoch
+        native = ex.native()
+        if native is not None:
+            whole = self.head_dim == 128 and q.dtype == torch.bfloat16
+            if not whole:
+                ex.inputs_written()       # before the arenas take this call's operands
+            res = native.forward(q, kv, self.head_dim, ex.scale)
+            if res is not None:
+                out, lse, entries = res
+                _lib.count(entries)
+                ex.kernel_launches += 1
+                ex._staging_valid = True
+                self._epoch = -1 if whole else ex.arena_epoch
+                return out, lse, self._epoch
         qk, kvk = self._as_kernel_rows(q), self._as_kernel_rows(kv, True)
         out, lse = ex.new_results()
         if self._in_place(qk, kvk):
@@ -249,6 +263,20 @@ class FusedPlanExecutor:
                 self._epoch = -1
             dq, dkv = self.backward(q, kv, out, dout.contiguous(), lse)
             return dq.clone(), dkv.clone()
+        native = ex.native()
+        if native is not None:
+            reload = token != ex.arena_epoch or not ex._staging_valid   # another call's operands took the arenas meanwhile
+            whole = self.head_dim == 128 and q.dtype == torch.bfloat16
+            if reload and not whole:
+                ex.inputs_written()
+            res = native.backward(q, kv, out, dout, lse, self.head_dim, reload, ex.scale)
+            if res is not None:
+                dq, dkv, entries = res
+                _lib.count(entries)
+                ex.kernel_launches += 2
+                if reload and not whole:
+                    self._epoch = ex.arena_epoch
+                return dq, dkv
         qk, kvk = self._as_kernel_rows(q), self._as_kernel_rows(kv, True)
         ok, dok = self._as_kernel_rows(out), self._as_kernel_rows(dout)
         lse = lse.reshape(ex.hq, ex.program.q_local_rows).to(ok.device, torch.float32).contiguous()

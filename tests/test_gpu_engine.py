@@ -397,3 +397,49 @@ def test_dcp_attention_reads_any_layout_and_keeps_calls_apart(head_dim, dtype):
         mine, other = call(q, kv), call(*second)
         same(grads(*mine, do), alone)
         same(grads(*other, torch.ones_like(ldo)), alone2)
+
+
+@pytest.mark.parametrize("head_dim,dtype,kv_dtype", [(128, torch.bfloat16, None), (128, torch.float16, None), (72, torch.bfloat16, None),
+                                                     (64, torch.float32, None), (128, torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("form", ["rows", "flat", "strided", "halves"])
+def test_native_calls_against_the_general_path(head_dim, dtype, kv_dtype, form):
+    """The same call with its host side in native code and in Python: same output bits, types and shapes, and gradients
+    that differ by the order of fp32 sums only (1e-5 of the largest, and one rounding of the result type).  Forms that the
+    native code does not take go the general way from inside the call; a wrong number of elements is refused by both."""
+    _need_gpu()
+    from dcp_b200.core.common import get_default_execution_context
+    from dcp_b200.ops import _lib
+    from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test
+    dev = torch.device("cuda", 0)
+    ex, lq, lkv, ldo, *_ = prepare_dcp_distributed_attn_for_test([300, 129], 4, 2, head_dim, 256, 4, get_default_execution_context(1, 1),
+                                                                 0, "causal", dtype, 3, device=dev, executor_impl="fused")
+    lkv = lkv.to(kv_dtype or dtype)
+    native = ex.impl.native()
+    assert native is not None
+    how = {"rows": lambda t: t, "flat": lambda t: t.flatten(1), "strided": lambda t: torch.stack([t, t], -1)[..., 0],
+           "halves": lambda t: t.flatten(0, 1).view(2, -1)}[form]
+
+    def call(with_native):
+        ex.impl._native = native if with_native else None
+        before, launches = _lib.LAUNCHES, ex.impl.kernel_launches
+        q, kv = how(lq.clone()).requires_grad_(True), how(lkv.clone()).requires_grad_(True)
+        out = DCPAttention.apply(ex, False, False, q, kv)
+        grads = torch.autograd.grad(out, (q, kv), ldo.to(out.dtype).view(out.shape))
+        torch.cuda.synchronize()
+        ex.impl.check_status()
+        assert grads[0].shape == q.shape and grads[1].shape == kv.shape
+        return (out.detach(), *grads), (_lib.LAUNCHES - before, ex.impl.kernel_launches - launches)
+
+    (got, counted), (want, counted_too) = call(True), call(False)
+    assert counted == counted_too and all(a.dtype == b.dtype and a.shape == b.shape for a, b in zip(got, want))
+    assert torch.equal(got[0], want[0])
+    for a, b in zip(got[1:], want[1:]):
+        ulp = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}.get(a.dtype, 0.0)
+        assert ((a.float() - b.float()).abs() <= ulp * b.float().abs() + 1e-5 * b.float().abs().max()).all()
+    for with_native in (True, False):
+        ex.impl._native = native if with_native else None
+        with pytest.raises(RuntimeError):
+            DCPAttention.apply(ex, False, False, lq[:-1], lkv)
+    ex.impl._native = native
+    ex.impl.time_calls = True        # the phases are looked at: the general path
+    assert ex.impl.native() is None
