@@ -2,12 +2,13 @@
 //
 // A pair of CTAs (a cluster of two, cta_group::2) takes one 256-row tile after another; the even CTA has query rows
 // 0-127 (tile A), the odd one 128-255 (tile B).  Warps of a CTA:
-//   0-3, 4-7  softmax of every second KV tile (one thread per query row), each half of the channels in the epilogue,
+//   0-3, 4-7  softmax of every second KV tile (one thread per query row),
 //   8         TMA producer: this CTA's Q rows and its halves of the K and V tiles,
 //   9         UMMA issuer (even CTA only: a product covers both CTAs' rows),
 //   10-11     fetch the next plan stage's remote operands (copy jobs: peer loads over NVLink into this
-//             GPU's staging rows, see copy_jobs.cuh) while the tiles are computed.
-// All four non-softmax warps donate registers (setmaxnreg).
+//             GPU's staging rows, see copy_jobs.cuh) while the tiles are computed,
+//   12-15     epilogue: O out of TMEM, divided by the row sums, stored.
+// All non-softmax warps donate registers (setmaxnreg).
 //   S(j) = Q K(j)^T   M = 256, each CTA holds 64 of the 128 keys             -> TMEM
 //   O   += P(j) V(j)  P as packed bf16 in the TMEM columns S(j) came from, each CTA holds 64 of the channels
 // TMEM (512 columns): three score buffers [0,384), O [384,512).  Per KV tile j the issuer emits PV(j), QK(j+3), also
@@ -35,12 +36,14 @@
 // What bounds it: the issuing thread and the softmax warps that share its scheduler.  Where both are in time a KV tile takes
 // 1250 cycles per CTA; the exponentials need 1024 of them and the products 1024.  Every look at a barrier costs the issuer
 // 200 cycles, so it asks for its three at once, and K(j+3) and V(j), which one step consumes, share a barrier.  Between
-// two tiles of a pair: the last product, the sums of the two warpgroups, O out of TMEM, about 4000 cycles; as a launch
-// with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
+// two tiles of a pair the epilogue has warps of its own: the softmax warps leave sums and references in shared memory and go on
+// with the next tile's scores, whose first product waits until O is in registers.  (With the epilogue in the softmax warps the
+// tensor core was idle for about 4000 cycles between two tiles: 16 heads, 16384 queries over 256 / 512 keys 110 -> 81 / 139
+// -> 107 us, causal 2048 x 2048 66.6 -> 62.5, 4096 x 4096 167 -> 159 us, sink + window 531 -> 514 us in long runs; full 8192 x
+// 16384 1.535 -> 1.542 ms.)  As a launch with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
 // Measured against two query tiles per CTA (32 / 8 heads, queries x keys; one box): full 8192 x 16384 1.71 -> 1.57 ms
 // (1283 -> 1404 TFLOP/s), causal 1.29 -> 1.17 ms (1397), sink + window 0.568 -> 0.505 ms, causal 4096 x 4096 0.163 ->
-// 0.153 ms; in long runs under the power cap full 2.01 -> 1.74 ms.  Slower where the tiles are many and short: causal
-// 2048 x 2048 0.059 -> 0.061 ms.  Tried and left: a pair per tile instead of persistent pairs (4096 x 4096 0.159 ms, 16384
+// 0.153 ms; in long runs under the power cap full 2.01 -> 1.74 ms (all with the epilogue in the softmax warps).  Tried and left: a pair per tile instead of persistent pairs (4096 x 4096 0.159 ms, 16384
 // tokens in sequences of 8192 6 % slower); the result written after the next tile's first exponentials (the longer loop
 // costs more than it hides: 1.57 -> 1.66 ms); the maximum taken beside the exponentials (1.75 ms).
 //
@@ -62,7 +65,7 @@
 
 namespace dcpk {
 
-static constexpr int kPairThreads = 384;  // 8 softmax warps + producer + UMMA issuer + 2 fetch warps (all four donate registers)
+static constexpr int kPairThreads = 512;  // 8 softmax warps, producer, UMMA issuer, 2 fetch warps, 4 epilogue warps
 static constexpr int kPairs = 148 / 2;    // one CTA per SM
 static constexpr int kSlots = 4;          // slot i holds this CTA's halves of K(i) and V(i-3): what one step of the issuer consumes
 static constexpr int kSBufs = 3;
@@ -74,10 +77,13 @@ static constexpr int kInfos = 4;
 static constexpr float kGap = 8.f;            // exponent (base 2) by which a score may exceed a reference that can still move
 static constexpr float kMaxSum = 1.8447e19f;  // 2^64: a row sum above it sends the tile through the second pass
 
-// What the softmax warps of a CTA need of a tile, put into shared memory by the TMA producer, which is some KV tiles
-// ahead of them: from the tables it would take three dependent trips to memory between two tiles.
+// What the softmax and epilogue warps of a CTA need of a tile, put into shared memory by the TMA producer, which is some
+// KV tiles ahead of them: from the tables it would take three dependent trips to memory between two tiles.  And what
+// they leave for one another.
 struct __align__(16) TileInfo {
   int4 mask[kTileM];        // ranges of this CTA's rows
+  float m[kTileM];          // reference of a row
+  float l[2][kTileM];       // its sums over the KV tiles of either warpgroup
   int4 first[2];            // first KV tiles
   __nv_bfloat16* out;       // where the first row goes
   float* lse;
@@ -88,15 +94,13 @@ struct __align__(1024) PairSmem {
   uint8_t q[2][2 * kQHalf];
   uint8_t k[kSlots][kKvBytes];      // 64 of the 128 keys, all channels
   uint8_t v[kSlots][kKvBytes];      // all 128 keys, 64 of the channels
-  uint8_t o_stage[8][32 * 64];      // per softmax warp: 32 rows x 32 channels on their way out
+  uint8_t o_stage[4][32 * 64];      // per epilogue warp: 32 rows x 32 channels on their way out
   TileInfo info[kInfos];
-  float m[kTileM];                  // reference of a row
-  float l[2][2][kTileM];            // its sums over the KV tiles of either warpgroup, of two tiles in turn
   uint32_t redo[kRedoWords];        // rounds that go through the second pass
   // of the even CTA (bytes and arrivals of both CTAs): q_full, kv_full, p_ready, o_empty; the others are signalled in
   // both
   uint64_t q_full[2], q_empty[2], kv_full[kSlots], kv_empty[kSlots], s_full[kSBufs], p_ready[kSBufs][2], o_empty, acc_full,
-      m_ready[4], l_ready[4], info_full[kInfos], info_empty[kInfos];
+      m_ready[kInfos][4], l_ready[kInfos][4], info_full[kInfos], info_empty[kInfos];
   uint32_t tmem_base;
   int abort_word;
   int any_redo;
@@ -115,10 +119,10 @@ __device__ __forceinline__ void for_each_barrier(PairSmem& sm, F f) {   // f(bar
   for (int i = 0; i < 2; ++i) { f(&sm.q_full[i], 1); f(&sm.q_empty[i], 1); }
   for (int i = 0; i < kSlots; ++i) { f(&sm.kv_full[i], 1); f(&sm.kv_empty[i], 1); }
   for (int i = 0; i < kSBufs; ++i) { f(&sm.s_full[i], 1); f(&sm.p_ready[i][0], 8); f(&sm.p_ready[i][1], 8); }   // four warps of either CTA
-  f(&sm.o_empty, 16);   // eight warps of either CTA
+  f(&sm.o_empty, 8);   // four warps of either CTA
   f(&sm.acc_full, 1);
-  for (int i = 0; i < 4; ++i) { f(&sm.m_ready[i], 1); f(&sm.l_ready[i], 2); }
-  for (int i = 0; i < kInfos; ++i) { f(&sm.info_full[i], 1); f(&sm.info_empty[i], 8); }
+  for (int i = 0; i < 4 * kInfos; ++i) { f(&sm.m_ready[i >> 2][i & 3], 1); f(&sm.l_ready[i >> 2][i & 3], 2); }
+  for (int i = 0; i < kInfos; ++i) { f(&sm.info_full[i], 1); f(&sm.info_empty[i], 12); }   // softmax and epilogue warps
 }
 
 // P = exp2(S * c - m) of 64 keys of a row, cut to bf16, to TMEM; `ps2` collects the row sum.  Packed fp32: one
@@ -211,11 +215,95 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     return true;
   };
 
-  // register rebalancing between warpgroups (setmaxnreg inside each role's branch): the four
-  // non-softmax warps give registers up, the softmax warps take them
-  // (256 x 216 + 128 x 72 = 64512 = 384 x 168, what the block is launched with)
-  if (warp >= 8) {
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  // register rebalancing between warpgroups (setmaxnreg inside each role's branch): the others give registers up, the
+  // softmax warps take them (256 x 200 + 128 x 64 + 128 x 48 = 65536 = 512 x 128, what the block is
+  // launched with)
+  if (warp >= 12) {
+    // ------------------------------------------------------------ epilogue: thread = query row
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    const int quad = warp & 3, r = threadIdx.x & 127;
+    const uint32_t o_addr = tmem + (uint32_t(quad * 32) << 16) + kSBufs * 128;
+    const uint32_t o_bar = cluster_addr(smem_u32(&sm.o_empty), 0);
+    uint8_t* stage = sm.o_stage[warp - 12];
+   for (int pass = 0;; ++pass) {
+    // O is in registers: the products of the tile in slot `info` may set it; false: there is no such tile
+    auto hand_over = [&](int info, int iph) -> bool {
+      const TileInfo& ti = sm.info[info];
+      if (!__all_sync(0xffffffffu, mbar_wait(&sm.info_full[info], iph, abort_word)) || ti.n_kv < 0) return false;
+      if (ti.n_kv > 0) {
+        if (!((ti.first[0].w >> X) & 1)) {   // then no product sets O of this query tile, they only add to it
+          uint32_t zero[32];
+#pragma unroll
+          for (int c = 0; c < 32; ++c) zero[c] = 0;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) tmem_st32(o_addr + c * 32, zero);
+          tmem_wait_st();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(o_bar);
+      }
+      return true;
+    };
+    int acc_ph = 0;  // parity of the tiles with a product so far
+    bool more = hand_over(0, 0);
+    for (int info = 0, iph = 0; more;) {
+      const TileInfo& ti = sm.info[info];
+      const int n = ti.n_kv, n_rows = ti.n_rows;
+      const int next = info + 1 == kInfos ? 0 : info + 1, next_ph = next == 0 ? iph ^ 1 : iph;
+      bool ok = mbar_wait(&sm.l_ready[info][quad], iph, abort_word);
+      const float l_sum = ti.l[0][r] + ti.l[1][r];
+      if (pass == 0 && __any_sync(0xffffffffu, r < n_rows && !(l_sum < kMaxSum)) && lane == 0) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
+          or_cluster_u32(smem_u32(&sm.redo[(ti.round >> 5) & (kRedoWords - 1)]), c, 1u << (ti.round & 31));
+        }
+      }
+      const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
+      if (ok && r < n_rows) ti.lse[r] = l_sum > 0.f ? ti.m[r] * scale + logf(l_sum) - kTruncLn : -INFINITY;
+      __nv_bfloat16* out = ti.out + size_t(quad * 32 + (lane >> 2)) * hq * kHeadDim + (lane & 3) * 8;
+      if (n > 0) {
+        ok = ok && mbar_wait(&sm.acc_full, acc_ph, abort_word);
+        acc_ph ^= 1;
+        tc_fence_after();
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {   // 32 channels: four 16-byte pieces per row, swizzled, out with four lanes per row
+        uint32_t oreg[32];
+        if (n > 0) {  // warp-uniform: the TMEM load is a warp-collective instruction
+          tmem_ld32(o_addr + c * 32, oreg);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) oreg[i] = 0;
+        }
+        if (c == 3) more = hand_over(next, next_ph);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t packed[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            packed[k] = pack_bf16x2(__uint_as_float(oreg[8 * i + 2 * k]) * inv_l, __uint_as_float(oreg[8 * i + 2 * k + 1]) * inv_l);
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = 8 * i + (lane >> 2);
+          const uint4 piece = *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4));
+          if (quad * 32 + row < n_rows) *reinterpret_cast<uint4*>(out + size_t(8 * i) * hq * kHeadDim + c * 32) = piece;
+        }
+        __syncwarp();
+      }
+      if (lane == 0) mbar_arrive(&sm.info_empty[info]);
+      info = next; iph = next_ph;
+    }
+    if (!next_pass(pass)) break;
+   }
+  } else if (warp >= 8) {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
    if (warp == 8) {
     // ------------------------------------------------------------ TMA producer: this CTA's rows and halves
    for (int pass = 0;; ++pass) {
@@ -363,7 +451,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const uint32_t hold_a = (flags & 1) - 1u, hold_b = ((flags >> 1) & 1) - 1u;   // all ones: the query tile sees none of the keys
           if (j + 1 < n) flags = subs[j + 1].w;
           if (!kv_there) ok = mbar_wait(&sm.kv_full[slot], ph, abort_word);
-          if (ok && j == 0 && n_tiles_done > 0) ok = mbar_wait(&sm.o_empty, (n_tiles_done - 1) & 1, abort_word);   // the last result is in registers
+          if (ok && j == 0) ok = mbar_wait(&sm.o_empty, n_tiles_done & 1, abort_word);   // the last result is in registers
           const uint32_t v0 = v_lo + slot * kKvStep, a = tmem + b * 128;
 #pragma unroll
           for (int h = 0; h < 2 && ok; ++h) {   // O += P V: the first 64 keys while the softmax warps still work on the others
@@ -393,8 +481,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // TMEM and operands stay until all has retired
       if (!ok) { umma_commit_pair(&sm.acc_full); ++n_tiles_done; }
       for (int spin = 0; spin < 200000 && n_tiles_done > 0 && !mbar_try_wait(&sm.acc_full, (n_tiles_done - 1) & 1); ++spin) {}
-      // ... and no arrival from the other CTA is on its way any more
-      if (ok && n_tiles_done > 0) mbar_wait(&sm.o_empty, (n_tiles_done - 1) & 1, abort_word);
     }
     __syncwarp();
     if (!next_pass(pass)) break;
@@ -406,8 +492,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (next_pass(0)) next_pass(1);
    }
   } else {
-    // ------------------------------------------------------------ softmax of every second KV tile, epilogue of half the channels
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    // ------------------------------------------------------------ softmax of every second KV tile
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     const int wg = warp >> 2, quad = warp & 3, r = threadIdx.x & 127;
     const uint32_t lane_base = uint32_t(quad * 32) << 16;
     const uint32_t o_addr = tmem + lane_base + kSBufs * 128;
@@ -417,11 +503,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     bool ok = true, ready = false;
     int b = wg, bph = 0;       // buffer of this warpgroup's next KV tile, counted over all tiles
     int g0 = 0;                // KV tiles before this tile
-    int published = 0;         // references handed on before this tile
-    int acc_ph = 0, turn = 0;  // parities of the tiles with a product and of all tiles so far
+    uint32_t published = 0;    // parities of the references handed on so far through either slot of `info`
     for (int info = 0, iph = 0;;) {
       // ---- next tile
-      const TileInfo& ti = sm.info[info];
+      TileInfo& ti = sm.info[info];
+      const uint32_t pub = published >> info;
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&sm.info_full[info], iph, abort_word));
       if (!ok || ti.n_kv < 0) break;
       const int n = ti.n_kv;
@@ -433,14 +519,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       float m_ref = sees ? -INFINITY : 0.f, l_run = 0.f;   // the row's reference, as far as this warpgroup knows; its own sum
       bool exchange = pass > 0 || __any_sync(0xffffffffu, m_ref == -INFINITY);
       int n_pub = exchange ? n : 0;
-      if (n > 0 && !((ti.first[0].w >> X) & 1)) {   // then no product sets O of this one; this warpgroup's channels here
-        uint32_t zero[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) zero[c] = 0;
-        tmem_st32(o_addr + wg * 64, zero);
-        tmem_st32(o_addr + wg * 64 + 32, zero);
-        tmem_wait_st();
-      }
       for (int j = first; j < n; j += 2) {
         const int4 sub = ahead;
         if (j + 2 < n) ahead = subs[j + 2];
@@ -472,9 +550,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           // what the warp that has the previous tile left behind
           float m_cur = m_ref;
           if (j > 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&sm.m_ready[quad], (published + j - 1) & 1, abort_word));
+            ok = __all_sync(0xffffffffu, mbar_wait(&sm.m_ready[info][quad], (pub + j - 1) & 1, abort_word));
             if (!ok) break;
-            m_cur = sm.m[r];
+            m_cur = ti.m[r];
           }
           float m_new = m_cur;
           if (pass == 0 && __all_sync(0xffffffffu, m_cur != -INFINITY)) {
@@ -492,9 +570,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                      fmaxf(fmaxf(mxp[4], mxp[5]), fmaxf(mxp[6], mxp[7])));
               m_new = (mx > m_cur + kGap / sl2) ? mx : m_cur;
             }
-            sm.m[r] = m_new;
+            ti.m[r] = m_new;
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.m_ready[quad]);
+            if (lane == 0) mbar_arrive(&sm.m_ready[info][quad]);
             exchange = pass > 0 || __any_sync(0xffffffffu, m_new == -INFINITY);
             if (!exchange) n_pub = j + 1;
             if (j > 0 && __any_sync(0xffffffffu, m_new != m_cur)) {
@@ -548,71 +626,19 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         b += 2;
         if (b >= kSBufs) { b -= kSBufs; bph ^= 1; }
       }
-      // ---- epilogue
+      // ---- the row's sum, for the reference it ends with
       float m_fin = m_ref;
-      if (n > 0 && ok) {
-        ok = mbar_wait(&sm.acc_full, acc_ph, abort_word);
-        acc_ph ^= 1;
-        tc_fence_after();
-        if (ok && exchange && ((g0 + n - 1) & 1) != wg) {
-          ok = mbar_wait(&sm.m_ready[quad], (published + n - 1) & 1, abort_word);
-          m_fin = sm.m[r];
-        }
+      if (n > 0 && ok && exchange && ((g0 + n - 1) & 1) != wg) {
+        ok = mbar_wait(&sm.m_ready[info][quad], (pub + n - 1) & 1, abort_word);
+        m_fin = ti.m[r];
       }
-      float (*sums)[kTileM] = sm.l[turn];
-      sums[wg][r] = l_run != 0.f ? l_run * fast_exp2((m_ref - m_fin) * sl2) : 0.f;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.l_ready[quad]);
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(&sm.l_ready[quad], turn, abort_word));
+      ti.l[wg][r] = l_run != 0.f ? l_run * fast_exp2((m_ref - m_fin) * sl2) : 0.f;
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      turn ^= 1;
-      published += n_pub;
+      published ^= uint32_t(n_pub & 1) << info;
       g0 += n;
-      uint32_t oreg[64];
-      if (n > 0) {  // warp-uniform: the TMEM load is a warp-collective instruction
-        tmem_ld32(o_addr + wg * 64, oreg);
-        tmem_ld32(o_addr + wg * 64 + 32, oreg + 32);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&sm.o_empty), 0));
-      } else {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) oreg[i] = 0;
-      }
-      const int n_rows = ti.n_rows;
-      const float l_sum = sums[0][r] + sums[1][r];
-      if (pass == 0 && __any_sync(0xffffffffu, r < n_rows && !(l_sum < kMaxSum)) && lane == 0) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
-          or_cluster_u32(smem_u32(&sm.redo[(ti.round >> 5) & (kRedoWords - 1)]), c, 1u << (ti.round & 31));
-        }
-      }
-      const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
-      if (r < n_rows && wg == 0) ti.lse[r] = l_sum > 0.f ? m_fin * scale + logf(l_sum) - kTruncLn : -INFINITY;
-      __nv_bfloat16* out = ti.out + size_t(quad * 32 + (lane >> 2)) * hq * kHeadDim + wg * 64 + (lane & 3) * 8;
-      uint8_t* stage = sm.o_stage[warp];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {   // 32 channels: four 16-byte pieces per row, swizzled, out with four lanes per row
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t packed[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            packed[k] = pack_bf16x2(__uint_as_float(oreg[32 * c + 8 * i + 2 * k]) * inv_l, __uint_as_float(oreg[32 * c + 8 * i + 2 * k + 1]) * inv_l);
-          *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = 8 * i + (lane >> 2);
-          const uint4 piece = *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4));
-          if (quad * 32 + row < n_rows) *reinterpret_cast<uint4*>(out + size_t(8 * i) * hq * kHeadDim + c * 32) = piece;
-        }
-        __syncwarp();
-      }
-      if (lane == 0) mbar_arrive(&sm.info_empty[info]);
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&sm.l_ready[info][quad]); mbar_arrive(&sm.info_empty[info]); }
       if (++info == kInfos) { info = 0; iph ^= 1; }
     }
     if (!next_pass(pass)) break;
