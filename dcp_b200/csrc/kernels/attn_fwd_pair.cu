@@ -180,8 +180,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   // The pairs of CTAs take the tiles, which are ordered by length, in rounds and every second round backwards.
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   auto index_of = [&](int round) { return round * n_pairs + ((round & 1) ? n_pairs - 1 - pair : pair); };
-  // the first tile from `round` on that has work for the pass and at least `min_kv` KV tiles; false: there is none
-  auto find_tile = [&](int pass, int& round, AttnTile& t, int min_kv) -> bool {
+  // the first tile from `round` on that has work for the pass and KV tiles, or none of them; false: there is none
+  int first_empty = -1;   // first round with a tile that has none
+  auto find_tile = [&](int pass, int& round, AttnTile& t, bool empty) -> bool {
     for (;; ++round) {
       const int i = index_of(round);
       if (i >= n_tiles) return false;
@@ -196,7 +197,9 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                        t.mask_row < 0 || t.mask_row + t.n_rows > n_mask_rows || t.kv_off < 0 ||
                        t.kv_off + t.n_kv > n_kv_subs;
       if (bad) atomicExch(status, kStatusBadArgs);
-      if (!bad && t.n_kv >= min_kv) return true;
+      if (bad) continue;
+      if ((t.n_kv == 0) == empty) return true;
+      if (!empty && first_empty < 0) first_empty = round;
     }
   };
   // End of a pass over the tiles, by all threads of both CTAs; true: a second pass follows.
@@ -326,9 +329,24 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         return true;
       };
       AttnTile tile;
+      // Tiles without keys come last: the last three V of a tile are loaded with the K of the next ones, and announcing a tile
+      // waits until the one kInfos before it is finished.
+      bool empty = false;
+      first_empty = -1;
       for (int round = 0; ok; ++round) {
-        const bool more = find_tile(pass, round, tile, 0);
-        ok = mbar_wait(&sm.info_empty[info], iph, abort_word);
+        bool more = find_tile(pass, round, tile, empty);
+        if (!more && !empty) {
+          // the last three V: slots 3, 4 and 5 at the earliest
+          if (behind > 0 && behind < 3) slot = 3;
+          for (; ok && behind > 0; --behind) {
+            if (behind < 3) { row3 = behind == 2 ? row2 : row1; head3 = behind == 2 ? head2 : head1; }
+            ok = load_slot(false, true, 0, 0);
+          }
+          empty = true;
+          round = first_empty;
+          more = round >= 0 && find_tile(pass, round, tile, empty);
+        }
+        ok = ok && mbar_wait(&sm.info_empty[info], iph, abort_word);
         if (!ok) break;
         TileInfo& ti = sm.info[info];
         if (!more) {
@@ -369,12 +387,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           head3 = head2; head2 = head1; head1 = kv_head;
         }
       }
-      // the last three V: slots 3, 4 and 5 at the earliest
-      if (behind > 0 && behind < 3) slot = 3;
-      for (; ok && behind > 0; --behind) {
-        if (behind < 3) { row3 = behind == 2 ? row2 : row1; head3 = behind == 2 ? head2 : head1; }
-        ok = load_slot(false, true, 0, 0);
-      }
       // arrivals from the even CTA's issuer have all come in before this CTA may retire
       for (int i = 0; ok && i < kSlots; ++i) {
         if ((used >> slot) & 1) ok = mbar_wait(&sm.kv_empty[slot], ph, abort_word);
@@ -412,7 +424,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       auto next_q = [&]() -> bool {
         if (q_left == 0) {
           q_left = -1;
-          if (find_tile(pass, q_round, t, 1)) {
+          if (find_tile(pass, q_round, t, false)) {
             ++q_round;
             q_left = t.n_kv;
             ok = mbar_wait(&sm.q_full[qi], qph, abort_word);
@@ -440,7 +452,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         umma_commit_pair(&sm.kv_empty[i]);
       }
       int slot = kSBufs, ph = 0, b = 0, bph = 0, n_tiles_done = 0;
-      for (int round = 0; ok && find_tile(pass, round, t, 1); ++round) {
+      for (int round = 0; ok && find_tile(pass, round, t, false); ++round) {
         const int n = t.n_kv;
         const int4* subs = kv_subs + t.kv_off;
         int flags = subs[0].w;

@@ -189,6 +189,29 @@ def test_attention_forward_pairs_of_tiles(dev, nkv, kind):
     assert out[nq:].abs().max() == 0
 
 
+@pytest.mark.parametrize("seeing", [0, 1, 700])
+def test_attention_forward_many_tiles_without_keys(dev, seeing):
+    """More tiles without any key per pair of CTAs than it holds records of, behind a tile that has some: zeros and -inf
+    there, and the others as above (2^-6 of the largest value)."""
+    nq, nkv, hq = 6400, 300, 16
+    torch.manual_seed(seeing)
+    q, kv = torch.randn(nq, hq, 128, device=dev).bfloat16(), torch.randn(nkv, 2, 4, 128, device=dev).bfloat16()
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:seeing, 1] = nkv
+    row = A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)
+    out, lse = torch.full_like(q, 7), torch.zeros(hq, nq, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 2048, dev), [out], [lse], 128 ** -0.5, status)
+    assert status.item() == 0
+    assert out[seeing:].abs().max() == 0 and torch.isinf(lse[:, seeing:]).all()
+    if seeing:
+        k64, v64 = (kv[:, j].double().repeat_interleave(hq // 4, 1).permute(1, 0, 2) for j in (0, 1))
+        s = q[:seeing].double().permute(1, 0, 2) @ k64.transpose(1, 2) * 128 ** -0.5
+        ref = (s.softmax(-1) @ v64).permute(1, 0, 2)
+        assert (out[:seeing].double() - ref).abs().max() <= 2.0 ** -6 * ref.abs().max()
+        assert (lse[:, :seeing] - torch.logsumexp(s, -1)).abs().max() < 1e-3
+
+
 @pytest.mark.parametrize("nq,nkv,kind,heads", [(1, 1, "causal", (4, 4)), (127, 129, "full", (4, 1)), (129, 127, "causal", (8, 2)),
                                                 (256, 255, "two", (4, 2)), (64, 640, "full", (8, 1)), (700, 700, "two", (8, 2))])
 def test_attention_backward_tile_edges(dev, nq, nkv, kind, heads):
