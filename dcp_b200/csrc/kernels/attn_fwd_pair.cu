@@ -40,7 +40,11 @@
 // with the next tile's scores, whose first product waits until O is in registers.  (With the epilogue in the softmax warps the
 // tensor core was idle for about 4000 cycles between two tiles: 16 heads, 16384 queries over 256 / 512 keys 110 -> 81 / 139
 // -> 107 us, causal 2048 x 2048 66.6 -> 62.5, 4096 x 4096 167 -> 159 us, sink + window 531 -> 514 us in long runs; full 8192 x
-// 16384 1.535 -> 1.542 ms.)  As a launch with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
+// 16384 1.535 -> 1.542 ms.)  They store rows straight from registers, a sector per lane and instruction: through shared memory,
+// in 64-byte pieces, O was in TMEM for 3500 cycles instead of 1900, as every look at shared memory queues behind the
+// exponentials (8192 queries over 1500 keys 213 -> 201 us, causal 6000 x 6000 280 -> 270, 16384 x 16384 1861 -> 1835 us, in long
+// runs; full 8192 x 16384 1836 -> 1820).  A copy per row by the copy engine takes 60 cycles to issue, 2000 for a half of 32 rows.
+// As a launch with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
 // Measured against two query tiles per CTA (32 / 8 heads, queries x keys; one box): full 8192 x 16384 1.71 -> 1.57 ms
 // (1283 -> 1404 TFLOP/s), causal 1.29 -> 1.17 ms (1397), sink + window 0.568 -> 0.505 ms, causal 4096 x 4096 0.163 ->
 // 0.153 ms; in long runs under the power cap full 2.01 -> 1.74 ms (all with the epilogue in the softmax warps).  Tried and left: a pair per tile instead of persistent pairs (4096 x 4096 0.159 ms, 16384
@@ -48,7 +52,7 @@
 // costs more than it hides: 1.57 -> 1.66 ms); the maximum taken beside the exponentials (1.75 ms).
 //
 // The partial (out, lse) of a tile is stored straight to its destination arena, which may be a
-// peer GPU's memory (plain st.global over the NVLink mapping), through shared memory in 64-byte pieces of a row.
+// peer GPU's memory (plain st.global over the NVLink mapping).
 //
 // Reference behaviour covered: the varlen forward with block tables and per-query KV ranges that
 // dcp/runtime/flash_attention/executor.py:884-913 calls.
@@ -94,7 +98,6 @@ struct __align__(1024) PairSmem {
   uint8_t q[2][2 * kQHalf];
   uint8_t k[kSlots][kKvBytes];      // 64 of the 128 keys, all channels
   uint8_t v[kSlots][kKvBytes];      // all 128 keys, 64 of the channels
-  uint8_t o_stage[4][32 * 64];      // per epilogue warp: 32 rows x 32 channels on their way out
   TileInfo info[kInfos];
   uint32_t redo[kRedoWords];        // rounds that go through the second pass
   // of the even CTA (bytes and arrivals of both CTAs): q_full, kv_full, p_ready, o_empty; the others are signalled in
@@ -227,12 +230,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int quad = warp & 3, r = threadIdx.x & 127;
     const uint32_t o_addr = tmem + (uint32_t(quad * 32) << 16) + kSBufs * 128;
     const uint32_t o_bar = cluster_addr(smem_u32(&sm.o_empty), 0);
-    uint8_t* stage = sm.o_stage[warp - 12];
    for (int pass = 0;; ++pass) {
-    // O is in registers: the products of the tile in slot `info` may set it; false: there is no such tile
-    auto hand_over = [&](int info, int iph) -> bool {
+    // O is in registers: the products of the tile in slot `info`, which is there, may set it; false: that is the end
+    auto hand_over = [&](int info) -> bool {
       const TileInfo& ti = sm.info[info];
-      if (!__all_sync(0xffffffffu, mbar_wait(&sm.info_full[info], iph, abort_word)) || ti.n_kv < 0) return false;
+      if (ti.n_kv < 0) return false;
       if (ti.n_kv > 0) {
         if (!((ti.first[0].w >> X) & 1)) {   // then no product sets O of this query tile, they only add to it
           uint32_t zero[32];
@@ -248,15 +250,17 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       return true;
     };
+    auto wait_info = [&](int info, int iph) { return __all_sync(0xffffffffu, mbar_wait(&sm.info_full[info], iph, abort_word)); };
     int acc_ph = 0;  // parity of the tiles with a product so far
-    bool more = hand_over(0, 0);
+    bool more = wait_info(0, 0) && hand_over(0);
     for (int info = 0, iph = 0; more;) {
       const TileInfo& ti = sm.info[info];
-      const int n = ti.n_kv, n_rows = ti.n_rows;
+      const int n = ti.n_kv;
       const int next = info + 1 == kInfos ? 0 : info + 1, next_ph = next == 0 ? iph ^ 1 : iph;
       bool ok = mbar_wait(&sm.l_ready[info][quad], iph, abort_word);
+      const bool next_there = __all_sync(0xffffffffu, mbar_test_wait(&sm.info_full[next], next_ph));   // asked while there is time
       const float l_sum = ti.l[0][r] + ti.l[1][r];
-      if (pass == 0 && __any_sync(0xffffffffu, r < n_rows && !(l_sum < kMaxSum)) && lane == 0) {
+      if (pass == 0 && __any_sync(0xffffffffu, r < ti.n_rows && !(l_sum < kMaxSum)) && lane == 0) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
@@ -264,42 +268,40 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
       }
       const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
-      if (ok && r < n_rows) ti.lse[r] = l_sum > 0.f ? ti.m[r] * scale + logf(l_sum) - kTruncLn : -INFINITY;
-      __nv_bfloat16* out = ti.out + size_t(quad * 32 + (lane >> 2)) * hq * kHeadDim + (lane & 3) * 8;
+      if (ok && r < ti.n_rows) ti.lse[r] = l_sum > 0.f ? ti.m[r] * scale + logf(l_sum) - kTruncLn : -INFINITY;
       if (n > 0) {
         ok = ok && mbar_wait(&sm.acc_full, acc_ph, abort_word);
         acc_ph ^= 1;
         tc_fence_after();
       }
       if (!__all_sync(0xffffffffu, ok)) break;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {   // 32 channels: four 16-byte pieces per row, swizzled, out with four lanes per row
-        uint32_t oreg[32];
+      // a row from TMEM to where it goes, 16 channels (a whole sector) per store
+      const bool mine = r < ti.n_rows;
+      __nv_bfloat16* out = ti.out + size_t(r) * hq * kHeadDim;
+      const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint32_t oreg[16], packed[8];
         if (n > 0) {  // warp-uniform: the TMEM load is a warp-collective instruction
-          tmem_ld32(o_addr + c * 32, oreg);
+          tmem_ld16(o_addr + c * 16, oreg);
           tmem_wait_ld();
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) oreg[i] = 0;
+          for (int i = 0; i < 16; ++i) oreg[i] = 0;
         }
-        if (c == 3) more = hand_over(next, next_ph);
+        if (c == 7) more = (next_there || wait_info(next, next_ph)) && hand_over(next);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t packed[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            packed[k] = pack_bf16x2(__uint_as_float(oreg[8 * i + 2 * k]) * inv_l, __uint_as_float(oreg[8 * i + 2 * k + 1]) * inv_l);
-          *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        for (int i = 0; i < 8; ++i) packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
+        if (mine) {
+          if (wide) {
+            st_global_v8(out + c * 16, packed);
+          } else {
+            reinterpret_cast<uint4*>(out)[2 * c] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            reinterpret_cast<uint4*>(out)[2 * c + 1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          }
         }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = 8 * i + (lane >> 2);
-          const uint4 piece = *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4));
-          if (quad * 32 + row < n_rows) *reinterpret_cast<uint4*>(out + size_t(8 * i) * hq * kHeadDim + c * 32) = piece;
-        }
-        __syncwarp();
       }
+      __syncwarp();
       if (lane == 0) mbar_arrive(&sm.info_empty[info]);
       info = next; iph = next_ph;
     }
