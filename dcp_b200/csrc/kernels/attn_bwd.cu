@@ -20,8 +20,10 @@
 // Warps: 0-15 gradient (warp = 32 key rows x 32 queries), 16-23 drain dQ (thread = 64 channels of a query row; a
 // [32 queries x 32 channels] fp32 tile per step, added to the accumulator with one tiled TMA
 // reduce-add, or to a peer's with a 128-byte bulk reduce-add per row), 24 TMA producer, 25 UMMA issuer, 26
-// per-query statistics, 27 idle.  dK/dV stay in TMEM for the CTA's lifetime and are added once
-// with red.global.add.v4.f32; the CTAs of a split head group first add their shares up through distributed
+// per-query statistics, 27 idle.  dK/dV stay in TMEM for the CTA's lifetime and are added once,
+// through shared memory with tiled TMA reduce-adds (with red.global.add.v4.f32, a row per lane, L2 took 11000 cycles for the
+// 128 KB of a key tile, 7000 now: one visit per CTA 15.4 -> 13.1 us per wave, 18944 keys x 1024 queries, 8 heads, 256 -> 232 us,
+// with 64 channels 180 -> 172; what is left of it is L2's rate of fp32 additions, 20 bytes per cycle and SM); the CTAs of a split head group first add their shares up through distributed
 // shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
 // (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
 // every key tile as it comes: its last bits may differ from run to run.
@@ -228,6 +230,7 @@ template <bool kTL, int kD>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_dq,
+                const __grid_constant__ CUtensorMap tm_dkv,
                 const BwdCta* __restrict__ ctas, const BwdItemDesc* __restrict__ items, const int4* __restrict__ masks,
                 const float* __restrict__ lse, const float* __restrict__ delta, BwdPtrs ptrs, int hq, int hkv,
                 int heads_per_cta, int stat_stride, int n_dst, int q_rows, int kv_rows, int n_mask_rows, int n_items_total,
@@ -548,11 +551,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         __syncwarp();
         if (cur.dq_dev == 0) {
           if (lane == 0) {
-            asm volatile(
-                "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-                ::"l"(reinterpret_cast<uint64_t>(&tm_dq)), "r"(smem_u32(stage)), "r"(ch0 + b * 32), "r"(cur.head),
-                "r"(cur.dq_row + quad * 32)
-                : "memory");
+            tma_reduce_add_3d(&tm_dq, stage, ch0 + b * 32, cur.head, cur.dq_row + quad * 32);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         } else if (quad * 32 + lane < cur.n_rows) {
@@ -639,6 +638,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int ch = (hf & 1) * 32 * kMine;
         float* dst = ptrs.dkv[cta.dkv_dev] + ((size_t(cta.dkv_row + r) * 2 + (hf >> 1)) * hkv + kv_head) * kHeadDim + ch;
         const uint32_t acc = tmem + lane_base + (hf >> 1 ? cdV : cdK) + ch;
+        // a whole key tile for this GPU's accumulator goes there in boxes of [32 keys x 32 channels], which take the place of K, V
+        // and Q; rows that may not be added to, and other GPUs' accumulators, go 16 bytes at a time
+        const bool whole = cta.dkv_dev == 0 && cta.n_valid == 128;
 #pragma unroll
         for (int c = 0; c < kMine; ++c) {
           if (ch + 32 * c >= kD) break;
@@ -651,6 +653,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int i = 0; i < 8; ++i)
               *reinterpret_cast<uint4*>(row + (((ch >> 2) + 8 * c + i) ^ (r & 7)) * 4) =
                   make_uint4(reg[4 * i], reg[4 * i + 1], reg[4 * i + 2], reg[4 * i + 3]);
+          } else if (whole) {
+            uint8_t* box = sm.k + warp * 8192 + c * 4096;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              *reinterpret_cast<uint4*>(box + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+                  make_uint4(reg[4 * i], reg[4 * i + 1], reg[4 * i + 2], reg[4 * i + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_reduce_add_3d(&tm_dkv, box, ch + 32 * c, (hf >> 1) * hkv + kv_head, cta.dkv_row + quad * 32);
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
           } else if (r < cta.n_valid) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
@@ -658,6 +672,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                          __uint_as_float(reg[4 * i + 2]), __uint_as_float(reg[4 * i + 3]));
           }
         }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
       }
     }
   }
@@ -723,8 +738,9 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
                              int job_stat_stride, int* status, void* stream) {
   if (n_ctas <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
   if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
-  CUtensorMap tm_q, tm_do, tm_kv, tm_dq;
+  CUtensorMap tm_q, tm_do, tm_kv, tm_dq, tm_dkv;
   if (encode_f32_tile_map(&tm_dq, dq_ptrs[0], uint64_t(q_rows), uint32_t(hq), kHeadDim, 32, 32)) return -1;
+  if (encode_f32_tile_map(&tm_dkv, dkv_ptrs[0], uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 32, 32)) return -1;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
   if (encode_arena_map(&tm_do, do_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
   if (encode_arena_map(&tm_kv, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 128)) return -1;
@@ -774,7 +790,7 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   cfg.attrs = &cluster;
   cfg.numAttrs = parts > 1 ? 1 : 0;
   const cudaError_t rc = cudaLaunchKernelEx(
-      &cfg, kernel, tm_q, tm_do, tm_kv, tm_dq, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
+      &cfg, kernel, tm_q, tm_do, tm_kv, tm_dq, tm_dkv, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
       static_cast<const int4*>(masks), lse, delta, pp, hq, hkv, heads_per_cta, stat_stride, n_dst, int(q_rows), int(kv_rows),
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;
