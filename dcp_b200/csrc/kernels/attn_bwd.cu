@@ -60,6 +60,8 @@
 #include <math.h>
 #include <stddef.h>
 
+#include <algorithm>
+
 #include "attn_common.cuh"
 #include "copy_jobs.cuh"
 #include "entries.h"
@@ -762,21 +764,23 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   }
   // about 16 fetch CTAs when there is something to fetch
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
-  // A CTA visits its items once per query head of the group, unless that would leave SMs idle: when the
-  // longest item list times the group is more than the average SM's share of all visits, the group is
-  // split over as many CTAs (a cluster, at most the portable 8, which adds its parts of dK / dV up in a fixed order)
-  // as it takes to get below that share.  CTAs that all run at once add to a row of dQ in the order of their items, which
-  // in practice gives a short batch the same bits in every run; they become more than one wave only where that takes 32
-  // visits (about 70 us) off the longest list.  Four sequences of 300 to 2100 tokens, 8 / 2 heads: 66 key tiles with up to
-  // 68 visits, 11 per SM on average: 171 us whole, 95 us in two parts (132 CTAs), 69 us in four, and the call, which waits
-  // for its launches, takes 231 us with two and 229 with four.  512 to 4096 tokens: 120 key tiles with up to 128 visits,
-  // 317 us whole, 163 us in four parts (480 CTAs), the call 457 and 319 us.
+  // A CTA visits its items once per query head of the group, or the group is split over several CTAs (a cluster, at most
+  // the portable 8, which adds its parts of dK / dV up in a fixed order): shorter longest lists, and more CTAs to begin and
+  // end, which takes one as long as 8 visits (2.2 us each).  The launch takes as long as its longest list, or as all visits
+  // spread over the SMs, whichever is more; the split for which that is least is taken, the smallest of equals.  Over 78
+  // batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128 channels) the
+  // choice is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was above the
+  // SMs' average, but seldom into more than one wave, was 9 % off, 54 % at worst.  Four sequences of 300 to 2100 tokens,
+  // 8 / 2 heads: 91 us in two parts, 64 in four; 2048 tokens, 32 / 8 heads: 152 us before, 109 in two parts; eight sequences,
+  // 9105 tokens, 8 / 2 heads: 147 and 107 us.
   const int group = hq / hkv;
+  constexpr long kBegin = 8;
+  auto visits = [&](int p) {   // times the SMs
+    return std::max(kSms * (long(max_items) * (group / p) + kBegin), long(n_items_total) * hq + kBegin * n_ctas * hkv * p);
+  };
   int parts = 1;
-  for (int p = 2; p <= group && p <= kMaxParts && long(max_items) * (group / parts) * kSms > long(n_items_total) * hq; ++p) {
-    const bool leaves_wave = long(n_ctas) * hkv * parts <= kSms && long(n_ctas) * hkv * p > kSms;
-    if (group % p == 0 && !(leaves_wave && long(max_items) * (group / parts - group / p) < 32)) parts = p;
-  }
+  for (int p = 2; max_items > 0 && p <= group && p <= kMaxParts; ++p)
+    if (group % p == 0 && visits(p) < visits(parts)) parts = p;
   const int heads_per_cta = group / parts;
   cudaLaunchAttribute cluster;
   cluster.id = cudaLaunchAttributeClusterDimension;
