@@ -189,6 +189,22 @@ def test_attention_forward_pairs_of_tiles(dev, nkv, kind):
     assert out[nq:].abs().max() == 0
 
 
+@pytest.mark.parametrize("nq,nkv", [(1, 1), (257, 300)])
+def test_attention_forward_result_at_16_bytes(dev, nq, nkv):
+    """A result whose rows begin 16 bytes off a sector: the same bits as at the start of one."""
+    torch.manual_seed(0)
+    q, kv = torch.randn(nq, 4, 128, device=dev).bfloat16(), torch.randn(nkv, 2, 2, 128, device=dev).bfloat16()
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = nkv
+    tables = A.build_fwd_tables([A.AttnRow(0, nq, list(range(4)), [(0, nkv)], rng)], 512, dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    flat = torch.zeros(2, q.numel() + 16, device=dev, dtype=torch.bfloat16)
+    for buf, off in zip(flat, (0, 8)):
+        A.attn_fwd(q, kv, tables, [buf[off:off + q.numel()].view_as(q)], [torch.zeros(4, nq, device=dev)], 128 ** -0.5, status)
+    assert status.item() == 0 and flat[0, :q.numel()].abs().max() > 0
+    assert torch.equal(flat[0, :q.numel()], flat[1, 8:8 + q.numel()]) and not flat[1, :8].any() and not flat[1, 8 + q.numel():].any()
+
+
 @pytest.mark.parametrize("seeing", [0, 1, 700])
 def test_attention_forward_many_tiles_without_keys(dev, seeing):
     """More tiles without any key per pair of CTAs than it holds records of, behind a tile that has some: zeros and -inf
@@ -365,6 +381,37 @@ def test_attention_backward_into_a_second_accumulator(dev):
     close = lambda a, b: (a - b).abs().max() <= 1e-5 * want.abs().max()
     assert close(first[(tile == 0) | (tile == 3)], want[(tile == 0) | (tile == 3)]) and close(second[other], want[other])
     assert first[other | (tile == 2)].abs().max() == 0 and second[~other].abs().max() == 0
+
+
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("nkv", [128, 256, 301])
+def test_attention_backward_whole_and_part_key_tiles(dev, d, nkv):
+    """Heads without a group, so that a CTA adds its dK and dV by itself: whole key tiles, and the part of one.  Added to what the
+    accumulators hold, nothing beyond the keys or the channels; bound as for the other backward tests (2^-6 of the largest)."""
+    nq, h = 200, 4
+    torch.manual_seed(nkv)
+    q, dout = torch.zeros(2, nq, h, 128, device=dev, dtype=torch.bfloat16)
+    kv = torch.zeros(nkv + 40, 2, h, 128, device=dev, dtype=torch.bfloat16)
+    for t in (q, dout, kv):
+        t[..., :d] = torch.randn(*t.shape[:-1], d, device=dev).bfloat16()
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = np.minimum(np.arange(nq) + nkv - 150, nkv).clip(0)
+    row = A.AttnRow(0, nq, list(range(h)), [(0, nkv)], rng)
+    out, lse, delta = torch.zeros_like(q), torch.zeros(h, nq, device=dev), torch.zeros(h, nq, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 512, dev), [out], [lse], d ** -0.5, status, channels=d)
+    A.attn_delta(out, dout, delta, 0, nq)
+    dq, dkv = torch.zeros(nq, h, 128, device=dev), torch.ones(nkv + 40, 2, h, 128, device=dev)
+    A.attn_bwd(q, dout, kv, lse, delta, A.build_bwd_tables([row], 512, h, h, dev), [dq], [dkv], d ** -0.5, status, channels=d)
+    assert status.item() == 0
+    assert (dkv[nkv:] == 1).all() and (dkv[..., d:] == 1).all()
+    q64, o64, k64, v64 = (t.double().permute(1, 0, 2) for t in (q, dout, kv[:nkv, 0], kv[:nkv, 1]))
+    s = (q64 @ k64.transpose(1, 2) * d ** -0.5).masked_fill(~A.ranges_to_dense(rng, nkv).to(dev), float("-inf"))
+    p = s.softmax(-1).nan_to_num(0.0)
+    ds = p * (o64 @ v64.transpose(1, 2) - ((p @ v64) * o64).sum(-1, keepdim=True)) * d ** -0.5
+    for got, want in ((dkv[:nkv, 0] - 1, ds.transpose(1, 2) @ q64), (dkv[:nkv, 1] - 1, p.transpose(1, 2) @ o64), (dq, ds @ k64)):
+        want = want.permute(1, 0, 2)
+        assert (got.double() - want).abs().max() <= 2.0 ** -6 * want.abs().max()
 
 
 @pytest.mark.parametrize("d", [8, 40, 64, 72, 96, 104])
