@@ -64,6 +64,7 @@
 #include "attn_common.cuh"
 #include "copy_jobs.cuh"
 #include "entries.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -176,6 +177,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   tc_fence_before();
   cluster_sync();   // barriers and TMEM of both CTAs are there
   tc_fence_after();
+  grid_let_next();
+  grid_wait();
   const uint32_t tmem = sm.tmem_base;
   volatile int* abort_word = &sm.abort_word;
   const int4 none = make_int4(0, 0, 0, 0);
@@ -701,9 +704,10 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
       return -4;
     g_pair_attr_set[v] = 1;
   }
-  kernel<<<2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
+  // short calls begin while the kernel before them ends (see kSmallPass in attn_edge.cu; a round is 5 us and more)
+  const cudaError_t rc = launch_overlapped(
+      kernel, 2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream), 1, n_tiles <= 8 * kPairs, tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
       static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, int(q_rows),
       n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

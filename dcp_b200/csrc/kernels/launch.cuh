@@ -1,0 +1,42 @@
+// Launches whose beginning overlaps the end of the kernel before them in the stream (programmatic dependent launch).
+//
+// An attention call is up to seven kernels that each need the one before.  As plain launches every one of them begins 1.5 to
+// 3 us after the last block of the one before has ended.  With this attribute a kernel's blocks come onto the SMs as those of
+// the one before leave, set up what needs no memory (barriers, TMEM) and wait in grid_wait().  Forward and backward of 4040
+// tokens, 8 heads: 114.5 -> 106 us (four kernels); 7680 tokens of 64 fp32 channels 224 -> 217 us (seven).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace dcpk {
+
+// Everything the kernels before this one in the stream have written is there.  Comes before the first access to global memory,
+// reading and writing, in every thread.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The next kernel's blocks may come (once all blocks of this one have called this or ended); they wait all the same until this
+// kernel is through.
+__device__ __forceinline__ void grid_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A kernel that calls grid_wait(), in clusters of `cluster` blocks where that is more than one; `overlapped` or as a plain launch.
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, unsigned cluster,
+                                     bool overlapped, A&&... args) {
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = overlapped;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = cluster;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attrs;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+}  // namespace dcpk
