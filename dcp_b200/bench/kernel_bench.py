@@ -276,7 +276,7 @@ def main():
     ap.add_argument("--hkv", type=int, default=8)
     ap.add_argument("--block", type=int, default=2048)
     ap.add_argument("--mask", default="causal", choices=["full", "causal", "lambda"])
-    ap.add_argument("--variant", type=int, default=2, help="forward kernel: 2 = two query tiles per CTA (default), 0 / 1 = one tile per CTA with P in TMEM / shared memory")
+    ap.add_argument("--variant", type=int, default=2, help="forward kernel: 2 = pairs of CTAs (default), 0 / 1 = one tile per CTA with P in TMEM / shared memory")
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--timeline", action="store_true", help="print per-phase cycle counts of one CTA (attn_bwd; attn_fwd with --variant 0 or 1)")
     ap.add_argument("--skip-dq", action="store_true", help="backward without the dQ drain (upper bound probe)")

@@ -39,12 +39,13 @@
 // 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
 // 13 stall cycles per issue; 0.5 of 19 now).  8 drain warps keep their part of dQ in registers, so the columns
 // are free before the shared-memory tile and the L2 have taken it (4 warps with half of it at a time: 7 % slower).
-// What bounds it now: the shared-memory pipe.  An item moves 2048 wavefronts of UMMA operands and 1870 of loads
-// and stores (dS^T, dQ staging, statistics).  Before dK took its operand from TMEM (256 more), over the whole kernel (causal, below, under ncu: 3.92 ms at 1.62
-// GHz, 1335 items per SM, so 4760 cycles per item with prologues, ends of CTAs and the last wave) the counters show
-// 49 and 40 % of that pipe and 56 % of the tensor pipe; inside the loop an item took 4100 to 4300 cycles, which the
-// 4174 wavefronts filled.  TMA traffic (128 KB per item: Q, dO, dQ) is in neither counter.  Without the dQ drain an item takes 15 %
-// less.
+// What bounds it now: an item takes 4100 to 4300 cycles for 2600 of tensor time, and the chain dS(t), dK(t), dQ(t), dQ to
+// registers, dP(t+1) is as long, because dP, dS and dQ share 128 TMEM columns.  L2 adds 64 KB of dQ in 2900 cycles when all
+// SMs add to tiles that are there (4300 when they are not), and shared memory moves 2048 wavefronts of UMMA operands and about
+// 1900 of loads and stores; without the dQ drain an item takes 15 % less.  Not what bounds it: the broadcast reads of lse and
+// delta (as a product of their own, three bf16 terms each: 4.85 -> 4.95 ms, and no faster with that product left out), the
+// conversions to bf16 (left out: the same), the order of a CTA's queries (reversed: the same).  In long runs the power limit
+// holds the clock at 1.3 to 1.6 GHz.  A pair of CTAs for 256 keys needs Q, dO and K in two layouts: 256 KB of shared memory.
 // Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104
 // TFLOP/s), causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
 //
