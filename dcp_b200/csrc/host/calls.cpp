@@ -80,25 +80,35 @@ class SingleRankAttention {
     return plain(t) && row_type(t) >= 0 && t.numel() == rows * heads * d;
   }
 
-  void launch_forward(const Tensor& q_in, const Tensor& kv_in, const Tensor& o, const Tensor& l, double scale) const {
+  void launch_forward(const Tensor& q_in, const Tensor& kv_in, const Tensor& o, const Tensor& l, double scale,
+                      int out_type = 2, int out_channels = kHeadDim) const {
     void* outs[2] = {part_out.data_ptr(), o.data_ptr()};
     float* lses[2] = {part_lse.data_ptr<float>(), l.data_ptr<float>()};
     check(dcpk_attn_fwd_pair(q_in.const_data_ptr(), q_in.size(0), kv_in.const_data_ptr(), kv_in.size(0), int(q.size(1)),
                              int(kv.size(2)), tiles.const_data_ptr(), n_tiles, kv_entries.const_data_ptr(),
                              int(kv_entries.size(0)), fwd_masks.const_data_ptr(), int(fwd_masks.size(0)), outs, lses, 2,
-                             int(part_lse.size(1)), int(l.size(1)), 1, block_size, float(scale), channels, nullptr, 0, nullptr,
+                             int(part_lse.size(1)), int(l.size(1)), 1, out_type, out_channels, block_size, float(scale), channels, nullptr, 0, nullptr,
                              nullptr, 0, status.data_ptr<int>(), stream()),
           "dcpk_attn_fwd_pair");
   }
 
-  // delta and cleared accumulators, then the gradients; `o` and `d_o`: at least the local rows
-  void launch_backward(const Tensor& q_in, const Tensor& d_o, const Tensor& kv_in, const Tensor& o, const Tensor& l, const Tensor& dl,
-                       double scale) const {
+  // delta and cleared accumulators, then the gradients; `o` and `d_in`: at least the local rows, of `d` channels.  Other than rows
+  // of 128 in bf16 go to the arena of dO on the way.
+  void launch_backward(const Tensor& q_in, const Tensor& d_in, const Tensor& kv_in, const Tensor& o, const Tensor& l, const Tensor& dl,
+                       int d, double scale) const {
     const long hq = q.size(1), hkv = kv.size(2);
-    check(dcpk_attn_bwd_prep(o.const_data_ptr(), d_o.const_data_ptr(), dl.data_ptr<float>(), int(q_local_rows), int(hq),
-                             int(dl.size(1)), dq.data_ptr<float>(), q_rows * hq * kHeadDim, dkv.data_ptr<float>(),
-                             kv_rows * 2 * hkv * kHeadDim, stream()),
-          "dcpk_attn_bwd_prep");
+    const bool in_place = d == kHeadDim && d_in.scalar_type() == at::kBFloat16;
+    const Tensor& d_o = in_place ? d_in : dout;
+    if (in_place)
+      check(dcpk_attn_bwd_prep(o.const_data_ptr(), d_in.const_data_ptr(), dl.data_ptr<float>(), int(q_local_rows), int(hq),
+                               int(dl.size(1)), dq.data_ptr<float>(), q_rows * hq * kHeadDim, dkv.data_ptr<float>(),
+                               kv_rows * 2 * hkv * kHeadDim, stream()),
+            "dcpk_attn_bwd_prep");
+    else
+      check(dcpk_attn_bwd_prep_cast(row_type(d_in), o.const_data_ptr(), d_in.const_data_ptr(), d, dout.data_ptr(), dl.data_ptr<float>(),
+                                    int(q_local_rows), int(hq), int(dl.size(1)), dq.data_ptr<float>(), q_rows * hq * kHeadDim,
+                                    dkv.data_ptr<float>(), kv_rows * 2 * hkv * kHeadDim, stream()),
+            "dcpk_attn_bwd_prep_cast");
     nvtxMarkA("bwd:dout copy, delta, zero accumulators");
     nvtxMarkA("bwd:wait inputs of peers");
     float* dqs[1] = {dq.data_ptr<float>()};
@@ -132,7 +142,7 @@ class SingleRankAttention {
         !arena_like(d_o, q_local_rows, q.size(1)) || d_o.size(0) != q_local_rows || !arena_like(o, q_local_rows, q.size(1)) || !statistics(l))
       return false;
     Range range("dcp.attention.bwd");
-    launch_backward(q_in, d_o, kv_in, o, l, dl ? *dl : at::empty_like(l), scale);
+    launch_backward(q_in, d_o, kv_in, o, l, dl ? *dl : at::empty_like(l), kHeadDim, scale);
     return true;
   }
 
@@ -146,11 +156,12 @@ class SingleRankAttention {
     const bool in_place = d == kHeadDim && q_in.scalar_type() == at::kBFloat16;
     int entries = 1;
     Tensor o, l;
+    const auto form = q.options().dtype(q_in.scalar_type());
     if (all_rows_written) {
-      o = at::empty({q_local_rows, hq, kHeadDim}, q.options());
+      o = at::empty({q_local_rows, hq, d}, form);
       l = at::empty({hq, q_local_rows}, lse.options());
     } else {
-      o = at::zeros({q_local_rows, hq, kHeadDim}, q.options());
+      o = at::zeros({q_local_rows, hq, d}, form);
       l = at::zeros({hq, q_local_rows}, lse.options());
     }
     if (!in_place) {
@@ -161,18 +172,10 @@ class SingleRankAttention {
     }
     nvtxMarkA("fwd:wait inputs of peers");
     if (in_place) launch_forward(q_in.view({q_local_rows, hq, kHeadDim}), kv_in.view({kv_local_rows, 2, hkv, kHeadDim}), o, l, scale);
-    else launch_forward(q, kv, o, l, scale);
+    else launch_forward(q, kv, o, l, scale, row_type(q_in), d);
     nvtxMarkA("fwd:kernels (with operand fetch)");
     nvtxMarkA("fwd:wait partials of peers");
     nvtxMarkA("fwd:merge");
-    if (!in_place) {
-      Tensor cut = at::empty({q_local_rows, hq, d}, q.options().dtype(q_in.scalar_type()));
-      check(dcpk_cut_cast_rows(0, row_type(cut), o.const_data_ptr(), cut.data_ptr(), q_local_rows * hq, nullptr, nullptr, 0, d,
-                               stream()),
-            "dcpk_cut_cast_rows");
-      ++entries;
-      o = cut;
-    }
     return std::make_tuple(o, l, entries);
   }
 
@@ -191,7 +194,6 @@ class SingleRankAttention {
     const Tensor l = l_in.view({hq, q_local_rows});
     Range range("dcp.attention.bwd");
     const bool in_place = d == kHeadDim && q_in.scalar_type() == at::kBFloat16;
-    const bool grads_in_place = d == kHeadDim && o_in.scalar_type() == at::kBFloat16;
     int entries = 3;
     if (!in_place && reload) {
       check(dcpk_pad_cast_rows(row_type(q_in), q_in.const_data_ptr(), q.data_ptr(), q_local_rows * hq, kv_in.const_data_ptr(),
@@ -199,14 +201,8 @@ class SingleRankAttention {
             "dcpk_pad_cast_rows");
       ++entries;
     }
-    if (!grads_in_place) {
-      check(dcpk_pad_cast_rows(row_type(o_in), o_in.const_data_ptr(), out.data_ptr(), q_local_rows * hq, do_in.const_data_ptr(),
-                               dout.data_ptr(), q_local_rows * hq, d, stream()),
-            "dcpk_pad_cast_rows");
-      ++entries;
-    }
-    launch_backward(in_place ? q_in : q, grads_in_place ? do_in : dout, in_place ? kv_in.view({kv_local_rows, 2, hkv, kHeadDim}) : kv,
-                    grads_in_place ? o_in : out, l, at::empty_like(l), scale);
+    launch_backward(in_place ? q_in : q, do_in, in_place ? kv_in.view({kv_local_rows, 2, hkv, kHeadDim}) : kv, o_in, l, at::empty_like(l),
+                    d, scale);
     Tensor gq = at::empty({q_local_rows, hq, d}, q.options().dtype(q_in.scalar_type()));
     Tensor gkv = at::empty({kv_local_rows, 2, hkv, d}, q.options().dtype(kv_in.scalar_type()));
     check(dcpk_cut_cast_rows(1, row_type(gq), dq.const_data_ptr(), gq.data_ptr(), q_local_rows * hq, dkv.const_data_ptr(),

@@ -3,13 +3,16 @@
 //
 //  pad_cast_rows   rows of d channels (fp32 / fp16 / bf16) -> bf16 rows of 128, zero-padded
 //  cut_cast_rows   rows of 128 (fp32 accumulators or bf16) -> rows of d channels in the caller's type
-//  attn_bwd_prep   delta = rowsum(dO * O) and cleared dQ / dKV accumulators, one launch
+//  attn_bwd_prep   delta = rowsum(dO * O) and cleared dQ / dKV accumulators, one launch; also from rows in the caller's form,
+//                  with dO converted on the way
 //
 // The two row kernels take up to two tensors per launch (Q and KV, O and dO, dQ and dKV).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "entries.h"
 #include "launch.cuh"
@@ -146,6 +149,53 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_
   for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
 }
 
+// The same for gradients in the caller's form (rows of d8 chunks of 8 channels): dO also goes to the arena's rows, rounded to
+// bf16 and zero-padded, and delta is that of the rounded values.  As a pass that converts O and dO and the one above
+// it took 22 us for 7680 tokens of 8 heads with 64 fp32 channels.
+template <typename T>
+__global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const T* __restrict__ o, const T* __restrict__ d_o, int d8,
+                                                                          __nv_bfloat16* __restrict__ rows, float* __restrict__ delta,
+                                                                          int n_rows, int hq, int stat_stride,
+                                                                          float4* __restrict__ zero0, size_t nz0,
+                                                                          float4* __restrict__ zero1, size_t nz1) {
+  constexpr int kInFlight = 2;
+  const size_t tid = size_t(blockIdx.x) * kEdgeThreads + threadIdx.x, n_thr = size_t(gridDim.x) * kEdgeThreads;
+  const int sub = threadIdx.x & 15;
+  const size_t n_items = size_t(n_rows) * hq, step = n_thr >> 4;
+  grid_let_next();
+  grid_wait();
+  // the trip count depends on the block only, so the shuffles below see whole warps
+  for (size_t base = size_t(blockIdx.x) * (kEdgeThreads / 16); base < n_items; base += kInFlight * step) {
+    float a[kInFlight][8], b[kInFlight][8];
+#pragma unroll
+    for (int u = 0; u < kInFlight; ++u) {
+      const size_t item = base + u * step + (threadIdx.x >> 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[u][i] = b[u][i] = 0.f;
+      if (item < n_items && sub < d8) {
+        load8(o + (item * d8 + sub) * 8, a[u]);
+        load8(d_o + (item * d8 + sub) * 8, b[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kInFlight; ++u) {
+      const size_t item = base + u * step + (threadIdx.x >> 4);
+      if (item < n_items) store8(rows + item * kEdgeHeadDim + sub * 8, b[u]);
+      float acc = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        acc += __bfloat162float(__float2bfloat16_rn(a[u][2 * i])) * __bfloat162float(__float2bfloat16_rn(b[u][2 * i])) +
+               __bfloat162float(__float2bfloat16_rn(a[u][2 * i + 1])) * __bfloat162float(__float2bfloat16_rn(b[u][2 * i + 1]));
+#pragma unroll
+      for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+      if (sub == 0 && item < n_items) delta[(item % hq) * size_t(stat_stride) + item / hq] = acc;
+    }
+  }
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (size_t i = tid; i < nz0; i += n_thr) zero0[i] = z;
+  for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
+}
+
 static int edge_grid(size_t chunks) {
   const size_t b = (chunks + kEdgeThreads - 1) / kEdgeThreads;
   return int(b < size_t(kEdgeBlocks) ? b : size_t(kEdgeBlocks));
@@ -211,5 +261,26 @@ extern "C" int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, 
   launch_overlapped(
       attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
       reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// o, d_o: [n_rows, hq, d] of an element type as above; d_o_rows: bf16 [n_rows, hq, 128]; the rest as dcpk_attn_bwd_prep
+extern "C" int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o, int d, void* d_o_rows, float* delta, int n_rows, int hq,
+                                       int stat_stride, float* zero0, long nz0, float* zero1, long nz1, void* stream) {
+  if (n_rows < 0 || hq <= 0 || n_rows > stat_stride || nz0 % 4 || nz1 % 4 || nz0 < 0 || nz1 < 0 || d <= 0 || d % 8 ||
+      d > kEdgeHeadDim || type < 0 || type > 2)
+    return -3;
+  const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
+  if (work == 0) return 0;
+  auto launch = [&](auto kernel, auto* as) {
+    using T = std::remove_pointer_t<decltype(as)>;
+    return launch_overlapped(kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass,
+                             static_cast<const T*>(o), static_cast<const T*>(d_o), d / 8, static_cast<__nv_bfloat16*>(d_o_rows), delta,
+                             n_rows, hq, stat_stride, reinterpret_cast<float4*>(zero0), size_t(nz0) / 4,
+                             reinterpret_cast<float4*>(zero1), size_t(nz1) / 4);
+  };
+  if (type == 0) launch(attn_bwd_prep_cast_kernel<float>, static_cast<float*>(nullptr));
+  else if (type == 1) launch(attn_bwd_prep_cast_kernel<__half>, static_cast<__half*>(nullptr));
+  else launch(attn_bwd_prep_cast_kernel<__nv_bfloat16>, static_cast<__nv_bfloat16*>(nullptr));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -56,6 +56,7 @@
 //
 // Reference behaviour covered: the varlen forward with block tables and per-query KV ranges that
 // dcp/runtime/flash_attention/executor.py:884-913 calls.
+#include <cuda_fp16.h>
 #include <limits.h>
 #include <math.h>
 
@@ -90,7 +91,8 @@ struct __align__(16) TileInfo {
   float m[kTileM];          // reference of a row
   float l[2][kTileM];       // its sums over the KV tiles of either warpgroup
   int4 first[2];            // first KV tiles
-  __nv_bfloat16* out;       // where the first row goes
+  uint8_t* out;             // where the first row goes
+  int out_type, out_channels;   // how (see store_channels)
   float* lse;
   int n_rows, n_kv, kv_off, round;  // rows of this CTA; n_kv < 0: there are no more tiles
 };
@@ -147,15 +149,54 @@ __device__ __forceinline__ void softmax_half(const uint32_t* s, uint64_t sl2_2, 
   tmem_st32(p_addr, preg);
 }
 
+// 16 channels of a row, from `ch` on, in the caller's type (0 float, 1 half, 2 bf16) where the row has them, a multiple of 8;
+// float and half hold what bf16 does
+__device__ __forceinline__ void store_channels(uint8_t* row, int type, int channels, int ch, uint32_t* packed) {
+  if (ch >= channels) return;
+  const bool both = ch + 16 <= channels;
+  uint8_t* p = row + ch * (type == 0 ? 4 : 2);
+  const bool wide = (reinterpret_cast<uintptr_t>(p) & 31) == 0;
+  if (type == 0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 1 && !both) break;
+      uint32_t f[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { f[2 * i] = packed[4 * h + i] << 16; f[2 * i + 1] = packed[4 * h + i] & 0xffff0000u; }
+      if (wide) {
+        st_global_v8(p + 32 * h, f);
+      } else {
+        reinterpret_cast<uint4*>(p)[2 * h] = make_uint4(f[0], f[1], f[2], f[3]);
+        reinterpret_cast<uint4*>(p)[2 * h + 1] = make_uint4(f[4], f[5], f[6], f[7]);
+      }
+    }
+    return;
+  }
+  if (type == 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __half2 v = __floats2half2_rn(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
+      packed[i] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+  if (wide && both) {
+    st_global_v8(p, packed);
+  } else {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    if (both) reinterpret_cast<uint4*>(p)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+  }
+}
+
 // kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and what S adds up over
 // zeros is left out.  PV stays as it is, so that the output's padding is written.  8192 queries x 16384 keys, 32 / 8 heads, against all 128
 // channels: 64 channels 1.43 -> 1.33 ms (causal 1.08 -> 1.04: the exponentials bound it then), 96 channels 1.51 -> 1.47 ms.
-template <int kD>
+// kForm: the results' type and width are arguments; rows of 128 in bf16 have an instance of their own, as a test per store cost
+// the calls that have them 1 to 4 %.
+template <int kD, bool kForm>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const AttnTile* __restrict__ tiles, int n_tiles,
                      const int4* __restrict__ kv_subs, const int4* __restrict__ masks, PeerPtrs ptrs, int hq, int hkv,
-                     int lse_stride_a, int lse_stride_b, int n_dst_a, int n_dst, int q_rows, int n_mask_rows,
+                     int lse_stride_a, int lse_stride_b, int n_dst_a, int n_dst, int out_type, int out_channels, int q_rows, int n_mask_rows,
                      int n_kv_subs, float scale, const CopyJob* __restrict__ jobs, int n_jobs,
                      const __grid_constant__ CopyCtx copy_ctx, int* __restrict__ status) {
   constexpr int kHalves = kD > 64 ? 2 : 1;   // of 64 channels of Q and K
@@ -280,7 +321,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (!__all_sync(0xffffffffu, ok)) break;
       // a row from TMEM to where it goes, 16 channels (a whole sector) per store
       const bool mine = r < ti.n_rows;
-      __nv_bfloat16* out = ti.out + size_t(r) * hq * kHeadDim;
+      const int type = kForm ? ti.out_type : 2, channels = kForm ? ti.out_channels : kHeadDim;
+      uint8_t* out = ti.out + size_t(r) * hq * channels * (type == 0 ? 4 : 2);
       const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -296,8 +338,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
         for (int i = 0; i < 8; ++i) packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
         if (mine) {
-          if (wide) {
-            st_global_v8(out + c * 16, packed);
+          if (kForm) {
+            store_channels(out, type, channels, c * 16, packed);
+          } else if (wide) {
+            st_global_v8(out + c * 32, packed);
           } else {
             reinterpret_cast<uint4*>(out)[2 * c] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             reinterpret_cast<uint4*>(out)[2 * c + 1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
@@ -368,7 +412,11 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         ti.kv_off = tile.kv_off;
         ti.round = round;
         ti.n_rows = tile.n_rows - X * kTileM;
-        ti.out = reinterpret_cast<__nv_bfloat16*>(ptrs.out[tile.out_dev]) + (size_t(tile.out_row + X * kTileM) * hq + tile.head) * kHeadDim;
+        const bool own_form = kForm && tile.out_dev >= n_dst_a;   // partial results are rows of 128 in bf16
+        ti.out_type = own_form ? out_type : 2;
+        ti.out_channels = own_form ? out_channels : kHeadDim;
+        ti.out = static_cast<uint8_t*>(ptrs.out[tile.out_dev]) +
+                 (size_t(tile.out_row + X * kTileM) * hq + tile.head) * ti.out_channels * (ti.out_type == 0 ? 4 : 2);
         ti.lse = ptrs.lse[tile.out_dev] + size_t(tile.head) * (tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b) + tile.out_row + X * kTileM;
         const int mask_bytes = 16 * min(max(tile.n_rows - X * kTileM, 0), kTileM);
         mbar_expect_tx(&sm.info_full[info], mask_bytes);
@@ -666,7 +714,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, kStatusBarrierTimeout);
 }
 
-static int g_pair_attr_set[3] = {0, 0, 0};
+static int g_pair_attr_set[6] = {0, 0, 0, 0, 0, 0};
 
 }  // namespace dcpk
 
@@ -676,15 +724,19 @@ using namespace dcpk;
 
 // Same contract as dcpk_attn_fwd, for tile tables built with 256-row tiles (AttnTile.n_rows <= 256):
 // `kv_entries` is the KvSub list (AttnTile.kv_off / n_kv index it), n_mask_rows / n_kv_entries are the
-// lengths of the mask table and of that list (bounds checks).
+// lengths of the mask table and of that list (bounds checks).  Destinations from n_dst_a on are rows of `out_channels` (a
+// multiple of 8, at most 128) of type `out_type` (0 fp32, 1 fp16, 2 bf16), those before it bf16 rows of 128; all 16-byte
+// aligned.  A pass of its own for the caller's form took 6.5 us of 218 for 7680 tokens of 64 fp32 channels, forward and backward.
 extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* kv_arena, long kv_rows, int hq,
                                   int hkv, const void* tiles, int n_tiles, const void* kv_entries, int n_kv_entries,
                                   const void* masks, int n_mask_rows, void* const* out_ptrs, float* const* lse_ptrs,
-                                  int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a, int block_size,
+                                  int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a, int out_type, int out_channels, int block_size,
                                   float scale, int channels, const void* jobs, int n_jobs, void* const* job_src_ptrs,
                                   void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream) {
   if (n_tiles <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
-  if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
+  if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim || out_type < 0 || out_type > 2 || out_channels < 8 ||
+      out_channels > kHeadDim || out_channels % 8 != 0)
+    return -3;
   CUtensorMap tm_q, tm_k, tm_v;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, 128)) return -1;
   if (encode_arena_map(&tm_k, kv_arena, uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 64)) return -1;
@@ -697,8 +749,10 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
   CopyCtx ctx;
   dcpk_fill_copy_ctx(&ctx, n_jobs > 0 ? job_src_ptrs : nullptr, n_jobs > 0 ? job_dst_ptrs : nullptr, job_stat_stride);
   const int smem = int(sizeof(PairSmem)) + 1024;
-  const int v = channels > 96 ? 0 : channels > 64 ? 1 : 2;
-  auto kernel = v == 2 ? attn_fwd_pair_kernel<64> : v == 1 ? attn_fwd_pair_kernel<96> : attn_fwd_pair_kernel<128>;
+  const bool form = out_type != 2 || out_channels != kHeadDim;
+  const int v = (channels > 96 ? 0 : channels > 64 ? 1 : 2) + 3 * form;
+  auto kernel = v == 5 ? attn_fwd_pair_kernel<64, true> : v == 4 ? attn_fwd_pair_kernel<96, true> : v == 3 ? attn_fwd_pair_kernel<128, true>
+              : v == 2 ? attn_fwd_pair_kernel<64, false> : v == 1 ? attn_fwd_pair_kernel<96, false> : attn_fwd_pair_kernel<128, false>;
   if (!g_pair_attr_set[v]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return -4;
@@ -707,7 +761,7 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
   // short calls begin while the kernel before them ends (see kSmallPass in attn_edge.cu; a round is 5 us and more)
   const cudaError_t rc = launch_overlapped(
       kernel, 2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream), 1, n_tiles <= 8 * kPairs, tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
-      static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, int(q_rows),
+      static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, out_type, out_channels, int(q_rows),
       n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

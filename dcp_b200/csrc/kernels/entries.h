@@ -6,7 +6,7 @@ extern "C" {
 int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* kv_arena, long kv_rows, int hq, int hkv, const void* tiles,
                        int n_tiles, const void* kv_entries, int n_kv_entries, const void* masks, int n_mask_rows,
                        void* const* out_ptrs, float* const* lse_ptrs, int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a,
-                       int block_size, float scale, int channels, const void* jobs, int n_jobs, void* const* job_src_ptrs,
+                       int out_type, int out_channels, int block_size, float scale, int channels, const void* jobs, int n_jobs, void* const* job_src_ptrs,
                        void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream);
 int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena, long kv_rows, int hq, int hkv,
                   const void* ctas, int n_ctas, const void* items, int n_items_total, int max_items, const void* masks,
@@ -15,6 +15,8 @@ int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const 
                   void* const* job_src_ptrs, void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream);
 int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int n_rows, int hq, int stat_stride, float* zero0, long nz0,
                        float* zero1, long nz1, void* stream);
+int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o, int d, void* d_o_rows, float* delta, int n_rows, int hq,
+                            int stat_stride, float* zero0, long nz0, float* zero1, long nz1, void* stream);
 int dcpk_pad_cast_rows(int type, const void* src0, void* dst0, long rows0, const void* src1, void* dst1, long rows1, int d,
                        void* stream);
 int dcpk_cut_cast_rows(int src_f32, int type, const void* src0, void* dst0, long rows0, const void* src1, void* dst1, long rows1,

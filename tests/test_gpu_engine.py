@@ -431,7 +431,8 @@ def test_native_calls_against_the_general_path(head_dim, dtype, kv_dtype, form):
         return (out.detach(), *grads), (_lib.LAUNCHES - before, ex.impl.kernel_launches - launches)
 
     (got, counted), (want, counted_too) = call(True), call(False)
-    assert counted == counted_too and all(a.dtype == b.dtype and a.shape == b.shape for a, b in zip(got, want))
+    assert counted[0] <= counted_too[0] and counted[1] == counted_too[1]   # conversions are part of other launches there
+    assert all(a.dtype == b.dtype and a.shape == b.shape for a, b in zip(got, want))
     assert torch.equal(got[0], want[0])
     for a, b in zip(got[1:], want[1:]):
         ulp = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}.get(a.dtype, 0.0)
