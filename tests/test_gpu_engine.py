@@ -400,7 +400,8 @@ def test_dcp_attention_reads_any_layout_and_keeps_calls_apart(head_dim, dtype):
 
 
 @pytest.mark.parametrize("head_dim,dtype,kv_dtype", [(128, torch.bfloat16, None), (128, torch.float16, None), (72, torch.bfloat16, None),
-                                                     (64, torch.float32, None), (128, torch.bfloat16, torch.float32)])
+                                                     (64, torch.float32, None), (24, torch.float32, None), (40, torch.float16, None),
+                                                     (128, torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("form", ["rows", "flat", "strided", "halves"])
 def test_native_calls_against_the_general_path(head_dim, dtype, kv_dtype, form):
     """The same call with its host side in native code and in Python: same output bits, types and shapes, and gradients
