@@ -26,7 +26,8 @@
 // with 64 channels 180 -> 172; what is left of it is L2's rate of fp32 additions, 20 bytes per cycle and SM); the CTAs of a split head group first add their shares up through distributed
 // shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
 // (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
-// every key tile as it comes: its last bits may differ from run to run.
+// every key tile as it comes: its last bits may differ from run to run where the CTAs are more than one wave or their lists
+// begin at the same query (see dcpk_attn_bwd_parts).
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
@@ -241,7 +242,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 float scale, const CopyJob* __restrict__ jobs, int n_jobs, const __grid_constant__ CopyCtx copy_ctx,
                 int n_copy_rows, int* __restrict__ status) {
   grid_let_next();
-  grid_wait();
   if (int(blockIdx.y) < n_copy_rows) {
     // ------------------------------------------------------------ operand fetch for the next stage
     run_copy_jobs(jobs, n_jobs, copy_ctx, blockIdx.y * gridDim.x + blockIdx.x, n_copy_rows * gridDim.x, threadIdx.x,
@@ -732,6 +732,38 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
   return cudaMemcpyToSymbol(g_bwd_timeline, &p, sizeof(p)) == cudaSuccess ? 0 : -5;
 }
 
+// Over how many CTAs a head group of `group` query heads is split, for `n_ctas` key tiles of `hkv` heads whose item lists have
+// n_items_total entries in all and at most max_items (0: not known, the group stays whole).
+//
+// A CTA visits its items once per query head of the group, or the group is split over several CTAs (a cluster, at most
+// the portable 8, which adds its parts of dK / dV up in a fixed order): shorter longest lists, and more CTAs to begin and
+// end, which takes one as long as 8 visits (2.2 us each).  The launch takes as long as its longest list, or as all visits
+// spread over the SMs, whichever is more; the split for which that is least is taken, the smallest of equals.  Over 78
+// batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128 channels) that
+// is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was above the SMs' average, but
+// seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads: 152 us before, 109 in two parts; eight
+// sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.
+// CTAs that all run at once add to a row of dQ in the order of their items, which in practice gives a short batch the same bits
+// in every run (300 of 300 for lists of up to 17 items that begin at different queries, as causal ones do).  They become more
+// than one wave only where that takes 32 visits (about 70 us) off the longest list; dQ's last bits differ from run to run then.
+// That has its price: four sequences of 300 to 2100 tokens, 8 / 2 heads, forward and backward, 131 us in two parts and one wave,
+// 117 in four parts; three of 640 to 1100 tokens, 16 / 4 heads, 143 and 118 us.
+extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total) {
+  constexpr long kBegin = 8;
+  auto visits = [&](int p) {   // times the SMs
+    return std::max(kSms * (long(max_items) * (group / p) + kBegin),
+                    long(n_items_total) * hkv * group + kBegin * n_ctas * hkv * p);
+  };
+  int parts = 1, in_one_wave = 0;   // the largest split whose CTAs all run at once, if there is one
+  for (int p = 1; max_items > 0 && p <= group && p <= kMaxParts; ++p) {
+    if (group % p != 0) continue;
+    if (long(n_ctas) * hkv * p <= kSms) in_one_wave = p;
+    else if (in_one_wave > 0 && long(max_items) * (group / in_one_wave - group / p) < 32) continue;
+    if (visits(p) < visits(parts)) parts = p;
+  }
+  return parts;
+}
+
 // Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  channels: of the arenas' 128, those that may be other
 // than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are the
 // lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
@@ -768,30 +800,15 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   }
   // about 16 fetch CTAs when there is something to fetch
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
-  // A CTA visits its items once per query head of the group, or the group is split over several CTAs (a cluster, at most
-  // the portable 8, which adds its parts of dK / dV up in a fixed order): shorter longest lists, and more CTAs to begin and
-  // end, which takes one as long as 8 visits (2.2 us each).  The launch takes as long as its longest list, or as all visits
-  // spread over the SMs, whichever is more; the split for which that is least is taken, the smallest of equals.  Over 78
-  // batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128 channels) the
-  // choice is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was above the
-  // SMs' average, but seldom into more than one wave, was 9 % off, 54 % at worst.  Four sequences of 300 to 2100 tokens,
-  // 8 / 2 heads: 91 us in two parts, 64 in four; 2048 tokens, 32 / 8 heads: 152 us before, 109 in two parts; eight sequences,
-  // 9105 tokens, 8 / 2 heads: 147 and 107 us.
-  const int group = hq / hkv;
-  constexpr long kBegin = 8;
-  auto visits = [&](int p) {   // times the SMs
-    return std::max(kSms * (long(max_items) * (group / p) + kBegin), long(n_items_total) * hq + kBegin * n_ctas * hkv * p);
-  };
-  int parts = 1;
-  for (int p = 2; max_items > 0 && p <= group && p <= kMaxParts; ++p)
-    if (group % p == 0 && visits(p) < visits(parts)) parts = p;
+  const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total);
   const int heads_per_cta = group / parts;
-  // Overlapped with the kernel before it only where all CTAs run at once: CTAs that begin together go through the queries
-  // together and find one another's tiles in L2, those that begin as the SMs come free do not (forward and backward of 121987
-  // tokens, mixed masks, 41.3 ms plain, 44.3 overlapped; 6168 tokens 1008 and 1050 us; 4040 tokens 116 and 108 us).
+  // A plain launch: CTAs that begin together go through the queries together and find one another's tiles in L2, those that begin as
+  // the SMs come free do not (forward and backward of 121987 tokens, mixed masks, 41.3 ms plain, 44.3 overlapped with the kernel
+  // before; 6168 tokens 1008 and 1050 us).  A single wave would gain 3 us of 134 (four sequences of 300 to 2100 tokens, 8 / 2
+  // heads), but its CTAs begin so far apart then that they add to dQ in another order in 1 to 24 of 60 runs.
   const dim3 grid(hkv * parts, n_ctas + n_copy_rows);
   const cudaError_t rc = launch_overlapped(
-      kernel, grid, kBwdThreads, smem, static_cast<cudaStream_t>(stream), unsigned(parts), long(grid.x) * grid.y <= kSms, tm_q, tm_do,
+      kernel, grid, kBwdThreads, smem, static_cast<cudaStream_t>(stream), unsigned(parts), false, tm_q, tm_do,
       tm_kv, tm_dq, tm_dkv, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
       static_cast<const int4*>(masks), lse, delta, pp, hq, hkv, heads_per_cta, stat_stride, n_dst, int(q_rows), int(kv_rows),
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);

@@ -335,3 +335,28 @@ def test_backward_of_an_earlier_call_gets_its_own_operands_on_several_ranks():
     for out, (q, kv) in zip(outs, calls):
         dq, dkv = torch.autograd.grad(out, (q, kv), torch.ones_like(out))
         assert torch.equal(dq, q) and torch.equal(dkv, kv)
+
+
+@pytest.mark.parametrize("raw,heads,kv_heads,want", [
+    ([1000, 300, 2100, 640], 8, 2, 2),    # 132 CTAs of at most 34 visits; four parts would be 264 and save 17
+    ([640, 1100, 900], 16, 4, 1),         # 88 CTAs in one part; 176 in two would save 18 visits
+    ([512, 1024, 2048, 4096], 8, 2, 4),   # 120 CTAs of 128 visits: 96 saved, so more than one wave
+    ([2048], 32, 8, 2),                   # 128 CTAs of 64 visits: 32 saved
+    ([700], 8, 2, 4),                     # 48 CTAs in four parts are one wave
+])
+def test_backward_of_a_short_batch_stays_in_one_wave(raw, heads, kv_heads, want):
+    """CTAs that all run at once give dQ the same bits in every run; a head group is split into more of them only where
+    that shortens the longest list by 32 visits."""
+    import ctypes
+    from dcp_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("the kernel library is not built")
+    block = 256
+    padded = pad_seqlens(raw, block)
+    ctx = get_default_execution_context(1, 1)
+    wl = generate_workload((sum(padded), heads, 128), (sum(padded), 2, kv_heads, 128), raw, padded, block, heads, ctx.comp_cost_model,
+                           masks.get_mask_fn("causal")(raw, padded, torch.int32), torch.bfloat16)
+    fw_wl, *_ = InstrCompiler(ctx, CompilerConfig()).compile(wl)
+    t = lower_all(ctx, fw_wl, build_backward=True)[ctx.devices()[0]].bwd[0]
+    got = _lib.load().dcpk_attn_bwd_parts(*(ctypes.c_int(x) for x in (t.n_ctas, kv_heads, heads // kv_heads, t.max_items, t.items.shape[0])))
+    assert got == want

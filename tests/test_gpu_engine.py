@@ -445,3 +445,24 @@ def test_native_calls_against_the_general_path(head_dim, dtype, kv_dtype, form):
     ex.impl._native = native
     ex.impl.time_calls = True        # the phases are looked at: the general path
     assert ex.impl.native() is None
+
+
+@pytest.mark.parametrize("raw,heads,kv_heads,head_dim,dtype", [([1000, 300, 2100, 640], 8, 2, 128, torch.bfloat16),
+                                                               ([1000, 300, 2100, 640], 8, 2, 64, torch.float32),
+                                                               ([640, 1100, 900], 16, 4, 128, torch.bfloat16)])
+def test_short_causal_calls_repeat_to_the_bit(raw, heads, kv_heads, head_dim, dtype):
+    """A backward whose CTAs all run at once adds to every row of dQ in the order of the CTAs' items (causal lists begin at
+    different queries): output and gradients have the same bits in every call."""
+    _need_gpu()
+    from dcp_b200.core.common import get_default_execution_context
+    from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test
+    dev = torch.device("cuda", 0)
+    ex, lq, lkv, ldo, *_ = prepare_dcp_distributed_attn_for_test(raw, heads, kv_heads, head_dim, 256, heads, get_default_execution_context(1, 1),
+                                                                 0, "causal", dtype, 3, device=dev, executor_impl="fused")
+    lq.requires_grad_(True), lkv.requires_grad_(True)
+    first = None
+    for _ in range(20):
+        out = DCPAttention.apply(ex, False, False, lq, lkv)
+        got = (out.detach(), *torch.autograd.grad(out, (lq, lkv), ldo))
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(got, first))
