@@ -466,3 +466,32 @@ def test_short_causal_calls_repeat_to_the_bit(raw, heads, kv_heads, head_dim, dt
         got = (out.detach(), *torch.autograd.grad(out, (lq, lkv), ldo))
         first = first or got
         assert all(torch.equal(a, b) for a, b in zip(got, first))
+
+
+@pytest.mark.parametrize("head_dim,dtype,rise,values", [(64, torch.float32, 54, 90), (64, torch.float16, 70, 0), (96, torch.bfloat16, 54, 90),
+                                                        (128, torch.float32, 70, 0), (128, torch.bfloat16, 54, 90)])
+def test_rising_scores_in_the_callers_form(head_dim, dtype, rise, values):
+    """Scores that rise by 2^rise behind the first key tile, with values of 2^values (a second pass over those tiles of queries), results
+    in the caller's type and width: within 2^-6 of the largest value of dense attention, as in the kernel's own tests."""
+    _need_gpu()
+    from dcp_b200.core.common import get_default_execution_context
+    from dcp_b200.planner import masks
+    from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test
+    from dcp_b200.runtime.layout import get_local_q_kv
+    from dcp_b200.runtime.simulate import dense_reference
+    dev, ctx, raw = torch.device("cuda", 0), get_default_execution_context(1, 1), [700, 260]
+    ex, _, _, _, q, kv, _, (wl, _), pad = prepare_dcp_distributed_attn_for_test(raw, 4, 2, head_dim, 256, 4, ctx, 0, "causal", dtype, 5,
+                                                                               device=dev, executor_impl="fused")
+    scale = head_dim ** -0.5
+    q[:, :2, 0] = 16.0
+    pos = torch.cat([torch.arange(n) for n in raw])
+    kv[:, 0, 0, 0] = ((pos >= 128) * (rise / (16.0 * scale * 1.4427))).to(dtype)
+    kv[:, 1] *= 2.0 ** values
+    q, kv = q.bfloat16().to(dtype), kv.bfloat16().to(dtype)
+    lq, lkv = (t.to(dev) for t in get_local_q_kv(q, kv, wl, ctx.devices()[0], raw))
+    out = DCPAttention.apply(ex, False, False, lq, lkv)
+    torch.cuda.synchronize()
+    ex.impl.check_status()
+    ref, *_ = dense_reference(q, kv, raw, pad, masks.get_mask_fn("causal")(raw, pad, torch.int32), scale)
+    assert out.dtype == dtype and out.shape == lq.shape
+    assert ((out.cpu().double() - ref).abs() <= 2.0 ** -6 * ref.abs().max()).all()

@@ -189,6 +189,34 @@ def test_attention_forward_pairs_of_tiles(dev, nkv, kind):
     assert out[nq:].abs().max() == 0
 
 
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("rise,values", [(54, 0), (54, 90), (80, 0), (80, 90)])
+def test_attention_forward_rising_scores_and_large_values(dev, d, rise, values):
+    """Scores that rise by 2^rise behind the first key tile, with values of 2^values: the row sum, or only O, leaves what the first
+    pass over a tile holds, and the result is representable all the same.  Bound as above, 2^-6 of the largest value."""
+    nq, nkv, hq = 300, 384, 4
+    g = torch.Generator().manual_seed(rise + values)
+    q, kv = torch.zeros(nq, hq, 128), torch.zeros(nkv, 2, 2, 128)
+    q[..., :d], kv[..., :d] = torch.randn(nq, hq, d, generator=g), torch.randn(nkv, 2, 2, d, generator=g)
+    kv[:, 1] *= 2.0 ** values
+    scale = d ** -0.5
+    q[:, :2, 0] = 16.0                                                                     # the first KV head's queries
+    kv[:, 0, 0, 0] = (torch.arange(nkv) >= 128) * (rise / (16.0 * scale * np.log2(np.e)))
+    q, kv = q.bfloat16().to(dev), kv.bfloat16().to(dev)
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = nkv
+    rng[7:11, 1] = 100                                                                     # rows that stay in the first key tile
+    out, lse = torch.zeros_like(q), torch.zeros(hq, nq, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)], 512, dev), [out], [lse], scale, status, channels=d)
+    assert status.item() == 0
+    k64, v64 = (kv[:, j].double().repeat_interleave(2, 1).permute(1, 0, 2) for j in (0, 1))
+    s = (q.double().permute(1, 0, 2) @ k64.transpose(1, 2) * scale).masked_fill(~A.ranges_to_dense(rng, nkv).to(dev), float("-inf"))
+    ref, rl = (s.softmax(-1) @ v64).permute(1, 0, 2), torch.logsumexp(s, -1)
+    assert ((out.double() - ref).abs() <= 2.0 ** -6 * ref.abs().max()).all()
+    assert ((lse - rl).abs() < 1e-3 + 2.0 ** -22 * rl.abs()).all()
+
+
 @pytest.mark.parametrize("nq,nkv", [(1, 1), (257, 300)])
 def test_attention_forward_result_at_16_bytes(dev, nq, nkv):
     """A result whose rows begin 16 bytes off a sector: the same bits as at the start of one."""
