@@ -69,6 +69,7 @@
 #include "entries.h"
 #include "launch.cuh"
 #include "ptx.cuh"
+#include "smem_limit.h"
 #include "tmap.cuh"
 
 namespace dcpk {
@@ -716,7 +717,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 }
 
 static constexpr int kSms = 148, kMaxParts = 8;
-static int g_bwd_attr_set[4] = {0, 0, 0, 0};
+static std::atomic<uint64_t> g_bwd_smem_raised[4];
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
 
 }  // namespace dcpk
@@ -794,10 +795,7 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   const int v = g_bwd_timeline_host ? 3 : channels > 96 ? 0 : channels > 64 ? 1 : 2;
   auto kernel = v == 3 ? attn_bwd_kernel<true, 128> : v == 2 ? attn_bwd_kernel<false, 64>
               : v == 1 ? attn_bwd_kernel<false, 96> : attn_bwd_kernel<false, 128>;
-  if (!g_bwd_attr_set[v]) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-    g_bwd_attr_set[v] = 1;
-  }
+  if (raise_smem_limit(kernel, smem, g_bwd_smem_raised[v]) != cudaSuccess) return -4;
   // about 16 fetch CTAs when there is something to fetch
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
   const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total);

@@ -22,6 +22,7 @@
 
 #include "attn_common.cuh"
 #include "ptx.cuh"
+#include "smem_limit.h"
 #include "tmap.cuh"
 
 namespace dcpk {
@@ -428,7 +429,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, kStatusBarrierTimeout);
 }
 
-static int g_fwd_attr_set[4] = {0, 0, 0, 0};
+static std::atomic<uint64_t> g_fwd_smem_raised[4];
 static long long* g_fwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
 
 }  // namespace dcpk
@@ -465,10 +466,7 @@ extern "C" int dcpk_attn_fwd(const void* q_arena, long q_rows, const void* kv_ar
                             int, int, int, int, int, int, int, int, int, int, float, int*);
   static const KernelFn kernels[4] = {attn_fwd_kernel<false, false>, attn_fwd_kernel<true, false>,
                                       attn_fwd_kernel<false, true>, attn_fwd_kernel<true, true>};
-  if (!g_fwd_attr_set[v]) {
-    if (cudaFuncSetAttribute(kernels[v], cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-    g_fwd_attr_set[v] = 1;
-  }
+  if (raise_smem_limit(kernels[v], smem, g_fwd_smem_raised[v]) != cudaSuccess) return -4;
   kernels[v]<<<n_tiles, kFwdThreads, smem, static_cast<cudaStream_t>(stream)>>>(
       tm_q, tm_kv, static_cast<const AttnTile*>(tiles), static_cast<const KvEntry*>(kv_entries),
       static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, int(q_rows), block_size,

@@ -71,6 +71,7 @@
 #include "entries.h"
 #include "launch.cuh"
 #include "ptx.cuh"
+#include "smem_limit.h"
 #include "tmap.cuh"
 
 namespace dcpk {
@@ -724,7 +725,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, kStatusBarrierTimeout);
 }
 
-static int g_pair_attr_set[6] = {0, 0, 0, 0, 0, 0};
+static std::atomic<uint64_t> g_pair_smem_raised[6];
 
 }  // namespace dcpk
 
@@ -763,11 +764,7 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
   const int v = (channels > 96 ? 0 : channels > 64 ? 1 : 2) + 3 * form;
   auto kernel = v == 5 ? attn_fwd_pair_kernel<64, true> : v == 4 ? attn_fwd_pair_kernel<96, true> : v == 3 ? attn_fwd_pair_kernel<128, true>
               : v == 2 ? attn_fwd_pair_kernel<64, false> : v == 1 ? attn_fwd_pair_kernel<96, false> : attn_fwd_pair_kernel<128, false>;
-  if (!g_pair_attr_set[v]) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -4;
-    g_pair_attr_set[v] = 1;
-  }
+  if (raise_smem_limit(kernel, smem, g_pair_smem_raised[v]) != cudaSuccess) return -4;
   // short calls begin while the kernel before them ends (see kSmallPass in attn_edge.cu; a round is 5 us and more)
   const cudaError_t rc = launch_overlapped(
       kernel, 2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream), 1, n_tiles <= 8 * kPairs, tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),

@@ -1,0 +1,39 @@
+"""Host-side pieces of the native libraries that need no GPU."""
+import subprocess
+from pathlib import Path
+
+from dcp_b200.csrc import build
+
+FAKE_RUNTIME = r"""
+#include <cstdio>
+#include <initializer_list>
+#include "smem_limit.h"
+static int device = 0, raised_on[70] = {}, fail = 0;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) {
+  if (fail) return cudaErrorInvalidValue;
+  ++raised_on[device];
+  return cudaSuccess;
+}
+static void kernel() {}
+int main() {
+  std::atomic<uint64_t> raised{0};
+  fail = 1;
+  if (dcpk::raise_smem_limit(kernel, 200000, raised) == cudaSuccess) return 1;   // a refusal is reported, and asked again
+  fail = 0;
+  for (int d : {0, 1, 0, 1, 63, 63, 0, 64, 64}) {
+    device = d;
+    if (dcpk::raise_smem_limit(kernel, 200000, raised) != cudaSuccess) return 2;
+  }
+  std::printf("%d %d %d %d\n", raised_on[0], raised_on[1], raised_on[63], raised_on[64]);
+}
+"""
+
+
+def test_shared_memory_limit_is_raised_once_on_each_device(tmp_path):
+    """Against a fake runtime: the limit belongs to a device, so a kernel's first launch on a second one raises it again."""
+    src, exe = tmp_path / "fake.cpp", tmp_path / "fake"
+    src.write_text(FAKE_RUNTIME)
+    cuda = Path(build._nvcc()).resolve().parent.parent / "include"
+    subprocess.run(["g++", "-std=c++17", "-I%s" % build.KERNEL_DIR, "-I%s" % cuda, str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], check=True, stdout=subprocess.PIPE, text=True).stdout.split() == ["1", "1", "1", "2"]
