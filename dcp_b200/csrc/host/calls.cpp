@@ -11,6 +11,7 @@
 // Only plain calls are taken: tensors on the arenas' device, contiguous, 16-byte aligned, of a type the row kernels read.
 // For anything else the functions return nothing before they launch anything, and the caller goes the general way.
 #include <ATen/ATen.h>
+#include <c10/core/DeviceGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <nvtx3/nvToolsExt.h>
 #include <pybind11/stl.h>
@@ -47,9 +48,11 @@ int row_type(const Tensor& t) {
   }
 }
 
-struct Range {
-  explicit Range(const char* name) { nvtxRangePushA(name); }
-  ~Range() { nvtxRangePop(); }
+// A call: on the arenas' device, whichever is current, and a range for a profiler.
+struct Call {
+  c10::DeviceGuard device;
+  Call(const char* name, const Tensor& arena) : device(arena.device()) { nvtxRangePushA(name); }
+  ~Call() { nvtxRangePop(); }
 };
 
 // One program's launches.  Holds its tables and the arenas; nothing in it changes after construction, so threads may
@@ -127,7 +130,7 @@ class SingleRankAttention {
     if (!arena_like(q_in, q_local_rows, q.size(1)) || !arena_like(kv_in, kv_local_rows, 2 * kv.size(2)) || kv_in.dim() != 4 ||
         !arena_like(o, q_local_rows, q.size(1)) || !statistics(l))
       return false;
-    Range range("dcp.attention.fwd");
+    Call call("dcp.attention.fwd", q);
     nvtxMarkA("fwd:wait inputs of peers");
     launch_forward(q_in, kv_in, o, l, scale);
     nvtxMarkA("fwd:kernels (with operand fetch)");
@@ -141,7 +144,7 @@ class SingleRankAttention {
     if (!has_bwd || !arena_like(q_in, q_local_rows, q.size(1)) || !arena_like(kv_in, kv_local_rows, 2 * kv.size(2)) || kv_in.dim() != 4 ||
         !arena_like(d_o, q_local_rows, q.size(1)) || d_o.size(0) != q_local_rows || !arena_like(o, q_local_rows, q.size(1)) || !statistics(l))
       return false;
-    Range range("dcp.attention.bwd");
+    Call call("dcp.attention.bwd", q);
     launch_backward(q_in, d_o, kv_in, o, l, dl ? *dl : at::empty_like(l), kHeadDim, scale);
     return true;
   }
@@ -152,7 +155,7 @@ class SingleRankAttention {
     const long hq = q.size(1), hkv = kv.size(2);
     if (!rows_of(q_in, q_local_rows, hq, d) || !rows_of(kv_in, kv_local_rows, 2 * hkv, d) || q_in.scalar_type() != kv_in.scalar_type())
       return std::nullopt;
-    Range range("dcp.attention.fwd");
+    Call call("dcp.attention.fwd", q);
     const bool in_place = d == kHeadDim && q_in.scalar_type() == at::kBFloat16;
     int entries = 1;
     Tensor o, l;
@@ -192,7 +195,7 @@ class SingleRankAttention {
         l_in.is_neg())
       return std::nullopt;
     const Tensor l = l_in.view({hq, q_local_rows});
-    Range range("dcp.attention.bwd");
+    Call call("dcp.attention.bwd", q);
     const bool in_place = d == kHeadDim && q_in.scalar_type() == at::kBFloat16;
     int entries = 3;
     if (!in_place && reload) {
