@@ -121,6 +121,8 @@ def build_calls(force: bool = False) -> Path:
 
     OBJ_DIR.mkdir(exist_ok=True)
     srcs = sorted(HOST_DIR.glob("*.cpp"))
+    if not srcs:
+        raise RuntimeError(f"no sources of the native attention calls in {HOST_DIR}: this copy of the package is incomplete")
     out = calls_lib_path()
     stamp = OBJ_DIR / "calls.stamp"
     digest = _digest(srcs + [KERNEL_DIR / "entries.h"]) + " " + torch.__version__

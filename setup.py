@@ -1,6 +1,7 @@
-"""`pip install -e . --no-build-isolation` builds the two native libraries in-tree
-(CUDA kernels for sm_100a with nvcc, the C++ planner with g++ + pybind11) before installing;
-the same build is available without pip as `python -m dcp_b200.csrc.build`."""
+"""`pip install -e . --no-build-isolation` builds the three native libraries in-tree (CUDA kernels for sm_100a with
+nvcc, the C++ planner with g++ + pybind11, the host side of attention calls with g++ + torch) before installing; without
+build isolation, because the last one is for the very torch it will run with.  The same build is available without pip as
+`python -m dcp_b200.csrc.build`."""
 import os
 import sys
 

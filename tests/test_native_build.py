@@ -1,6 +1,10 @@
 """Host-side pieces of the native libraries that need no GPU."""
+import fnmatch
 import subprocess
+import tomllib
 from pathlib import Path
+
+import pytest
 
 from dcp_b200.csrc import build
 
@@ -37,3 +41,16 @@ def test_shared_memory_limit_is_raised_once_on_each_device(tmp_path):
     cuda = Path(build._nvcc()).resolve().parent.parent / "include"
     subprocess.run(["g++", "-std=c++17", "-I%s" % build.KERNEL_DIR, "-I%s" % cuda, str(src), "-o", str(exe)], check=True)
     assert subprocess.run([str(exe)], check=True, stdout=subprocess.PIPE, text=True).stdout.split() == ["1", "1", "1", "2"]
+
+
+def test_package_data_holds_every_native_source():
+    """An installed copy can rebuild all of its libraries."""
+    patterns = tomllib.loads((build.PKG.parent / "pyproject.toml").read_text())["tool"]["setuptools"]["package-data"]["dcp_b200"]
+    sources = [p.relative_to(build.PKG).as_posix() for p in build.HERE.rglob("*") if p.suffix in (".cu", ".cuh", ".h", ".hpp", ".cpp")]
+    assert len(sources) > 20 and [s for s in sources if not any(fnmatch.fnmatch(s, p) for p in patterns)] == []
+
+
+def test_build_of_an_incomplete_copy_says_so(monkeypatch, tmp_path):
+    monkeypatch.setattr(build, "HOST_DIR", tmp_path)
+    with pytest.raises(RuntimeError, match="incomplete"):
+        build.build_calls(force=True)
