@@ -7,6 +7,7 @@ is an error, never a silent fallback to eager PyTorch.
 from __future__ import annotations
 
 import ctypes
+import sysconfig
 from pathlib import Path
 
 import torch
@@ -48,13 +49,21 @@ def stream_handle():
 LAUNCHES = 0  # kernel-entry calls made through this library since import (each launches >= 1 kernel)
 
 
+def calls_path() -> Path:
+    return lib_path().parent / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
 def calls():
     """The native host side of single-rank attention calls (``csrc/host/calls.cpp``)."""
     load()
+    p = calls_path()
+    if not p.exists():
+        raise RuntimeError(f"{p} is missing: build it with `python -m dcp_b200.csrc.build`")
     try:
         from .. import _calls
-    except ImportError as e:
-        raise RuntimeError("dcp_b200/_calls is missing: build it with `python -m dcp_b200.csrc.build`") from e
+    except ImportError as e:   # it is there: most likely built for another torch
+        raise RuntimeError(f"{p} does not load with torch {torch.__version__} ({e}): rebuild it with "
+                           "`python -m dcp_b200.csrc.build --force`") from e
     return _calls
 
 

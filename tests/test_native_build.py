@@ -1,12 +1,15 @@
 """Host-side pieces of the native libraries that need no GPU."""
 import fnmatch
 import subprocess
+import sys
 import tomllib
 from pathlib import Path
 
 import pytest
 
+import dcp_b200
 from dcp_b200.csrc import build
+from dcp_b200.ops import _lib
 
 FAKE_RUNTIME = r"""
 #include <cstdio>
@@ -54,3 +57,15 @@ def test_build_of_an_incomplete_copy_says_so(monkeypatch, tmp_path):
     monkeypatch.setattr(build, "HOST_DIR", tmp_path)
     with pytest.raises(RuntimeError, match="incomplete"):
         build.build_calls(force=True)
+
+
+def test_missing_and_unloadable_native_calls_are_told_apart(monkeypatch, tmp_path):
+    monkeypatch.setattr(_lib, "load", lambda: None)
+    monkeypatch.setattr(_lib, "calls_path", lambda: tmp_path / "_calls.so")
+    with pytest.raises(RuntimeError, match="missing"):
+        _lib.calls()
+    (tmp_path / "_calls.so").touch()
+    monkeypatch.delattr(dcp_b200, "_calls", raising=False)
+    monkeypatch.setitem(sys.modules, "dcp_b200._calls", None)      # the import fails
+    with pytest.raises(RuntimeError, match="does not load"):
+        _lib.calls()
