@@ -59,9 +59,9 @@ struct Call {
 // share it (what they compute shares the arenas all the same).
 class SingleRankAttention {
  public:
-  Tensor q, kv, dout, out, lse, delta, dq, dkv, part_out, part_lse, status;                // arenas
-  Tensor tiles, kv_entries, fwd_masks, ctas, items, bwd_masks;                             // tables
-  int n_tiles = 0, block_size = 0, n_ctas = 0, max_items = 0;
+  Tensor q, kv, dout, lse, dq, dkv, part_out, part_lse, status;      // arenas
+  Tensor tiles, kv_entries, fwd_masks, ctas, items, bwd_masks;       // tables
+  int n_tiles = 0, n_ctas = 0, max_items = 0;
   long q_local_rows = 0, kv_local_rows = 0, q_rows = 0, kv_rows = 0;
   bool has_bwd = false, all_rows_written = true;
   int channels = kHeadDim;
@@ -90,8 +90,8 @@ class SingleRankAttention {
     check(dcpk_attn_fwd_pair(q_in.const_data_ptr(), q_in.size(0), kv_in.const_data_ptr(), kv_in.size(0), int(q.size(1)),
                              int(kv.size(2)), tiles.const_data_ptr(), n_tiles, kv_entries.const_data_ptr(),
                              int(kv_entries.size(0)), fwd_masks.const_data_ptr(), int(fwd_masks.size(0)), outs, lses, 2,
-                             int(part_lse.size(1)), int(l.size(1)), 1, out_type, out_channels, block_size, float(scale), channels, nullptr, 0, nullptr,
-                             nullptr, 0, status.data_ptr<int>(), stream()),
+                             int(part_lse.size(1)), int(l.size(1)), 1, out_type, out_channels, float(scale), channels, nullptr, 0, nullptr, nullptr, 0,
+                             status.data_ptr<int>(), stream()),
           "dcpk_attn_fwd_pair");
   }
 
@@ -224,8 +224,8 @@ PYBIND11_MODULE(_calls, m) {
       .def(py::init([](const py::dict& d) {
         auto a = std::make_unique<A>();
         auto tensor = [&](const char* k) { return d[k].cast<Tensor>(); };
-        for (auto [k, t] : {std::pair<const char*, Tensor*>{"q", &a->q}, {"kv", &a->kv}, {"dout", &a->dout}, {"out", &a->out},
-                            {"lse", &a->lse}, {"dq", &a->dq}, {"dkv", &a->dkv}, {"part_out", &a->part_out},
+        for (auto [k, t] : {std::pair<const char*, Tensor*>{"q", &a->q}, {"kv", &a->kv}, {"dout", &a->dout}, {"lse", &a->lse},
+                            {"dq", &a->dq}, {"dkv", &a->dkv}, {"part_out", &a->part_out},
                             {"part_lse", &a->part_lse}, {"status", &a->status}, {"tiles", &a->tiles},
                             {"kv_entries", &a->kv_entries}, {"fwd_masks", &a->fwd_masks}})
           *t = tensor(k);
@@ -234,7 +234,7 @@ PYBIND11_MODULE(_calls, m) {
           a->ctas = tensor("ctas"), a->items = tensor("items"), a->bwd_masks = tensor("bwd_masks");
           a->n_ctas = d["n_ctas"].cast<int>(), a->max_items = d["max_items"].cast<int>();
         }
-        a->n_tiles = d["n_tiles"].cast<int>(), a->block_size = d["block_size"].cast<int>();
+        a->n_tiles = d["n_tiles"].cast<int>();
         a->q_local_rows = d["q_local_rows"].cast<long>(), a->kv_local_rows = d["kv_local_rows"].cast<long>();
         a->q_rows = d["q_rows"].cast<long>(), a->kv_rows = d["kv_rows"].cast<long>();
         a->all_rows_written = d["all_rows_written"].cast<bool>(), a->channels = d["channels"].cast<int>();

@@ -741,7 +741,7 @@ using namespace dcpk;
 extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* kv_arena, long kv_rows, int hq,
                                   int hkv, const void* tiles, int n_tiles, const void* kv_entries, int n_kv_entries,
                                   const void* masks, int n_mask_rows, void* const* out_ptrs, float* const* lse_ptrs,
-                                  int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a, int out_type, int out_channels, int block_size,
+                                  int n_dst, int lse_stride_a, int lse_stride_b, int n_dst_a, int out_type, int out_channels,
                                   float scale, int channels, const void* jobs, int n_jobs, void* const* job_src_ptrs,
                                   void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream) {
   if (n_tiles <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on

@@ -251,7 +251,8 @@ def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, o
             ctypes.c_int(len(out_dsts)), ctypes.c_int(lse_stride),
             ctypes.c_int(lse_stride if lse_stride_b is None else lse_stride_b),
             ctypes.c_int(len(out_dsts) if n_dst_a is None else n_dst_a), ctypes.c_int(2), ctypes.c_int(HEAD_DIM),
-            ctypes.c_int(tables.block_size), ctypes.c_float(scale), ctypes.c_int(channels), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
+            ctypes.c_float(scale), ctypes.c_int(channels), *_job_args(jobs, job_ctx), _lib.ptr(status),
+            _lib.stream_handle())
         _lib.check(rc, "dcpk_attn_fwd_pair")
         return
     assert jobs is None or jobs.shape[0] == 0, "only the two-tile forward kernel carries copy jobs"

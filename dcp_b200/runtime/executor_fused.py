@@ -152,9 +152,9 @@ class FusedAttentionExecutor:
         if self.world > 1 or p.n_stages != 1 or self.merge_ops.shape[0] or f[0] is None or f[0].tile_m != attn_ops.TILE_M_PAIR:
             return None
         f, b = f[0], b[0] if len(b) else None
-        d = {"q": self.q, "kv": self.kv, "dout": self.dout, "out": self.out, "lse": self.lse, "dq": self.dq, "dkv": self.dkv,
+        d = {"q": self.q, "kv": self.kv, "dout": self.dout, "lse": self.lse, "dq": self.dq, "dkv": self.dkv,
              "part_out": self.part_out, "part_lse": self.part_lse, "status": self.arena.status, "tiles": f.tiles,
-             "kv_entries": f.kv_entries, "fwd_masks": f.masks, "n_tiles": f.n_tiles, "block_size": f.block_size,
+             "kv_entries": f.kv_entries, "fwd_masks": f.masks, "n_tiles": f.n_tiles,
              "q_local_rows": p.q_local_rows, "kv_local_rows": p.kv_local_rows, "q_rows": p.q_rows, "kv_rows": p.kv_rows,
              "all_rows_written": self._all_rows_written, "channels": self.channels}
         if b is not None:
