@@ -61,7 +61,7 @@ class SingleRankAttention {
  public:
   Tensor q, kv, dout, lse, dq, dkv, part_out, part_lse, status;      // arenas
   Tensor tiles, kv_entries, fwd_masks, ctas, items, bwd_masks;       // tables
-  int n_tiles = 0, n_ctas = 0, max_items = 0;
+  int n_tiles = 0, n_ctas = 0, max_items = 0, dq_levels = 0;
   long q_local_rows = 0, kv_local_rows = 0, q_rows = 0, kv_rows = 0;
   bool has_bwd = false, all_rows_written = true;
   int channels = kHeadDim;
@@ -114,12 +114,15 @@ class SingleRankAttention {
             "dcpk_attn_bwd_prep_cast");
     nvtxMarkA("bwd:dout copy, delta, zero accumulators");
     nvtxMarkA("bwd:wait inputs of peers");
+    const long bytes = dcpk_attn_bwd_workspace(int(items.size(0)), q_local_rows, int(hq), channels, dq_levels);
+    Tensor workspace;
+    if (bytes > 0) workspace = at::empty({bytes}, q.options().dtype(at::kByte));
     float* dqs[1] = {dq.data_ptr<float>()};
     float* dkvs[1] = {dkv.data_ptr<float>()};
     check(dcpk_attn_bwd(q_in.const_data_ptr(), d_o.const_data_ptr(), q_local_rows, kv_in.const_data_ptr(), kv_in.size(0), int(hq),
                         int(hkv), ctas.const_data_ptr(), n_ctas, items.const_data_ptr(), int(items.size(0)), max_items,
                         bwd_masks.const_data_ptr(), int(bwd_masks.size(0)), l.const_data_ptr<float>(), dl.const_data_ptr<float>(),
-                        int(l.size(1)), dqs, dkvs, 1, float(scale), channels, nullptr, 0, nullptr, nullptr, 0,
+                        int(l.size(1)), dqs, dkvs, 1, float(scale), channels, dq_levels, bytes > 0 ? workspace.data_ptr() : nullptr, nullptr, 0, nullptr, nullptr, 0,
                         status.data_ptr<int>(), stream()),
           "dcpk_attn_bwd");
     nvtxMarkA("bwd:kernels (with operand fetch)");
@@ -233,6 +236,7 @@ PYBIND11_MODULE(_calls, m) {
         if (a->has_bwd) {
           a->ctas = tensor("ctas"), a->items = tensor("items"), a->bwd_masks = tensor("bwd_masks");
           a->n_ctas = d["n_ctas"].cast<int>(), a->max_items = d["max_items"].cast<int>();
+          a->dq_levels = d["dq_levels"].cast<int>();
         }
         a->n_tiles = d["n_tiles"].cast<int>();
         a->q_local_rows = d["q_local_rows"].cast<long>(), a->kv_local_rows = d["kv_local_rows"].cast<long>();

@@ -26,8 +26,8 @@
 // with 64 channels 180 -> 172; what is left of it is L2's rate of fp32 additions, 20 bytes per cycle and SM); the CTAs of a split head group first add their shares up through distributed
 // shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
 // (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
-// every key tile as it comes: its last bits may differ from run to run where the CTAs are more than one wave or their lists
-// begin at the same query (see dcpk_attn_bwd_parts).
+// every key tile as it comes, in short launches through buffers of at most two additions each, which are summed afterwards (see
+// dq_level): these give the same bits in every run, the last bits of longer ones differ.
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
@@ -117,6 +117,14 @@ __device__ __forceinline__ bool item_ok(const BwdItem& it, int q_rows, int stat_
            it.q_row + it.n_rows > stat_stride || it.dq_dev >= n_dst || it.mask_row < 0 ||
            (!it.full && it.mask_row + it.n_rows > n_mask_rows) ||
            (it.dq_dev >= 0 && (it.dq_row < 0 || it.dq_row + it.n_rows > q_rows)));
+}
+
+// A row of dQ is added to by every key tile that it sees, as these come.  Two additions to zero give the same bits in either order,
+// three do not: with a workspace each 256 keys (of the positions of an item's concatenated KV) have a buffer of their own, a level,
+// and the levels are summed afterwards, in their order.  Level 0 is the accumulator itself, and the only one without a workspace.
+__device__ __forceinline__ int dq_level(int kv_pos0, int n_levels) {
+  const int level = kv_pos0 >> 8;
+  return level > 0 && level < n_levels ? level : 0;
 }
 
 struct BwdPtrs {
@@ -236,7 +244,7 @@ template <bool kTL, int kD>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_kv, const __grid_constant__ CUtensorMap tm_dq,
-                const __grid_constant__ CUtensorMap tm_dkv,
+                const __grid_constant__ CUtensorMap tm_dkv, const __grid_constant__ CUtensorMap tm_levels, int n_levels,
                 const BwdCta* __restrict__ ctas, const BwdItemDesc* __restrict__ items, const int4* __restrict__ masks,
                 const float* __restrict__ lse, const float* __restrict__ delta, BwdPtrs ptrs, int hq, int hkv,
                 int heads_per_cta, int stat_stride, int n_dst, int q_rows, int kv_rows, int n_mask_rows, int n_items_total,
@@ -558,7 +566,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         __syncwarp();
         if (cur.dq_dev == 0) {
           if (lane == 0) {
-            tma_reduce_add_3d(&tm_dq, stage, ch0 + b * 32, cur.head, cur.dq_row + quad * 32);
+            const int level = dq_level(cur.kv_pos0, n_levels), row = cur.dq_row + quad * 32;
+            tma_reduce_add_3d(level > 0 ? &tm_levels : &tm_dq, stage, ch0 + b * 32, cur.head, level > 0 ? (level - 1) * q_rows + row : row);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         } else if (quad * 32 + lane < cur.n_rows) {
@@ -716,7 +725,64 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-static constexpr int kSms = 148, kMaxParts = 8;
+// The levels of dQ above the first, [n_levels - 1, q_rows, hq, kPitch]: zeroed where they will be added to, or summed into dQ.  Bound by
+// L2.  A CTA takes kLevelRows rows; which levels these have is in the items that cover them, so it looks through the whole table.
+static constexpr int kLevelRows = 4;
+
+template <int kPitch, bool kSum>
+__global__ void __launch_bounds__(256) dq_levels_kernel(const BwdItemDesc* __restrict__ items, int n_items, float* __restrict__ levels,
+                                                        int n_levels, float* __restrict__ dq, int q_rows, int hq, int channels) {
+  __shared__ uint32_t present[kLevelRows][2];   // a bit per level
+  const int row0 = blockIdx.x * kLevelRows;
+  if (threadIdx.x < 2 * kLevelRows) present[threadIdx.x >> 1][threadIdx.x & 1] = 0;
+  __syncthreads();
+  grid_let_next();
+  grid_wait();
+  for (int i = threadIdx.x; i < n_items; i += 256) {
+    const BwdItemDesc d = items[i];
+    if (d.dq_dev != 0) continue;
+    const int level = dq_level(d.kv_pos0, n_levels);
+    for (int row = max(d.dq_row, row0); row < min(min(d.dq_row + d.n_rows, q_rows), row0 + kLevelRows); ++row)
+      atomicOr(&present[row - row0][level >> 5], 1u << (level & 31));
+  }
+  __syncthreads();
+  const size_t level_size = size_t(q_rows) * hq * kPitch;
+  for (int r = 0; r < kLevelRows; ++r) {
+    const uint64_t above = (uint64_t(present[r][1]) << 32 | present[r][0]) & ~uint64_t(1);
+    if (above == 0) continue;
+    for (int c = threadIdx.x; c < hq * (kPitch / 4); c += 256) {   // four channels of a head
+      const int head = c / (kPitch / 4), ch = c % (kPitch / 4) * 4;
+      if (ch >= channels) continue;
+      const size_t in_row = size_t(row0 + r) * hq + head;
+      float* at = levels + in_row * kPitch + ch;
+      float4* acc = reinterpret_cast<float4*>(dq + in_row * kHeadDim + ch);
+      float4 sum = kSum ? *acc : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint64_t left = above; left != 0;) {
+        float4 v[4];   // of four levels in flight
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool there = left != 0;
+          float4* p = reinterpret_cast<float4*>(at + size_t(there ? __ffsll(left) - 2 : 0) * level_size);
+          left &= left - 1;
+          if (kSum) v[u] = there ? *p : make_float4(0.f, 0.f, 0.f, 0.f);
+          else if (there) *p = sum;
+        }
+        if (kSum)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) { sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w; }
+      }
+      if (kSum) *acc = sum;
+    }
+  }
+}
+
+static constexpr int kSms = 148, kMaxParts = 8, kMaxLevels = 64;
+// Launches of up to so many bytes of dQ tiles (one per visit) have levels, if these take no more than the other number.  Levels cost
+// what it takes to clear and to sum them: four sequences of 300 to 2100 tokens, 8 / 2 heads, 110 MB, forward and backward, 107 us
+// without and 135 with them, 2048 tokens, 71 MB, 96 and 108.  Above, what is added to no longer stays in L2: 2048 tokens, 32 / 8 heads, 285 MB,
+// 169 and 280 us, 4096 tokens, 8 / 2 heads, 277 MB, 152 and 235.  (Tiles of their own for all visits, stored and then summed, took
+// 150 us for the first.)
+static constexpr long kMaxVisitBytes = 128l << 20, kMaxWorkspace = 512l << 20;
 static std::atomic<uint64_t> g_bwd_smem_raised[4];
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
 
@@ -733,6 +799,16 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
   return cudaMemcpyToSymbol(g_bwd_timeline, &p, sizeof(p)) == cudaSuccess ? 0 : -5;
 }
 
+static int level_pitch(int channels) { return channels > 64 ? kHeadDim : 64; }
+
+// Bytes of the workspace of dcpk_attn_bwd for item lists of `n_levels` levels (see dq_level; 0: not known); 0: there is none.
+extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, int channels, int n_levels) {
+  if (n_levels < 2 || n_levels > kMaxLevels) return 0;
+  const long pitch = level_pitch(channels) * long(sizeof(float));
+  const long bytes = (n_levels - 1) * q_rows * hq * pitch;
+  return long(n_items_total) * hq * kQTile * pitch <= kMaxVisitBytes && bytes <= kMaxWorkspace ? bytes : 0;
+}
+
 // Over how many CTAs a head group of `group` query heads is split, for `n_ctas` key tiles of `hkv` heads whose item lists have
 // n_items_total entries in all and at most max_items (0: not known, the group stays whole).
 //
@@ -744,12 +820,10 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
 // is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was above the SMs' average, but
 // seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads: 152 us before, 109 in two parts; eight
 // sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.
-// CTAs that all run at once add to a row of dQ in the order of their items, which in practice gives a short batch the same bits
-// in every run (300 of 300 for lists of up to 17 items that begin at different queries, as causal ones do).  They become more
-// than one wave only where that takes 32 visits (about 70 us) off the longest list; dQ's last bits differ from run to run then.
-// That has its price: four sequences of 300 to 2100 tokens, 8 / 2 heads, forward and backward, 131 us in two parts and one wave,
-// 117 in four parts; three of 640 to 1100 tokens, 16 / 4 heads, 143 and 118 us.
-extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total) {
+// CTAs that all run at once add to a row of dQ in the order of their items, and as long as their lists are short and begin at
+// different queries that is nearly the same in every run.  Without `any_wave` (dQ has levels, whose order does not matter) they
+// become more than one wave only where that takes 32 visits (about 70 us) off the longest list.
+extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total, int any_wave) {
   constexpr long kBegin = 8;
   auto visits = [&](int p) {   // times the SMs
     return std::max(kSms * (long(max_items) * (group / p) + kBegin),
@@ -759,7 +833,7 @@ extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items
   for (int p = 1; max_items > 0 && p <= group && p <= kMaxParts; ++p) {
     if (group % p != 0) continue;
     if (long(n_ctas) * hkv * p <= kSms) in_one_wave = p;
-    else if (in_one_wave > 0 && long(max_items) * (group / in_one_wave - group / p) < 32) continue;
+    else if (!any_wave && in_one_wave > 0 && long(max_items) * (group / in_one_wave - group / p) < 32) continue;
     if (visits(p) < visits(parts)) parts = p;
   }
   return parts;
@@ -768,17 +842,22 @@ extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items
 // Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  channels: of the arenas' 128, those that may be other
 // than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are the
 // lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
-// length of the longest item list (0: not known, the head groups stay whole).
+// length of the longest item list (0: not known, the head groups stay whole).  workspace: as many bytes as dcpk_attn_bwd_workspace
+// says, contents of no matter; null: dQ has no levels.
 extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena,
                              long kv_rows, int hq, int hkv, const void* ctas, int n_ctas, const void* items,
                              int n_items_total, int max_items, const void* masks, int n_mask_rows, const float* lse, const float* delta,
                              int stat_stride, float* const* dq_ptrs, float* const* dkv_ptrs, int n_dst, float scale, int channels,
-                             const void* jobs, int n_jobs, void* const* job_src_ptrs, void* const* job_dst_ptrs,
+                             int n_levels, void* workspace, const void* jobs, int n_jobs, void* const* job_src_ptrs, void* const* job_dst_ptrs,
                              int job_stat_stride, int* status, void* stream) {
   if (n_ctas <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
   if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
-  CUtensorMap tm_q, tm_do, tm_kv, tm_dq, tm_dkv;
+  const bool levels = workspace != nullptr && dcpk_attn_bwd_workspace(n_items_total, q_rows, hq, channels, n_levels) > 0;
+  CUtensorMap tm_q, tm_do, tm_kv, tm_dq, tm_dkv, tm_levels;
   if (encode_f32_tile_map(&tm_dq, dq_ptrs[0], uint64_t(q_rows), uint32_t(hq), kHeadDim, 32, 32)) return -1;
+  tm_levels = tm_dq;
+  if (levels && encode_f32_tile_map(&tm_levels, workspace, uint64_t(n_levels - 1) * q_rows, uint32_t(hq), uint32_t(level_pitch(channels)), 32, 32))
+    return -1;
   if (encode_f32_tile_map(&tm_dkv, dkv_ptrs[0], uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 32, 32)) return -1;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
   if (encode_arena_map(&tm_do, do_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
@@ -798,17 +877,26 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   if (raise_smem_limit(kernel, smem, g_bwd_smem_raised[v]) != cudaSuccess) return -4;
   // about 16 fetch CTAs when there is something to fetch
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
-  const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total);
+  const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total, levels || n_levels == 1);
   const int heads_per_cta = group / parts;
   // A plain launch: CTAs that begin together go through the queries together and find one another's tiles in L2, those that begin as
   // the SMs come free do not (forward and backward of 121987 tokens, mixed masks, 41.3 ms plain, 44.3 overlapped with the kernel
   // before; 6168 tokens 1008 and 1050 us).  A single wave would gain 3 us of 134 (four sequences of 300 to 2100 tokens, 8 / 2
-  // heads), but its CTAs begin so far apart then that they add to dQ in another order in 1 to 24 of 60 runs.
+  // heads).
   const dim3 grid(hkv * parts, n_ctas + n_copy_rows);
+  const bool narrow = level_pitch(channels) == 64;
+  auto pass_over_levels = [&](auto kernel) {
+    return launch_overlapped(kernel, unsigned((q_rows + kLevelRows - 1) / kLevelRows), 256, 0, static_cast<cudaStream_t>(stream), 1, true,
+                             static_cast<const BwdItemDesc*>(items), n_items_total, static_cast<float*>(workspace), n_levels,
+                             dq_ptrs[0], int(q_rows), hq, channels);
+  };
+  if (levels && pass_over_levels(narrow ? dq_levels_kernel<64, false> : dq_levels_kernel<128, false>) != cudaSuccess) return -5;
   const cudaError_t rc = launch_overlapped(
       kernel, grid, kBwdThreads, smem, static_cast<cudaStream_t>(stream), unsigned(parts), false, tm_q, tm_do,
-      tm_kv, tm_dq, tm_dkv, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
+      tm_kv, tm_dq, tm_dkv, tm_levels, levels ? n_levels : 1, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
       static_cast<const int4*>(masks), lse, delta, pp, hq, hkv, heads_per_cta, stat_stride, n_dst, int(q_rows), int(kv_rows),
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);
-  return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;
+  if (rc != cudaSuccess || cudaGetLastError() != cudaSuccess) return -5;
+  if (levels && pass_over_levels(narrow ? dq_levels_kernel<64, true> : dq_levels_kernel<128, true>) != cudaSuccess) return -5;
+  return 0;
 }

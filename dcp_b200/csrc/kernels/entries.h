@@ -11,8 +11,10 @@ int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* kv_arena, l
 int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena, long kv_rows, int hq, int hkv,
                   const void* ctas, int n_ctas, const void* items, int n_items_total, int max_items, const void* masks,
                   int n_mask_rows, const float* lse, const float* delta, int stat_stride, float* const* dq_ptrs,
-                  float* const* dkv_ptrs, int n_dst, float scale, int channels, const void* jobs, int n_jobs,
+                  float* const* dkv_ptrs, int n_dst, float scale, int channels, int n_levels, void* workspace, const void* jobs, int n_jobs,
                   void* const* job_src_ptrs, void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream);
+long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, int channels, int n_levels);
+int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total, int any_wave);
 int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int n_rows, int hq, int stat_stride, float* zero0, long nz0,
                        float* zero1, long nz1, void* stream);
 int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o, int d, void* d_o_rows, float* delta, int n_rows, int hq,

@@ -131,7 +131,7 @@ def plan_iteration_all(spec: PlanSpec, iteration: int) -> Dict[int, RankPlan]:
 
 # Part of the key of a cached plan: raised whenever what a plan file holds, or what the kernels expect of the tables in
 # it, changes.  2: rows of the packed batch in place of the token arrays.
-PLAN_FORMAT = 2
+PLAN_FORMAT = 3
 
 
 def batch_signature(spec: PlanSpec, rank: int, seqlens: Sequence[int], mask_fn_info, group_members) -> str:

@@ -308,15 +308,16 @@ class BwdTables:
     n_items: int
     flops: float = 0.0
     max_items: int = 0    # items of the longest key tile (0: not known, head groups are not split over CTAs)
+    dq_levels: int = 0    # buffers that take at most two additions per row of dQ each (see _dq_levels; 0: not known)
 
     def to(self, device, non_blocking: bool = True) -> "BwdTables":
         mv = lambda t: t.to(device, non_blocking=non_blocking)
         return BwdTables(mv(self.ctas), mv(self.items), mv(self.masks), self.n_ctas, self.n_items, self.flops,
-                         self.max_items)
+                         self.max_items, self.dq_levels)
 
     def pin(self) -> "BwdTables":
         return BwdTables(self.ctas.pin_memory(), self.items.pin_memory(), self.masks.pin_memory(), self.n_ctas,
-                         self.n_items, self.flops, self.max_items)
+                         self.n_items, self.flops, self.max_items, self.dq_levels)
 
 
 def _tile_bounds(rng: np.ndarray, tile: int):
@@ -338,6 +339,16 @@ def _tile_bounds(rng: np.ndarray, tile: int):
     return n_t, (u0s, u0e, u1s, u1e, i0s, i0e, i1s, i1e)
 
 
+def _dq_levels(items: np.ndarray) -> int:
+    """How many buffers dQ needs for each to take the additions of two key tiles at most: one per 256 positions of the items'
+    concatenated KV, if key tiles begin at multiples of 128 of these (block sizes that are multiples of 128).  0: not known, as
+    for longer lists, which have none (see dcpk_attn_bwd_workspace)."""
+    if not 0 < items.shape[0] <= 4096:
+        return 0
+    pos = items[:, 2]
+    return 0 if (pos & 127).any() else int(pos.max() >> 8) + 1
+
+
 def build_bwd_tables(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: int, device) -> BwdTables:
     """Backward kernel tables (see ``build_bwd_tables_py`` for the layout); built by the C++ planner module."""
     native = _native_planner()
@@ -346,7 +357,7 @@ def build_bwd_tables(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: int
     c_np, i_np, m_np, pairs = native.build_bwd_tables(_row_tuples(rows), int(block_size), int(hq))
     to = lambda a: torch.from_numpy(a).to(device, non_blocking=True)
     return BwdTables(to(c_np), to(i_np), to(m_np), int(c_np.shape[0]), int(i_np.shape[0]), flops=10.0 * pairs * HEAD_DIM,
-                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0)
+                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0, dq_levels=_dq_levels(i_np))
 
 
 def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: int, device) -> BwdTables:
@@ -422,7 +433,7 @@ def build_bwd_tables_py(rows: Sequence[AttnRow], block_size: int, hq: int, hkv: 
     m_np = np.concatenate(masks, axis=0) if masks else np.zeros((0, 4), np.int32)
     to = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device, non_blocking=True)
     return BwdTables(to(c_np), to(i_np), to(m_np), len(ctas), int(off), flops=10.0 * pairs * HEAD_DIM,
-                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0)
+                     max_items=int(c_np[0, 3]) if c_np.shape[0] else 0, dq_levels=_dq_levels(i_np))
 
 
 def attn_bwd_prep(out: torch.Tensor, dout: torch.Tensor, delta: torch.Tensor, n_rows: int, row0: int = 0, zero=()) -> None:
@@ -494,6 +505,10 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
     lib = _lib.load()
     hq, hkv = q_arena.shape[1], kv_arena.shape[2]
     assert q_arena.shape == do_arena.shape and lse.shape == delta.shape
+    lib.dcpk_attn_bwd_workspace.restype = ctypes.c_long
+    n_bytes = lib.dcpk_attn_bwd_workspace(ctypes.c_int(tables.items.shape[0]), ctypes.c_long(q_arena.shape[0]), ctypes.c_int(hq),
+                                          ctypes.c_int(channels), ctypes.c_int(tables.dq_levels))
+    workspace = torch.empty(n_bytes, dtype=torch.uint8, device=q_arena.device) if n_bytes else None
     rc = lib.dcpk_attn_bwd(
         _lib.ptr(q_arena), _lib.ptr(do_arena), ctypes.c_long(q_arena.shape[0]), _lib.ptr(kv_arena),
         ctypes.c_long(kv_arena.shape[0]), ctypes.c_int(hq), ctypes.c_int(hkv), _lib.ptr(tables.ctas),
@@ -501,7 +516,8 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
         ctypes.c_int(tables.max_items), _lib.ptr(tables.masks),
         ctypes.c_int(tables.masks.shape[0]), _lib.ptr(lse), _lib.ptr(delta),
         ctypes.c_int(lse.shape[1]), _ptr_array(dq_dsts), _ptr_array(dkv_dsts), ctypes.c_int(len(dq_dsts)),
-        ctypes.c_float(scale), ctypes.c_int(channels), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
+        ctypes.c_float(scale), ctypes.c_int(channels), ctypes.c_int(tables.dq_levels),
+        ctypes.c_void_p(workspace.data_ptr() if n_bytes else 0), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
     _lib.check(rc, "dcpk_attn_bwd")
 
 

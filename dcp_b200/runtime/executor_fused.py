@@ -158,7 +158,8 @@ class FusedAttentionExecutor:
              "q_local_rows": p.q_local_rows, "kv_local_rows": p.kv_local_rows, "q_rows": p.q_rows, "kv_rows": p.kv_rows,
              "all_rows_written": self._all_rows_written, "channels": self.channels}
         if b is not None:
-            d.update(ctas=b.ctas, items=b.items, bwd_masks=b.masks, n_ctas=b.n_ctas, max_items=b.max_items)
+            d.update(ctas=b.ctas, items=b.items, bwd_masks=b.masks, n_ctas=b.n_ctas, max_items=b.max_items,
+                     dq_levels=b.dq_levels)
         return _lib.calls().SingleRankAttention(d)
 
     def native(self):

@@ -337,16 +337,16 @@ def test_backward_of_an_earlier_call_gets_its_own_operands_on_several_ranks():
         assert torch.equal(dq, q) and torch.equal(dkv, kv)
 
 
-@pytest.mark.parametrize("raw,heads,kv_heads,want", [
-    ([1000, 300, 2100, 640], 8, 2, 2),    # 132 CTAs of at most 34 visits; four parts would be 264 and save 17
-    ([640, 1100, 900], 16, 4, 1),         # 88 CTAs in one part; 176 in two would save 18 visits
-    ([512, 1024, 2048, 4096], 8, 2, 4),   # 120 CTAs of 128 visits: 96 saved, so more than one wave
-    ([2048], 32, 8, 2),                   # 128 CTAs of 64 visits: 32 saved
-    ([700], 8, 2, 4),                     # 48 CTAs in four parts are one wave
+@pytest.mark.parametrize("raw,heads,kv_heads,one_wave,any_wave,levels", [
+    ([1000, 300, 2100, 640], 8, 2, 2, 4, 9),    # 132 CTAs of at most 34 visits; four parts are 264 and save 17
+    ([640, 1100, 900], 16, 4, 1, 2, 5),         # 88 CTAs in one part; 176 in two save 18 visits
+    ([512, 1024, 2048, 4096], 8, 2, 4, 4, 16),  # 120 CTAs of 128 visits: 96 saved, so more than one wave
+    ([2048], 32, 8, 2, 2, 8),                   # 128 CTAs of 64 visits: 32 saved
+    ([700], 8, 2, 4, 4, 3),                     # 48 CTAs in four parts are one wave
 ])
-def test_backward_of_a_short_batch_stays_in_one_wave(raw, heads, kv_heads, want):
-    """CTAs that all run at once give dQ the same bits in every run; a head group is split into more of them only where
-    that shortens the longest list by 32 visits."""
+def test_split_of_head_groups_and_levels_of_dq(raw, heads, kv_heads, one_wave, any_wave, levels):
+    """CTAs that add to dQ as they come are more than one wave only where that shortens the longest list by 32 visits; where every
+    256 positions of a query's keys have a buffer of their own, waves do not matter, and no buffer takes more than two key tiles."""
     import ctypes
     from dcp_b200.ops import _lib
     if not _lib.available():
@@ -358,5 +358,11 @@ def test_backward_of_a_short_batch_stays_in_one_wave(raw, heads, kv_heads, want)
                            masks.get_mask_fn("causal")(raw, padded, torch.int32), torch.bfloat16)
     fw_wl, *_ = InstrCompiler(ctx, CompilerConfig()).compile(wl)
     t = lower_all(ctx, fw_wl, build_backward=True)[ctx.devices()[0]].bwd[0]
-    got = _lib.load().dcpk_attn_bwd_parts(*(ctypes.c_int(x) for x in (t.n_ctas, kv_heads, heads // kv_heads, t.max_items, t.items.shape[0])))
-    assert got == want
+    args = (t.n_ctas, kv_heads, heads // kv_heads, t.max_items, t.items.shape[0])
+    assert [_lib.load().dcpk_attn_bwd_parts(*(ctypes.c_int(x) for x in (*args, o))) for o in (0, 1)] == [one_wave, any_wave]
+    assert t.dq_levels == levels
+    adders = {}
+    for q_row, n_rows, kv_pos0, _, _, dq_row, *_ in t.items.tolist():
+        for row in range(dq_row, dq_row + n_rows):
+            adders.setdefault((row, kv_pos0 >> 8), []).append(kv_pos0)
+    assert all(len(set(a)) == len(a) <= 2 for a in adders.values()) and max(k[1] for k in adders) == levels - 1

@@ -474,25 +474,30 @@ def test_native_calls_against_the_general_path(head_dim, dtype, kv_dtype, form):
     assert ex.impl.native() is None
 
 
-@pytest.mark.parametrize("raw,heads,kv_heads,head_dim,dtype", [([1000, 300, 2100, 640], 8, 2, 128, torch.bfloat16),
-                                                               ([1000, 300, 2100, 640], 8, 2, 64, torch.float32),
-                                                               ([640, 1100, 900], 16, 4, 128, torch.bfloat16)])
-def test_short_causal_calls_repeat_to_the_bit(raw, heads, kv_heads, head_dim, dtype):
-    """A backward whose CTAs all run at once adds to every row of dQ in the order of the CTAs' items (causal lists begin at
-    different queries): output and gradients have the same bits in every call."""
+@pytest.mark.parametrize("raw,heads,kv_heads,head_dim,dtype,mask", [([1000, 300, 2100, 640], 8, 2, 128, torch.bfloat16, "causal"),
+                                                                    ([1000, 300, 2100, 640], 8, 2, 64, torch.float32, "causal"),
+                                                                    ([640, 1100, 900], 16, 4, 96, torch.float16, "shared_question"),
+                                                                    ([700], 4, 1, 128, torch.bfloat16, "lambda")])
+def test_short_calls_repeat_to_the_bit(raw, heads, kv_heads, head_dim, dtype, mask):
+    """Output and gradients of a short batch have the same bits in every call, whatever goes on in between."""
     _need_gpu()
     from dcp_b200.core.common import get_default_execution_context
     from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test
     dev = torch.device("cuda", 0)
     ex, lq, lkv, ldo, *_ = prepare_dcp_distributed_attn_for_test(raw, heads, kv_heads, head_dim, 256, heads, get_default_execution_context(1, 1),
-                                                                 0, "causal", dtype, 3, device=dev, executor_impl="fused")
+                                                                 0, mask, dtype, 3, device=dev, executor_impl="fused")
     lq.requires_grad_(True), lkv.requires_grad_(True)
     first = None
-    for _ in range(20):
+    for i in range(40):
+        if i % 3 == 0:
+            torch.full((1 << 26,), float("nan"), device=dev)       # other lines in L2, other bytes in what a call allocates
         out = DCPAttention.apply(ex, False, False, lq, lkv)
         got = (out.detach(), *torch.autograd.grad(out, (lq, lkv), ldo))
+        if i % 2:
+            got[1].cpu()
         first = first or got
         assert all(torch.equal(a, b) for a, b in zip(got, first))
+    ex.impl.check_status()
 
 
 @pytest.mark.parametrize("head_dim,dtype,rise,values", [(64, torch.float32, 54, 90), (64, torch.float16, 70, 0), (96, torch.bfloat16, 54, 90),
@@ -571,7 +576,7 @@ def test_native_calls_leave_idle_rows_zero(head_dim, dtype):
 @pytest.mark.parametrize("head_dim,dtype", [(128, torch.bfloat16), (64, torch.float32)])
 def test_native_calls_on_another_stream_and_in_a_graph(head_dim, dtype):
     """The whole call on a stream of its own, behind work of that stream, and captured and replayed on other inputs: the same
-    bits (a short causal batch; see test_short_causal_calls_repeat_to_the_bit)."""
+    bits (a short batch)."""
     _need_gpu()
     from dcp_b200.core.common import get_default_execution_context
     from dcp_b200.runtime.interface import DCPAttention, prepare_dcp_distributed_attn_for_test

@@ -880,3 +880,58 @@ def test_adamw_and_reduce_scatter_single_rank(dev):
         ref.step()
     assert (opt.master - ref_p.detach()).abs().max() < 1e-5
     assert torch.equal(bufs.params, opt.master.bfloat16())
+
+
+@pytest.mark.parametrize("d,heads", [(128, (8, 2)), (128, (5, 1)), (64, (8, 2)), (64, (6, 6)), (96, (4, 1))])
+@pytest.mark.parametrize("kind", ["full", "causal", "two"])
+def test_attention_backward_levels_of_dq(dev, d, heads, kind):
+    """dQ through a buffer per 256 keys: the same bits in every run where it was cleared, also where all key tiles begin at the same
+    query; elsewhere added to what dQ holds; within rounding of additions to one buffer (8 of 2^-24 of the largest partial sum,
+    and 2^-20 of the largest element, which is at least 1 here).  Rows without keys keep what they hold, and so do channels beyond the
+    heads'."""
+    import dataclasses
+    (hq, hkv), nq, nkv = heads, 520, 1100
+    torch.manual_seed(d + hq)
+    q, dout = torch.zeros(2, nq, hq, 128, device=dev, dtype=torch.bfloat16)
+    kv = torch.zeros(nkv, 2, hkv, 128, device=dev, dtype=torch.bfloat16)
+    for t in (q, dout, kv):
+        t[..., :d] = torch.randn(*t.shape[:-1], d, device=dev).bfloat16()
+    rng = np.zeros((nq, 4), np.int32)
+    rng[:, 1] = nkv if kind == "full" else np.arange(nq) + 581
+    if kind == "two":
+        rng[:, 1], rng[:, 2], rng[:, 3] = 200, 600, np.arange(nq) + 581
+        rng[100:140] = 0
+    row = A.AttnRow(0, nq, list(range(hq)), [(0, nkv)], rng)
+    out, lse, delta = torch.zeros_like(q), torch.zeros(hq, nq, device=dev), torch.zeros(hq, nq, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    A.attn_fwd(q, kv, A.build_fwd_tables([row], 1152, dev), [out], [lse], d ** -0.5, status, channels=d)
+    A.attn_delta(out, dout, delta, 0, nq)
+    levels = A.build_bwd_tables([row], 1152, hq, hkv, dev)
+    assert levels.dq_levels == 5
+    first = None
+    for tables in [levels] * 12 + [dataclasses.replace(levels, dq_levels=0)]:
+        junk = torch.full((5 * nq * hq * 128,), float("nan"), device=dev)
+        del junk                                            # the buffers' memory
+        dq, dkv = torch.zeros(nq, hq, 128, device=dev), torch.zeros(nkv, 2, hkv, 128, device=dev)
+        dq[:, :, 3] = 1.0
+        dq[..., d:] = 5.0
+        A.attn_bwd(q, dout, kv, lse, delta, tables, [dq], [dkv], d ** -0.5, status, channels=d)
+        first = first or (dq, dkv)
+        assert torch.equal(dkv, first[1])
+        if tables is levels:
+            assert torch.equal(dq[..., :3], first[0][..., :3]) and torch.equal(dq[..., 4:], first[0][..., 4:])
+            assert (dq[..., 3] - first[0][..., 3]).abs().max() <= 2.0 ** -20 * dq[..., :d].abs().max()
+    assert status.item() == 0 and (first[0][..., d:] == 5.0).all()
+    assert (dq - first[0]).abs().max() <= 2.0 ** -20 * dq[..., :d].abs().max()
+    if kind == "two":
+        assert (first[0][100:140, :, 3] == 1.0).all() and not first[0][100:140, :, :3].any()
+
+
+def test_levels_of_dq_need_whole_key_tiles():
+    """Key tiles that begin anywhere may share 256 positions with two others: no levels then."""
+    rng = np.zeros((200, 4), np.int32)
+    rng[:, 1] = 400
+    rows = lambda bs: [A.AttnRow(0, 200, [0], [(0, min(bs, 400)), (400, 100)], rng)]
+    assert A.build_bwd_tables(rows(200), 200, 1, 1, "cpu").dq_levels == 0
+    assert A.build_bwd_tables(rows(256), 256, 1, 1, "cpu").dq_levels == 2
+    assert A.build_bwd_tables([], 256, 1, 1, "cpu").dq_levels == 0
