@@ -22,6 +22,7 @@
 #include <stdexcept>
 #include <string>
 #include <tuple>
+#include <utility>
 
 #include "entries.h"
 
@@ -95,34 +96,41 @@ class SingleRankAttention {
           "dcpk_attn_fwd_pair");
   }
 
+  // The levels of dQ, in memory of this call's own (null: none).
+  std::pair<Tensor, DcpkDqLevels> levels_of_call() const {
+    const long bytes = dcpk_attn_bwd_workspace(int(items.size(0)), q_local_rows, int(q.size(1)), channels, dq_levels);
+    Tensor memory;
+    if (bytes > 0) memory = at::empty({bytes}, q.options().dtype(at::kByte));
+    return {memory, {items.const_data_ptr(), int(items.size(0)), dq_levels, int(q_local_rows), int(q.size(1)), channels,
+                     bytes > 0 ? memory.data_ptr() : nullptr}};
+  }
+
   // delta and cleared accumulators, then the gradients; `o` and `d_in`: at least the local rows, of `d` channels.  Other than rows
   // of 128 in bf16 go to the arena of dO on the way.
   void launch_backward(const Tensor& q_in, const Tensor& d_in, const Tensor& kv_in, const Tensor& o, const Tensor& l, const Tensor& dl,
-                       int d, double scale) const {
+                       int d, const DcpkDqLevels& levels, bool sum_levels, double scale) const {
     const long hq = q.size(1), hkv = kv.size(2);
     const bool in_place = d == kHeadDim && d_in.scalar_type() == at::kBFloat16;
     const Tensor& d_o = in_place ? d_in : dout;
     if (in_place)
       check(dcpk_attn_bwd_prep(o.const_data_ptr(), d_in.const_data_ptr(), dl.data_ptr<float>(), int(q_local_rows), int(hq),
                                int(dl.size(1)), dq.data_ptr<float>(), q_rows * hq * kHeadDim, dkv.data_ptr<float>(),
-                               kv_rows * 2 * hkv * kHeadDim, stream()),
+                               kv_rows * 2 * hkv * kHeadDim, &levels, stream()),
             "dcpk_attn_bwd_prep");
     else
       check(dcpk_attn_bwd_prep_cast(row_type(d_in), o.const_data_ptr(), d_in.const_data_ptr(), d, dout.data_ptr(), dl.data_ptr<float>(),
                                     int(q_local_rows), int(hq), int(dl.size(1)), dq.data_ptr<float>(), q_rows * hq * kHeadDim,
-                                    dkv.data_ptr<float>(), kv_rows * 2 * hkv * kHeadDim, stream()),
+                                    dkv.data_ptr<float>(), kv_rows * 2 * hkv * kHeadDim, &levels, stream()),
             "dcpk_attn_bwd_prep_cast");
     nvtxMarkA("bwd:dout copy, delta, zero accumulators");
     nvtxMarkA("bwd:wait inputs of peers");
-    const long bytes = dcpk_attn_bwd_workspace(int(items.size(0)), q_local_rows, int(hq), channels, dq_levels);
-    Tensor workspace;
-    if (bytes > 0) workspace = at::empty({bytes}, q.options().dtype(at::kByte));
     float* dqs[1] = {dq.data_ptr<float>()};
     float* dkvs[1] = {dkv.data_ptr<float>()};
     check(dcpk_attn_bwd(q_in.const_data_ptr(), d_o.const_data_ptr(), q_local_rows, kv_in.const_data_ptr(), kv_in.size(0), int(hq),
                         int(hkv), ctas.const_data_ptr(), n_ctas, items.const_data_ptr(), int(items.size(0)), max_items,
                         bwd_masks.const_data_ptr(), int(bwd_masks.size(0)), l.const_data_ptr<float>(), dl.const_data_ptr<float>(),
-                        int(l.size(1)), dqs, dkvs, 1, float(scale), channels, dq_levels, bytes > 0 ? workspace.data_ptr() : nullptr, nullptr, 0, nullptr, nullptr, 0,
+                        int(l.size(1)), dqs, dkvs, 1, float(scale), channels, dq_levels, levels.workspace,
+                        sum_levels ? 2 : 0, nullptr, 0, nullptr, nullptr, 0,
                         status.data_ptr<int>(), stream()),
           "dcpk_attn_bwd");
     nvtxMarkA("bwd:kernels (with operand fetch)");
@@ -148,7 +156,8 @@ class SingleRankAttention {
         !arena_like(d_o, q_local_rows, q.size(1)) || d_o.size(0) != q_local_rows || !arena_like(o, q_local_rows, q.size(1)) || !statistics(l))
       return false;
     Call call("dcp.attention.bwd", q);
-    launch_backward(q_in, d_o, kv_in, o, l, dl ? *dl : at::empty_like(l), kHeadDim, scale);
+    const auto [memory, levels] = levels_of_call();
+    launch_backward(q_in, d_o, kv_in, o, l, dl ? *dl : at::empty_like(l), kHeadDim, levels, true, scale);
     return true;
   }
 
@@ -207,13 +216,19 @@ class SingleRankAttention {
             "dcpk_pad_cast_rows");
       ++entries;
     }
+    const auto [memory, levels] = levels_of_call();
     launch_backward(in_place ? q_in : q, do_in, in_place ? kv_in.view({kv_local_rows, 2, hkv, kHeadDim}) : kv, o_in, l, at::empty_like(l),
-                    d, scale);
+                    d, levels, false, scale);
     Tensor gq = at::empty({q_local_rows, hq, d}, q.options().dtype(q_in.scalar_type()));
     Tensor gkv = at::empty({kv_local_rows, 2, hkv, d}, q.options().dtype(kv_in.scalar_type()));
-    check(dcpk_cut_cast_rows(1, row_type(gq), dq.const_data_ptr(), gq.data_ptr(), q_local_rows * hq, dkv.const_data_ptr(),
-                             gkv.data_ptr(), kv_local_rows * 2 * hkv, d, stream()),
-          "dcpk_cut_cast_rows");
+    if (levels.workspace)
+      check(dcpk_cut_cast_gradients(row_type(gq), &levels, dq.const_data_ptr<float>(), gq.data_ptr(), dkv.const_data_ptr<float>(),
+                                    gkv.data_ptr(), kv_local_rows * 2 * hkv, d, stream()),
+            "dcpk_cut_cast_gradients");
+    else
+      check(dcpk_cut_cast_rows(1, row_type(gq), dq.const_data_ptr(), gq.data_ptr(), q_local_rows * hq, dkv.const_data_ptr(),
+                               gkv.data_ptr(), kv_local_rows * 2 * hkv, d, stream()),
+            "dcpk_cut_cast_rows");
     return std::make_tuple(gq, gkv, entries);
   }
 };

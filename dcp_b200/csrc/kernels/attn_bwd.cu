@@ -27,7 +27,7 @@
 // shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
 // (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
 // every key tile as it comes, in short launches through buffers of at most two additions each, which are summed afterwards (see
-// dq_level): these give the same bits in every run, the last bits of longer ones differ.
+// attn_levels.cuh): these give the same bits in every run, the last bits of longer ones differ.
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
@@ -65,6 +65,7 @@
 #include <algorithm>
 
 #include "attn_common.cuh"
+#include "attn_levels.cuh"
 #include "copy_jobs.cuh"
 #include "entries.h"
 #include "launch.cuh"
@@ -77,19 +78,6 @@ namespace dcpk {
 static constexpr int kBwdThreads = 896;  // 16 gradient warps, 8 drain warps, TMA producer, UMMA issuer, statistics, 1 idle
 static constexpr int kQTile = 128;            // query rows per item
 static constexpr int kHalf = 128 * 64 * 2;  // [128 x 64] bf16 half tile, 16 KB
-
-// One item = one query tile (up to 128 rows) that attends to the CTA's key tile; a CTA visits it once per
-// query head it covers, so the table does not grow with the head count.
-struct BwdItemDesc {
-  int q_row;     // arena row of the query tile (same row addresses Q, dO, lse, delta)
-  int n_rows;    // valid queries
-  int kv_pos0;   // position of this CTA's first key inside the item's concatenated KV
-  int mask_row;  // row in the range table
-  int dq_dev;    // destination index of the dQ accumulator
-  int dq_row;    // arena row in that accumulator
-  int full;      // 1: every (query, key) pair of the tile is allowed
-  int pad;
-};
 
 struct BwdItem {  // descriptor + the query head of the current visit
   int q_row, n_rows, head, kv_pos0, mask_row, dq_dev, dq_row, full;
@@ -117,14 +105,6 @@ __device__ __forceinline__ bool item_ok(const BwdItem& it, int q_rows, int stat_
            it.q_row + it.n_rows > stat_stride || it.dq_dev >= n_dst || it.mask_row < 0 ||
            (!it.full && it.mask_row + it.n_rows > n_mask_rows) ||
            (it.dq_dev >= 0 && (it.dq_row < 0 || it.dq_row + it.n_rows > q_rows)));
-}
-
-// A row of dQ is added to by every key tile that it sees, as these come.  Two additions to zero give the same bits in either order,
-// three do not: with a workspace each 256 keys (of the positions of an item's concatenated KV) have a buffer of their own, a level,
-// and the levels are summed afterwards, in their order.  Level 0 is the accumulator itself, and the only one without a workspace.
-__device__ __forceinline__ int dq_level(int kv_pos0, int n_levels) {
-  const int level = kv_pos0 >> 8;
-  return level > 0 && level < n_levels ? level : 0;
 }
 
 struct BwdPtrs {
@@ -251,6 +231,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 float scale, const CopyJob* __restrict__ jobs, int n_jobs, const __grid_constant__ CopyCtx copy_ctx,
                 int n_copy_rows, int* __restrict__ status) {
   grid_let_next();
+  grid_wait();
   if (int(blockIdx.y) < n_copy_rows) {
     // ------------------------------------------------------------ operand fetch for the next stage
     run_copy_jobs(jobs, n_jobs, copy_ctx, blockIdx.y * gridDim.x + blockIdx.x, n_copy_rows * gridDim.x, threadIdx.x,
@@ -725,63 +706,37 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-// The levels of dQ above the first, [n_levels - 1, q_rows, hq, kPitch]: zeroed where they will be added to, or summed into dQ.  Bound by
-// L2.  A CTA takes kLevelRows rows; which levels these have is in the items that cover them, so it looks through the whole table.
-static constexpr int kLevelRows = 4;
-
-template <int kPitch, bool kSum>
-__global__ void __launch_bounds__(256) dq_levels_kernel(const BwdItemDesc* __restrict__ items, int n_items, float* __restrict__ levels,
-                                                        int n_levels, float* __restrict__ dq, int q_rows, int hq, int channels) {
-  __shared__ uint32_t present[kLevelRows][2];   // a bit per level
+// The passes over the levels of dQ as launches of their own (kSum: they are added to dQ; else they are cleared).  Bound by L2.
+template <bool kSum>
+__global__ void __launch_bounds__(256) dq_levels_kernel(const __grid_constant__ DqLevels lv, float* __restrict__ dq) {
+  __shared__ RowLevels present;
   const int row0 = blockIdx.x * kLevelRows;
-  if (threadIdx.x < 2 * kLevelRows) present[threadIdx.x >> 1][threadIdx.x & 1] = 0;
-  __syncthreads();
   grid_let_next();
   grid_wait();
-  for (int i = threadIdx.x; i < n_items; i += 256) {
-    const BwdItemDesc d = items[i];
-    if (d.dq_dev != 0) continue;
-    const int level = dq_level(d.kv_pos0, n_levels);
-    for (int row = max(d.dq_row, row0); row < min(min(d.dq_row + d.n_rows, q_rows), row0 + kLevelRows); ++row)
-      atomicOr(&present[row - row0][level >> 5], 1u << (level & 31));
+  if (!kSum) {
+    clear_levels(lv, row0, present);
+    return;
   }
-  __syncthreads();
-  const size_t level_size = size_t(q_rows) * hq * kPitch;
-  for (int r = 0; r < kLevelRows; ++r) {
-    const uint64_t above = (uint64_t(present[r][1]) << 32 | present[r][0]) & ~uint64_t(1);
-    if (above == 0) continue;
-    for (int c = threadIdx.x; c < hq * (kPitch / 4); c += 256) {   // four channels of a head
-      const int head = c / (kPitch / 4), ch = c % (kPitch / 4) * 4;
-      if (ch >= channels) continue;
-      const size_t in_row = size_t(row0 + r) * hq + head;
-      float* at = levels + in_row * kPitch + ch;
-      float4* acc = reinterpret_cast<float4*>(dq + in_row * kHeadDim + ch);
-      float4 sum = kSum ? *acc : make_float4(0.f, 0.f, 0.f, 0.f);
-      for (uint64_t left = above; left != 0;) {
-        float4 v[4];   // of four levels in flight
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const bool there = left != 0;
-          float4* p = reinterpret_cast<float4*>(at + size_t(there ? __ffsll(left) - 2 : 0) * level_size);
-          left &= left - 1;
-          if (kSum) v[u] = there ? *p : make_float4(0.f, 0.f, 0.f, 0.f);
-          else if (there) *p = sum;
-        }
-        if (kSum)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) { sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w; }
-      }
-      if (kSum) *acc = sum;
-    }
+  find_levels(lv, row0, present);
+  const int quads = lv.pitch / 4, per_row = lv.hq * quads;
+  for (int c = threadIdx.x; c < kLevelRows * per_row; c += 256) {
+    const int r = c / per_row, k = c % quads * 4;
+    const uint64_t above = levels_above(present, r);
+    if (above == 0 || k >= lv.channels) continue;
+    const size_t head_row = size_t(row0 + r) * lv.hq + c % per_row / quads;
+    float4* acc = reinterpret_cast<float4*>(dq + head_row * kHeadDim + k);
+    float4 sum = *acc;
+    add_levels(lv, above, head_row * lv.pitch + k, sum);
+    *acc = sum;
   }
 }
 
 static constexpr int kSms = 148, kMaxParts = 8, kMaxLevels = 64;
 // Launches of up to so many bytes of dQ tiles (one per visit) have levels, if these take no more than the other number.  Levels cost
-// what it takes to clear and to sum them: four sequences of 300 to 2100 tokens, 8 / 2 heads, 110 MB, forward and backward, 107 us
-// without and 135 with them, 2048 tokens, 71 MB, 96 and 108.  Above, what is added to no longer stays in L2: 2048 tokens, 32 / 8 heads, 285 MB,
-// 169 and 280 us, 4096 tokens, 8 / 2 heads, 277 MB, 152 and 235.  (Tiles of their own for all visits, stored and then summed, took
-// 150 us for the first.)
+// what it takes to clear and to sum them, in the passes before and after the kernel or in launches of their own: four sequences of
+// 300 to 2100 tokens, 8 / 2 heads, 110 MB, forward and backward, 107 us without, 130 and 135 with them; 2048 tokens, 71 MB, 96, 101
+// and 108.  Above, what is added to no longer stays in L2: 2048 tokens, 32 / 8 heads, 285 MB, 169 and 280 us, 4096 tokens, 8 / 2
+// heads, 277 MB, 152 and 235.  (A tile of its own for every visit, stored and then summed, took 150 us for the first.)
 static constexpr long kMaxVisitBytes = 128l << 20, kMaxWorkspace = 512l << 20;
 static std::atomic<uint64_t> g_bwd_smem_raised[4];
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
@@ -798,8 +753,6 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
   g_bwd_timeline_host = p;
   return cudaMemcpyToSymbol(g_bwd_timeline, &p, sizeof(p)) == cudaSuccess ? 0 : -5;
 }
-
-static int level_pitch(int channels) { return channels > 64 ? kHeadDim : 64; }
 
 // Bytes of the workspace of dcpk_attn_bwd for item lists of `n_levels` levels (see dq_level; 0: not known); 0: there is none.
 extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, int channels, int n_levels) {
@@ -843,13 +796,14 @@ extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items
 // than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are the
 // lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
 // length of the longest item list (0: not known, the head groups stay whole).  workspace: as many bytes as dcpk_attn_bwd_workspace
-// says, contents of no matter; null: dQ has no levels.
+// says; null: dQ has no levels.  level_passes: 1 they are cleared here (else dcpk_attn_bwd_prep did), + 2 and summed here (else
+// dcpk_cut_cast_gradients does).
 extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena,
                              long kv_rows, int hq, int hkv, const void* ctas, int n_ctas, const void* items,
                              int n_items_total, int max_items, const void* masks, int n_mask_rows, const float* lse, const float* delta,
                              int stat_stride, float* const* dq_ptrs, float* const* dkv_ptrs, int n_dst, float scale, int channels,
-                             int n_levels, void* workspace, const void* jobs, int n_jobs, void* const* job_src_ptrs, void* const* job_dst_ptrs,
-                             int job_stat_stride, int* status, void* stream) {
+                             int n_levels, void* workspace, int level_passes, const void* jobs, int n_jobs,
+                             void* const* job_src_ptrs, void* const* job_dst_ptrs, int job_stat_stride, int* status, void* stream) {
   if (n_ctas <= 0) return n_jobs > 0 ? -6 : 0;   // copy jobs need a kernel to ride on
   if (n_dst > kMaxPeers || hq % hkv != 0 || channels < 1 || channels > kHeadDim) return -3;
   const bool levels = workspace != nullptr && dcpk_attn_bwd_workspace(n_items_total, q_rows, hq, channels, n_levels) > 0;
@@ -877,26 +831,30 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   if (raise_smem_limit(kernel, smem, g_bwd_smem_raised[v]) != cudaSuccess) return -4;
   // about 16 fetch CTAs when there is something to fetch
   const int n_copy_rows = n_jobs > 0 ? (16 + hkv - 1) / hkv : 0;
-  const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total, levels || n_levels == 1);
+  const bool any_order = levels || n_levels == 1;   // of the additions to dQ
+  const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total, any_order);
   const int heads_per_cta = group / parts;
-  // A plain launch: CTAs that begin together go through the queries together and find one another's tiles in L2, those that begin as
-  // the SMs come free do not (forward and backward of 121987 tokens, mixed masks, 41.3 ms plain, 44.3 overlapped with the kernel
-  // before; 6168 tokens 1008 and 1050 us).  A single wave would gain 3 us of 134 (four sequences of 300 to 2100 tokens, 8 / 2
-  // heads).
+  // Overlapped with the kernel before it only where all CTAs run at once: CTAs that begin together go through the queries
+  // together and find one another's tiles in L2, those that begin as the SMs come free do not (forward and backward of 121987
+  // tokens, mixed masks, 41.3 ms plain, 44.3 overlapped; 6168 tokens 1008 and 1050 us; 4040 tokens in one wave 134 and 131 us).  And only
+  // where dQ has levels, as the CTAs of an overlapped wave begin so far apart that they add to dQ in another order each time.
   const dim3 grid(hkv * parts, n_ctas + n_copy_rows);
-  const bool narrow = level_pitch(channels) == 64;
-  auto pass_over_levels = [&](auto kernel) {
-    return launch_overlapped(kernel, unsigned((q_rows + kLevelRows - 1) / kLevelRows), 256, 0, static_cast<cudaStream_t>(stream), 1, true,
-                             static_cast<const BwdItemDesc*>(items), n_items_total, static_cast<float*>(workspace), n_levels,
-                             dq_ptrs[0], int(q_rows), hq, channels);
-  };
-  if (levels && pass_over_levels(narrow ? dq_levels_kernel<64, false> : dq_levels_kernel<128, false>) != cudaSuccess) return -5;
+  const DcpkDqLevels of_call = {items, n_items_total, n_levels, int(q_rows), hq, channels, levels ? workspace : nullptr};
+  const unsigned level_blocks = unsigned((q_rows + kLevelRows - 1) / kLevelRows);
+  if (levels && (level_passes & 1) &&
+      launch_overlapped(dq_levels_kernel<false>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, true, make_levels(&of_call),
+                        dq_ptrs[0]) != cudaSuccess)
+    return -5;
   const cudaError_t rc = launch_overlapped(
-      kernel, grid, kBwdThreads, smem, static_cast<cudaStream_t>(stream), unsigned(parts), false, tm_q, tm_do,
+      kernel, grid, kBwdThreads, smem, static_cast<cudaStream_t>(stream), unsigned(parts),
+      any_order && long(grid.x) * grid.y <= kSms, tm_q, tm_do,
       tm_kv, tm_dq, tm_dkv, tm_levels, levels ? n_levels : 1, static_cast<const BwdCta*>(ctas), static_cast<const BwdItemDesc*>(items),
       static_cast<const int4*>(masks), lse, delta, pp, hq, hkv, heads_per_cta, stat_stride, n_dst, int(q_rows), int(kv_rows),
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);
   if (rc != cudaSuccess || cudaGetLastError() != cudaSuccess) return -5;
-  if (levels && pass_over_levels(narrow ? dq_levels_kernel<64, true> : dq_levels_kernel<128, true>) != cudaSuccess) return -5;
+  if (levels && (level_passes & 2) &&
+      launch_overlapped(dq_levels_kernel<true>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, true, make_levels(&of_call),
+                        dq_ptrs[0]) != cudaSuccess)
+    return -5;
   return 0;
 }

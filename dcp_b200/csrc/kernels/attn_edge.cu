@@ -14,6 +14,7 @@
 
 #include <type_traits>
 
+#include "attn_levels.cuh"
 #include "entries.h"
 #include "launch.cuh"
 
@@ -104,6 +105,36 @@ __global__ void __launch_bounds__(kEdgeThreads) cut_cast_kernel(const S* __restr
   }
 }
 
+// The same of dQ and dKV where dQ has levels, which are added on the way.  The first `row_blocks` blocks take dQ, kLevelRows rows each.
+// As a launch of its own the sum took 13 us of 135 (42 MB of levels and 16 of dQ; four sequences of 300 to 2100 tokens, 8 / 2 heads).
+template <typename T>
+__global__ void __launch_bounds__(kEdgeThreads) cut_cast_levels_kernel(const __grid_constant__ DqLevels lv, const float* __restrict__ dq,
+                                                                       T* __restrict__ gq, const float* __restrict__ dkv,
+                                                                       T* __restrict__ gkv, size_t n_kv, int d8, int row_blocks) {
+  __shared__ RowLevels present;
+  grid_let_next();
+  grid_wait();
+  if (int(blockIdx.x) >= row_blocks) {
+    for (size_t c = size_t(blockIdx.x - row_blocks) * kEdgeThreads + threadIdx.x; c < n_kv; c += size_t(gridDim.x - row_blocks) * kEdgeThreads)
+      cut_chunk(dkv, gkv, c, d8);
+    return;
+  }
+  const int row0 = blockIdx.x * kLevelRows, per_row = lv.hq * d8;
+  find_levels(lv, row0, present);
+  for (int c = threadIdx.x; c < kLevelRows * per_row; c += kEdgeThreads) {
+    const int r = c / per_row, k = c % d8;
+    if (row0 + r >= lv.q_rows) break;
+    const size_t head_row = size_t(row0 + r) * lv.hq + c % per_row / d8;
+    const float4* src = reinterpret_cast<const float4*>(dq + head_row * kEdgeHeadDim + 8 * k);
+    const uint64_t above = levels_above(present, r);
+    float4 a = src[0], b = src[1];
+    add_levels(lv, above, head_row * lv.pitch + 8 * k, a);
+    add_levels(lv, above, head_row * lv.pitch + 8 * k + 4, b);
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    store8(gq + (head_row * d8 + k) * 8, f);
+  }
+}
+
 // delta[h][row] = sum_d dO[row][h][d] * O[row][h][d]: sixteen lanes per (row, head), 16 bytes each of both
 // operands, four (row, head) pairs in flight per thread; then the grid clears the two accumulators.
 // One warp per pair with 8-byte loads read at 3.7 TB/s and the two fills were launches of their own.
@@ -111,7 +142,8 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_
                                                                      const __nv_bfloat16* __restrict__ d_o,
                                                                      float* __restrict__ delta, int n_rows, int hq,
                                                                      int stat_stride, float4* __restrict__ zero0, size_t nz0,
-                                                                     float4* __restrict__ zero1, size_t nz1) {
+                                                                     float4* __restrict__ zero1, size_t nz1,
+                                                                     const __grid_constant__ DqLevels levels) {
   const size_t tid = size_t(blockIdx.x) * kEdgeThreads + threadIdx.x, n_thr = size_t(gridDim.x) * kEdgeThreads;
   const int sub = threadIdx.x & 15;
   const size_t n_items = size_t(n_rows) * hq, step = n_thr >> 4;
@@ -147,6 +179,9 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (size_t i = tid; i < nz0; i += n_thr) zero0[i] = z;
   for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
+  __shared__ RowLevels present;
+  if (levels.n_levels > 1)
+    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
 }
 
 // The same for gradients in the caller's form (rows of d8 chunks of 8 channels): dO also goes to the arena's rows, rounded to
@@ -157,7 +192,8 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const 
                                                                           __nv_bfloat16* __restrict__ rows, float* __restrict__ delta,
                                                                           int n_rows, int hq, int stat_stride,
                                                                           float4* __restrict__ zero0, size_t nz0,
-                                                                          float4* __restrict__ zero1, size_t nz1) {
+                                                                          float4* __restrict__ zero1, size_t nz1,
+                                                                          const __grid_constant__ DqLevels levels) {
   constexpr int kInFlight = 2;
   const size_t tid = size_t(blockIdx.x) * kEdgeThreads + threadIdx.x, n_thr = size_t(gridDim.x) * kEdgeThreads;
   const int sub = threadIdx.x & 15;
@@ -194,6 +230,9 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const 
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (size_t i = tid; i < nz0; i += n_thr) zero0[i] = z;
   for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
+  __shared__ RowLevels present;
+  if (levels.n_levels > 1)
+    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
 }
 
 static int edge_grid(size_t chunks) {
@@ -251,22 +290,43 @@ extern "C" int dcpk_cut_cast_rows(int src_f32, int type, const void* src0, void*
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+// The gradients of a call whose dQ has levels (these with items, workspace and the rest of dcpk_attn_bwd's call): dq fp32
+// [levels->q_rows, levels->hq, 128] and dkv fp32 [rows1, 128] -> rows of d channels of element type `type`.
+extern "C" int dcpk_cut_cast_gradients(int type, const DcpkDqLevels* levels, const float* dq, void* gq, const float* dkv, void* gkv,
+                                       long rows1, int d, void* stream) {
+  if (!levels || !levels->workspace || levels->n_levels < 2 || rows1 < 0 || d <= 0 || d % 8 || d > kEdgeHeadDim || d > levels->channels ||
+      type < 0 || type > 2)
+    return -3;
+  const int d8 = d / 8, row_blocks = (levels->q_rows + kLevelRows - 1) / kLevelRows;
+  const size_t n_kv = size_t(rows1) * d8;
+  auto launch = [&](auto kernel, auto* as) {
+    using T = std::remove_pointer_t<decltype(as)>;
+    return launch_overlapped(kernel, unsigned(row_blocks + edge_grid(n_kv)), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, true,
+                             make_levels(levels), dq, static_cast<T*>(gq), dkv, static_cast<T*>(gkv), n_kv, d8, row_blocks);
+  };
+  if (type == 0) launch(cut_cast_levels_kernel<float>, static_cast<float*>(nullptr));
+  else if (type == 1) launch(cut_cast_levels_kernel<__half>, static_cast<__half*>(nullptr));
+  else launch(cut_cast_levels_kernel<__nv_bfloat16>, static_cast<__nv_bfloat16*>(nullptr));
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
 // o, d_o: bf16 [n_rows, hq, 128]; delta fp32 [hq, stat_stride]; zero0 / zero1: fp32 buffers of nz0 / nz1 elements
-// (multiples of 4)
+// (multiples of 4); levels (may be null): of the dQ of the backward that follows, cleared where it will add to them
 extern "C" int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, int n_rows, int hq, int stat_stride,
-                                  float* zero0, long nz0, float* zero1, long nz1, void* stream) {
+                                  float* zero0, long nz0, float* zero1, long nz1, const DcpkDqLevels* levels, void* stream) {
   if (n_rows < 0 || hq <= 0 || n_rows > stat_stride || nz0 % 4 || nz1 % 4 || nz0 < 0 || nz1 < 0) return -3;
   const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
   if (work == 0) return 0;
   launch_overlapped(
       attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
-      reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4);
+      reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 // o, d_o: [n_rows, hq, d] of an element type as above; d_o_rows: bf16 [n_rows, hq, 128]; the rest as dcpk_attn_bwd_prep
 extern "C" int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o, int d, void* d_o_rows, float* delta, int n_rows, int hq,
-                                       int stat_stride, float* zero0, long nz0, float* zero1, long nz1, void* stream) {
+                                       int stat_stride, float* zero0, long nz0, float* zero1, long nz1,
+                                       const DcpkDqLevels* levels, void* stream) {
   if (n_rows < 0 || hq <= 0 || n_rows > stat_stride || nz0 % 4 || nz1 % 4 || nz0 < 0 || nz1 < 0 || d <= 0 || d % 8 ||
       d > kEdgeHeadDim || type < 0 || type > 2)
     return -3;
@@ -277,7 +337,7 @@ extern "C" int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o,
     return launch_overlapped(kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass,
                              static_cast<const T*>(o), static_cast<const T*>(d_o), d / 8, static_cast<__nv_bfloat16*>(d_o_rows), delta,
                              n_rows, hq, stat_stride, reinterpret_cast<float4*>(zero0), size_t(nz0) / 4,
-                             reinterpret_cast<float4*>(zero1), size_t(nz1) / 4);
+                             reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
   };
   if (type == 0) launch(attn_bwd_prep_cast_kernel<float>, static_cast<float*>(nullptr));
   else if (type == 1) launch(attn_bwd_prep_cast_kernel<__half>, static_cast<__half*>(nullptr));

@@ -448,7 +448,7 @@ def attn_bwd_prep(out: torch.Tensor, dout: torch.Tensor, delta: torch.Tensor, n_
         assert t is None or (t.is_contiguous() and t.dtype == torch.float32 and t.numel() % 4 == 0)
         args += [ctypes.c_void_p(0), ctypes.c_long(0)] if t is None else [_lib.ptr(t), ctypes.c_long(t.numel())]
     rc = lib.dcpk_attn_bwd_prep(_lib.ptr(out[row0:]), _lib.ptr(dout[row0:]), ctypes.c_void_p(delta.data_ptr() + 4 * row0),
-                                ctypes.c_int(n_rows), ctypes.c_int(hq), ctypes.c_int(delta.shape[1]), *args,
+                                ctypes.c_int(n_rows), ctypes.c_int(hq), ctypes.c_int(delta.shape[1]), *args, ctypes.c_void_p(0),
                                 _lib.stream_handle())
     _lib.check(rc, "dcpk_attn_bwd_prep")
 
@@ -517,7 +517,7 @@ def attn_bwd(q_arena, do_arena, kv_arena, lse, delta, tables: BwdTables, dq_dsts
         ctypes.c_int(tables.masks.shape[0]), _lib.ptr(lse), _lib.ptr(delta),
         ctypes.c_int(lse.shape[1]), _ptr_array(dq_dsts), _ptr_array(dkv_dsts), ctypes.c_int(len(dq_dsts)),
         ctypes.c_float(scale), ctypes.c_int(channels), ctypes.c_int(tables.dq_levels),
-        ctypes.c_void_p(workspace.data_ptr() if n_bytes else 0), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
+        ctypes.c_void_p(workspace.data_ptr() if n_bytes else 0), ctypes.c_int(3), *_job_args(jobs, job_ctx), _lib.ptr(status), _lib.stream_handle())
     _lib.check(rc, "dcpk_attn_bwd")
 
 
