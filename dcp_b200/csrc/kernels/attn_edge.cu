@@ -235,6 +235,10 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const 
     for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
 }
 
+// Passes over levels are plain launches: overlapped, both took longer (2048 tokens, 8 / 2 heads, forward and backward in a graph, 88
+// and 93 us; four sequences of 300 to 2100 tokens 119 and 122).
+static bool small_pass(size_t work, const DcpkDqLevels* levels) { return work <= kSmallPass && !(levels && levels->workspace); }
+
 static int edge_grid(size_t chunks) {
   const size_t b = (chunks + kEdgeThreads - 1) / kEdgeThreads;
   return int(b < size_t(kEdgeBlocks) ? b : size_t(kEdgeBlocks));
@@ -301,7 +305,7 @@ extern "C" int dcpk_cut_cast_gradients(int type, const DcpkDqLevels* levels, con
   const size_t n_kv = size_t(rows1) * d8;
   auto launch = [&](auto kernel, auto* as) {
     using T = std::remove_pointer_t<decltype(as)>;
-    return launch_overlapped(kernel, unsigned(row_blocks + edge_grid(n_kv)), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, true,
+    return launch_overlapped(kernel, unsigned(row_blocks + edge_grid(n_kv)), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, false,
                              make_levels(levels), dq, static_cast<T*>(gq), dkv, static_cast<T*>(gkv), n_kv, d8, row_blocks);
   };
   if (type == 0) launch(cut_cast_levels_kernel<float>, static_cast<float*>(nullptr));
@@ -318,7 +322,7 @@ extern "C" int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, 
   const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
   if (work == 0) return 0;
   launch_overlapped(
-      attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass, static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
+      attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels), static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
       reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -334,7 +338,7 @@ extern "C" int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o,
   if (work == 0) return 0;
   auto launch = [&](auto kernel, auto* as) {
     using T = std::remove_pointer_t<decltype(as)>;
-    return launch_overlapped(kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, work <= kSmallPass,
+    return launch_overlapped(kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels),
                              static_cast<const T*>(o), static_cast<const T*>(d_o), d / 8, static_cast<__nv_bfloat16*>(d_o_rows), delta,
                              n_rows, hq, stat_stride, reinterpret_cast<float4*>(zero0), size_t(nz0) / 4,
                              reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
