@@ -1,15 +1,15 @@
 // Host side of attention calls with a single rank, in native code.
 //
-// A call is three to six launches.  Driven from Python it took 46 us of host time forward and 107 us backward (8 query
-// heads, 4040 tokens in four sequences) against 30 and 105 us of device time, so small calls waited for the host; most of
-// it went into checks, slices, argument objects and result tensors between the launches.  Here the pieces that do not change
-// between calls (tables, arenas, sizes) are laid out once per program, and a call checks its tensors, allocates its results
-// and launches: 13 us and 21 us.  The whole call, autograd's 48 us included, took 229 us and
-// takes 105 of host time, so it now waits for the device (212 -> 143 us); fp32 tensors of 64 channels, two launches and three
-// tensors more, 304 -> 116 us of host time (284 -> 230).
+// A forward is one or two launches, a backward three or four.  Driven from Python small calls waited for the host; most
+// of its time went into checks, slices, argument objects and result tensors between the launches.  Here the pieces that
+// do not change between calls (tables, arenas, sizes) are laid out once per program, and a call checks its tensors,
+// allocates its results and launches. Host time (8 query heads, 4040 tokens in four sequences): forward 37 -> 13 us,
+// backward 105 -> 27, the whole call with autograd 221 -> 97; 7680 tokens of 64 fp32 channels 71 -> 10, 110 -> 16 and
+// 302 -> 96.
 //
-// Only plain calls are taken: tensors on the arenas' device, contiguous, 16-byte aligned, of a type the row kernels read.
-// For anything else the functions return nothing before they launch anything, and the caller goes the general way.
+// Only plain calls are taken: tensors on the arenas' device, contiguous, 16-byte aligned, of a type the row kernels
+// read. For anything else the functions return nothing before they launch anything, and the caller goes the general
+// way.
 #include <ATen/ATen.h>
 #include <c10/core/DeviceGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -91,8 +91,8 @@ class SingleRankAttention {
     check(dcpk_attn_fwd_pair(q_in.const_data_ptr(), q_in.size(0), kv_in.const_data_ptr(), kv_in.size(0), int(q.size(1)),
                              int(kv.size(2)), tiles.const_data_ptr(), n_tiles, kv_entries.const_data_ptr(),
                              int(kv_entries.size(0)), fwd_masks.const_data_ptr(), int(fwd_masks.size(0)), outs, lses, 2,
-                             int(part_lse.size(1)), int(l.size(1)), 1, out_type, out_channels, float(scale), channels, nullptr, 0, nullptr, nullptr, 0,
-                             status.data_ptr<int>(), stream()),
+                             int(part_lse.size(1)), int(l.size(1)), 1, out_type, out_channels, float(scale), channels, nullptr, 0, nullptr,
+                             nullptr, 0, status.data_ptr<int>(), stream()),
           "dcpk_attn_fwd_pair");
   }
 
@@ -105,8 +105,8 @@ class SingleRankAttention {
                      bytes > 0 ? memory.data_ptr() : nullptr}};
   }
 
-  // delta and cleared accumulators, then the gradients; `o` and `d_in`: at least the local rows, of `d` channels.  Other than rows
-  // of 128 in bf16 go to the arena of dO on the way.
+  // delta and cleared accumulators, then the gradients; `o` and `d_in`: at least the local rows, of `d` channels.
+  // Other than rows of 128 in bf16 go to the arena of dO on the way.
   void launch_backward(const Tensor& q_in, const Tensor& d_in, const Tensor& kv_in, const Tensor& o, const Tensor& l, const Tensor& dl,
                        int d, const DcpkDqLevels& levels, bool sum_levels, double scale) const {
     const long hq = q.size(1), hkv = kv.size(2);

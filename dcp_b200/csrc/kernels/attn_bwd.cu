@@ -21,34 +21,38 @@
 // [32 queries x 32 channels] fp32 tile per step, added to the accumulator with one tiled TMA
 // reduce-add, or to a peer's with a 128-byte bulk reduce-add per row), 24 TMA producer, 25 UMMA issuer, 26
 // per-query statistics, 27 idle.  dK/dV stay in TMEM for the CTA's lifetime and are added once,
-// through shared memory with tiled TMA reduce-adds (with red.global.add.v4.f32, a row per lane, L2 took 11000 cycles for the
-// 128 KB of a key tile, 7000 now: one visit per CTA 15.4 -> 13.1 us per wave, 18944 keys x 1024 queries, 8 heads, 256 -> 232 us,
-// with 64 channels 180 -> 172; what is left of it is L2's rate of fp32 additions, 20 bytes per cycle and SM); the CTAs of a split head group first add their shares up through distributed
-// shared memory, in the order of their heads, so that an element has one adder and the same bits in every run
-// (with an atomic addition per CTA, three and more of them gave other last bits each time).  dQ is added to by
-// every key tile as it comes, in short launches through buffers of at most two additions each, which are summed afterwards (see
-// attn_levels.cuh): these give the same bits in every run, the last bits of longer ones differ.
+// through shared memory with tiled TMA reduce-adds (with red.global.add.v4.f32, a row per lane, L2 took 11000 cycles
+// for the 128 KB of a key tile, 7000 now: one visit per CTA 15.4 -> 13.1 us per wave, 18944 keys x 1024 queries, 8
+// heads, 256 -> 232 us, with 64 channels 180 -> 172; what is left of it is L2's rate of fp32 additions, 20 bytes per
+// cycle and SM); the CTAs of a split head group first add their shares up through distributed shared memory, in the
+// order of their heads, so that an element has one adder and the same bits in every run (with an atomic addition per
+// CTA, three and more of them gave other last bits each time).  dQ is added to by every key tile as it comes, in short
+// launches through buffers of at most two additions each, which are summed afterwards (see attn_levels.cuh): these give
+// the same bits in every run, the last bits of longer ones differ.
 //
 // Why 128 x 128: a UMMA with N = 64 occupies the tensor pipe almost as long as one with N = 128 (61 and 72
 // cycles with both operands in shared memory, 64 with A in TMEM), so with 64-query items three of the five
 // products ran at half rate.  The issuer is one thread, taken by elect.sync: with a test on the lane number
-// each UMMA took about 90 cycles to issue (128 x 128 tiles: 839 against 1053 TFLOP/s).  Its descriptors cost an addition of 32
-// bits each, and it asks for operands that are long there while it has something to issue: an answer takes 200 cycles and
-// more, behind the exponentials of the warps that share its scheduler (full 5.52 -> 5.45 ms, causal 4.18 -> 4.13, sink +
-// window 1.52 -> 1.51 in long runs; 1000 queries x 2100 keys, causal, 101 -> 99 us).  Handing dS^T to dK before it is stored
-// for dQ costs more registers than it gains time (5.69 ms).  16 gradient warps of
-// 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
+// each UMMA took about 90 cycles to issue (128 x 128 tiles: 839 against 1053 TFLOP/s).  Its descriptors cost an
+// addition of 32 bits each, and it asks for operands that are long there while it has something to issue: an answer
+// takes 200 cycles and more, behind the exponentials of the warps that share its scheduler (full 5.52 -> 5.45 ms,
+// causal 4.18 -> 4.13, sink + window 1.52 -> 1.51 in long runs; 1000 queries x 2100 keys, causal, 101 -> 99 us).
+// Handing dS^T to dK before it is stored for dQ costs more registers than it gains time (5.69 ms).  16 gradient warps
+// of 32 queries instead of 8 of 64: the unrolled loops of 8 warps did not stay in the instruction cache (5 of
 // 13 stall cycles per issue; 0.5 of 19 now).  8 drain warps keep their part of dQ in registers, so the columns
 // are free before the shared-memory tile and the L2 have taken it (4 warps with half of it at a time: 7 % slower).
-// What bounds it now: an item takes 4100 to 4300 cycles for 2600 of tensor time, and the chain dS(t), dK(t), dQ(t), dQ to
-// registers, dP(t+1) is as long, because dP, dS and dQ share 128 TMEM columns.  L2 adds 64 KB of dQ in 2900 cycles when all
-// SMs add to tiles that are there (4300 when they are not), and shared memory moves 2048 wavefronts of UMMA operands and about
-// 1900 of loads and stores; without the dQ drain an item takes 15 % less.  Not what bounds it: the broadcast reads of lse and
-// delta (as a product of their own, three bf16 terms each: 4.85 -> 4.95 ms, and no faster with that product left out), the
-// conversions to bf16 (left out: the same), the order of a CTA's queries (reversed: the same).  In long runs the power limit
-// holds the clock at 1.3 to 1.6 GHz.  A pair of CTAs for 256 keys needs Q, dO and K in two layouts: 256 KB of shared memory.
-// Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104
-// TFLOP/s), causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
+// What bounds it now: an item takes 4100 to 4300 cycles for 2600 of tensor time, and the chain dS(t), dK(t), dQ(t), dQ
+// to registers, dP(t+1) is as long, because dP, dS and dQ share 128 TMEM columns.  L2 adds 64 KB of dQ in 2900 cycles
+// when all SMs add to tiles that are there (4300 when they are not), and shared memory moves 2048 wavefronts of UMMA
+// operands and about 1900 of loads and stores; without the dQ drain an item takes 15 % less.  Not what bounds it: the
+// broadcast reads of lse and delta (as a product of their own, three bf16 terms each: 4.85 -> 4.95 ms, and no faster
+// with that product left out), the conversions to bf16 (left out: the same), the order of a CTA's queries (reversed:
+// the same).  In long runs the power limit holds the clock at 1.3 to 1.6 GHz.  Not tried: a pair of CTAs for 256 keys
+// (cta_group::2), which would add half as much to dQ.  It needs Q, dO and K in two layouts, by count 208 KB of shared
+// memory per CTA: K and V 32 each, K for dQ 32, Q and dO for S and dP 16 each, for dK and dV 16 each, dS for dQ 32, dQ
+// staging 16.
+// Measured (8192 queries x 16384 keys, 32 / 8 heads, against 64-query items): full 6.68 -> 4.98 ms (1104 TFLOP/s),
+// causal 4.99 -> 3.77 ms (1095), sink + window 1.84 -> 1.38 ms (1009).
 //
 // The first `n_copy_rows` rows of the grid are fetch CTAs: they compute nothing and bring the next plan
 // stage's remote operands (Q, dO, KV rows and the lse / delta statistics of the queries) from peer
@@ -215,11 +219,11 @@ __device__ __forceinline__ void grad_scores(const uint32_t* p, const uint32_t* d
   }
 }
 
-// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and products over zeros
-// and accumulators of zeros are left out: for up to 64 channels half of S and dP (K steps), half of dK, dV and dQ (N) and
-// of their traffic; for up to 96 a quarter of S, dP and the drain of dQ (N stays 128: an operand that is not K-major comes in
-// 64s).  8192 queries x 16384 keys, 32 / 8 heads, causal, against all 128
-// channels: 64 channels 3.56 -> 2.61 ms, 96 channels 3.99 -> 3.45 ms; 1000 x 2100: 110 -> 83 us and 122 -> 110 us.
+// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and products over
+// zeros and accumulators of zeros are left out: for up to 64 channels half of S and dP (K steps), half of dK, dV and dQ
+// (N) and of their traffic; for up to 96 a quarter of S, dP and the drain of dQ (N stays 128: an operand that is not
+// K-major comes in 64s).  8192 queries x 16384 keys, 32 / 8 heads, causal, against all 128 channels: 64 channels 3.56
+// -> 2.61 ms, 96 channels 3.99 -> 3.45 ms; 1000 x 2100: 110 -> 83 us and 122 -> 110 us.
 template <bool kTL, int kD>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -424,7 +428,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         constexpr uint32_t idesc_sdp = make_idesc_bf16(128, 128, 0, 0);
         constexpr uint32_t idesc_acc = make_idesc_bf16(128, 64 * kHalves, 0, 1);
         constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64 * kHalves, 1, 1);
-        // descriptors: K-major operands and MN-major ones differ in the leading offset, all others in the address field only
+        // descriptors: K-major operands and MN-major ones differ in the leading offset, all others in the address field
+        // only
         const uint64_t some = make_sdesc_sw128(0, 16, 1024), some_mn = make_sdesc_sw128(0, kHalf, 1024);
         const uint32_t hi = uint32_t(some >> 32), lo = uint32_t(some), lo_mn = uint32_t(some_mn);
         auto desc = [&](uint32_t low) { return (uint64_t(hi) << 32) | low; };
@@ -464,7 +469,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k)  // 16 queries per step; P^T: queries 32 i .. 32 i + 31 in columns [32 i, 32 i + 16) of S^T
-            umma_ts(tmem + cdV, tmem + cS + (k >> 1) * 32 + (k & 1) * 8, desc(lo_mn + do_at + k * 128), idesc_acc, (t > 0 || k > 0) ? 1u : 0u);
+            umma_ts(tmem + cdV, tmem + cS + (k >> 1) * 32 + (k & 1) * 8, desc(lo_mn + do_at + k * 128), idesc_acc,
+                    (t > 0 || k > 0) ? 1u : 0u);
           umma_commit(&sm.do_empty);
           TL_ADD(7, tl_t);
           return true;
@@ -548,7 +554,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (cur.dq_dev == 0) {
           if (lane == 0) {
             const int level = dq_level(cur.kv_pos0, n_levels), row = cur.dq_row + quad * 32;
-            tma_reduce_add_3d(level > 0 ? &tm_levels : &tm_dq, stage, ch0 + b * 32, cur.head, level > 0 ? (level - 1) * q_rows + row : row);
+            if (level > 0) tma_reduce_add_3d(&tm_levels, stage, ch0 + b * 32, cur.head, (level - 1) * q_rows + row);
+            else tma_reduce_add_3d(&tm_dq, stage, ch0 + b * 32, cur.head, row);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         } else if (quad * 32 + lane < cur.n_rows) {
@@ -635,8 +642,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int ch = (hf & 1) * 32 * kMine;
         float* dst = ptrs.dkv[cta.dkv_dev] + ((size_t(cta.dkv_row + r) * 2 + (hf >> 1)) * hkv + kv_head) * kHeadDim + ch;
         const uint32_t acc = tmem + lane_base + (hf >> 1 ? cdV : cdK) + ch;
-        // a whole key tile for this GPU's accumulator goes there in boxes of [32 keys x 32 channels], which take the place of K, V
-        // and Q; rows that may not be added to, and other GPUs' accumulators, go 16 bytes at a time
+        // a whole key tile for this GPU's accumulator goes there in boxes of [32 keys x 32 channels], which take the
+        // place of K, V and Q; rows that may not be added to, and other GPUs' accumulators, go 16 bytes at a time
         const bool whole = cta.dkv_dev == 0 && cta.n_valid == 128;
 #pragma unroll
         for (int c = 0; c < kMine; ++c) {
@@ -706,7 +713,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-// The passes over the levels of dQ as launches of their own (kSum: they are added to dQ; else they are cleared).  Bound by L2.
+// The passes over the levels of dQ as launches of their own (kSum: they are added to dQ; else they are cleared).  Bound
+// by L2.
 template <bool kSum>
 __global__ void __launch_bounds__(256) dq_levels_kernel(const __grid_constant__ DqLevels lv, float* __restrict__ dq) {
   __shared__ RowLevels present;
@@ -732,11 +740,12 @@ __global__ void __launch_bounds__(256) dq_levels_kernel(const __grid_constant__ 
 }
 
 static constexpr int kSms = 148, kMaxParts = 8, kMaxLevels = 64;
-// Launches of up to so many bytes of dQ tiles (one per visit) have levels, if these take no more than the other number.  Levels cost
-// what it takes to clear and to sum them, in the passes before and after the kernel or in launches of their own: four sequences of
-// 300 to 2100 tokens, 8 / 2 heads, 110 MB, forward and backward, 107 us without, 130 and 135 with them; 2048 tokens, 71 MB, 96, 101
-// and 108.  Above, what is added to no longer stays in L2: 2048 tokens, 32 / 8 heads, 285 MB, 169 and 280 us, 4096 tokens, 8 / 2
-// heads, 277 MB, 152 and 235.  (A tile of its own for every visit, stored and then summed, took 150 us for the first.)
+// Launches of up to so many bytes of dQ tiles (one per visit) have levels, if these take no more than the other number.
+// Levels cost what it takes to clear and to sum them, in the passes before and after the kernel or in launches of their
+// own: four sequences of 300 to 2100 tokens, 8 / 2 heads, 110 MB, forward and backward, 107 us without, 130 and 135
+// with them; 2048 tokens, 71 MB, 96, 101 and 108.  Above, what is added to no longer stays in L2: 2048 tokens, 32 / 8
+// heads, 285 MB, 169 and 280 us, 4096 tokens, 8 / 2 heads, 277 MB, 152 and 235.  (A tile of its own for every visit,
+// stored and then summed, took 150 us for the first.)
 static constexpr long kMaxVisitBytes = 128l << 20, kMaxWorkspace = 512l << 20;
 static std::atomic<uint64_t> g_bwd_smem_raised[4];
 static long long* g_bwd_timeline_host = nullptr;  // non-null selects the instrumented build of the kernel
@@ -754,7 +763,8 @@ extern "C" int dcpk_attn_bwd_set_timeline(void* buf) {
   return cudaMemcpyToSymbol(g_bwd_timeline, &p, sizeof(p)) == cudaSuccess ? 0 : -5;
 }
 
-// Bytes of the workspace of dcpk_attn_bwd for item lists of `n_levels` levels (see dq_level; 0: not known); 0: there is none.
+// Bytes of the workspace of dcpk_attn_bwd for item lists of `n_levels` levels (see dq_level; 0: not known); 0: there is
+// none.
 extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, int channels, int n_levels) {
   if (n_levels < 2 || n_levels > kMaxLevels) return 0;
   const long pitch = level_pitch(channels) * long(sizeof(float));
@@ -762,20 +772,20 @@ extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, 
   return long(n_items_total) * hq * kQTile * pitch <= kMaxVisitBytes && bytes <= kMaxWorkspace ? bytes : 0;
 }
 
-// Over how many CTAs a head group of `group` query heads is split, for `n_ctas` key tiles of `hkv` heads whose item lists have
-// n_items_total entries in all and at most max_items (0: not known, the group stays whole).
+// Over how many CTAs a head group of `group` query heads is split, for `n_ctas` key tiles of `hkv` heads whose item
+// lists have n_items_total entries in all and at most max_items (0: not known, the group stays whole).
 //
 // A CTA visits its items once per query head of the group, or the group is split over several CTAs (a cluster, at most
-// the portable 8, which adds its parts of dK / dV up in a fixed order): shorter longest lists, and more CTAs to begin and
-// end, which takes one as long as 8 visits (2.2 us each).  The launch takes as long as its longest list, or as all visits
-// spread over the SMs, whichever is more; the split for which that is least is taken, the smallest of equals.  Over 78
-// batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128 channels) that
-// is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was above the SMs' average, but
-// seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads: 152 us before, 109 in two parts; eight
-// sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.
-// CTAs that all run at once add to a row of dQ in the order of their items, and as long as their lists are short and begin at
-// different queries that is nearly the same in every run.  Without `any_wave` (dQ has levels, whose order does not matter) they
-// become more than one wave only where that takes 32 visits (about 70 us) off the longest list.
+// the portable 8, which adds its parts of dK / dV up in a fixed order): shorter longest lists, and more CTAs to begin
+// and end, which takes one as long as 8 visits (2.2 us each).  The launch takes as long as its longest list, or as all
+// visits spread over the SMs, whichever is more; the split for which that is least is taken, the smallest of equals.
+// Over 78 batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128
+// channels) that is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was
+// above the SMs' average, but seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads:
+// 152 us before, 109 in two parts; eight sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us. CTAs that all run at once
+// add to a row of dQ in the order of their items, and as long as their lists are short and begin at
+// different queries that is nearly the same in every run.  Without `any_wave` (dQ has levels, whose order does not
+// matter) they become more than one wave only where that takes 32 visits (about 70 us) off the longest list.
 extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total, int any_wave) {
   constexpr long kBegin = 8;
   auto visits = [&](int p) {   // times the SMs
@@ -792,12 +802,12 @@ extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items
   return parts;
 }
 
-// Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  channels: of the arenas' 128, those that may be other
-// than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are the
-// lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
-// length of the longest item list (0: not known, the head groups stay whole).  workspace: as many bytes as dcpk_attn_bwd_workspace
-// says; null: dQ has no levels.  level_passes: 1 they are cleared here (else dcpk_attn_bwd_prep did), + 2 and summed here (else
-// dcpk_cut_cast_gradients does).
+// Launches the backward kernel: one CTA per (entry of `ctas`, KV head).  channels: of the arenas' 128, those that may
+// be other than zero (the first); the gradients of the others are left as they are.  n_items_total / n_mask_rows are
+// the lengths of the item and mask tables; entries that point past them are reported (status 3), not read.  max_items:
+// length of the longest item list (0: not known, the head groups stay whole).  workspace: as many bytes as
+// dcpk_attn_bwd_workspace says; null: dQ has no levels.  level_passes: 1 they are cleared here (else dcpk_attn_bwd_prep
+// did), + 2 and summed here (else dcpk_cut_cast_gradients does).
 extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_rows, const void* kv_arena,
                              long kv_rows, int hq, int hkv, const void* ctas, int n_ctas, const void* items,
                              int n_items_total, int max_items, const void* masks, int n_mask_rows, const float* lse, const float* delta,
@@ -810,7 +820,8 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   CUtensorMap tm_q, tm_do, tm_kv, tm_dq, tm_dkv, tm_levels;
   if (encode_f32_tile_map(&tm_dq, dq_ptrs[0], uint64_t(q_rows), uint32_t(hq), kHeadDim, 32, 32)) return -1;
   tm_levels = tm_dq;
-  if (levels && encode_f32_tile_map(&tm_levels, workspace, uint64_t(n_levels - 1) * q_rows, uint32_t(hq), uint32_t(level_pitch(channels)), 32, 32))
+  if (levels && encode_f32_tile_map(&tm_levels, workspace, uint64_t(n_levels - 1) * q_rows, uint32_t(hq),
+                                    uint32_t(level_pitch(channels)), 32, 32))
     return -1;
   if (encode_f32_tile_map(&tm_dkv, dkv_ptrs[0], uint64_t(kv_rows), uint32_t(2 * hkv), kHeadDim, 32, 32)) return -1;
   if (encode_arena_map(&tm_q, q_arena, uint64_t(q_rows), uint32_t(hq), kHeadDim, kQTile)) return -1;
@@ -834,10 +845,11 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   const bool any_order = levels || n_levels == 1;   // of the additions to dQ
   const int group = hq / hkv, parts = dcpk_attn_bwd_parts(n_ctas, hkv, group, max_items, n_items_total, any_order);
   const int heads_per_cta = group / parts;
-  // Overlapped with the kernel before it only where all CTAs run at once: CTAs that begin together go through the queries
-  // together and find one another's tiles in L2, those that begin as the SMs come free do not (forward and backward of 121987
-  // tokens, mixed masks, 41.3 ms plain, 44.3 overlapped; 6168 tokens 1008 and 1050 us; 4040 tokens in one wave 134 and 131 us).  And only
-  // where dQ has levels, as the CTAs of an overlapped wave begin so far apart that they add to dQ in another order each time.
+  // Overlapped with the kernel before it only where all CTAs run at once: CTAs that begin together go through the
+  // queries together and find one another's tiles in L2, those that begin as the SMs come free do not (forward and
+  // backward of 121987 tokens, mixed masks, 41.3 ms plain, 44.3 overlapped; 6168 tokens 1008 and 1050 us; 4040 tokens
+  // in one wave 134 and 131 us).  And only where dQ has levels, as the CTAs of an overlapped wave begin so far apart
+  // that they add to dQ in another order each time.
   const dim3 grid(hkv * parts, n_ctas + n_copy_rows);
   const DcpkDqLevels of_call = {items, n_items_total, n_levels, int(q_rows), hq, channels, levels ? workspace : nullptr};
   const unsigned level_blocks = unsigned((q_rows + kLevelRows - 1) / kLevelRows);

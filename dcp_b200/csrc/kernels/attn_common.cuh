@@ -39,7 +39,7 @@ struct KvEntry {
 };
 
 struct PeerPtrs {
-  void* out[kMaxPeers];   // bf16 [rows, hq, d] per destination
+  void* out[kMaxPeers];   // per destination: bf16 [rows, hq, 128], final buffers perhaps of another type and width
   float* lse[kMaxPeers];  // fp32 [hq, rows] per destination
 };
 

@@ -24,7 +24,7 @@ static constexpr int kEdgeHeadDim = 128;
 static constexpr int kEdgeThreads = 256;
 static constexpr int kEdgeBlocks = 148 * 8;   // every SM full (2048 threads)
 // Passes over up to so many chunks of 16 bytes (about 10 us) begin while the kernel before them ends.  Longer ones gain
-// nothing from it (6168 tokens of 32 heads, seven kernels: 1008 -> 1010 us; 121987 tokens 41.4 -> 41.9 ms).
+// nothing from it (6168 tokens of 32 heads, forward and backward, 1008 -> 1010 us; 121987 tokens 41.4 -> 41.9 ms).
 static constexpr size_t kSmallPass = size_t(1) << 21;
 
 __device__ __forceinline__ void load8(const float* p, float* f) {
@@ -105,17 +105,19 @@ __global__ void __launch_bounds__(kEdgeThreads) cut_cast_kernel(const S* __restr
   }
 }
 
-// The same of dQ and dKV where dQ has levels, which are added on the way.  The first `row_blocks` blocks take dQ, kLevelRows rows each.
-// As a launch of its own the sum took 13 us of 135 (42 MB of levels and 16 of dQ; four sequences of 300 to 2100 tokens, 8 / 2 heads).
+// The same of dQ and dKV where dQ has levels, which are added on the way.  The first `row_blocks` blocks take dQ,
+// kLevelRows rows each. As a launch of its own the sum took 13 us of 135 (42 MB of levels and 16 of dQ; four sequences
+// of 300 to 2100 tokens, 8 / 2 heads).
 template <typename T>
-__global__ void __launch_bounds__(kEdgeThreads) cut_cast_levels_kernel(const __grid_constant__ DqLevels lv, const float* __restrict__ dq,
-                                                                       T* __restrict__ gq, const float* __restrict__ dkv,
-                                                                       T* __restrict__ gkv, size_t n_kv, int d8, int row_blocks) {
+__global__ void __launch_bounds__(kEdgeThreads)
+cut_cast_levels_kernel(const __grid_constant__ DqLevels lv, const float* __restrict__ dq, T* __restrict__ gq,
+                       const float* __restrict__ dkv, T* __restrict__ gkv, size_t n_kv, int d8, int row_blocks) {
   __shared__ RowLevels present;
   grid_let_next();
   grid_wait();
   if (int(blockIdx.x) >= row_blocks) {
-    for (size_t c = size_t(blockIdx.x - row_blocks) * kEdgeThreads + threadIdx.x; c < n_kv; c += size_t(gridDim.x - row_blocks) * kEdgeThreads)
+    const size_t stride = size_t(gridDim.x - row_blocks) * kEdgeThreads;
+    for (size_t c = size_t(blockIdx.x - row_blocks) * kEdgeThreads + threadIdx.x; c < n_kv; c += stride)
       cut_chunk(dkv, gkv, c, d8);
     return;
   }
@@ -184,9 +186,9 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_
     for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
 }
 
-// The same for gradients in the caller's form (rows of d8 chunks of 8 channels): dO also goes to the arena's rows, rounded to
-// bf16 and zero-padded, and delta is that of the rounded values.  As a pass that converts O and dO and the one above
-// it took 22 us for 7680 tokens of 8 heads with 64 fp32 channels.
+// The same for gradients in the caller's form (rows of d8 chunks of 8 channels): dO also goes to the arena's rows,
+// rounded to bf16 and zero-padded, and delta is that of the rounded values.  As a pass that converts O and dO and the
+// one above it took 22 us for 7680 tokens of 8 heads with 64 fp32 channels.
 template <typename T>
 __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const T* __restrict__ o, const T* __restrict__ d_o, int d8,
                                                                           __nv_bfloat16* __restrict__ rows, float* __restrict__ delta,
@@ -235,8 +237,8 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const 
     for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
 }
 
-// Passes over levels are plain launches: overlapped, both took longer (2048 tokens, 8 / 2 heads, forward and backward in a graph, 88
-// and 93 us; four sequences of 300 to 2100 tokens 119 and 122).
+// Passes over levels are plain launches: overlapped, both took longer (2048 tokens, 8 / 2 heads, forward and backward
+// in a graph, 88 and 93 us; four sequences of 300 to 2100 tokens 119 and 122).
 static bool small_pass(size_t work, const DcpkDqLevels* levels) { return work <= kSmallPass && !(levels && levels->workspace); }
 
 static int edge_grid(size_t chunks) {
@@ -251,8 +253,8 @@ static void launch_pad(const void* s0, void* d0, size_t n0, const void* s1, void
 }
 template <typename S, typename T>
 static void launch_cut(const void* s0, void* d0, size_t n0, const void* s1, void* d1, size_t n1, int d8, cudaStream_t st) {
-  launch_overlapped(cut_cast_kernel<S, T>, edge_grid(n0 + n1), kEdgeThreads, 0, st, 1, n0 + n1 <= kSmallPass, static_cast<const S*>(s0), static_cast<T*>(d0),
-                    n0, static_cast<const S*>(s1), static_cast<T*>(d1), n1, d8);
+  launch_overlapped(cut_cast_kernel<S, T>, edge_grid(n0 + n1), kEdgeThreads, 0, st, 1, n0 + n1 <= kSmallPass,
+                    static_cast<const S*>(s0), static_cast<T*>(d0), n0, static_cast<const S*>(s1), static_cast<T*>(d1), n1, d8);
 }
 
 }  // namespace dcpk
@@ -294,12 +296,12 @@ extern "C" int dcpk_cut_cast_rows(int src_f32, int type, const void* src0, void*
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// The gradients of a call whose dQ has levels (these with items, workspace and the rest of dcpk_attn_bwd's call): dq fp32
-// [levels->q_rows, levels->hq, 128] and dkv fp32 [rows1, 128] -> rows of d channels of element type `type`.
+// The gradients of a call whose dQ has levels (these with items, workspace and the rest of dcpk_attn_bwd's call): dq
+// fp32 [levels->q_rows, levels->hq, 128] and dkv fp32 [rows1, 128] -> rows of d channels of element type `type`.
 extern "C" int dcpk_cut_cast_gradients(int type, const DcpkDqLevels* levels, const float* dq, void* gq, const float* dkv, void* gkv,
                                        long rows1, int d, void* stream) {
-  if (!levels || !levels->workspace || levels->n_levels < 2 || rows1 < 0 || d <= 0 || d % 8 || d > kEdgeHeadDim || d > levels->channels ||
-      type < 0 || type > 2)
+  if (!levels || !levels->workspace || levels->n_levels < 2 || rows1 < 0 || d <= 0 || d % 8 || d > kEdgeHeadDim ||
+      d > levels->channels || type < 0 || type > 2)
     return -3;
   const int d8 = d / 8, row_blocks = (levels->q_rows + kLevelRows - 1) / kLevelRows;
   const size_t n_kv = size_t(rows1) * d8;
@@ -322,7 +324,8 @@ extern "C" int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, 
   const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
   if (work == 0) return 0;
   launch_overlapped(
-      attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels), static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
+      attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels),
+      static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
       reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

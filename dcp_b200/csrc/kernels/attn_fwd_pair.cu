@@ -16,44 +16,48 @@
 // taken O to registers.
 //
 // Why pairs: with one query tile per CTA there is room for three score buffers, so a softmax warp finds its next scores
-// ready.  (Two query tiles per CTA, the earlier form, leave one buffer each: scores, exponentials and both products of a
-// tile were one serial chain of 3200 cycles per 2180 of tensor time.)  One query tile per CTA alone would read every K
-// and V tile twice as often from L2; in a pair each CTA reads half of it, and the tensor core reads half as much of
-// B from shared memory.
+// ready.  (Two query tiles per CTA leave one buffer each: scores, exponentials and both products of a tile are one
+// serial chain of 3200 cycles per 2180 of tensor time.)  One query tile per CTA alone would read every K and V tile
+// twice as often from L2; in a pair each CTA reads half of it, and the tensor core reads half as much of B from shared
+// memory.
 //
-// Why no running maximum: out = O / l and lse = m + ln l are exact for any reference m, and bf16 has the exponent range of
-// fp32, so m has to be near the row's largest score only within what fp32 holds.  A row keeps the maximum of the first
-// tile it sees anything of; while some row of a warp has none, the two warps that share the rows hand the references on
-// from KV tile to KV tile.  Afterwards no maximum is taken and nothing is handed on.  Where a row's sum exceeds 2^64 (a
-// score 44 above the reference), or the sum or an element of O is not finite (values of 2^64 and more overflow O before the sum
-// does), the pair goes through the tile again when it is done with all tiles, with the reference following the maximum to
-// within 2^8 and O rescaled in TMEM where it moves.  That pass takes longer than the first, as references are handed on at every
-// KV tile: 32 / 8 heads, all rows rising by 2^80 behind their first 128 keys, full 8192 x 16384 3.71 ms against 1.55 without the
-// rise, causal 4096 x 4096 0.302 against 0.142 (a kernel that kept the running maximum throughout took 1.86 and 0.161 ms for them).
-// Looking at O costs nothing that can be measured.
+// Why no running maximum: out = O / l and lse = m + ln l are exact for any reference m, and bf16 has the exponent range
+// of fp32, so m has to be near the row's largest score only within what fp32 holds.  A row keeps the maximum of the
+// first tile it sees anything of; while some row of a warp has none, the two warps that share the rows hand the
+// references on from KV tile to KV tile.  Afterwards no maximum is taken and nothing is handed on.  Where a row's sum
+// exceeds 2^64 (a score 44 above the reference), or the sum or an element of O is not finite (values of 2^64 and more
+// overflow O before the sum does), the pair goes through the tile again when it is done with all tiles, with the
+// reference following the maximum to within 2^8 and O rescaled in TMEM where it moves.  That pass takes longer than the
+// first, as references are handed on at every KV tile: 32 / 8 heads, all rows rising by 2^80 behind their first 128
+// keys, full 8192 x 16384 3.71 ms against 1.55 without the rise, causal 4096 x 4096 0.302 against 0.142 (a kernel that
+// kept the running maximum throughout took 1.86 and 0.161 ms for them).  Looking at O costs nothing that can be
+// measured.
 //
 // P of the first 64 keys is handed over while the softmax works on the other 64, so half of PV runs under it.  The next
 // scores' barrier is asked before the last probabilities are stored: a look at shared memory queues behind the
-// exponentials of the other warp, 200 cycles and more.  Arrivals on the other CTA's barriers carry no release at cluster
-// scope (a fence that waits for everything the warp has stored; 1.6 times slower): what they announce is in TMEM.
+// exponentials of the other warp, 200 cycles and more.  Arrivals on the other CTA's barriers carry no release at
+// cluster scope (a fence that waits for everything the warp has stored; 1.6 times slower): what they announce is in
+// TMEM.
 //
-// What bounds it: the issuing thread and the softmax warps that share its scheduler.  Where both are in time a KV tile takes
-// 1250 cycles per CTA; the exponentials need 1024 of them and the products 1024.  Every look at a barrier costs the issuer
-// 200 cycles, so it asks for its three at once, and K(j+3) and V(j), which one step consumes, share a barrier.  Between
-// two tiles of a pair the epilogue has warps of its own: the softmax warps leave sums and references in shared memory and go on
-// with the next tile's scores, whose first product waits until O is in registers.  (With the epilogue in the softmax warps the
-// tensor core was idle for about 4000 cycles between two tiles: 16 heads, 16384 queries over 256 / 512 keys 110 -> 81 / 139
-// -> 107 us, causal 2048 x 2048 66.6 -> 62.5, 4096 x 4096 167 -> 159 us, sink + window 531 -> 514 us in long runs; full 8192 x
-// 16384 1.535 -> 1.542 ms.)  They store rows straight from registers, a sector per lane and instruction: through shared memory,
-// in 64-byte pieces, O was in TMEM for 3500 cycles instead of 1900, as every look at shared memory queues behind the
-// exponentials (8192 queries over 1500 keys 213 -> 201 us, causal 6000 x 6000 280 -> 270, 16384 x 16384 1861 -> 1835 us, in long
-// runs; full 8192 x 16384 1836 -> 1820).  A copy per row by the copy engine takes 60 cycles to issue, 2000 for a half of 32 rows.
-// As a launch with a pair per tile (table look-ups, barriers, TMEM, first loads, exit) it was 14000.
-// Measured against two query tiles per CTA (32 / 8 heads, queries x keys; one box): full 8192 x 16384 1.71 -> 1.57 ms
-// (1283 -> 1404 TFLOP/s), causal 1.29 -> 1.17 ms (1397), sink + window 0.568 -> 0.505 ms, causal 4096 x 4096 0.163 ->
-// 0.153 ms; in long runs under the power cap full 2.01 -> 1.74 ms (all with the epilogue in the softmax warps).  Tried and left: a pair per tile instead of persistent pairs (4096 x 4096 0.159 ms, 16384
-// tokens in sequences of 8192 6 % slower); the result written after the next tile's first exponentials (the longer loop
-// costs more than it hides: 1.57 -> 1.66 ms); the maximum taken beside the exponentials (1.75 ms).
+// What bounds it: the issuing thread and the softmax warps that share its scheduler.  Where both are in time a KV tile
+// takes 1250 cycles per CTA; the exponentials need 1024 of them and the products 1024.  Every look at a barrier costs
+// the issuer 200 cycles, so it asks for its three at once, and K(j+3) and V(j), which one step consumes, share a
+// barrier.
+//
+// Why the epilogue has warps of its own: the softmax warps leave sums and references in shared memory and go on with
+// the next tile's scores, whose first product waits until O is in registers, about 2000 cycles; with the epilogue in
+// the softmax warps the tensor core was idle for 4000 (16 heads, 16384 queries over 512 keys 139 -> 107 us, causal 4096
+// x 4096 167 -> 159 us).  It stores rows straight from registers, a sector per lane and instruction: through shared
+// memory O was in TMEM for 3500 cycles instead of 1900, as every look at shared memory queues behind the exponentials
+// (8192 queries over 1500 keys 213 -> 201 us).  A copy per row by the copy engine takes 60 cycles to issue, 2000 for a
+// half of 32 rows.
+//
+// Measured against two query tiles per CTA (32 / 8 heads, queries x keys; one box, L2 flushed between calls): full 8192
+// x 16384 1.69 -> 1.55 ms (1415 TFLOP/s), causal 1.42 -> 1.26 ms, causal 4096 x 4096 0.169 -> 0.142, 2048 x 2048 equal,
+// 8192 over 1500 keys 0.224 -> 0.177; 16 heads, 16384 over 512 keys 0.122 -> 0.095 ms; 8 heads, causal 1024 x 1024 27.5
+// -> 19.5 us.  Tried and left: a launch with a pair per tile (4096 x 4096 4 % slower, 16384 tokens in sequences of 8192
+// 6 %); the result written after the next tile's first exponentials (full 6 % slower); the maximum taken beside the
+// exponentials (11 % slower).
 //
 // The partial (out, lse) of a tile is stored straight to its destination arena, which may be a
 // peer GPU's memory (plain st.global over the NVLink mapping).
@@ -88,9 +92,9 @@ static constexpr int kInfos = 4;
 static constexpr float kGap = 8.f;            // exponent (base 2) by which a score may exceed a reference that can still move
 static constexpr float kMaxSum = 1.8447e19f;  // 2^64: a row sum above it sends the tile through the second pass
 
-// What the softmax and epilogue warps of a CTA need of a tile, put into shared memory by the TMA producer, which is some
-// KV tiles ahead of them: from the tables it would take three dependent trips to memory between two tiles.  And what
-// they leave for one another.
+// What the softmax and epilogue warps of a CTA need of a tile, put into shared memory by the TMA producer, which is
+// some KV tiles ahead of them: from the tables it would take three dependent trips to memory between two tiles.  And
+// what they leave for one another.
 struct __align__(16) TileInfo {
   int4 mask[kTileM];        // ranges of this CTA's rows
   float m[kTileM];          // reference of a row
@@ -129,8 +133,9 @@ template <typename F>
 __device__ __forceinline__ void for_each_barrier(PairSmem& sm, F f) {   // f(barrier, arrivals)
   for (int i = 0; i < 2; ++i) { f(&sm.q_full[i], 1); f(&sm.q_empty[i], 1); }
   for (int i = 0; i < kSlots; ++i) { f(&sm.kv_full[i], 1); f(&sm.kv_empty[i], 1); }
-  for (int i = 0; i < kSBufs; ++i) { f(&sm.s_full[i], 1); f(&sm.p_ready[i][0], 8); f(&sm.p_ready[i][1], 8); }   // four warps of either CTA
-  f(&sm.o_empty, 8);   // four warps of either CTA
+  // of P and O: four warps of either CTA
+  for (int i = 0; i < kSBufs; ++i) { f(&sm.s_full[i], 1); f(&sm.p_ready[i][0], 8); f(&sm.p_ready[i][1], 8); }
+  f(&sm.o_empty, 8);
   f(&sm.acc_full, 1);
   for (int i = 0; i < 4 * kInfos; ++i) { f(&sm.m_ready[i >> 2][i & 3], 1); f(&sm.l_ready[i >> 2][i & 3], 2); }
   for (int i = 0; i < kInfos; ++i) { f(&sm.info_full[i], 1); f(&sm.info_empty[i], 12); }   // softmax and epilogue warps
@@ -154,8 +159,8 @@ __device__ __forceinline__ void softmax_half(const uint32_t* s, uint64_t sl2_2, 
   tmem_st32(p_addr, preg);
 }
 
-// 16 channels of a row, from `ch` on, in the caller's type (0 float, 1 half, 2 bf16) where the row has them, a multiple of 8;
-// float and half hold what bf16 does
+// 16 channels of a row, from `ch` on, in the caller's type (0 float, 1 half, 2 bf16) where the row has them, a multiple
+// of 8: the bf16 result, which float holds as it is, and half rounded once more (beyond 65504 it is infinite there)
 __device__ __forceinline__ void store_channels(uint8_t* row, int type, int channels, int ch, uint32_t* packed) {
   if (ch >= channels) return;
   const bool both = ch + 16 <= channels;
@@ -191,11 +196,11 @@ __device__ __forceinline__ void store_channels(uint8_t* row, int type, int chann
   }
 }
 
-// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and what S adds up over
-// zeros is left out.  PV stays as it is, so that the output's padding is written.  8192 queries x 16384 keys, 32 / 8 heads, against all 128
-// channels: 64 channels 1.43 -> 1.33 ms (causal 1.08 -> 1.04: the exponentials bound it then), 96 channels 1.51 -> 1.47 ms.
-// kForm: the results' type and width are arguments; rows of 128 in bf16 have an instance of their own, as a test per store cost
-// the calls that have them 1 to 4 %.
+// kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and what S adds up
+// over zeros is left out.  PV stays as it is, so that the output's padding is written.  8192 queries x 16384 keys, 32 /
+// 8 heads, against all 128 channels: 64 channels 1.43 -> 1.33 ms (causal 1.08 -> 1.04: the exponentials bound it then),
+// 96 channels 1.51 -> 1.47 ms. kForm: the results' type and width are arguments; rows of 128 in bf16 have an instance
+// of their own, as a test per store cost the calls that have them 1 to 4 %.
 template <int kD, bool kForm>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -338,7 +343,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int i = 0; i < 8; ++i)
           zeros_2 = fma_f32x2(pack_f32x2(__uint_as_float(oreg[2 * i]), __uint_as_float(oreg[2 * i + 1])), 0ull, zeros_2);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
+        for (int i = 0; i < 8; ++i)
+          packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
         if (mine) {
           if (kForm) {
             store_channels(out, type, channels, c * 16, packed);
@@ -389,8 +395,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         return true;
       };
       AttnTile tile;
-      // Tiles without keys come last: the last three V of a tile are loaded with the K of the next ones, and announcing a tile
-      // waits until the one kInfos before it is finished.
+      // Tiles without keys come last: the last three V of a tile are loaded with the K of the next ones, and announcing
+      // a tile waits until the one kInfos before it is finished.
       bool empty = false;
       first_empty = -1;
       for (int round = 0; ok; ++round) {
@@ -428,7 +434,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         ti.out_channels = own_form ? out_channels : kHeadDim;
         ti.out = static_cast<uint8_t*>(ptrs.out[tile.out_dev]) +
                  (size_t(tile.out_row + X * kTileM) * hq + tile.head) * ti.out_channels * (ti.out_type == 0 ? 4 : 2);
-        ti.lse = ptrs.lse[tile.out_dev] + size_t(tile.head) * (tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b) + tile.out_row + X * kTileM;
+        ti.lse = ptrs.lse[tile.out_dev] + size_t(tile.head) * (tile.out_dev < n_dst_a ? lse_stride_a : lse_stride_b) +
+                 tile.out_row + X * kTileM;
         const int mask_bytes = 16 * min(max(tile.n_rows - X * kTileM, 0), kTileM);
         mbar_expect_tx(&sm.info_full[info], mask_bytes);
         if (mask_bytes > 0) bulk_load(ti.mask, masks + tile.mask_row + X * kTileM, mask_bytes, &sm.info_full[info]);
@@ -541,7 +548,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             } else {
 #pragma unroll 1
               for (int k = 4 * h; k < 4 * h + 4; ++k)
-                umma_ts_pair_hold(tmem + kSBufs * 128, a + k * 8, desc(v0 + k * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u, hold_a, hold_b);
+                umma_ts_pair_hold(tmem + kSBufs * 128, a + k * 8, desc(v0 + k * 128), idesc_pv, (j > 0 || k > 0) ? 1u : 0u,
+                                  hold_a, hold_b);
             }
           }
           if (!ok) break;
@@ -652,8 +660,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             exchange = pass > 0 || __any_sync(0xffffffffu, m_new == -INFINITY);
             if (!exchange) n_pub = j + 1;
             if (j > 0 && __any_sync(0xffffffffu, m_new != m_cur)) {
-              // no product may be adding to O; that of KV tile j - 3 has retired, as S(j) came after it, so the phase is
-              // unambiguous
+              // no product may be adding to O; that of KV tile j - 3 has retired, as S(j) came after it, so the phase
+              // is unambiguous
               const int i = g0 + j - 1 + kSBufs;   // its slot
               ok = __all_sync(0xffffffffu, mbar_wait(&sm.kv_empty[i % kSlots], (i / kSlots) & 1, abort_word));
               if (!ok) break;
@@ -735,9 +743,10 @@ using namespace dcpk;
 
 // Same contract as dcpk_attn_fwd, for tile tables built with 256-row tiles (AttnTile.n_rows <= 256):
 // `kv_entries` is the KvSub list (AttnTile.kv_off / n_kv index it), n_mask_rows / n_kv_entries are the
-// lengths of the mask table and of that list (bounds checks).  Destinations from n_dst_a on are rows of `out_channels` (a
-// multiple of 8, at most 128) of type `out_type` (0 fp32, 1 fp16, 2 bf16), those before it bf16 rows of 128; all 16-byte
-// aligned.  A pass of its own for the caller's form took 6.5 us of 218 for 7680 tokens of 64 fp32 channels, forward and backward.
+// lengths of the mask table and of that list (bounds checks).  Destinations from n_dst_a on are rows of `out_channels`
+// (a multiple of 8, at most 128) of type `out_type` (0 fp32, 1 fp16, 2 bf16), those before it bf16 rows of 128; all
+// 16-byte aligned.  A pass of its own for the caller's form took 6.5 us of 218 for 7680 tokens of 64 fp32 channels,
+// forward and backward.
 extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* kv_arena, long kv_rows, int hq,
                                   int hkv, const void* tiles, int n_tiles, const void* kv_entries, int n_kv_entries,
                                   const void* masks, int n_mask_rows, void* const* out_ptrs, float* const* lse_ptrs,
@@ -762,12 +771,14 @@ extern "C" int dcpk_attn_fwd_pair(const void* q_arena, long q_rows, const void* 
   const int smem = int(sizeof(PairSmem)) + 1024;
   const bool form = out_type != 2 || out_channels != kHeadDim;
   const int v = (channels > 96 ? 0 : channels > 64 ? 1 : 2) + 3 * form;
-  auto kernel = v == 5 ? attn_fwd_pair_kernel<64, true> : v == 4 ? attn_fwd_pair_kernel<96, true> : v == 3 ? attn_fwd_pair_kernel<128, true>
-              : v == 2 ? attn_fwd_pair_kernel<64, false> : v == 1 ? attn_fwd_pair_kernel<96, false> : attn_fwd_pair_kernel<128, false>;
+  auto kernel = v == 5 ? attn_fwd_pair_kernel<64, true> : v == 4 ? attn_fwd_pair_kernel<96, true>
+              : v == 3 ? attn_fwd_pair_kernel<128, true> : v == 2 ? attn_fwd_pair_kernel<64, false>
+              : v == 1 ? attn_fwd_pair_kernel<96, false> : attn_fwd_pair_kernel<128, false>;
   if (raise_smem_limit(kernel, smem, g_pair_smem_raised[v]) != cudaSuccess) return -4;
   // short calls begin while the kernel before them ends (see kSmallPass in attn_edge.cu; a round is 5 us and more)
   const cudaError_t rc = launch_overlapped(
-      kernel, 2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream), 1, n_tiles <= 8 * kPairs, tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
+      kernel, 2 * std::min(n_tiles, kPairs), kPairThreads, smem, static_cast<cudaStream_t>(stream), 1, n_tiles <= 8 * kPairs,
+      tm_q, tm_k, tm_v, static_cast<const AttnTile*>(tiles), n_tiles, static_cast<const int4*>(kv_entries),
       static_cast<const int4*>(masks), pp, hq, hkv, lse_stride_a, lse_stride_b, n_dst_a, n_dst, out_type, out_channels, int(q_rows),
       n_mask_rows, n_kv_entries, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, status);
   return rc == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -5;

@@ -1,8 +1,9 @@
 // Levels of dQ: buffers that make its sums the same in every run.
 //
-// A row of dQ is added to by every key tile that it sees, as these come.  Two additions to zero give the same bits in either order,
-// three do not: with a workspace each 256 keys (of the positions of an item's concatenated KV) have a buffer of their own, a level,
-// and the levels are summed afterwards, in their order.  Level 0 is the accumulator itself, and the only one without a workspace.
+// A row of dQ is added to by every key tile that it sees, as these come.  Two additions to zero give the same bits in
+// either order, three do not: with a workspace each 256 keys (of the positions of an item's concatenated KV) have a
+// buffer of their own, a level, and the levels are summed afterwards, in their order.  Level 0 is the accumulator
+// itself, and the only one without a workspace.
 #pragma once
 #include <stdint.h>
 
@@ -10,8 +11,8 @@
 
 namespace dcpk {
 
-// One item of the backward kernel = one query tile (up to 128 rows) that attends to a key tile; a CTA visits it once per
-// query head it covers, so the table does not grow with the head count.
+// One item of the backward kernel = one query tile (up to 128 rows) that attends to a key tile; a CTA visits it once
+// per query head it covers, so the table does not grow with the head count.
 struct BwdItemDesc {
   int q_row;     // arena row of the query tile (same row addresses Q, dO, lse, delta)
   int n_rows;    // valid queries
@@ -39,12 +40,13 @@ struct DqLevels {
 
 inline DqLevels make_levels(const DcpkDqLevels* l) {
   if (!l || !l->workspace) return DqLevels{};
-  return DqLevels{static_cast<const BwdItemDesc*>(l->items), static_cast<float*>(l->workspace), l->n_items, l->n_levels, l->q_rows, l->hq,
-                  l->channels, level_pitch(l->channels)};
+  return DqLevels{static_cast<const BwdItemDesc*>(l->items), static_cast<float*>(l->workspace), l->n_items, l->n_levels,
+                  l->q_rows, l->hq, l->channels, level_pitch(l->channels)};
 }
 
-// A block works on so many rows at a time; which levels they have is in the items that cover them, so it looks through the whole
-// table (a row at a time per warp, with a look each: 13 and 14 us for clearing and summing 42 MB, 10.5 and 13 this way).
+// A block works on so many rows at a time; which levels they have is in the items that cover them, so it looks through
+// the whole table (a row at a time per warp, with a look each: 13 and 14 us for clearing and summing 42 MB, 10.5 and 13
+// this way).
 static constexpr int kLevelRows = 4;
 struct RowLevels { uint32_t bits[kLevelRows][2]; };   // in shared memory
 
@@ -91,7 +93,8 @@ __device__ __forceinline__ void add_levels(const DqLevels& lv, uint64_t left, si
     float4 v[4];   // of four levels in flight
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      v[u] = left != 0 ? *reinterpret_cast<const float4*>(lv.buf + (__ffsll(left) - 2) * size + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (left != 0) v[u] = *reinterpret_cast<const float4*>(lv.buf + (__ffsll(left) - 2) * size + at);
       left &= left - 1;
     }
 #pragma unroll

@@ -2,7 +2,8 @@
 // compares the two.  All return 0, or a negative code when nothing ran.
 #pragma once
 
-// The levels of dQ of a backward call (see attn_levels.cuh), with that call's items, rows, heads and channels.  A null workspace: none.
+// The levels of dQ of a backward call (see attn_levels.cuh), with that call's items, rows, heads and channels.  A null
+// workspace: none.
 struct DcpkDqLevels {
   const void* items;
   int n_items, n_levels, q_rows, hq, channels;

@@ -103,9 +103,9 @@ __global__ void adamw_all_gather_kernel(float* __restrict__ master, float* __res
 }
 
 // squared norm of the scaled, rank-summed gradient slice; nothing is written but the scalar.  Bound by reading.
-// One rank (kOne): a vector at a time in 148 x 4 CTAs whose loads leave L1 alone reads 436M gradients at 6.2 TB/s (141 us);
-// four vectors of a thread in flight, which over peers' buffers hide the link, 4.4 TB/s (197 us; a grid apart or 4 KB apart,
-// in twice as many CTAs or half as many: 152 to 350 us), and 32-byte loads 5.7 TB/s.
+// One rank (kOne): a vector at a time in 148 x 4 CTAs whose loads leave L1 alone reads 436M gradients at 6.2 TB/s (141
+// us); four vectors of a thread in flight, which over peers' buffers hide the link, 4.4 TB/s (197 us; a grid apart or 4
+// KB apart, in twice as many CTAs or half as many: 152 to 350 us), and 32-byte loads 5.7 TB/s.
 template <bool kOne>
 __global__ void __launch_bounds__(256) grad_sqnorm_kernel(GradPtrs grads, int world, size_t shard_off, size_t shard_len,
                                                           float scale, double* __restrict__ sq_norm) {

@@ -7,8 +7,8 @@
 
 namespace dcpk {
 
-// `raised`: of one kernel, a bit per device on which the limit has been raised (devices from 64 on: on every call).  Two threads that
-// come at once both raise it, which does no harm.
+// `raised`: of one kernel, a bit per device on which the limit has been raised (devices from 64 on: on every call).
+// Two threads that come at once both raise it, which does no harm.
 template <typename K>
 inline cudaError_t raise_smem_limit(K kernel, int bytes, std::atomic<uint64_t>& raised) {
   int device = 0;

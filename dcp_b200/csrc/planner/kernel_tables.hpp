@@ -1,6 +1,6 @@
 // Work tables of the sm_100a attention kernels, built from the attention rows of one stage of one
 // device (a row = one Q block with the KV blocks it attends to and its per-query key ranges).
-// Forward: CTA tiles of 256 (two-tile kernel) or 128 query rows, with the walk over 128-key tiles
+// Forward: tiles of 256 (pairs of CTAs) or 128 query rows, with the walk over 128-key tiles
 // each CTA makes; backward: one entry per 128-key tile listing the 64-query tiles that see it.
 // The layouts are the ones dcp_b200/ops/attention.py documents (its Python builders are the
 // oracle of this file).

@@ -17,7 +17,7 @@ import torch
 from . import _lib
 
 TILE_M = 128          # query rows per softmax warpgroup
-TILE_M_PAIR = 256     # query rows per CTA of the two-tile forward kernel (the default)
+TILE_M_PAIR = 256     # query rows per pair of CTAs of the default forward kernel
 TILE_N = 128
 HEAD_DIM = 128
 
@@ -52,7 +52,7 @@ class FwdTables:
     n_tiles: int
     block_size: int
     flops: float = 0.0
-    tile_m: int = TILE_M_PAIR   # 256: two-tile kernel (attn_fwd_pair.cu); 128: one tile per CTA (attn_fwd.cu)
+    tile_m: int = TILE_M_PAIR   # 256: pairs of CTAs (attn_fwd_pair.cu); 128: one tile per CTA (attn_fwd.cu)
 
     def to(self, device, non_blocking: bool = True) -> "FwdTables":
         mv = lambda t: t.to(device, non_blocking=non_blocking)
@@ -99,12 +99,12 @@ def build_fwd_tables(rows: Sequence[AttnRow], block_size: int, device, tile_m: i
 
 
 def build_fwd_tables_py(rows: Sequence[AttnRow], block_size: int, device, tile_m: int = TILE_M_PAIR) -> FwdTables:
-    """Flatten Q blocks into CTA tiles of ``tile_m`` query rows.
+    """Flatten Q blocks into tiles of ``tile_m`` query rows.
 
     tile_m = 128: one tile per CTA (attn_fwd.cu, attn_fwd_split.cu); ``kv_entries`` lists the KV blocks
     (arena row, tokens) and the kernel derives the 128-key tiles it needs from the mask bounds.
 
-    tile_m = 256: two 128-row tiles per CTA that share every K/V tile (attn_fwd_pair.cu);
+    tile_m = 256: a pair of CTAs, 128 rows each, that share every K/V tile (attn_fwd_pair.cu);
     ``kv_entries`` then is the ready-made walk of the CTA: one int32 x 4 entry per 128-key tile that
     at least one of the two query tiles can see = (arena row, position of its first key, valid keys,
     flags) with flags bit 0 / 1 = query tile A / B sees a key of it, bit 2 / 3 = A / B sees every
@@ -151,7 +151,7 @@ def build_fwd_tables_py(rows: Sequence[AttnRow], block_size: int, device, tile_m
 
 
 def _kv_walks(row: AttnRow, rng: np.ndarray, block_size: int) -> List[np.ndarray]:
-    """Per 256-row CTA tile of a Q block: int32 [n, 4] list of the 128-key tiles it visits (see
+    """Per 256-row tile of a Q block: int32 [n, 4] list of the 128-key tiles it visits (see
     build_fwd_tables).  Visibility comes from the union / intersection of the two key ranges over each
     128-row query tile, the same test the one-tile kernels run on the device."""
     n_qt, (u0s, u0e, u1s, u1e, i0s, i0e, i1s, i1e) = _tile_bounds(rng, TILE_M)
@@ -227,13 +227,13 @@ def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, o
              job_ctx: Optional[CopyContext] = None, channels: int = HEAD_DIM):
     """Run the forward kernel the tables were built for (``tables.tile_m``); ``variant`` only applies to
     the one-tile kernel (0: P in TMEM, 1: P through shared memory).  ``jobs`` (int32 [n, 4] on the
-    device, see copy_jobs.cuh) is a list of peer -> local copies the two-tile kernel performs with
+    device, see copy_jobs.cuh) is a list of peer -> local copies the pair kernel performs with
     two spare warps per CTA while it computes; ``job_ctx`` names the regions they refer to.
 
     q_arena: bf16 [rows, hq, 128]; kv_arena: bf16 [rows, 2, hkv, 128]; out_dsts / lse_dsts: lists of
     destination arenas (tensors or raw device addresses; index 0 = this rank), every out arena
     bf16 [rows_o, hq, 128] with its lse fp32 [hq, rows_o].  ``channels``: all channels of Q and K from there on are zero,
-    and the products need not go over them (the two-tile kernel makes use of it).
+    and the products need not go over them (the pair kernel makes use of it).
     """
     lib = _lib.load()
     assert q_arena.dtype == torch.bfloat16 and kv_arena.dtype == torch.bfloat16
@@ -255,7 +255,7 @@ def attn_fwd(q_arena: torch.Tensor, kv_arena: torch.Tensor, tables: FwdTables, o
             _lib.stream_handle())
         _lib.check(rc, "dcpk_attn_fwd_pair")
         return
-    assert jobs is None or jobs.shape[0] == 0, "only the two-tile forward kernel carries copy jobs"
+    assert jobs is None or jobs.shape[0] == 0, "only the pair forward kernel carries copy jobs"
     rc = lib.dcpk_attn_fwd(
         _lib.ptr(q_arena), ctypes.c_long(q_arena.shape[0]), _lib.ptr(kv_arena), ctypes.c_long(kv_arena.shape[0]),
         ctypes.c_int(hq), ctypes.c_int(hkv), _lib.ptr(tables.tiles), ctypes.c_int(tables.n_tiles),
