@@ -713,8 +713,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0 && sm.abort_word) atomicExch(status, sm.abort_word);  // 1 = wait timeout, 3 = bad table
 }
 
-// The passes over the levels of dQ as launches of their own (kSum: they are added to dQ; else they are cleared).  Bound
-// by L2.
+// The passes over the levels of dQ as launches of their own, plain ones (kSum: they are added to dQ; else they are
+// cleared).  Bound by L2.
 template <bool kSum>
 __global__ void __launch_bounds__(256) dq_levels_kernel(const __grid_constant__ DqLevels lv, float* __restrict__ dq) {
   __shared__ RowLevels present;
@@ -854,7 +854,7 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
   const DcpkDqLevels of_call = {items, n_items_total, n_levels, int(q_rows), hq, channels, levels ? workspace : nullptr};
   const unsigned level_blocks = unsigned((q_rows + kLevelRows - 1) / kLevelRows);
   if (levels && (level_passes & 1) &&
-      launch_overlapped(dq_levels_kernel<false>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, true, make_levels(&of_call),
+      launch_overlapped(dq_levels_kernel<false>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, false, make_levels(&of_call),
                         dq_ptrs[0]) != cudaSuccess)
     return -5;
   const cudaError_t rc = launch_overlapped(
@@ -865,7 +865,7 @@ extern "C" int dcpk_attn_bwd(const void* q_arena, const void* do_arena, long q_r
       n_mask_rows, n_items_total, scale, static_cast<const CopyJob*>(jobs), n_jobs, ctx, n_copy_rows, status);
   if (rc != cudaSuccess || cudaGetLastError() != cudaSuccess) return -5;
   if (levels && (level_passes & 2) &&
-      launch_overlapped(dq_levels_kernel<true>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, true, make_levels(&of_call),
+      launch_overlapped(dq_levels_kernel<true>, level_blocks, 256, 0, static_cast<cudaStream_t>(stream), 1, false, make_levels(&of_call),
                         dq_ptrs[0]) != cudaSuccess)
     return -5;
   return 0;

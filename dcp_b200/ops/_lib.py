@@ -56,12 +56,13 @@ def calls_path() -> Path:
 def calls():
     """The native host side of single-rank attention calls (``csrc/host/calls.cpp``)."""
     load()
-    p = calls_path()
-    if not p.exists():
-        raise RuntimeError(f"{p} is missing: build it with `python -m dcp_b200.csrc.build`")
     try:
         from .. import _calls
-    except ImportError as e:   # it is there: most likely built for another torch
+    except ImportError as e:
+        p = calls_path()
+        if not p.exists():
+            raise RuntimeError(f"{p} is missing: build it with `python -m dcp_b200.csrc.build`") from e
+        # it is there: most likely built for another torch
         raise RuntimeError(f"{p} does not load with torch {torch.__version__} ({e}): rebuild it with "
                            "`python -m dcp_b200.csrc.build --force`") from e
     return _calls

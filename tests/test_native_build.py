@@ -62,10 +62,10 @@ def test_build_of_an_incomplete_copy_says_so(monkeypatch, tmp_path):
 def test_missing_and_unloadable_native_calls_are_told_apart(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "load", lambda: None)
     monkeypatch.setattr(_lib, "calls_path", lambda: tmp_path / "_calls.so")
+    monkeypatch.delattr(dcp_b200, "_calls", raising=False)
+    monkeypatch.setitem(sys.modules, "dcp_b200._calls", None)      # the import fails
     with pytest.raises(RuntimeError, match="missing"):
         _lib.calls()
     (tmp_path / "_calls.so").touch()
-    monkeypatch.delattr(dcp_b200, "_calls", raising=False)
-    monkeypatch.setitem(sys.modules, "dcp_b200._calls", None)      # the import fails
     with pytest.raises(RuntimeError, match="does not load"):
         _lib.calls()
