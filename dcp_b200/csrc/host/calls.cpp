@@ -3,12 +3,11 @@
 // A forward is one or two launches, a backward three or four.  Driven from Python small calls waited for the host; most
 // of its time went into checks, slices, argument objects and result tensors between the launches.  Here the pieces that
 // do not change between calls (tables, arenas, sizes) are laid out once per program, and a call checks its tensors,
-// allocates its results and launches. Host time (8 query heads, 4040 tokens in four sequences): forward 37 -> 13 us,
-// backward 105 -> 27, the whole call with autograd 221 -> 97; 7680 tokens of 64 fp32 channels 71 -> 10, 110 -> 16 and
-// 302 -> 96.
+// allocates its results and launches.  Host time (8 query heads, 4040 tokens in four sequences): forward 37 -> 8 us,
+// backward 105 -> 17, the whole call with autograd 221 -> 100; with 64 fp32 channels 71 -> 9, 110 -> 17 and 302 -> 100.
 //
 // Only plain calls are taken: tensors on the arenas' device, contiguous, 16-byte aligned, of a type the row kernels
-// read. For anything else the functions return nothing before they launch anything, and the caller goes the general
+// read.  For anything else the functions return nothing before they launch anything, and the caller goes the general
 // way.
 #include <ATen/ATen.h>
 #include <c10/core/DeviceGuard.h>

@@ -782,7 +782,7 @@ extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, 
 // Over 78 batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128
 // channels) that is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was
 // above the SMs' average, but seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads:
-// 152 us before, 109 in two parts; eight sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us. CTAs that all run at once
+// 152 us before, 109 in two parts; eight sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.  CTAs that all run at once
 // add to a row of dQ in the order of their items, and as long as their lists are short and begin at
 // different queries that is nearly the same in every run.  Without `any_wave` (dQ has levels, whose order does not
 // matter) they become more than one wave only where that takes 32 visits (about 70 us) off the longest list.

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kEdgeThreads) cut_cast_kernel(const S* __restr
 }
 
 // The same of dQ and dKV where dQ has levels, which are added on the way.  The first `row_blocks` blocks take dQ,
-// kLevelRows rows each. As a launch of its own the sum took 13 us of 135 (42 MB of levels and 16 of dQ; four sequences
+// kLevelRows rows each.  As a launch of its own the sum took 13 us of 135 (42 MB of levels and 16 of dQ; four sequences
 // of 300 to 2100 tokens, 8 / 2 heads).
 template <typename T>
 __global__ void __launch_bounds__(kEdgeThreads)
