@@ -782,12 +782,16 @@ extern "C" long dcpk_attn_bwd_workspace(int n_items_total, long q_rows, int hq, 
 // Over 78 batches of 700 to 22000 tokens (causal, full, sink + window; 8 to 32 heads, groups of 4 and 8, 64 and 128
 // channels) that is within 0.8 % of the best split on average, 12 % at worst; splitting while the longest list was
 // above the SMs' average, but seldom into more than one wave, was 9 % off, 54 % at worst.  2048 tokens, 32 / 8 heads:
-// 152 us before, 109 in two parts; eight sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.  CTAs that all run at once
-// add to a row of dQ in the order of their items, and as long as their lists are short and begin at
-// different queries that is nearly the same in every run.  Without `any_wave` (dQ has levels, whose order does not
-// matter) they become more than one wave only where that takes 32 visits (about 70 us) off the longest list.
+// 152 us before, 109 in two parts; eight sequences, 9105 tokens, 8 / 2 heads: 147 and 107 us.
+// CTAs that all run at once add to a row of dQ in the order of their items, and as long as their lists are short and
+// begin at different queries, as causal ones do, that is nearly the same in every run (ten sequences of 800 tokens or
+// seven of 1200, 8 / 2 heads, 2000 tokens, 16 / 4 heads: the same bits in 100 of 100; from 17 items on, 2100 to 3900
+// tokens, in 97 to 2).  Unless `any_wave` (dQ has levels, whose order does not matter) or some list is longer than
+// that, they become more than one wave only where that takes 32 visits (about 70 us) off the longest list, which costs
+// up to 10 % (1500 tokens, 32 / 8 heads, forward and backward, 126 -> 139 us).
 extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items, int n_items_total, int any_wave) {
   constexpr long kBegin = 8;
+  constexpr int kRepeats = 16;
   auto visits = [&](int p) {   // times the SMs
     return std::max(kSms * (long(max_items) * (group / p) + kBegin),
                     long(n_items_total) * hkv * group + kBegin * n_ctas * hkv * p);
@@ -796,7 +800,8 @@ extern "C" int dcpk_attn_bwd_parts(int n_ctas, int hkv, int group, int max_items
   for (int p = 1; max_items > 0 && p <= group && p <= kMaxParts; ++p) {
     if (group % p != 0) continue;
     if (long(n_ctas) * hkv * p <= kSms) in_one_wave = p;
-    else if (!any_wave && in_one_wave > 0 && long(max_items) * (group / in_one_wave - group / p) < 32) continue;
+    else if (!any_wave && max_items <= kRepeats && in_one_wave > 0 && long(max_items) * (group / in_one_wave - group / p) < 32)
+      continue;
     if (visits(p) < visits(parts)) parts = p;
   }
   return parts;
