@@ -25,6 +25,8 @@ static constexpr int kEdgeThreads = 256;
 static constexpr int kEdgeBlocks = 148 * 8;   // every SM full (2048 threads)
 // Passes over up to so many chunks of 16 bytes (about 10 us) begin while the kernel before them ends.  Longer ones gain
 // nothing from it (6168 tokens of 32 heads, forward and backward, 1008 -> 1010 us; 121987 tokens 41.4 -> 41.9 ms).
+// Passes over levels of dQ are plain launches: overlapped, both took longer (2048 tokens, 8 / 2 heads, forward and
+// backward in a graph, 88 and 93 us; four sequences of 300 to 2100 tokens 119 and 122).
 static constexpr size_t kSmallPass = size_t(1) << 21;
 
 __device__ __forceinline__ void load8(const float* p, float* f) {
@@ -140,6 +142,7 @@ cut_cast_levels_kernel(const __grid_constant__ DqLevels lv, const float* __restr
 // delta[h][row] = sum_d dO[row][h][d] * O[row][h][d]: sixteen lanes per (row, head), 16 bytes each of both
 // operands, four (row, head) pairs in flight per thread; then the grid clears the two accumulators.
 // One warp per pair with 8-byte loads read at 3.7 TB/s and the two fills were launches of their own.
+template <bool kLevels>
 __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
                                                                      const __nv_bfloat16* __restrict__ d_o,
                                                                      float* __restrict__ delta, int n_rows, int hq,
@@ -181,15 +184,17 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_kernel(const __nv_
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (size_t i = tid; i < nz0; i += n_thr) zero0[i] = z;
   for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
-  __shared__ RowLevels present;
-  if (levels.n_levels > 1)
-    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
+  if constexpr (kLevels) {
+    __shared__ RowLevels present;
+    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows)
+      clear_levels(levels, row0, present);
+  }
 }
 
 // The same for gradients in the caller's form (rows of d8 chunks of 8 channels): dO also goes to the arena's rows,
 // rounded to bf16 and zero-padded, and delta is that of the rounded values.  As a pass that converts O and dO and the
 // one above it took 22 us for 7680 tokens of 8 heads with 64 fp32 channels.
-template <typename T>
+template <typename T, bool kLevels>
 __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const T* __restrict__ o, const T* __restrict__ d_o, int d8,
                                                                           __nv_bfloat16* __restrict__ rows, float* __restrict__ delta,
                                                                           int n_rows, int hq, int stat_stride,
@@ -232,14 +237,12 @@ __global__ void __launch_bounds__(kEdgeThreads) attn_bwd_prep_cast_kernel(const 
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
   for (size_t i = tid; i < nz0; i += n_thr) zero0[i] = z;
   for (size_t i = tid; i < nz1; i += n_thr) zero1[i] = z;
-  __shared__ RowLevels present;
-  if (levels.n_levels > 1)
-    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows) clear_levels(levels, row0, present);
+  if constexpr (kLevels) {
+    __shared__ RowLevels present;
+    for (int row0 = blockIdx.x * kLevelRows; row0 < levels.q_rows; row0 += gridDim.x * kLevelRows)
+      clear_levels(levels, row0, present);
+  }
 }
-
-// Passes over levels are plain launches: overlapped, both took longer (2048 tokens, 8 / 2 heads, forward and backward
-// in a graph, 88 and 93 us; four sequences of 300 to 2100 tokens 119 and 122).
-static bool small_pass(size_t work, const DcpkDqLevels* levels) { return work <= kSmallPass && !(levels && levels->workspace); }
 
 static int edge_grid(size_t chunks) {
   const size_t b = (chunks + kEdgeThreads - 1) / kEdgeThreads;
@@ -323,8 +326,10 @@ extern "C" int dcpk_attn_bwd_prep(const void* o, const void* d_o, float* delta, 
   if (n_rows < 0 || hq <= 0 || n_rows > stat_stride || nz0 % 4 || nz1 % 4 || nz0 < 0 || nz1 < 0) return -3;
   const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
   if (work == 0) return 0;
+  const bool clear = levels && levels->workspace;
   launch_overlapped(
-      attn_bwd_prep_kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels),
+      clear ? attn_bwd_prep_kernel<true> : attn_bwd_prep_kernel<false>, edge_grid(work), kEdgeThreads, 0,
+      static_cast<cudaStream_t>(stream), 1, work <= kSmallPass && !clear,
       static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), delta, n_rows, hq, stat_stride,
       reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
@@ -339,15 +344,18 @@ extern "C" int dcpk_attn_bwd_prep_cast(int type, const void* o, const void* d_o,
     return -3;
   const size_t work = size_t(n_rows) * hq * 16 + size_t(nz0 + nz1) / 4;
   if (work == 0) return 0;
-  auto launch = [&](auto kernel, auto* as) {
+  const bool clear = levels && levels->workspace;
+  auto launch = [&](auto* as) {
     using T = std::remove_pointer_t<decltype(as)>;
-    return launch_overlapped(kernel, edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1, small_pass(work, levels),
-                             static_cast<const T*>(o), static_cast<const T*>(d_o), d / 8, static_cast<__nv_bfloat16*>(d_o_rows), delta,
-                             n_rows, hq, stat_stride, reinterpret_cast<float4*>(zero0), size_t(nz0) / 4,
-                             reinterpret_cast<float4*>(zero1), size_t(nz1) / 4, make_levels(levels));
+    return launch_overlapped(clear ? attn_bwd_prep_cast_kernel<T, true> : attn_bwd_prep_cast_kernel<T, false>,
+                             edge_grid(work), kEdgeThreads, 0, static_cast<cudaStream_t>(stream), 1,
+                             work <= kSmallPass && !clear, static_cast<const T*>(o), static_cast<const T*>(d_o), d / 8,
+                             static_cast<__nv_bfloat16*>(d_o_rows), delta, n_rows, hq, stat_stride,
+                             reinterpret_cast<float4*>(zero0), size_t(nz0) / 4, reinterpret_cast<float4*>(zero1),
+                             size_t(nz1) / 4, make_levels(levels));
   };
-  if (type == 0) launch(attn_bwd_prep_cast_kernel<float>, static_cast<float*>(nullptr));
-  else if (type == 1) launch(attn_bwd_prep_cast_kernel<__half>, static_cast<__half*>(nullptr));
-  else launch(attn_bwd_prep_cast_kernel<__nv_bfloat16>, static_cast<__nv_bfloat16*>(nullptr));
+  if (type == 0) launch(static_cast<float*>(nullptr));
+  else if (type == 1) launch(static_cast<__half*>(nullptr));
+  else launch(static_cast<__nv_bfloat16*>(nullptr));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

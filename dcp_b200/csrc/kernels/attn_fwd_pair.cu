@@ -25,13 +25,13 @@
 // of fp32, so m has to be near the row's largest score only within what fp32 holds.  A row keeps the maximum of the
 // first tile it sees anything of; while some row of a warp has none, the two warps that share the rows hand the
 // references on from KV tile to KV tile.  Afterwards no maximum is taken and nothing is handed on.  Where a row's sum
-// exceeds 2^64 (a score 44 above the reference), or the sum or an element of O is not finite (values of 2^64 and more
-// overflow O before the sum does), the pair goes through the tile again when it is done with all tiles, with the
-// reference following the maximum to within 2^8 and O rescaled in TMEM where it moves.  That pass takes longer than the
-// first, as references are handed on at every KV tile: 32 / 8 heads, all rows rising by 2^80 behind their first 128
-// keys, full 8192 x 16384 3.71 ms against 1.55 without the rise, causal 4096 x 4096 0.302 against 0.142 (a kernel that
-// kept the running maximum throughout took 1.86 and 0.161 ms for them).  Looking at O costs nothing that can be
-// measured.
+// exceeds 2^64 (a score 44 above the reference), or the sum or an element of the result is not finite (values of 2^64
+// and more overflow O before the sum does; looked for where the sum exceeds 2^16, in what has been stored: a look in
+// passing made the epilogue 350 cycles longer per tile), the pair goes through the tile again when it is done with all
+// tiles, with the reference following the maximum to within 2^8 and O rescaled in TMEM where it moves.  That pass takes
+// longer than the first, as references are handed on at every KV tile: 32 / 8 heads, all rows rising by 2^80 behind
+// their first 128 keys, full 8192 x 16384 3.71 ms against 1.55 without the rise, causal 4096 x 4096 0.302 against 0.142
+// (a kernel that kept the running maximum throughout took 1.86 and 0.161 ms for them).
 //
 // P of the first 64 keys is handed over while the softmax works on the other 64, so half of PV runs under it.  The next
 // scores' barrier is asked before the last probabilities are stored: a look at shared memory queues behind the
@@ -90,6 +90,7 @@ static constexpr int kKvBytes = 64 * 128 * 2;    // a CTA's half of a K or V til
 static constexpr int kRedoWords = 16;
 static constexpr int kInfos = 4;
 static constexpr float kGap = 8.f;            // exponent (base 2) by which a score may exceed a reference that can still move
+static constexpr float kSafeSum = 65536.f;    // up to this row sum O is finite where values are below 2^112
 static constexpr float kMaxSum = 1.8447e19f;  // 2^64: a row sum above it sends the tile through the second pass
 
 // What the softmax and epilogue warps of a CTA need of a tile, put into shared memory by the TMA producer, which is
@@ -194,6 +195,20 @@ __device__ __forceinline__ void store_channels(uint8_t* row, int type, int chann
     reinterpret_cast<uint4*>(p)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     if (both) reinterpret_cast<uint4*>(p)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
   }
+}
+
+// no element of a row that this thread has stored is infinite or not a number; its form as above
+__device__ __forceinline__ bool finite_row(const uint8_t* row, int type, int channels) {
+  // the exponent's bits and one more at their lowest: a carry into the sign's place where all are set
+  const uint32_t exponent = type == 0 ? 0x7f800000u : type == 1 ? 0x7c007c00u : 0x7f807f80u;
+  const uint32_t one = type == 0 ? 0x00800000u : type == 1 ? 0x04000400u : 0x00800080u;
+  uint32_t carries = 0;
+#pragma unroll 1
+  for (const uint8_t* p = row; p < row + channels * (type == 0 ? 4 : 2); p += 16) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    carries |= ((v.x & exponent) + one) | ((v.y & exponent) + one) | ((v.z & exponent) + one) | ((v.w & exponent) + one);
+  }
+  return (carries & (type == 0 ? 0x80000000u : 0x80008000u)) == 0;
 }
 
 // kD: channels that are computed.  The arenas' rows have 128; heads of fewer are zero-padded there, and what S adds up
@@ -327,7 +342,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int type = kForm ? ti.out_type : 2, channels = kForm ? ti.out_channels : kHeadDim;
       uint8_t* out = ti.out + size_t(r) * hq * channels * (type == 0 ? 4 : 2);
       const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
-      uint64_t zeros_2 = 0ull;   // sums of O x 0: not a number from the first element on that is not finite
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         uint32_t oreg[16], packed[8];
@@ -339,9 +353,6 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           for (int i = 0; i < 16; ++i) oreg[i] = 0;
         }
         if (c == 7) more = (next_there || wait_info(next, next_ph)) && hand_over(next);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          zeros_2 = fma_f32x2(pack_f32x2(__uint_as_float(oreg[2 * i]), __uint_as_float(oreg[2 * i + 1])), 0ull, zeros_2);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           packed[i] = pack_bf16x2(__uint_as_float(oreg[2 * i]) * inv_l, __uint_as_float(oreg[2 * i + 1]) * inv_l);
@@ -356,13 +367,14 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
         }
       }
-      float zero0, zero1;
-      unpack_f32x2(zeros_2, zero0, zero1);
-      if (pass == 0 && __any_sync(0xffffffffu, mine && !(l_sum < kMaxSum && zero0 + zero1 == 0.f)) && lane == 0) {
+      if (pass == 0 && __any_sync(0xffffffffu, mine && !(l_sum <= kSafeSum))) {
+        const bool again = mine && (!(l_sum < kMaxSum) || !finite_row(out, type, channels));
+        if (__any_sync(0xffffffffu, again) && lane == 0) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
-          or_cluster_u32(smem_u32(&sm.redo[(ti.round >> 5) & (kRedoWords - 1)]), c, 1u << (ti.round & 31));
+          for (int c = 0; c < 2; ++c) {
+            st_cluster_u32(smem_u32(&sm.any_redo), c, 1u);
+            or_cluster_u32(smem_u32(&sm.redo[(ti.round >> 5) & (kRedoWords - 1)]), c, 1u << (ti.round & 31));
+          }
         }
       }
       __syncwarp();
